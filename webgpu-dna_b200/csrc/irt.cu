@@ -96,20 +96,62 @@ __device__ __forceinline__ float erfcx_f(float z) {
         return s * 0.5641895835f * iz;
     }
     float t = __fdividef(2.0f, 2.0f + z), ty = 4.0f * t - 2.0f, d = 0.0f, dd = 0.0f;
-    for (int j = 13; j > 0; --j) { float tmp = d; d = ty * d - dd + c_erfcx_f[j]; dd = tmp; }
-    return t * __expf(0.5f * (c_erfcx_f[0] + ty * d) - dd);
+    for (int j = 13; j > 0; --j) { float tmp = d; d = fmaf(ty, d, c_erfcx_f[j] - dd); dd = tmp; }
+    return t * __expf(0.5f * fmaf(ty, d, c_erfcx_f[0]) - dd);
 }
 
-// SamplePDC (:91-113) for one pair, 32 trials at a time across the warp; the
-// first accepted trial in trial order wins, as in the sequential loop.  Must
-// be called by all 32 lanes with the same arguments.
+// SamplePDC (:91-113): what a trial needs of its pair.  The f64 members give
+// the winner's X and the undecided trials; the f32 ones the brackets.
+struct PdcPair {
+    double pq, M;                      // p + q M and M (:92-95)
+    float thr, pqf, Mf, t2f, bbf, af, bf;
+};
+__device__ __forceinline__ PdcPair pdc_pair(double a, double b) {
+    const double r = sqrt(2.0 * b / a);
+    const double p = 2.0 * r, q = 2.0 / r;
+    PdcPair P;
+    P.M = fmax(1.0 / (a * a), 3.0 * b / a);
+    P.pq = p + q * P.M;
+    P.thr = (float)(p / P.pq);
+    P.pqf = (float)P.pq; P.Mf = (float)P.M; P.t2f = (float)(2.0 * b / a); P.bbf = (float)(b * b);
+    P.af = (float)a; P.bf = (float)b;
+    return P;
+}
+// X of a trial (:97-103) from its first two words
+__device__ __forceinline__ double pdc_x(double a, double b, double pq, double M, uint32_t wx, uint32_t wy) {
+    const double U1 = u01d(wx, wy), p = 2.0 * sqrt(2.0 * b / a);
+    if (U1 < p / pq) { const double h = U1 * pq / 2; return h * h; }
+    const double h = 2 / ((1 - U1) * pq / M);
+    return h * h;
+}
+
+// The first accepted trial of lane `src`'s pair (qi, qj), 32 trials at a time
+// across the warp: in trial order, as in the sequential loop.  All 32 lanes call;
+// P, a and b are read from lane src.  Returns the trial's first two words (the
+// caller turns them into X), or ~0 when 10,000 trials are rejected.
+//
+// What bounds it: the issue slots of 60 evaluated trials per pair (42 up to the
+// accepted one, 2.4 % of them accepted).  The pair's f64 square root and divisions
+// are therefore done once per pair by its own lane, not by all lanes of the
+// call, and a trial first meets an upper bound of lambdax that costs 30
+// instructions beside its Philox block:
+//   Q >= (1 - beta) (1 - h), so 1 - Q <= beta + h   (h, beta as below; any z > 0,
+//   the asymptotic series of erfcx alternates), which rejects all but 2.43 %.
+//   Its draws are the upper words alone (U1 and 1 - U1 within 2^-27, so X to 2.2e-4
+//   and e to 2.2e-4 b^2/X relative when both exceed 1.2e-4, else the trial goes on;
+//   U2 rounded down); 3 % + 1e-3 b^2/X covers that.
+// Only a warp with a trial left evaluates the bracket (54 % of the rounds).
+// Measured in the pairing kernel (4096 x 10 keV, 6.5 M calls): 4.5 ms; 5.1 ms
+// with the bracket in every round and 6 ms with the f64 set-up in every lane.
 //
 // A trial is accepted when U2 <= lambdax (X <= 2b/a) or U2 M / X <= lambdax
 // (X >= 2b/a), lambdax = e (1 - Q), e = exp(-b^2/X), Q = a sqrt(pi X)
-// erfcx(b/sqrt(X) + a sqrt(X)).  Each trial first brackets the f64 lambdax
-// with f32 arithmetic (the fast reciprocal, rsqrt, divide and exp2
-// instructions, 2 ulp each; ex2 adds |x| 8.6e-8 for exp(x)):
-//   X to 7e-7 relative, so b^2/X to 1.7e-6 and e to (4e-6 b^2/X + 2e-6);
+// erfcx(b/sqrt(X) + a sqrt(X)).  Each trial brackets the f64 lambdax with f32
+// arithmetic (the fast reciprocal, rsqrt, divide and exp2 instructions, 2 ulp
+// each; ex2 adds |x| 8.6e-8 for exp(x)):
+//   U1, 1 - U1 and U2 are the 53-bit draws rounded to f32 (1.2e-7 relative, from
+//   the exact integers), a draw within 1e-6 of the branch point is undecided;
+//   X to 1.2e-6 relative, so b^2/X to 2e-6 and e to (4e-6 b^2/X + 2e-6);
 //   z to 1e-6 relative, which moves erfcx by at most 1.2e-6 (|d ln erfcx/dz|
 //   <= 1.13 and <= 1/z); with the 3.3e-7 of erfcx_f (8e-7 with the fast
 //   exp) the prefactor Q is known to 4e-6, taken as 2e-5, 1 - Q to that
@@ -122,91 +164,109 @@ __device__ __forceinline__ float erfcx_f(float z) {
 //   within 2.2e-7 of h s); taken as 2e-5.  The f64 1 - Q it must bound
 //   carries the rounding of Q near 1 (about 7 ulp, the continued fraction
 //   of erfcx_pos within 2.2e-16), so 1e-14 is added on both sides;
-// and decides when U2 (or U2 M against lambdax X) lies outside the bracket
-// with a further 1e-6 (3e-6) margin.  Trials inside the bracket, near
-// X = 2b/a, with e below exp(-80) in case B, z < 0, or a zero draw are
-// evaluated exactly in f64; only the winner's X is computed in f64.
-__device__ __noinline__ double pdc_warp(uint32_t i, uint32_t j, uint32_t pid, uint32_t k0, uint32_t k1, double a, double b,
-                           int lane) {
-    double p = 2.0 * sqrt(2.0 * b / a);
-    double q = 2.0 / sqrt(2.0 * b / a);
-    double M = fmax(1.0 / (a * a), 3.0 * b / a);
-    const double pq = p + q * M, thr = p / pq, t2 = 2.0 * b / a;
-    const float pqf = (float)pq, Mf = (float)M, t2f = (float)t2, bbf = (float)(b * b);
-    const float af = (float)a, bf = (float)b;
+// and decides when U2 (or U2 M against lambdax X) lies outside the bracket,
+// itself widened by 2e-6 relative and 1e-30, with a further margin of 1e-6
+// (5e-6).  Trials inside the bracket, near X = 2b/a, z < 0, or with a zero draw
+// are evaluated exactly in f64.
+__device__ __forceinline__ float rcp_fast(float x) { return __fdividef(1.0f, x); }
+
+template <class Philox>
+__device__ __forceinline__ uint64_t pdc_find(int src, uint32_t i, uint32_t j, uint32_t pid, const PdcPair& P, double a,
+                                             double b, int lane, Philox philox_pdc) {
+    const uint32_t qi = __shfl_sync(0xffffffffu, i, src), qj = __shfl_sync(0xffffffffu, j, src);
+    const float thr = __shfl_sync(0xffffffffu, P.thr, src), pqf = __shfl_sync(0xffffffffu, P.pqf, src);
+    const float Mf = __shfl_sync(0xffffffffu, P.Mf, src), t2f = __shfl_sync(0xffffffffu, P.t2f, src);
+    const float bbf = __shfl_sync(0xffffffffu, P.bbf, src), af = __shfl_sync(0xffffffffu, P.af, src);
+    const float bf = __shfl_sync(0xffffffffu, P.bf, src);
+    const float hpq = 0.5f * pqf, qpq = __fdividef(0.5f * pqf, Mf);
     for (uint32_t t0 = 0; t0 < 10000; t0 += 32) {
-        uint32_t trial = t0 + lane;
+        const uint32_t trial = t0 + lane;
+        const u4 w = philox_pdc(qi, qj, pid, 4u | (trial << 4));
         int st = 0;                               // 0 rejected, 1 accepted, 2 undecided
-        double U1 = 0, U2 = 0;
-        if (trial < 10000) {
-            u4 w = philox(i, j, pid, 4u | (trial << 4), k0, k1);
-            U1 = u01d(w.x, w.y);
-            U2 = u01d(w.z, w.w);
-            st = 2;
-            float xf;
-            if (U1 < thr) { float h = (float)U1 * pqf * 0.5f; xf = h * h; }
-            else { float h = __fdividef(2.0f * Mf, (float)(1.0 - U1) * pqf); xf = h * h; }
-            const bool ca = xf < t2f * 0.99999f, cb = xf > t2f * 1.00001f;
-            if (U2 > 0.0 && xf > 1e-30f && xf < 1.0e30f && (ca || cb)) {
-                const float rs = rsqrtf(xf);
-                const float argf = bbf * rs * rs;
-                float elo = 0.0f, ehi = 1e-30f;
-                if (argf <= 80.0f) {
-                    const float ef = __expf(-argf), re = argf * 4e-6f + 2e-6f;
-                    elo = ef * (1.0f - re); ehi = ef * (1.0f + re);
+        {
+            const float u = __uint2float_rd(w.x) * 0x1p-32f, v = 1.0f - u;
+            const bool ca = u < thr;
+            const float q = ca ? u * hpq : v * qpq;             // sqrt(X), or its reciprocal
+            const float r = rcp_fast(q);
+            const float hx = ca ? q : r, rs = ca ? r : q;
+            const float y = bf * rs, arg = y * y, iz = rcp_fast(fmaf(af, hx, y));
+            const float lam = fmaxf(__expf(-arg), 1e-30f) * iz * fmaf(0.5f, iz, y) * fmaf(1e-3f, arg, 1.03f);
+            const float mult = hx * hx < t2f * 1.001f ? 1.0f : Mf * rs * rs;
+            const bool rej = __uint2float_rd(w.z) * 0x1p-32f * mult > lam;
+            if (trial < 10000 && !(rej && fminf(u, v) > 1.2e-4f && bf >= 0.0f)) st = 2;
+        }
+        if (!__any_sync(0xffffffffu, st != 0)) continue;
+        const uint32_t ah = w.x >> 5, al = w.y >> 6;
+        const float u1 = fmaf((float)ah, 0x1p-27f, (float)al * 0x1p-53f);
+        const float v1 = fmaf((float)(0x7ffffffu - ah), 0x1p-27f, (float)(0x4000000u - al) * 0x1p-53f);   // 1 - U1
+        const float u2 = fmaf((float)(w.z >> 5), 0x1p-27f, (float)(w.w >> 6) * 0x1p-53f);
+        const float hx = u1 < thr ? u1 * pqf * 0.5f : __fdividef(2.0f * Mf, v1 * pqf);
+        const float xf = hx * hx;
+        const bool ca = xf < t2f * 0.99999f, cb = xf > t2f * 1.00001f;
+        if (st != 0 && u2 > 0.0f && xf > 1e-30f && xf < 1.0e30f && (ca || cb) && fabsf(u1 - thr) > thr * 1e-6f) {
+            const float rs = rsqrtf(xf);
+            const float argf = bbf * rs * rs;
+            float elo = 0.0f, ehi = 1e-30f;
+            if (argf <= 80.0f) {
+                const float ef = __expf(-argf), re = argf * 4e-6f + 2e-6f;
+                elo = ef * (1.0f - re); ehi = ef * (1.0f + re);
+            }
+            const float sx = xf * rs;
+            const float zf = bf * rs + af * sx;
+            if (zf >= 0.0f) {
+                float flo, fhi;
+                if (zf >= 6.0f && bf >= 0.0f) {
+                    const float iz = __frcp_rn(zf), h = 0.5f * iz * iz;
+                    float s = 1.0f - 13.0f * h;
+                    s = 1.0f - 11.0f * h * s; s = 1.0f - 9.0f * h * s; s = 1.0f - 7.0f * h * s;
+                    s = 1.0f - 5.0f * h * s; s = 1.0f - 3.0f * h * s;
+                    const float omq = fmaf(af * sx * iz, h * s, bf * rs * iz);
+                    flo = omq * 0.99998f - 1e-14f; fhi = omq * 1.00002f + 1e-14f;
+                } else {
+                    const float Q = af * 1.7724539f * sx * erfcx_f(zf);
+                    flo = 1.0f - Q * 1.00002f - 1e-6f; fhi = 1.0f - Q * 0.99998f + 1e-6f;
                 }
-                const float sx = xf * rs;
-                const float zf = bf * rs + af * sx;
-                if (zf >= 0.0f) {
-                    float flo, fhi;
-                    if (zf >= 6.0f && bf >= 0.0f) {
-                        const float iz = __frcp_rn(zf), h = 0.5f * iz * iz;
-                        float s = 1.0f - 13.0f * h;
-                        s = 1.0f - 11.0f * h * s; s = 1.0f - 9.0f * h * s; s = 1.0f - 7.0f * h * s;
-                        s = 1.0f - 5.0f * h * s; s = 1.0f - 3.0f * h * s;
-                        const float omq = fmaf(af * sx * iz, h * s, bf * rs * iz);
-                        flo = omq * 0.99998f - 1e-14f; fhi = omq * 1.00002f + 1e-14f;
-                    } else {
-                        const float Q = af * 1.7724539f * sx * erfcx_f(zf);
-                        flo = 1.0f - Q * 1.00002f - 1e-6f; fhi = 1.0f - Q * 0.99998f + 1e-6f;
-                    }
-                    const double Llo = (double)(elo * fmaxf(flo, 0.0f)) * (1.0 - 1e-6);
-                    const double Lhi = (double)(ehi * fmaxf(fhi, 0.0f)) * (1.0 + 1e-6) + 1e-37;
-                    if (ca) st = U2 <= Llo ? 1 : (U2 > Lhi ? 0 : 2);
-                    else {
-                        const double lhs = U2 * M;
-                        st = lhs <= Llo * (double)xf * (1.0 - 3e-6) ? 1 : (lhs > Lhi * (double)xf * (1.0 + 3e-6) ? 0 : 2);
-                    }
+                const float Llo = elo * fmaxf(flo, 0.0f) * (1.0f - 2e-6f) - 1e-30f;
+                const float Lhi = ehi * fmaxf(fhi, 0.0f) * (1.0f + 2e-6f) + 1e-30f;
+                if (ca) st = u2 <= Llo * (1.0f - 1e-6f) ? 1 : (u2 > Lhi * (1.0f + 1e-6f) ? 0 : 2);
+                else {
+                    const float lhs = u2 * Mf;
+                    st = lhs <= Llo * xf * (1.0f - 5e-6f) ? 1 : (lhs > Lhi * xf * (1.0f + 5e-6f) ? 0 : 2);
                 }
             }
         }
-        if (__any_sync(0xffffffffu, st == 2) && st == 2) {
-            double X;
-            if (U1 < thr) { double h = U1 * pq / 2; X = h * h; }
-            else { double h = 2 / ((1 - U1) * pq / M); X = h * h; }
-            // lambdax <= e: a trial that fails against e alone is rejected
-            // without evaluating erfcx (same decision as the full test)
-            double e = exp_(-b * b / X);
-            double v = U2 * M / X;
-            st = 0;
-            if ((X <= t2 && U2 <= e) || (X >= t2 && v <= e)) {
-                double sqX = sqrt(X);
-                double lambdax = e * (1.0 - a * sqrt(3.141592653589793 * X) * erfcx_(b / sqX + a * sqX));
-                st = ((X <= t2 && U2 <= lambdax) || (X >= t2 && v <= lambdax)) ? 1 : 0;
+        if (__any_sync(0xffffffffu, st == 2)) {
+            const double da = __shfl_sync(0xffffffffu, a, src), db = __shfl_sync(0xffffffffu, b, src);
+            if (st == 2) {
+                const double t2 = 2.0 * db / da, r = sqrt(t2), M = fmax(1.0 / (da * da), 3.0 * db / da);
+                const double pq = 2.0 * r + 2.0 / r * M;
+                const double X = pdc_x(da, db, pq, M, w.x, w.y), U2 = u01d(w.z, w.w);
+                // lambdax <= e: a trial that fails against e alone is rejected
+                // without evaluating erfcx (same decision as the full test)
+                const double e = exp_(-db * db / X);
+                const double v = U2 * M / X;
+                st = 0;
+                if ((X <= t2 && U2 <= e) || (X >= t2 && v <= e)) {
+                    const double sqX = sqrt(X);
+                    const double lambdax = e * (1.0 - da * sqrt(3.141592653589793 * X) * erfcx_(db / sqX + da * sqX));
+                    st = ((X <= t2 && U2 <= lambdax) || (X >= t2 && v <= lambdax)) ? 1 : 0;
+                }
             }
         }
-        unsigned m = __ballot_sync(0xffffffffu, st == 1);
+        const unsigned m = __ballot_sync(0xffffffffu, st == 1);
         if (m) {
-            const int src = __ffs(m) - 1;
-            double X = 0;
-            if (lane == src) {
-                if (U1 < thr) { double h = U1 * pq / 2; X = h * h; }
-                else { double h = 2 / ((1 - U1) * pq / M); X = h * h; }
-            }
-            return __shfl_sync(0xffffffffu, X, src);
+            const int win = __ffs(m) - 1;
+            return ((uint64_t)__shfl_sync(0xffffffffu, w.x, win) << 32) | __shfl_sync(0xffffffffu, w.y, win);
         }
     }
-    return -1.0;
+    return ~0ull;
+}
+
+// the event kernel's copy, out of line (its two call sites in one place)
+__device__ __noinline__ uint64_t pdc_find_nc(int src, uint32_t i, uint32_t j, uint32_t pid, uint32_t k0, uint32_t k1,
+                                             const PdcPair P, double a, double b, int lane) {
+    return pdc_find(src, i, j, pid, P, a, b, lane,
+                    [k0, k1](uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) { return philox(c0, c1, c2, c3, k0, k1); });
 }
 
 // sampleIRT (:116-184) with the acceptance draw U supplied.  Returns the
@@ -431,7 +491,9 @@ __global__ void __launch_bounds__(IB) k_irt_load(IArgs A) {
             A.th2[p] = h2;
             // |f32 shadow distance - f64 distance| <= 3.1e-7 * extent; 1e-6 * extent + 1e-4 nm bounds it
             A.tdel[p] = mext * 1e-6f + 1e-4f;
-            A.ttiles[p] = (n + 31) / 32;
+            uint32_t tiles = 0;                    // the pairing kernel's tiles: 32 particles of one species
+            for (int q = 0; q < 6; ++q) tiles += (cnt[q] + 31) / 32;
+            A.ttiles[p] = tiles;
             A.tev[p] = 0;
         }
         if (n) { n_tracks++; n_part += n; }
@@ -440,73 +502,74 @@ __global__ void __launch_bounds__(IB) k_irt_load(IArgs A) {
     if (lane == 0 && n_tracks) { atomicAdd(&A.acc[12], n_tracks); atomicAdd(&A.acc[13], n_part); }
 }
 
-// Cheap test that a pair may pass the exact acceptance-radius test r2 <= R^2
-// of r_acc: f32 shadow distance r2f (error below del), acceptance word w
-// with U = (w + 0.5) / 2^32 >= Uf.  Never false when the exact test is true:
-//   R = max(s, s c / U) + add  (times 1 + 1e-6, plus 1e-6), so either
-//   rf <= (s + add)(1+1e-6) + 1e-6 + del, or (rf - kb) U <= s c (1+1e-6)^2
-//   with kb = add (1+1e-6) + 1e-6 + del, which holds for Uf <= U as well;
-// both are squared, with a 1e-4 relative margin for the f32 arithmetic.
-__device__ __forceinline__ bool pair_maybe(const IrtConst& C, int ri, float r2f, float del, uint32_t w) {
-    float ta = (C.fa0[ri] + del) * 1.000001f;
-    if (r2f <= ta * ta * 1.0001f) return true;
-    float uf = __uint2float_rd(w) * 2.3283064365386963e-10f;
-    float kb = (C.fkb0[ri] + del) * 1.000001f;
-    float rhs = fmaf(kb, uf, C.fk[ri]);
-    return r2f * uf * uf <= rhs * rhs * 1.0001f;
-}
-
 __device__ __forceinline__ u4 philox_accept(uint32_t blk, uint32_t i, uint32_t pid, const uint32_t* rk) {
     return philox_rk(blk, i, pid, 3u, rk);
 }
 
-// 2) initial pairing (:539-558): one warp per (track, tile of 32 particles).
-//    The tile's particles sit in lane registers as f32 shadows; partners come
-//    32 at a time through shared memory and are read as broadcasts.  The f32
-//    distance settles the R_CUT test and the acceptance prefilter for almost
-//    every pair; the rare candidates (and pairs within rounding of R_CUT) are
-//    queued per warp and redone exactly in f64, 32 at a time, one per lane.
-constexpr int IQ = 64;                   // candidate queue per warp
+// 2) initial pairing (:539-558): one warp per (track, tile of 32 particles of one
+//    species).  What bounds it is the number of instructions per pair: every
+//    pair inside R_CUT needs its own Philox word (4 partners to a block), so
+//    everything else is kept off the pair.  The tile's particles sit in lane
+//    registers; 32 partners at a time are staged in shared memory with the
+//    constants of their reaction with the tile's species (a tile of one
+//    species needs one table row), and those that cannot react with it, or do
+//    not exist, are staged so far away that no test passes.  A pair is a
+//    candidate when
+//      R_CUT may hold and (U, r) may pass the exact test r2 <= R^2 of r_acc.
+//    With R = max(s, s c / U) + add (times 1 + 1e-6, plus 1e-6) and the shadow
+//    distance within del of the exact one, that is
+//      r <= (s + add)(1+1e-6) + 1e-6 + del             (rare: `ta2`), or
+//      (r - kb) U <= s c (1+1e-6)^2,  kb = add (1+1e-6) + 1e-6 + del,
+//    which holds for any lower bound of U as well: the word's upper 16 bits,
+//    which cost a byte permute instead of a conversion and admit 1 % more
+//    candidates.  Both sides are squared, with a 1e-4 margin for the f32
+//    arithmetic.  Each lane keeps its candidates in its own column of shared memory
+//    (no vote per pair); a full column makes the warp pack all columns and
+//    evaluate them exactly in f64, 32 at a time, one per lane.
+//    Measured at 4096 x 10 keV: 10.5 ms; 14.9 ms with tiles in index order, one
+//    table gather per pair and queue votes per partner (5, 6, 7 blocks per SM:
+//    10.8, 10.5, 10.5 ms).
+constexpr int IQ = 64;                   // partner queue per warp of the event kernel
+constexpr int QCAP = 16;                 // candidates per lane
+constexpr float FAR = 1e18f;             // shadow coordinate of a partner that cannot react
 
 struct InitTrack {
     const double *px, *py, *pz;
+    const float4* pf;
+    const int8_t* sp;
     double* ET;
     uint32_t* EAB;
     uint32_t* tev;
     uint32_t ecp, pid;
+    float lo2;                           // shadow distance^2 below which a pair is certainly inside R_CUT
 };
 
-// exact evaluation of queued candidates [0, cnt): one per lane; returns the
-// reactive pairs inside R_CUT found among the near-R_CUT entries
-__device__ __forceinline__ uint32_t init_batch(const IrtConst& C, const InitTrack& T, const uint32_t* qij,
-                                               const uint32_t* qw, const uint16_t* qk, int cnt, int lane,
-                                               uint32_t k0, uint32_t k1, bool& ev_over) {
+// exact evaluation of queued candidates [0, cnt), one per lane; returns the
+// reactive pairs inside R_CUT found among those within rounding of it
+__device__ __forceinline__ uint32_t init_batch(const IrtConst& C, const InitTrack& T, const uint32_t* qij, int cnt,
+                                               int lane, const uint32_t* rk, bool& ev_over) {
     const unsigned lt = (1u << lane) - 1u;
     bool acc = false, pdcq = false;
-    double t = 0, pa = 0, pb = 0, pD = 0;
+    double t = 0, pa = 1, pb = 1, pD = 1;
     uint32_t i = 0, j = 0, np = 0;
     if (lane < cnt) {
-        const uint32_t ij = qij[lane], k = qk[lane];
-        uint32_t wd = qw[lane];
+        const uint32_t ij = qij[lane];
         i = ij >> 16; j = ij & 0xffffu;
-        const int kind = (int)(k & 3u), ri = (int)((k >> 2) & 15u);
-        const int si = (int)((k >> 6) & 7u), sj = (int)((k >> 9) & 7u);
-        double dx = T.px[i] - T.px[j], dy = T.py[i] - T.py[j], dz = T.pz[i] - T.pz[j];
-        double r2 = dx * dx + dy * dy + dz * dz;
-        bool inside = true;
-        if (kind == 2) {
-            inside = r2 <= C.r_cut2;
-            if (inside) {
-                np = 1;
-                u4 w4 = philox(j >> 2, i, T.pid, 3u, k0, k1);
-                wd = (j & 3) == 0 ? w4.x : (j & 3) == 1 ? w4.y : (j & 3) == 2 ? w4.z : w4.w;
-            }
-        }
+        const float4 a = T.pf[i], q = T.pf[j];
+        const int si = __float_as_int(a.w), sj = __float_as_int(q.w);
+        const int ri = C.map[si * 6 + sj];
+        const float fx = a.x - q.x, fy = a.y - q.y, fz = a.z - q.z;
+        const bool sure = fmaf(fz, fz, fmaf(fy, fy, fx * fx)) < T.lo2;     // counted by the scan
+        const double dx = T.px[i] - T.px[j], dy = T.py[i] - T.py[j], dz = T.pz[i] - T.pz[j];
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        const bool inside = sure || r2 <= C.r_cut2;
         if (inside) {
-            double U = u01d32(wd);
-            double R = r_acc(C, ri, U);
+            if (!sure) np = 1;
+            const u4 w4 = philox_accept(j >> 2, i, T.pid, rk);
+            const double U = u01d32((j & 3) == 0 ? w4.x : (j & 3) == 1 ? w4.y : (j & 3) == 2 ? w4.z : w4.w);
+            const double R = r_acc(C, ri, U);
             if (r2 <= R * R) {
-                double D = C.D[si] + C.D[sj];
+                const double D = C.D[si] + C.D[sj];
                 t = sample_pre(C, sqrt(r2), ri, D, U, &pa, &pb);
                 if (t == -2.0) { pdcq = true; pD = D; }
                 else acc = (t >= 0 && t < 1000);
@@ -514,20 +577,27 @@ __device__ __forceinline__ uint32_t init_batch(const IrtConst& C, const InitTrac
         }
     }
     unsigned pm = __ballot_sync(FULL, pdcq);
-    while (pm) {
-        int src = __ffs(pm) - 1;
-        pm &= pm - 1;
-        uint32_t qi = __shfl_sync(FULL, i, src), qj = __shfl_sync(FULL, j, src);
-        double qa = __shfl_sync(FULL, pa, src), qb = __shfl_sync(FULL, pb, src);
-        double X = pdc_warp(qi, qj, T.pid, k0, k1, qa, qb, lane);
-        if (lane == src && X > 0) { t = X / pD; acc = t < 1000; }
+    if (pm) {
+        const PdcPair P = pdc_pair(pa, pb);
+        uint64_t words = ~0ull;
+        while (pm) {
+            const int src = __ffs(pm) - 1;
+            pm &= pm - 1;
+            const uint64_t wd = pdc_find(src, i, j, T.pid, P, pa, pb, lane,
+                                         [rk](uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) { return philox_rk(c0, c1, c2, c3, rk); });
+            if (lane == src) words = wd;
+        }
+        if (pdcq && words != ~0ull) {
+            const double X = pdc_x(pa, pb, P.pq, P.M, (uint32_t)(words >> 32), (uint32_t)words);
+            if (X > 0) { t = X / pD; acc = t < 1000; }
+        }
     }
-    unsigned m = __ballot_sync(FULL, acc);
+    const unsigned m = __ballot_sync(FULL, acc);
     if (m) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(T.tev, (uint32_t)__popc(m));
         base = __shfl_sync(FULL, base, 0);
-        uint32_t slot = base + __popc(m & lt);
+        const uint32_t slot = base + __popc(m & lt);
         if (acc) {
             if (slot < T.ecp) { T.ET[slot] = t; T.EAB[slot] = (i << 16) | j; }
             else ev_over = true;
@@ -536,36 +606,23 @@ __device__ __forceinline__ uint32_t init_batch(const IrtConst& C, const InitTrac
     return np;
 }
 
-// One out-of-line copy of the exact evaluation for the pairing kernel's two
-// call sites (measured faster than two inlined copies: less code and fewer
-// spills in the partner loop).
-struct IbOut { uint32_t np; uint32_t over; };
-__device__ __noinline__ IbOut init_batch_nc(const IrtConst& C, InitTrack T, const uint32_t* qij, const uint32_t* qw,
-                                            const uint16_t* qk, int cnt, int lane, uint32_t k0, uint32_t k1) {
-    bool over = false;
-    const uint32_t np = init_batch(C, T, qij, qw, qk, cnt, lane, k0, k1, over);
-    return IbOut{np, over ? 1u : 0u};
-}
-
 #ifndef WG_INIT_MINB
-#define WG_INIT_MINB 7
+#define WG_INIT_MINB 6
 #endif
-__global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(IArgs A) {
+__global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(const __grid_constant__ IArgs A) {
     __shared__ IrtConst s_c;
     __shared__ uint32_t s_row[6];
-    __shared__ float4 s_pj[IB / 32][32];
-    __shared__ uint32_t s_qij[IB / 32][IQ], s_qw[IB / 32][IQ];
-    __shared__ uint16_t s_qk[IB / 32][IQ];
+    // partners of a chunk: shadow x, y, z and the bound's kb and fk (scaled to 16-bit U)
+    __shared__ __align__(16) float s_p[IB / 32][5][32];
+    __shared__ uint16_t s_q[IB / 32][QCAP][32];
+    __shared__ uint32_t s_d[IB / 32][QCAP * 32 + 32];
     load_consts(&s_c, s_row);
     const IrtConst& C = s_c;
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const unsigned lt = (1u << lane) - 1u;
     const unsigned long long nitems = A.toff[A.nseg];
     const float rcut = (float)sqrt(C.r_cut2);
-    const uint32_t k0 = A.k0, k1 = A.k1;
-    uint32_t* qij = s_qij[wl];
-    uint32_t* qw = s_qw[wl];
-    uint16_t* qk = s_qk[wl];
+    float (*sp)[32] = s_p[wl];
+    uint32_t* dq = s_d[wl];
     unsigned long long n_pairs = 0;
     bool ev_over = false;
     for (;;) {
@@ -577,101 +634,129 @@ __global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(IArgs A) {
         while (hi - lo > 1) { uint32_t mid = (lo + hi) >> 1; if (A.toff[mid] <= item) lo = mid; else hi = mid; }
         const uint32_t p = lo;
         const uint32_t n = A.tn[p];
-        const uint32_t i0 = 32u * (uint32_t)(item - A.toff[p]);
+        // the item's species and its place in that species' list
+        uint32_t tile = (uint32_t)(item - A.toff[p]), len = 0;
+        int s = 0;
+        for (; s < 6; ++s) {
+            len = A.tlc[6 * p + s];
+            const uint32_t nt = (len + 31) / 32;
+            if (tile < nt) break;
+            tile -= nt;
+        }
+        if (s == 6) break;                            // not reached: ttiles is the sum of these
+        const uint32_t row = s_row[s];
         const unsigned long long tb0 = tbase(A, p);
+        const uint32_t cap = tcap(A, p);
         const float4* pf = A.pf + tb0;
         const float del = A.tdel[p];
         const float clo = (rcut - del) * 0.99999f, chi = (rcut + del) * 1.00001f;
-        const float lo2 = clo * clo, hi2 = chi * chi;
-        InitTrack T{A.px + tb0, A.py + tb0, A.pz + tb0, A.ev_t + ebase(A, p), A.ev_ab + ebase(A, p), &A.tev[p],
-                    ecap(A, p), A.pid_base + p};
-        const uint32_t i = i0 + lane;
-        const bool hi_ = i < n;
-        float4 me = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (hi_) me = pf[i];
-        const int si = hi_ ? __float_as_int(me.w) : 0;
-        const uint32_t row = s_row[si];
-        int qn = 0;
-        for (uint32_t j0 = i0; j0 < n; j0 += 32) {
-            __syncwarp();
-            if (j0 + lane < n) s_pj[wl][lane] = pf[j0 + lane];
-            __syncwarp();
-            const uint32_t kmax = min(32u, n - j0);
-            // partners in groups of 4 = one Philox block of acceptance words
-            // (j0 is a multiple of 32): 4 distances, at most one Philox call
-            for (uint32_t kk = 0; kk < kmax; kk += 4) {
-                float r2[4];
-                int rr[4], sv[4];
-                bool ok[4];
-                bool need = false;
+        const float lo2 = clo * clo, hi2 = chi * chi, lo2s = lo2 * 0x1p100f, hi2s = hi2 * 0x1p100f;
+        const InitTrack T{A.px + tb0, A.py + tb0, A.pz + tb0, pf, A.sp + tb0, A.ev_t + ebase(A, p), A.ev_ab + ebase(A, p),
+                          &A.tev[p], ecap(A, p), A.pid_base + p, lo2};
+        const uint32_t at = 32u * tile + lane;
+        const bool have = at < len;
+        const uint32_t i = have ? A.lst[6 * tb0 + (size_t)s * cap + at] : 0xffffu;
+        float4 me = make_float4(-3.0f * FAR, 0.f, 0.f, 0.f);
+        if (have) me = A.rec[6 * tb0 + (size_t)s * cap + at];
+        float ta2 = 0.0f;                             // (r_acc's radius for U -> 1)^2, over the row's reactions
+        for (int q = 0; q < 6; ++q) {
+            const int r = (int)((row >> (4 * q)) & 15u);
+            if (r != 15) { const float ta = (C.fa0[r] + del) * 1.000001f; ta2 = fmaxf(ta2, ta * ta * 1.0001f); }
+        }
+        const uint32_t imin = __shfl_sync(FULL, i, 0);
+        const uint32_t imax = __shfl_sync(FULL, i, min(31u, len - 32u * tile - 1u));
+        uint32_t cnt = 0, rem = 0;
+        float np = 0.0f;                              // at most 32,735 partners: exact
+        const uint32_t gend = (n + 3) >> 2;           // groups of 4 partners = one Philox block
+        for (uint32_t g = (imin >> 5) << 3; g < gend; ++g) {
+            if ((g & 7u) == 0) {
+                __syncwarp();
+                const uint32_t j = 4 * g + lane;
+                float4 q = make_float4(FAR, 0.f, 0.f, 0.f);
+                float kb = 0.0f, fk = 0.0f;
+                if (j < n) {
+                    q = pf[j];
+                    const int r = (int)((row >> (4 * __float_as_int(q.w))) & 15u);
+                    if (r == 15) q.x = FAR;
+                    else { kb = (C.fkb0[r] + del) * 1.00006f; fk = C.fk[r] * (65536.0f * 1.00006f); }
+                }
+                sp[0][lane] = q.x; sp[1][lane] = q.y; sp[2][lane] = q.z; sp[3][lane] = kb; sp[4][lane] = fk;
+                __syncwarp();
+            }
+            const uint32_t k = (g & 7u) * 4u;
+            const float4 X = *reinterpret_cast<const float4*>(&sp[0][k]), Y = *reinterpret_cast<const float4*>(&sp[1][k]);
+            const float4 Z = *reinterpret_cast<const float4*>(&sp[2][k]);
+            float r2[4];
+            {
+                const float qx[4] = {X.x, X.y, X.z, X.w}, qy[4] = {Y.x, Y.y, Y.z, Y.w}, qz[4] = {Z.x, Z.y, Z.z, Z.w};
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const uint32_t j = j0 + kk + u;
-                    const float4 q = s_pj[wl][kk + u];
-                    const bool in = kk + u < kmax;
-                    sv[u] = in ? __float_as_int(q.w) : 0;
-                    rr[u] = (int)((row >> (4 * sv[u])) & 15u);
-                    ok[u] = in && hi_ && j > i && rr[u] != 15;
-                    const float dx = me.x - q.x, dy = me.y - q.y, dz = me.z - q.z;
+                    const float dx = me.x - qx[u], dy = me.y - qy[u], dz = me.z - qz[u];
                     r2[u] = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                    need |= ok[u] && r2[u] < lo2;
-                }
-                u4 cw = {0, 0, 0, 0};
-                if (need) cw = philox_accept((j0 + kk) >> 2, i, T.pid, A.rk);
-                int kind[4];                            // 1: candidate, 2: near R_CUT
-                bool any = false;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const uint32_t wd = u == 0 ? cw.x : u == 1 ? cw.y : u == 2 ? cw.z : cw.w;
-                    kind[u] = 0;
-                    if (ok[u]) {
-                        if (r2[u] < lo2) {
-                            n_pairs++;
-                            if (pair_maybe(C, rr[u], r2[u], del, wd)) kind[u] = 1;
-                        } else if (r2[u] <= hi2) kind[u] = 2;
-                    }
-                    any |= kind[u] != 0;
-                }
-                if (!__any_sync(FULL, any)) continue;
-                // queue entries of the four partners, 12 bits each (kind | rr << 2 | sv << 6);
-                // the queueing loop is kept rolled (one copy of its code, fewer spills:
-                // measured faster than four unrolled copies)
-                uint64_t pk = 0;
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    pk |= (uint64_t)((uint32_t)kind[u] | ((uint32_t)rr[u] << 2) | ((uint32_t)sv[u] << 6)) << (12 * u);
-#pragma unroll 1
-                for (int u = 0; u < 4; ++u) {
-                    const uint32_t f = (uint32_t)(pk >> (12 * u)) & 0xfffu;
-                    const unsigned m = __ballot_sync(FULL, (f & 3u) != 0u);
-                    if (!m) continue;
-                    if (f & 3u) {
-                        const int at = qn + __popc(m & lt);
-                        qij[at] = (i << 16) | (j0 + kk + u);
-                        qw[at] = u == 0 ? cw.x : u == 1 ? cw.y : u == 2 ? cw.z : cw.w;
-                        qk[at] = (uint16_t)((f & 3u) | (((f >> 2) & 15u) << 2) | (si << 6) | ((f >> 6) << 9));
-                    }
-                    qn += __popc(m);
-                    if (qn >= 32) {
-                        __syncwarp();
-                        const IbOut o = init_batch_nc(C, T, qij, qw, qk, 32, lane, k0, k1);
-                        n_pairs += o.np;
-                        ev_over |= o.over != 0u;
-                        __syncwarp();
-                        if (lane < qn - 32) { qij[lane] = qij[32 + lane]; qw[lane] = qw[32 + lane]; qk[lane] = qk[32 + lane]; }
-                        qn -= 32;
-                        __syncwarp();
-                    }
                 }
             }
+            if (4 * g <= imax) {                      // partners not after i do not count
+#pragma unroll
+                for (int u = 0; u < 4; ++u) r2[u] = 4 * g + u > i ? r2[u] : FAR * FAR;
+            }
+            // pairs surely inside R_CUT, and those that may be: sums of saturated
+            // differences (the sign decides, 2^100 makes any difference 1), which run on the
+            // FP32 pipe; a compare and a count would each take two cycles of the integer one
+            float nlo = 0.0f, nhi = 0.0f;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                nlo += __saturatef(fmaf(r2[u], -0x1p100f, lo2s));
+                nhi += __saturatef(fmaf(r2[u], -0x1p100f, hi2s));
+            }
+            if (nhi > 0.0f) {
+                const float4 KB = *reinterpret_cast<const float4*>(&sp[3][k]), FK = *reinterpret_cast<const float4*>(&sp[4][k]);
+                const float kb[4] = {KB.x, KB.y, KB.z, KB.w}, fk[4] = {FK.x, FK.y, FK.z, FK.w};
+                const u4 cw = philox_accept(g, i, T.pid, A.rk);
+                const uint32_t wd[4] = {cw.x, cw.y, cw.z, cw.w};
+                np += nlo;
+                float v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    // 2^23 + the word's upper 16 bits, minus 2^23
+                    const float uf = __uint_as_float(__byte_perm(wd[u], 0x4B000000u, 0x7632)) - 8388608.0f;
+                    const float rhs = fmaf(kb[u], uf, fk[u]);
+                    v[u] = fmaf(rhs, rhs, -(r2[u] * (uf * uf)));
+                }
+                const float mn = fminf(fminf(fminf(r2[0], r2[1]), r2[2]), r2[3]);
+                if (fmaxf(fmaxf(fmaxf(v[0], v[1]), v[2]), v[3]) >= 0.0f || nhi != nlo || mn <= ta2) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if ((v[u] >= 0.0f || !(r2[u] < lo2) || r2[u] <= ta2) && r2[u] <= hi2) {
+                            s_q[wl][cnt][lane] = (uint16_t)(4 * g + u);
+                            cnt++;
+                        }
+                }
+            }
+            const bool last = g + 1 == gend;
+            if (last || __any_sync(FULL, cnt > QCAP - 4)) {
+                __syncwarp();
+                uint32_t off = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const uint32_t v = __shfl_up_sync(FULL, off, o); if (lane >= o) off += v; }
+                const uint32_t total = rem + __shfl_sync(FULL, off, 31);
+                off += rem - cnt;
+                for (uint32_t c = 0; c < cnt; ++c) dq[off + c] = (i << 16) | s_q[wl][c][lane];
+                cnt = 0;
+                __syncwarp();
+                uint32_t b = 0;
+                for (; b + (last ? 1u : 32u) <= total; b += 32)
+                    n_pairs += init_batch(C, T, dq + b, (int)min(32u, total - b), lane, A.rk, ev_over);
+                rem = 0;
+                if (b < total) {
+                    rem = total - b;
+                    const uint32_t v = (uint32_t)lane < rem ? dq[b + lane] : 0u;
+                    __syncwarp();
+                    if ((uint32_t)lane < rem) dq[lane] = v;
+                }
+                __syncwarp();
+            }
         }
-        if (qn) {
-            __syncwarp();
-            const IbOut o = init_batch_nc(C, T, qij, qw, qk, qn, lane, k0, k1);
-            n_pairs += o.np;
-            ev_over |= o.over != 0u;
-            __syncwarp();
-        }
+        n_pairs += (unsigned long long)np;
     }
     if (__any_sync(FULL, ev_over) && lane == 0) atomicOr(A.err, DERR_HEAP);
     for (int o = 16; o; o >>= 1) n_pairs += __shfl_xor_sync(FULL, n_pairs, o);
@@ -705,7 +790,7 @@ struct ProdCtx {
 __device__ __forceinline__ bool prod_batch(const IrtConst& C, const ProdCtx& P, const uint32_t* pq, int cnt, int lane,
                                         const Heap& H, uint32_t& hn, uint32_t hcap) {
     bool acc = false, pdcq = false, over = false;
-    double ta = 0, pa = 0, pb = 0, pD = 0;
+    double ta = 0, pa = 1, pb = 1, pD = 1;
     uint32_t jj = 0;
     const double pnx = P.px[P.id], pny = P.py[P.id], pnz = P.pz[P.id], pet = P.tb[P.id];
     if (lane < cnt) {
@@ -749,13 +834,19 @@ __device__ __forceinline__ bool prod_batch(const IrtConst& C, const ProdCtx& P, 
         }
     }
     unsigned pm = __ballot_sync(FULL, pdcq);
-    while (pm) {
-        int src = __ffs(pm) - 1;
-        pm &= pm - 1;
-        uint32_t qj = __shfl_sync(FULL, jj, src);
-        double qa = __shfl_sync(FULL, pa, src), qb = __shfl_sync(FULL, pb, src);
-        double X = pdc_warp(P.id, qj, P.pid, P.k0, P.k1, qa, qb, lane);
-        if (lane == src && X > 0) { ta = pet + X / pD; acc = ta < 1000; }
+    if (pm) {
+        const PdcPair PP = pdc_pair(pa, pb);
+        uint64_t words = ~0ull;
+        while (pm) {
+            const int src = __ffs(pm) - 1;
+            pm &= pm - 1;
+            const uint64_t wd = pdc_find_nc(src, P.id, jj, P.pid, P.k0, P.k1, PP, pa, pb, lane);
+            if (lane == src) words = wd;
+        }
+        if (pdcq && words != ~0ull) {
+            const double X = pdc_x(pa, pb, PP.pq, PP.M, (uint32_t)(words >> 32), (uint32_t)words);
+            if (X > 0) { ta = pet + X / pD; acc = ta < 1000; }
+        }
     }
     unsigned m = __ballot_sync(FULL, acc);
     while (m) {
