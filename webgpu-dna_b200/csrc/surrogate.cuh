@@ -16,47 +16,34 @@ constexpr int SG_OFF_W3 = SG_OFF_B2 + SG_HID, SG_OFF_B3 = SG_OFF_W3 + SG_HID * S
 constexpr int SG_OFF_W4 = SG_OFF_B3 + SG_HID, SG_OFF_B4 = SG_OFF_W4 + SG_OUT * SG_HID;
 constexpr int SG_NPARAM = SG_OFF_B4 + SG_OUT;
 
-// bf16 copies of the weights: W_l as [out][in] and transposed [in][out]
+// bf16 copies of the weights, W_l [out][in] and transposed [in][out], each laid out
+// as the tensor cores' K-major shared-memory operand (surrogate.cu coff)
 struct SgWeights {
     const __nv_bfloat16 *W[4], *WT[4];
     const float* p;                          // f32 parameters (biases read from here)
 };
 
-struct SgFwdArgs {
-    const float* X;                          // n x 64 standardised inputs
+struct SgArgs {
+    const float* X;                          // n x 64 inputs
+    const float *xmean, *xinv;               // standardise on load ((x - xmean) * xinv), or null
     const uint32_t* rows;                    // optional gather (batch -> row of X / T)
     uint32_t n;
     SgWeights w;
-    float* Y;                                // n x 80 outputs
-    // training: saved activations of the batch (bf16 inputs of each layer, f32 pre-activations)
-    __nv_bfloat16 *H0, *H1, *H2, *H3;
-    float *Z1, *Z2, *Z3;
     uint32_t* err;
-    unsigned long long mma_ns;               // bound of a tensor-core wait
+    unsigned long long mma_ns;               // bound of a tensor-core or bulk-copy wait
     uint32_t give_up_first;                  // test switch: a tile's first wait gives up at once
-    // optional fusions of the chemistry path: standardise X on load
-    // ((x - xmean) * xinv), and add the energy-weighted de-standardised outputs
-    // ((y * ystd + ymean) * E_track, then E_track) to acc[0..80] (Y may be null)
-    const float *xmean, *xinv;
+    // forward: outputs y * ystd + ymean to Y (n x 80, may be null), and / or their
+    // energy-weighted sums ((y * ystd + ymean) * E_track, then E_track) added to acc[0..80]
+    float* Y;
     const float *ymean, *ystd;
     const float* E;                          // per-row energy, or null for E0
     float E0;
     double* acc;
-};
-
-struct SgBwdArgs {
-    const float* T;                          // targets (standardised), rows gathered like X
-    const uint32_t* rows;
-    uint32_t n;                              // batch size
-    SgWeights w;
-    const float* Y;
-    const __nv_bfloat16 *H0, *H1, *H2, *H3;
-    const float *Z1, *Z2, *Z3;
-    float* grad;                             // f32, SG_NPARAM, accumulated with atomics
-    double* loss;                            // sum of squared errors
-    uint32_t* err;
-    unsigned long long mma_ns;
-    uint32_t give_up_first;
+    // training: targets (standardised, gathered like X), the CTAs' partial gradients
+    // (sg_parts(n) x SG_NPARAM, overwritten) and the sum of squared errors (added to)
+    const float* T;
+    float* part;
+    double* loss;
 };
 
 // descriptors of the tracks of a canonical rad_buf
@@ -67,23 +54,27 @@ struct DescArgs {
     const float* E;                          // per-track energy (eV) or null
     float E0;                                // energy when E is null
     float* out;                              // nseg x 64
+    const float2* dbin;                      // the distance bins' table (launch_dbin_table)
 };
 
+// the table of the descriptors' distance bins, SG_DBIN entries
+constexpr int SG_DBIN = 25;
+cudaError_t launch_dbin_table(float2* tab, cudaStream_t s);
 cudaError_t launch_descriptors(const DescArgs& a, cudaStream_t s);
-cudaError_t launch_sg_forward(const SgFwdArgs& a, cudaStream_t s);
-cudaError_t launch_sg_backward(const SgBwdArgs& a, cudaStream_t s);
-// Adam on the f32 parameters, then the bf16 weight copies; zeroes the gradient
-cudaError_t launch_sg_adam(float* p, float* m, float* v, float* grad, float lr, float b1t, float b2t,
-                           __nv_bfloat16* Wcat, __nv_bfloat16* WTcat, cudaStream_t s);
+cudaError_t launch_sg_forward(const SgArgs& a, cudaStream_t s);
+// loss and partial gradients of n rows, by sg_parts(n) CTAs of the current device
+cudaError_t launch_sg_train(const SgArgs& a, cudaStream_t s);
+uint32_t sg_parts(uint32_t n);
+// Adam on the f32 parameters with the sum of the partial gradients, then the bf16 weight copies
+cudaError_t launch_sg_adam(float* p, float* m, float* v, const float* part, uint32_t nparts, float lr, float b1t,
+                           float b2t, __nv_bfloat16* Wcat, __nv_bfloat16* WTcat, cudaStream_t s);
+// that sum alone
+cudaError_t launch_sg_grad(const float* part, uint32_t nparts, float* g, cudaStream_t s);
 // bf16 copies of the weights only
 cudaError_t launch_sg_convert(const float* p, __nv_bfloat16* Wcat, __nv_bfloat16* WTcat, cudaStream_t s);
 // standardise rows: out = (in - mean) / std
 cudaError_t launch_sg_standardise(const float* in, float* out, uint64_t n, int dim, const float* mean,
                                   const float* inv_std, cudaStream_t s);
-// energy-weighted sums of de-standardised outputs: acc[k] += (y * std + mean)[k] * E_track
-cudaError_t launch_sg_reduce(const float* Y, uint32_t n, const float* ymean, const float* ystd, const float* E,
-                             float E0, double* acc, cudaStream_t s);
-
 // offsets of W_l (and WT_l) inside the concatenated bf16 arrays
 constexpr int SG_WOFF[4] = {0, SG_HID * SG_IN, SG_HID * SG_IN + SG_HID * SG_HID, SG_HID * SG_IN + 2 * SG_HID * SG_HID};
 constexpr int SG_WTOTAL = SG_HID * SG_IN + 2 * SG_HID * SG_HID + SG_OUT * SG_HID;

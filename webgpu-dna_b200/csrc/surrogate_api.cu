@@ -19,21 +19,21 @@ struct SgState {
     __nv_bfloat16 *W = nullptr, *WT = nullptr;
     float *xmean = nullptr, *xinv = nullptr, *ymean = nullptr, *ystd = nullptr;
     float h_xmean[SG_IN], h_xstd[SG_IN], h_ymean[SG_OUT], h_ystd[SG_OUT];
-    // training data (standardised) and batch buffers
+    // training data (standardised) and a training call's buffers
     float *X = nullptr, *T = nullptr;
     uint64_t ndata = 0, data_cap = 0;
-    uint32_t* rows = nullptr;
-    float* Y = nullptr;
-    __nv_bfloat16 *H0 = nullptr, *H1 = nullptr, *H2 = nullptr, *H3 = nullptr;
-    float *Z1 = nullptr, *Z2 = nullptr, *Z3 = nullptr;
-    uint64_t batch_cap = 0;
+    uint32_t* perm = nullptr;             // the epoch's order of the rows
+    uint64_t perm_cap = 0;
+    float* part = nullptr;                // partial gradients of a batch's CTAs
+    uint32_t part_cap = 0;
     double* loss = nullptr;
     uint32_t* err = nullptr;
     uint64_t step = 0;
     // descriptors / predictions of the last transport
-    float *desc = nullptr, *xs = nullptr, *pred = nullptr;
+    float *desc = nullptr, *pred = nullptr;
     uint64_t desc_n = 0, desc_cap = 0;
     double* acc = nullptr;
+    float2* dbin = nullptr;               // the descriptors' distance bins
     // bound of the kernels' tensor-core waits and the test switch (from the context)
     unsigned long long mma_ns = WG_MMA_WAIT_NS;
     uint32_t give_up_first = 0;
@@ -43,8 +43,7 @@ struct SgState {
 void sg_free(SgState* s) {
     if (!s) return;
     void* ptrs[] = {s->p, s->m, s->v, s->g, s->W, s->WT, s->xmean, s->xinv, s->ymean, s->ystd, s->X, s->T,
-                    s->rows, s->Y, s->H0, s->H1, s->H2, s->H3, s->Z1, s->Z2, s->Z3, s->loss, s->err,
-                    s->desc, s->xs, s->pred, s->acc};
+                    s->perm, s->part, s->loss, s->err, s->desc, s->pred, s->acc, s->dbin};
     for (void* q : ptrs) if (q) cudaFree(q);
     for (cudaEvent_t e : s->ev) if (e) cudaEventDestroy(e);
     delete s;
@@ -75,6 +74,16 @@ uint64_t smix(uint64_t& s) {
 }
 double u01(uint64_t& s) { return (double)(smix(s) >> 11) * (1.0 / 9007199254740992.0); }
 
+int upload_norm(SgState* s, cudaStream_t st) {
+    float xinv[SG_IN];
+    for (int k = 0; k < SG_IN; ++k) xinv[k] = s->h_xstd[k] > 0 ? 1.0f / s->h_xstd[k] : 1.0f;
+    WG_CUDA_OK(cudaMemcpyAsync(s->xmean, s->h_xmean, sizeof s->h_xmean, cudaMemcpyHostToDevice, st));
+    WG_CUDA_OK(cudaMemcpyAsync(s->xinv, xinv, sizeof xinv, cudaMemcpyHostToDevice, st));
+    WG_CUDA_OK(cudaMemcpyAsync(s->ymean, s->h_ymean, sizeof s->h_ymean, cudaMemcpyHostToDevice, st));
+    WG_CUDA_OK(cudaMemcpyAsync(s->ystd, s->h_ystd, sizeof s->h_ystd, cudaMemcpyHostToDevice, st));
+    return WGDNA_OK;
+}
+
 int ensure_state(wgdna_ctx* c, CtxView& v, SgState** out) {
     ctx_view(c, &v);
     WG_CUDA_OK(cudaSetDevice(v.device));
@@ -94,22 +103,15 @@ int ensure_state(wgdna_ctx* c, CtxView& v, SgState** out) {
     STRY(salloc(&s->xmean, SG_IN)); STRY(salloc(&s->xinv, SG_IN));
     STRY(salloc(&s->ymean, SG_OUT)); STRY(salloc(&s->ystd, SG_OUT));
     STRY(salloc(&s->loss, 1)); STRY(salloc(&s->err, 1)); STRY(salloc(&s->acc, SG_OUT + 1));
+    STRY(salloc(&s->dbin, SG_DBIN));
+    WG_CUDA_OK(launch_dbin_table(s->dbin, v.stream));
     WG_CUDA_OK(cudaMemset(s->m, 0, SG_NPARAM * 4)); WG_CUDA_OK(cudaMemset(s->v, 0, SG_NPARAM * 4));
     WG_CUDA_OK(cudaMemset(s->g, 0, SG_NPARAM * 4)); WG_CUDA_OK(cudaMemset(s->p, 0, SG_NPARAM * 4));
     WG_CUDA_OK(cudaMemset(s->err, 0, 4));
     for (int k = 0; k < SG_IN; ++k) { s->h_xmean[k] = 0.0f; s->h_xstd[k] = 1.0f; }
     for (int k = 0; k < SG_OUT; ++k) { s->h_ymean[k] = 0.0f; s->h_ystd[k] = 1.0f; }
+    STRY(upload_norm(s, v.stream));
     *out = s;
-    return WGDNA_OK;
-}
-
-int upload_norm(SgState* s, cudaStream_t st) {
-    float xinv[SG_IN];
-    for (int k = 0; k < SG_IN; ++k) xinv[k] = s->h_xstd[k] > 0 ? 1.0f / s->h_xstd[k] : 1.0f;
-    WG_CUDA_OK(cudaMemcpyAsync(s->xmean, s->h_xmean, sizeof s->h_xmean, cudaMemcpyHostToDevice, st));
-    WG_CUDA_OK(cudaMemcpyAsync(s->xinv, xinv, sizeof xinv, cudaMemcpyHostToDevice, st));
-    WG_CUDA_OK(cudaMemcpyAsync(s->ymean, s->h_ymean, sizeof s->h_ymean, cudaMemcpyHostToDevice, st));
-    WG_CUDA_OK(cudaMemcpyAsync(s->ystd, s->h_ystd, sizeof s->h_ystd, cudaMemcpyHostToDevice, st));
     return WGDNA_OK;
 }
 
@@ -120,13 +122,11 @@ SgWeights weights(SgState* s) {
     return w;
 }
 
-int ensure_batch(SgState* s, uint64_t n) {
-    if (n <= s->batch_cap) return WGDNA_OK;
-    STRY(salloc(&s->rows, n)); STRY(salloc(&s->Y, n * SG_OUT));
-    STRY(salloc(&s->H0, n * SG_IN)); STRY(salloc(&s->H1, n * SG_HID)); STRY(salloc(&s->H2, n * SG_HID));
-    STRY(salloc(&s->H3, n * SG_HID)); STRY(salloc(&s->Z1, n * SG_HID)); STRY(salloc(&s->Z2, n * SG_HID));
-    STRY(salloc(&s->Z3, n * SG_HID));
-    s->batch_cap = n;
+int ensure_parts(SgState* s, uint32_t n) {
+    const uint32_t k = sg_parts(n);
+    if (k <= s->part_cap) return WGDNA_OK;
+    STRY(salloc(&s->part, (size_t)k * SG_NPARAM));
+    s->part_cap = k;
     return WGDNA_OK;
 }
 
@@ -142,18 +142,17 @@ int check_err(SgState* s, cudaStream_t st, const char* who) {
     return WGDNA_OK;
 }
 
-// forward + backward over rows [rows] of the loaded data (n of them), gradients accumulated in s->g
+SgArgs sg_args(SgState* s, const float* X, uint32_t n) {
+    SgArgs f{};
+    f.X = X; f.n = n; f.w = weights(s); f.err = s->err; f.mma_ns = s->mma_ns; f.give_up_first = s->give_up_first;
+    return f;
+}
+
+// loss and partial gradients over rows [d_rows] of the loaded data (n of them) in s->part
 int fwd_bwd(SgState* s, cudaStream_t st, const uint32_t* d_rows, uint32_t n) {
-    SgFwdArgs f{};
-    f.X = s->X; f.rows = d_rows; f.n = n; f.w = weights(s); f.Y = s->Y;
-    f.H0 = s->H0; f.H1 = s->H1; f.H2 = s->H2; f.H3 = s->H3; f.Z1 = s->Z1; f.Z2 = s->Z2; f.Z3 = s->Z3;
-    f.err = s->err; f.mma_ns = s->mma_ns; f.give_up_first = s->give_up_first;
-    WG_CUDA_OK(launch_sg_forward(f, st));
-    SgBwdArgs b{};
-    b.T = s->T; b.rows = d_rows; b.n = n; b.w = f.w; b.Y = s->Y;
-    b.H0 = s->H0; b.H1 = s->H1; b.H2 = s->H2; b.H3 = s->H3; b.Z1 = s->Z1; b.Z2 = s->Z2; b.Z3 = s->Z3;
-    b.grad = s->g; b.loss = s->loss; b.err = s->err; b.mma_ns = s->mma_ns; b.give_up_first = s->give_up_first;
-    WG_CUDA_OK(launch_sg_backward(b, st));
+    SgArgs f = sg_args(s, s->X, n);
+    f.rows = d_rows; f.T = s->T; f.part = s->part; f.loss = s->loss;
+    WG_CUDA_OK(launch_sg_train(f, st));
     return WGDNA_OK;
 }
 
@@ -253,15 +252,14 @@ extern "C" int wgdna_surrogate_grad(wgdna_ctx* c, uint64_t n, float* grad, doubl
     SgState* s;
     STRY(ensure_state(c, v, &s));
     if (n == 0 || n > s->ndata || n > 0xffffffffull) { wg_set_error("wgdna_surrogate_grad: bad row count"); return WGDNA_ERR_ARG; }
-    STRY(ensure_batch(s, n));
-    WG_CUDA_OK(cudaMemsetAsync(s->g, 0, SG_NPARAM * 4, v.stream));
+    STRY(ensure_parts(s, (uint32_t)n));
     WG_CUDA_OK(cudaMemsetAsync(s->loss, 0, 8, v.stream));
     STRY(fwd_bwd(s, v.stream, nullptr, (uint32_t)n));
+    WG_CUDA_OK(launch_sg_grad(s->part, sg_parts((uint32_t)n), s->g, v.stream));
     STRY(check_err(s, v.stream, "wgdna_surrogate_grad"));
     if (grad) WG_CUDA_OK(cudaMemcpyAsync(grad, s->g, SG_NPARAM * 4, cudaMemcpyDeviceToHost, v.stream));
     double l = 0;
     WG_CUDA_OK(cudaMemcpyAsync(&l, s->loss, 8, cudaMemcpyDeviceToHost, v.stream));
-    WG_CUDA_OK(cudaMemsetAsync(s->g, 0, SG_NPARAM * 4, v.stream));
     WG_CUDA_OK(cudaStreamSynchronize(v.stream));
     if (loss) *loss = l / ((double)n * SG_OUT);
     return WGDNA_OK;
@@ -276,9 +274,12 @@ extern "C" int wgdna_surrogate_train(wgdna_ctx* c, uint32_t epochs, uint32_t bat
     if (s->ndata == 0) { wg_set_error("wgdna_surrogate_train: no data loaded"); return WGDNA_ERR_STATE; }
     const uint64_t n = s->ndata;
     const uint32_t B = (uint32_t)(batch < n ? batch : n);
-    STRY(ensure_batch(s, B));
-    uint32_t* d_perm = nullptr;
-    STRY(salloc(&d_perm, n));
+    STRY(ensure_parts(s, B));
+    if (n > s->perm_cap) {
+        STRY(salloc(&s->perm, n));
+        s->perm_cap = n;
+    }
+    const uint32_t nparts = sg_parts(B);
     std::vector<uint32_t> perm(n);
     uint64_t st = seed ^ 0xA5A5A5A5ull;
     for (uint32_t e = 0; e < epochs; ++e) {
@@ -287,21 +288,20 @@ extern "C" int wgdna_surrogate_train(wgdna_ctx* c, uint32_t epochs, uint32_t bat
             uint64_t j = smix(st) % (i + 1);
             uint32_t t = perm[i]; perm[i] = perm[j]; perm[j] = t;
         }
-        WG_CUDA_OK(cudaMemcpyAsync(d_perm, perm.data(), n * 4, cudaMemcpyHostToDevice, v.stream));
+        WG_CUDA_OK(cudaMemcpyAsync(s->perm, perm.data(), n * 4, cudaMemcpyHostToDevice, v.stream));
         WG_CUDA_OK(cudaMemsetAsync(s->loss, 0, 8, v.stream));
         const uint64_t nb = n / B;                                   // full batches
         for (uint64_t b = 0; b < nb; ++b) {
-            STRY(fwd_bwd(s, v.stream, d_perm + b * B, B));
+            STRY(fwd_bwd(s, v.stream, s->perm + b * B, B));
             s->step++;
             const float b1t = (float)std::pow(0.9, (double)s->step), b2t = (float)std::pow(0.999, (double)s->step);
-            WG_CUDA_OK(launch_sg_adam(s->p, s->m, s->v, s->g, lr, b1t, b2t, s->W, s->WT, v.stream));
+            WG_CUDA_OK(launch_sg_adam(s->p, s->m, s->v, s->part, nparts, lr, b1t, b2t, s->W, s->WT, v.stream));
         }
         double l = 0;
         WG_CUDA_OK(cudaMemcpyAsync(&l, s->loss, 8, cudaMemcpyDeviceToHost, v.stream));
         STRY(check_err(s, v.stream, "wgdna_surrogate_train"));
         if (losses) losses[e] = (float)(l / ((double)nb * B * SG_OUT));
     }
-    cudaFree(d_perm);
     return WGDNA_OK;
 }
 
@@ -315,7 +315,7 @@ extern "C" int wgdna_surrogate_predict(wgdna_ctx* c, const float* X, uint64_t n,
     const float* src = s->desc;
     if (X) {
         if (n > s->desc_cap) {
-            STRY(salloc(&s->desc, n * SG_IN)); STRY(salloc(&s->xs, n * SG_IN)); STRY(salloc(&s->pred, n * SG_OUT));
+            STRY(salloc(&s->desc, n * SG_IN)); STRY(salloc(&s->pred, n * SG_OUT));
             s->desc_cap = n;
         }
         WG_CUDA_OK(cudaMemcpyAsync(s->desc, X, n * SG_IN * 4, cudaMemcpyHostToDevice, v.stream));
@@ -326,18 +326,13 @@ extern "C" int wgdna_surrogate_predict(wgdna_ctx* c, const float* X, uint64_t n,
     }
     if (n == 0) return WGDNA_OK;
     if (n > 0xffffffffull) { wg_set_error("wgdna_surrogate_predict: too many rows"); return WGDNA_ERR_ARG; }
-    WG_CUDA_OK(launch_sg_standardise(src, s->xs, n, SG_IN, s->xmean, s->xinv, v.stream));
-    SgFwdArgs f{};
-    f.X = s->xs; f.n = (uint32_t)n; f.w = weights(s); f.Y = s->pred; f.err = s->err;
-    f.mma_ns = s->mma_ns; f.give_up_first = s->give_up_first;
+    SgArgs f = sg_args(s, src, (uint32_t)n);
+    f.xmean = s->xmean; f.xinv = s->xinv; f.ymean = s->ymean; f.ystd = s->ystd; f.Y = s->pred;
     WG_CUDA_OK(launch_sg_forward(f, v.stream));
     STRY(check_err(s, v.stream, "wgdna_surrogate_predict"));
     if (G) {
-        std::vector<float> y(n * SG_OUT);
-        WG_CUDA_OK(cudaMemcpyAsync(y.data(), s->pred, n * SG_OUT * 4, cudaMemcpyDeviceToHost, v.stream));
+        WG_CUDA_OK(cudaMemcpyAsync(G, s->pred, n * SG_OUT * 4, cudaMemcpyDeviceToHost, v.stream));
         WG_CUDA_OK(cudaStreamSynchronize(v.stream));
-        for (uint64_t i = 0; i < n; ++i)
-            for (int k = 0; k < SG_OUT; ++k) G[i * SG_OUT + k] = y[i * SG_OUT + k] * s->h_ystd[k] + s->h_ymean[k];
     }
     return WGDNA_OK;
 }
@@ -350,10 +345,10 @@ extern "C" int wgdna_track_descriptors(wgdna_ctx* c, float* out, uint64_t cap, u
     if (!v.have_transport) { wg_set_error("wgdna_track_descriptors: no transport result in the context"); return WGDNA_ERR_STATE; }
     const uint64_t n = v.nseg;
     if (n > s->desc_cap) {
-        STRY(salloc(&s->desc, n * SG_IN)); STRY(salloc(&s->xs, n * SG_IN)); STRY(salloc(&s->pred, n * SG_OUT));
+        STRY(salloc(&s->desc, n * SG_IN)); STRY(salloc(&s->pred, n * SG_OUT));
         s->desc_cap = n;
     }
-    DescArgs a{v.rad, v.seg_off, v.nseg, v.Eprim, v.E0, s->desc};
+    DescArgs a{v.rad, v.seg_off, v.nseg, v.Eprim, v.E0, s->desc, s->dbin};
     WG_CUDA_OK(launch_descriptors(a, v.stream));
     s->desc_n = n;
     if (n_tracks) *n_tracks = n;
@@ -378,7 +373,7 @@ extern "C" int wgdna_surrogate_chemistry(wgdna_ctx* c, double* G, float* ms) {
     if (!v.have_transport) { wg_set_error("wgdna_surrogate_chemistry: no transport result in the context"); return WGDNA_ERR_STATE; }
     const uint64_t n = v.nseg;
     if (n > s->desc_cap) {
-        STRY(salloc(&s->desc, n * SG_IN)); STRY(salloc(&s->xs, n * SG_IN)); STRY(salloc(&s->pred, n * SG_OUT));
+        STRY(salloc(&s->desc, n * SG_IN)); STRY(salloc(&s->pred, n * SG_OUT));
         s->desc_cap = n;
     }
     if (!s->ev[0]) {
@@ -387,12 +382,10 @@ extern "C" int wgdna_surrogate_chemistry(wgdna_ctx* c, double* G, float* ms) {
     }
     WG_CUDA_OK(cudaEventRecord(s->ev[0], v.stream));
     WG_CUDA_OK(cudaMemsetAsync(s->acc, 0, (SG_OUT + 1) * sizeof(double), v.stream));
-    DescArgs da{v.rad, v.seg_off, v.nseg, v.Eprim, v.E0, s->desc};
+    DescArgs da{v.rad, v.seg_off, v.nseg, v.Eprim, v.E0, s->desc, s->dbin};
     WG_CUDA_OK(launch_descriptors(da, v.stream));
     s->desc_n = n;
-    SgFwdArgs f{};
-    f.X = s->desc; f.n = (uint32_t)n; f.w = weights(s); f.Y = nullptr; f.err = s->err;
-    f.mma_ns = s->mma_ns; f.give_up_first = s->give_up_first;
+    SgArgs f = sg_args(s, s->desc, (uint32_t)n);
     f.xmean = s->xmean; f.xinv = s->xinv; f.ymean = s->ymean; f.ystd = s->ystd;
     f.E = v.Eprim; f.E0 = v.E0; f.acc = s->acc;
     WG_CUDA_OK(launch_sg_forward(f, v.stream));
