@@ -1,0 +1,37 @@
+"""The grid chemistry's cell-ordered neighbour search: sizes at the edges of a warp
+and a block, and steps with an overfull cell (more than 128 radicals in 0.75 nm),
+which walk the reference's lists; against the oracle, whose claims run in radical
+order."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle
+from wgdna import _lib
+
+
+def clusters(n, k, sigma, seed):
+    g = np.random.default_rng(seed)
+    centre = np.arange(k)[:, None] * np.array([[400.0, -250.0, 130.0]])
+    pos = centre[g.integers(0, k, n)] + g.normal(0, sigma, (n, 3))
+    code = g.choice([0, 1, 2, 3, 5, 6, 7], n, p=[0.3, 0.2, 0.1, 0.2, 0.1, 0.05, 0.05])
+    return np.ascontiguousarray(np.concatenate([pos, code[:, None]], axis=1), np.float32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,k,sigma", [
+    (1, 1, 1.0), (31, 3, 0.5), (33, 2, 0.5), (257, 20, 0.8),
+    (30_000, 600, 1.5),        # about 50 radicals per cluster: no overfull cell
+    (30_000, 15, 0.4),         # 2000 per cluster within a nanometre: overfull until they spread
+])
+def test_yields_against_oracle(ctx, n, k, sigma):
+    """t = 0 exactly; later within 2 % (the order of the claims, as in
+    test_grid_chemistry_gpu_against_oracle) and 4 standard deviations of a count."""
+    rad = clusters(n, k, sigma, n + k)
+    ref, _, _ = oracle.chem_grid(rad, seed=9)
+    r = _lib.ChemGridResult()
+    _lib.check("grid", _lib.lib().wgdna_chem_grid(ctx.h, _lib.ptr(rad), n, 16, 1000.0, 9, C.byref(r), None, None, 0))
+    got, ref = np.array(r.counts).astype(float), ref.astype(float)
+    np.testing.assert_array_equal(got[0], ref[0])
+    assert np.all(np.abs(got - ref) <= 0.02 * ref + 4 * np.sqrt(ref + 1)), (got, ref)

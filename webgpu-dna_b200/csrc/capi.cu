@@ -76,7 +76,9 @@ struct wgdna_ctx {
     float4 *d_cg_pos = nullptr, *d_cg_rad = nullptr;
     uint32_t *d_cg_alive = nullptr, *d_cg_prod = nullptr, *d_cg_counts = nullptr;
     int *d_cg_head = nullptr, *d_cg_next = nullptr;
-    wg::CgStep* d_cg_step = nullptr;
+    uint32_t *d_cg_tab = nullptr, *d_cg_cell = nullptr, *d_cg_rank = nullptr;
+    float4* d_cg_sorted = nullptr;
+    wg::CgState* d_cg_state = nullptr;
     size_t cg_cap = 0, cg_rad_cap = 0;
     cudaGraphExec_t cg_graph = nullptr;
     wg::CgGraphKey cg_key{};
@@ -319,7 +321,8 @@ extern "C" void wgdna_destroy(wgdna_ctx* c) {
                     c->sc.fib, c->d_px, c->d_py, c->d_pz, c->d_tb, c->d_sp, c->d_alive8, c->d_lst, c->d_lpos, c->d_evt, c->d_evab,
                     c->d_hov_t, c->d_hov_ab, c->d_track, c->d_toff, c->d_irt_cnt, c->d_pf, c->d_rec, c->d_tdel, c->d_curves, c->d_acc_tl, c->d_acc, c->d_maxpid,
                     c->d_dose_in, c->d_lambda, c->d_hits_in, c->d_dres, c->d_cg_pos, c->d_cg_rad, c->d_cg_alive,
-                    c->d_cg_prod, c->d_cg_counts, c->d_cg_head, c->d_cg_next, c->d_cg_step};
+                    c->d_cg_prod, c->d_cg_counts, c->d_cg_head, c->d_cg_next, c->d_cg_tab,
+                    c->d_cg_cell, c->d_cg_rank, c->d_cg_sorted, c->d_cg_state};
     if (c->cg_graph) cudaGraphExecDestroy(c->cg_graph);
     if (c->irt_graph.exec) cudaGraphExecDestroy(c->irt_graph.exec);
     for (void* p : ptrs) if (p) cudaFree(p);
@@ -1028,15 +1031,19 @@ extern "C" int wgdna_chem_grid(wgdna_ctx* c, const float* rad, uint64_t rad_n, u
     memset(out, 0, sizeof *out);
     if (n == 0) return WGDNA_OK;
     if (n > c->cg_cap) {
+        c->cg_cap = 0;                   // until every buffer has its new size
         TRY(dalloc(&c->d_cg_pos, n)); TRY(dalloc(&c->d_cg_alive, n)); TRY(dalloc(&c->d_cg_next, n));
+        TRY(dalloc(&c->d_cg_cell, 2 * (size_t)n)); TRY(dalloc(&c->d_cg_rank, n)); TRY(dalloc(&c->d_cg_sorted, n));
         c->cg_cap = n;
     }
-    if (!c->d_cg_head) {
+    if (!c->d_cg_tab) {                  // the last of them
         TRY(dalloc(&c->d_cg_head, wg::CG_HASH_SIZE)); TRY(dalloc(&c->d_cg_prod, 2));
-        TRY(dalloc(&c->d_cg_counts, 40)); TRY(dalloc(&c->d_cg_step, 1));
+        TRY(dalloc(&c->d_cg_counts, 40)); TRY(dalloc(&c->d_cg_state, 1));
+        TRY(dalloc(&c->d_cg_tab, 2 * (size_t)wg::CG_HASH_SIZE));
     }
-    wg::CgArgs a{src, n, (uint32_t)seed, (uint32_t)(seed >> 32), c->d_cg_pos, c->d_cg_alive, c->d_cg_head,
-                 c->d_cg_next, c->d_cg_prod, c->d_cg_counts, c->d_cg_step};
+    wg::CgArgs a{src, n, (uint32_t)seed, (uint32_t)(seed >> 32), c->d_cg_pos, c->d_cg_alive, c->d_cg_tab,
+                 c->d_cg_cell, c->d_cg_rank, c->d_cg_sorted, c->d_cg_head, c->d_cg_next, c->d_cg_prod, c->d_cg_counts,
+                 c->d_cg_state};
     WG_CUDA_OK(cudaEventRecord(c->ev[4], s));
     WG_CUDA_OK(wg::cg_run(a, s, &c->cg_graph, &c->cg_key));
     WG_CUDA_OK(cudaEventRecord(c->ev[5], s));

@@ -5,8 +5,21 @@
 // with a contact probability, each thread claiming both radicals with
 // compare-and-swap (so, as in the reference, which of several competing
 // pairs reacts depends on thread timing).  The 7-stage schedule (133 steps of
-// diffuse / clear / build / react, plus the counts at each checkpoint) is
+// diffuse / place / sort / react, plus the counts at each checkpoint) is
 // captured once into a CUDA graph and replayed with one launch.
+//
+// What bounds a step: 27 table lookups per radical, and at the common start of all
+// tracks, where a reference cell holds hundreds of radicals, the pair tests.  The
+// neighbours are therefore found in cells of half the reference's edge (0.75 nm,
+// still above the largest reaction radius, so the same pairs are in contact and
+// there are 6 times fewer to test), the radicals of a cell are stored side by side
+// (a counting sort per step) instead of chained, and are read four at a time.
+// Measured at 4096 x 1 keV (0.63 M radicals): 1614 us per react kernel with lists of
+// 1.5 nm cells, 137 us now; 1640 and 165 us per whole step.
+//
+// The reference's walk stops after 1024 entries of a 1.5 nm cell.  While no such cell
+// (eight of 0.75 nm) holds more, no walk is stopped and the results are those of the
+// lists; a step with a fuller one walks the lists as the reference does.
 //
 // Random numbers: Philox4x32-10 with counter (radical, step, 0, 6) and the
 // call's key; the f32 Gaussians use this build's own log / sincos
@@ -97,91 +110,213 @@ __global__ void k_cg_init(const float4* rad, uint32_t n, uint32_t k0, uint32_t k
     pos[i] = p;
 }
 
-// diffuse (chemistry.wgsl:32-56)
-__global__ void k_cg_diffuse(float4* pos, const uint32_t* alive, uint32_t n, const CgStep* st, uint32_t k0, uint32_t k1) {
+constexpr float CG_FINE = 0.75f;                 // nm
+constexpr uint32_t CG_NONE = 0xffffffffu;
+constexpr uint32_t CG_WALK = 1024;               // the reference's bound on a walk through a cell
+__device__ __forceinline__ int cg_fine(float x) { return (int)floorf(x / CG_FINE); }
+
+// 1) diffuse (chemistry.wgsl:32-56) and take a place in the fine cell's bucket
+__global__ void k_cg_diffuse(float4* pos, const uint32_t* alive, uint32_t n, float dt, uint32_t step, uint32_t k0,
+                             uint32_t k1, uint32_t* tab, uint32_t* cell, uint32_t* rank, CgState* st) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || alive[i] == 0u) return;
+    if (i == 0) { st->placed = 0u; st->dense = 0u; }
+    if (i >= n) return;
+    if (alive[i] == 0u) { cell[i] = CG_NONE; return; }
     float4 p = pos[i];
     const int kind = (int)rintf(p.w);
-    float D;
+    float D = 0.0f;
     if (kind == 0) D = 2.2f;
     else if (kind == 1) D = 4.9f;
     else if (kind == 2) D = 7.0f;
     else if (kind == 3) D = 9.0f;
-    else return;
-    const float sigma = sqrtf(2.0f * D * st->dt);
-    const u4 w = philox(i, st->step, 0u, 6u, k0, k1);
-    const float2 g01 = cg_gauss2(u01f(w.x), u01f(w.y));
-    const float2 g23 = cg_gauss2(u01f(w.z), u01f(w.w));
-    p.x += sigma * g01.x;
-    p.y += sigma * g01.y;
-    p.z += sigma * g23.x;
-    pos[i] = p;
+    if (kind >= 0 && kind <= 3) {
+        const float sigma = sqrtf(2.0f * D * dt);
+        const u4 w = philox(i, step, 0u, 6u, k0, k1);
+        const float2 g01 = cg_gauss2(u01f(w.x), u01f(w.y));
+        const float2 g23 = cg_gauss2(u01f(w.z), u01f(w.w));
+        p.x += sigma * g01.x;
+        p.y += sigma * g01.y;
+        p.z += sigma * g23.x;
+        pos[i] = p;
+    }
+    const uint32_t h = cg_hash(cg_fine(p.x), cg_fine(p.y), cg_fine(p.z));
+    cell[i] = h;
+    rank[i] = atomicAdd(&tab[h], 1u);
 }
 
-__global__ void k_cg_clear(int* head) {
+// count of a bucket whose word may already hold its first entry as well
+__device__ __forceinline__ uint32_t cg_count(uint32_t v) { return (v >> 23) ? v >> 23 : v; }
+
+// 2) the first radical of each bucket reserves the bucket's entries: one atomic
+//    per block, so buckets keep the order of the tracks.  The table word becomes
+//    first entry | count << 23.  A fine cell with more than an eighth of CG_WALK has
+//    its coarse cell counted.
+constexpr int CG_RB = 512;
+__global__ void __launch_bounds__(CG_RB) k_cg_reserve(const float4* pos, uint32_t n, uint32_t* tab, const uint32_t* cell,
+                                                      const uint32_t* rank, CgState* st) {
+    __shared__ uint32_t wsum[CG_RB / 32], s_base;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const uint32_t h = i < n ? cell[i] : CG_NONE;
+    const bool lead = h != CG_NONE && rank[i] == 0u;
+    const uint32_t c = lead ? tab[h] : 0u;
+    uint32_t off = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t v = __shfl_up_sync(0xffffffffu, off, o); if (lane >= o) off += v; }
+    if (lane == 31) wsum[wl] = off;
+    __syncthreads();
+    if (wl == 0) {
+        const uint32_t own = lane < CG_RB / 32 ? wsum[lane] : 0u;
+        uint32_t v = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+        if (lane < CG_RB / 32) wsum[lane] = v - own;
+        if (lane == 31) s_base = v ? atomicAdd(&st->placed, v) : 0u;
+    }
+    __syncthreads();
+    if (!lead) return;
+    bool dense = c > 511u;                           // does not fit the word
+    if (c > CG_WALK / 8 && !dense) {
+        const float4 p = pos[i];
+        const int ix = cg_fine(p.x) & ~1, iy = cg_fine(p.y) & ~1, iz = cg_fine(p.z) & ~1;
+        uint32_t sum = 0;
+        for (int o = 0; o < 8; ++o)
+            sum += cg_count(*(volatile uint32_t*)&tab[cg_hash(ix + (o & 1), iy + ((o >> 1) & 1), iz + (o >> 2))]);
+        dense = sum > CG_WALK;
+    }
+    if (dense) st->dense = 1u;
+    tab[h] = (s_base + wsum[wl] + off - c) | (min(c, 511u) << 23);
+}
+
+// 3) radicals in bucket order; the other table is emptied for the next step
+__global__ void k_cg_sort(const float4* pos, uint32_t n, const uint32_t* tab, const uint32_t* cell, const uint32_t* rank,
+                          float4* sorted, uint32_t* tab_old, const uint32_t* cell_old) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (cell_old) { const uint32_t o = cell_old[i]; if (o != CG_NONE) tab_old[o] = 0u; }
+    const uint32_t h = cell[i];
+    if (h == CG_NONE) return;
+    const float4 p = pos[i];
+    const uint32_t kind = (uint32_t)(int)rintf(p.w) & 7u;
+    sorted[(tab[h] & 0x7fffffu) + rank[i]] = make_float4(p.x, p.y, p.z, __uint_as_float(i | (kind << 23)));
+}
+
+// a pair within R_max: the contact test (with i's kind when its walk began and j's kind
+// of now, as the reference reads them), the roll, the claim.  0: go on, 1: radical i is
+// done with this step
+__device__ __forceinline__ int cg_contact(float4* pos, uint32_t* alive, uint32_t i, int ki, uint32_t j, float d2, uint32_t step,
+                                          uint32_t k0, uint32_t k1, uint32_t& draw, u4& w, uint32_t* prod) {
+    if (alive[j] == 0u) return 0;
+    const int kj = (int)rintf(pos[j].w);
+    if (kj < 0 || kj > 3) return 0;
+    const float R = cg_sigma_react(ki, kj);
+    if (R <= 0.0f || d2 > R * R) return 0;
+    if ((draw & 3u) == 0u) w = philox(i, step, 1u + (draw >> 2), 6u, k0, k1);
+    const uint32_t word = (draw & 3u) == 0u ? w.x : (draw & 3u) == 1u ? w.y : (draw & 3u) == 2u ? w.z : w.w;
+    draw++;
+    if (u01f(word) >= cg_pcontact(ki, kj)) return 0;
+    if (atomicCAS(&alive[i], 1u, 0u) != 1u) return 1;
+    if (atomicCAS(&alive[j], 1u, 0u) != 1u) { atomicExch(&alive[i], 1u); return 0; }
+    const int pr = cg_product(ki, kj);
+    if (pr == 1) atomicAdd(&prod[0], 1u);
+    else if (pr == 2) atomicAdd(&prod[1], 1u);
+    else if (pr == 3) {
+        const uint32_t e = ki == 1 ? i : j;         // the e-aq becomes an H
+        pos[e].w = 2.0f;
+        atomicExch(&alive[e], 1u);
+    }
+    return 1;
+}
+
+// 4) react (chemistry.wgsl:194-266): contact within the reaction radius, a
+//    contact-probability roll from the radical's step stream, claim both
+//    radicals with compare-and-swap.  The pair belongs to its lower index.  Threads
+//    take the radicals in index order: which of several contacts is claimed
+//    depends on when threads run, and cell order shifts the yields of a crowded
+//    origin by 0.1 % for 5 % of the time.
+__global__ void k_cg_react(float4* pos, uint32_t* alive, uint32_t n, const uint32_t* tab, const float4* sorted,
+                           const CgState* st, uint32_t step, uint32_t k0, uint32_t k1, uint32_t* prod) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || st->dense || alive[i] == 0u) return;
+    const float4 me = pos[i];
+    const int ki = (int)rintf(me.w);
+    if (ki < 0 || ki > 3) return;
+    const int ix = cg_fine(me.x), iy = cg_fine(me.y), iz = cg_fine(me.z);
+    constexpr float R2_MAX = 0.61f * 0.61f * 1.0001f;            // cg_sigma_react's largest
+    uint32_t draw = 0;
+    u4 w = {0, 0, 0, 0};
+    for (int dz = -1; dz <= 1; ++dz)
+        for (int dy = -1; dy <= 1; ++dy) {
+            uint32_t word[3];                                    // three lookups in flight
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) word[dx] = tab[cg_hash(ix + dx - 1, iy + dy, iz + dz)];
+#pragma unroll 1
+            for (int dx = 0; dx < 3; ++dx) {
+                const uint32_t v = dx == 0 ? word[0] : dx == 1 ? word[1] : word[2];
+                const float4* S = sorted + (v & 0x7fffffu);
+                // four entries in flight; the last inserted first, as in the lists
+                for (int c = (int)(v >> 23) - 1; c >= 0; c -= 4) {
+                    float d2[4];
+                    uint32_t j[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float4 q = S[max(c - u, 0)];
+                        const float ddx = me.x - q.x, ddy = me.y - q.y, ddz = me.z - q.z;
+                        d2[u] = c >= u ? ddx * ddx + ddy * ddy + ddz * ddz : 1e30f;
+                        j[u] = __float_as_uint(q.w) & 0x7fffffu;
+                    }
+                    if (fminf(fminf(d2[0], d2[1]), fminf(d2[2], d2[3])) > R2_MAX) continue;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (d2[u] <= R2_MAX && j[u] > i && cg_contact(pos, alive, i, ki, j[u], d2[u], step, k0, k1, draw, w, prod))
+                            return;
+                }
+            }
+        }
+}
+
+// Steps with an overfull cell: the reference's lists (build_hash and react,
+// chemistry.wgsl:111-122, 194-266) over 1.5 nm cells, walked at most 1024 deep.
+__global__ void k_cg_clear(const CgState* st, int* head) {
+    if (!st->dense) return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < CG_HASH; i += gridDim.x * blockDim.x) head[i] = -1;
 }
 
 __device__ __forceinline__ int cg_cell(float x) { return (int)floorf(x / CG_CELL); }
 
-// build_hash (chemistry.wgsl:111-122)
-__global__ void k_cg_build(const float4* pos, const uint32_t* alive, uint32_t n, int* head, int* next) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (alive[i] == 0u) { next[i] = -1; return; }
-    const float4 p = pos[i];
-    const uint32_t h = cg_hash(cg_cell(p.x), cg_cell(p.y), cg_cell(p.z));
-    next[i] = atomicExch(&head[h], (int)i);
+__global__ void k_cg_list(const CgState* st, const float4* pos, const uint32_t* alive, uint32_t n, int* head, int* next) {
+    if (!st->dense) return;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        if (alive[i] == 0u) { next[i] = -1; continue; }
+        const float4 p = pos[i];
+        next[i] = atomicExch(&head[cg_hash(cg_cell(p.x), cg_cell(p.y), cg_cell(p.z))], (int)i);
+    }
 }
 
-// react (chemistry.wgsl:194-266): contact within the reaction radius, a
-// contact-probability roll from the radical's step stream, claim both
-// radicals with compare-and-swap
-__global__ void k_cg_react(float4* pos, uint32_t* alive, uint32_t n, const int* head, const int* next,
-                           const CgStep* st, uint32_t k0, uint32_t k1, uint32_t* prod) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || alive[i] == 0u) return;
-    const float4 pi = pos[i];
-    const int ki = (int)rintf(pi.w);
-    if (ki < 0 || ki > 3) return;
-    const int ix = cg_cell(pi.x), iy = cg_cell(pi.y), iz = cg_cell(pi.z);
-    uint32_t draw = 0;
-    u4 w = {0, 0, 0, 0};
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) {
-                int j = head[cg_hash(ix + dx, iy + dy, iz + dz)];
-                for (uint32_t it = 0; it < 1024u && j >= 0; ++it) {
-                    const uint32_t ju = (uint32_t)j;
-                    const int jn = next[ju];
-                    if (ju <= i || alive[ju] == 0u) { j = jn; continue; }
-                    const float4 pj = pos[ju];
-                    const int kj = (int)rintf(pj.w);
-                    if (kj < 0 || kj > 3) { j = jn; continue; }
-                    const float R = cg_sigma_react(ki, kj);
-                    if (R <= 0.0f) { j = jn; continue; }
-                    const float ddx = pi.x - pj.x, ddy = pi.y - pj.y, ddz = pi.z - pj.z;
-                    if (ddx * ddx + ddy * ddy + ddz * ddz > R * R) { j = jn; continue; }
-                    if ((draw & 3u) == 0u) w = philox(i, st->step, 1u + (draw >> 2), 6u, k0, k1);
-                    const uint32_t word = (draw & 3u) == 0u ? w.x : (draw & 3u) == 1u ? w.y : (draw & 3u) == 2u ? w.z : w.w;
-                    draw++;
-                    if (u01f(word) >= cg_pcontact(ki, kj)) { j = jn; continue; }
-                    if (atomicCAS(&alive[i], 1u, 0u) != 1u) return;
-                    if (atomicCAS(&alive[ju], 1u, 0u) != 1u) { atomicExch(&alive[i], 1u); j = jn; continue; }
-                    const int pr = cg_product(ki, kj);
-                    if (pr == 1) atomicAdd(&prod[0], 1u);
-                    else if (pr == 2) atomicAdd(&prod[1], 1u);
-                    else if (pr == 3) {
-                        const uint32_t e = ki == 1 ? i : ju;        // the e-aq becomes an H
-                        float4 q = pos[e];
-                        q.w = 2.0f;
-                        pos[e] = q;
-                        atomicExch(&alive[e], 1u);
-                    }
-                    return;
-                }
+__global__ void k_cg_react_list(const CgState* st, float4* pos, uint32_t* alive, uint32_t n, const int* head,
+                                const int* next, uint32_t step, uint32_t k0, uint32_t k1, uint32_t* prod) {
+    if (!st->dense) return;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        if (alive[i] == 0u) continue;
+        const float4 pi = pos[i];
+        const int ki = (int)rintf(pi.w);
+        if (ki < 0 || ki > 3) continue;
+        const int ix = cg_cell(pi.x), iy = cg_cell(pi.y), iz = cg_cell(pi.z);
+        uint32_t draw = 0;
+        u4 w = {0, 0, 0, 0};
+        bool done = false;
+        for (int c = 0; c < 27 && !done; ++c) {
+            int j = head[cg_hash(ix + c % 3 - 1, iy + c / 3 % 3 - 1, iz + c / 9 - 1)];
+            for (uint32_t it = 0; it < 1024u && j >= 0 && !done; ++it) {
+                const uint32_t ju = (uint32_t)j;
+                j = next[ju];
+                if (ju <= i) continue;
+                const float4 pj = pos[ju];
+                const float ddx = pi.x - pj.x, ddy = pi.y - pj.y, ddz = pi.z - pj.z;
+                done = cg_contact(pos, alive, i, ki, ju, ddx * ddx + ddy * ddy + ddz * ddz, step, k0, k1, draw, w, prod) != 0;
             }
+        }
+    }
 }
 
 // count_alive (chemistry.wgsl:270-281) into checkpoint slot k: OH, e-aq, H
@@ -201,8 +336,6 @@ __global__ void k_cg_count(const float4* pos, const uint32_t* alive, uint32_t n,
     if (blockIdx.x == 0 && threadIdx.x == 0) { out[3] = prod[0]; out[4] = prod[1]; }
 }
 
-__global__ void k_cg_set_step(CgStep* st, float dt, uint32_t step) { st->dt = dt; st->step = step; }
-
 // The schedule of schedule.ts:38-46: [dt ns, steps]
 static const float CG_DT[7] = {0.0001f, 0.001f, 0.005f, 0.05f, 0.5f, 3.0f, 30.0f};
 static const int CG_NS[7] = {10, 9, 18, 18, 18, 30, 30};
@@ -215,8 +348,13 @@ cudaError_t cg_run(const CgArgs& a, cudaStream_t s, cudaGraphExec_t* cache, CgGr
     { cudaError_t me_ = cudaMemsetAsync(a.counts, 0, 8 * 5 * sizeof(uint32_t), s); if (me_ != cudaSuccess) return me_; }
     { cudaError_t me_ = cudaMemsetAsync(a.prod, 0, 2 * sizeof(uint32_t), s); if (me_ != cudaSuccess) return me_; }
     k_cg_count<<<296, 256, 0, s>>>(a.pos, a.alive, n, a.prod, a.counts);
+    if ((e = cudaMemsetAsync(a.tab, 0, 2 * (size_t)CG_HASH * sizeof(uint32_t), s)) != cudaSuccess) return e;
     // the schedule as one graph; rebuilt when the buffers or sizes change
-    const CgGraphKey want{a.pos, a.alive, a.head, a.next, a.prod, a.counts, a.st, n, a.k0, a.k1};
+    CgGraphKey want;
+    memset(&want, 0, sizeof want);
+    want.pos = a.pos; want.sorted = a.sorted; want.alive = a.alive; want.tab = a.tab; want.cell = a.cell;
+    want.rank = a.rank; want.prod = a.prod; want.counts = a.counts; want.head = a.head; want.next = a.next;
+    want.st = a.st; want.n = n; want.k0 = a.k0; want.k1 = a.k1;
     if (!*cache || memcmp(key, &want, sizeof want) != 0) {
         if (*cache) { cudaGraphExecDestroy(*cache); *cache = nullptr; }
         cudaStream_t cs;
@@ -226,11 +364,16 @@ cudaError_t cg_run(const CgArgs& a, cudaStream_t s, cudaGraphExec_t* cache, CgGr
         uint32_t step = 0;
         for (int stage = 0; stage < 7; ++stage) {
             for (int k = 0; k < CG_NS[stage]; ++k) {
-                k_cg_set_step<<<1, 1, 0, cs>>>(a.st, CG_DT[stage], ++step);
-                k_cg_diffuse<<<nb, 256, 0, cs>>>(a.pos, a.alive, n, a.st, a.k0, a.k1);
-                k_cg_clear<<<2048, 256, 0, cs>>>(a.head);
-                k_cg_build<<<nb, 256, 0, cs>>>(a.pos, a.alive, n, a.head, a.next);
-                k_cg_react<<<nb, 256, 0, cs>>>(a.pos, a.alive, n, a.head, a.next, a.st, a.k0, a.k1, a.prod);
+                ++step;
+                uint32_t *tab = a.tab + (size_t)(step & 1u) * CG_HASH, *tab_old = a.tab + (size_t)((step + 1) & 1u) * CG_HASH;
+                uint32_t *cell = a.cell + (size_t)(step & 1u) * n, *cell_old = a.cell + (size_t)((step + 1) & 1u) * n;
+                k_cg_diffuse<<<nb, 256, 0, cs>>>(a.pos, a.alive, n, CG_DT[stage], step, a.k0, a.k1, tab, cell, a.rank, a.st);
+                k_cg_reserve<<<(n + CG_RB - 1) / CG_RB, CG_RB, 0, cs>>>(a.pos, n, tab, cell, a.rank, a.st);
+                k_cg_sort<<<nb, 256, 0, cs>>>(a.pos, n, tab, cell, a.rank, a.sorted, tab_old, step > 1 ? cell_old : nullptr);
+                k_cg_react<<<nb, 256, 0, cs>>>(a.pos, a.alive, n, tab, a.sorted, a.st, step, a.k0, a.k1, a.prod);
+                k_cg_clear<<<592, 256, 0, cs>>>(a.st, a.head);
+                k_cg_list<<<592, 256, 0, cs>>>(a.st, a.pos, a.alive, n, a.head, a.next);
+                k_cg_react_list<<<592, 256, 0, cs>>>(a.st, a.pos, a.alive, n, a.head, a.next, step, a.k0, a.k1, a.prod);
             }
             k_cg_count<<<296, 256, 0, cs>>>(a.pos, a.alive, n, a.prod, a.counts + 5 * (stage + 1));
         }

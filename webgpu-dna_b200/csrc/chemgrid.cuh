@@ -6,23 +6,31 @@
 
 namespace wg {
 
-struct CgStep { float dt; uint32_t step; };
+struct CgState { uint32_t placed, dense; };    // entries in the cell-ordered copy; a cell too full for it
 
 struct CgArgs {
     const float4* rad;       // the first n rad_buf entries
     uint32_t n, k0, k1;
     float4* pos;             // n: x, y, z, kind
     uint32_t* alive;         // n
-    int* head;               // 2^23 bucket heads
-    int* next;               // n
+    uint32_t* tab;           // 2 x 2^23 buckets, for odd and even steps: entries, then first entry and count
+    uint32_t* cell;          // 2 x n: bucket of each radical in the step's grid
+    uint32_t* rank;          // n: its place in the bucket
+    float4* sorted;          // n: x, y, z, index and kind in bucket order
+    int* head;               // 2^23 list heads and
+    int* next;               // n links, for steps with an overfull cell
     uint32_t* prod;          // 2: H2O2, H2 made
     uint32_t* counts;        // 8 x 5: t = 0 and the 7 checkpoints
-    CgStep* st;
+    CgState* st;
 };
 
+// what the captured schedule depends on (compared as bytes: no padding)
 struct CgGraphKey {
-    float4* pos; uint32_t* alive; int* head; int* next; uint32_t* prod; uint32_t* counts; CgStep* st;
-    uint32_t n, k0, k1;
+    float4 *pos, *sorted;
+    uint32_t *alive, *tab, *cell, *rank, *prod, *counts;
+    int *head, *next;
+    CgState* st;
+    uint32_t n, k0, k1, pad;
 };
 
 constexpr uint32_t CG_HASH_SIZE = 8388608u;
