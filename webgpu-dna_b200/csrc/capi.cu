@@ -31,6 +31,8 @@ void wg_set_error(const char* fmt, ...) {
 extern "C" const char* wgdna_last_error(void) { return g_err; }
 extern "C" int wgdna_version(void) { return 10000; }
 
+constexpr size_t H_PIN = 4096;
+
 struct wgdna_ctx {
     int device = 0;
     cudaStream_t stream = nullptr, own = nullptr;
@@ -115,7 +117,11 @@ struct wgdna_ctx {
     unsigned long long* d_acc = nullptr;
     uint32_t* d_maxpid = nullptr;
     IrtGraph irt_graph;                   // the IRT launch sequence, captured once per argument set
-    cudaEvent_t ev[11]{};
+    cudaEvent_t ev[13]{};
+    // small results land here (page-locked, so that a readback is a stream operation)
+    unsigned char* h_pin = nullptr;       // H_PIN bytes
+    uint32_t* h_fib = nullptr;            // 3 per fibre
+    size_t h_fib_cap = 0;
 };
 
 static std::string lib_dir() {
@@ -270,6 +276,12 @@ extern "C" int wgdna_create(const wgdna_cfg* cfg, wgdna_ctx** out) {
     if (r == WGDNA_OK) r = dalloc(&c->d_err, 1);
     if (r == WGDNA_OK) r = ensure_segments(c, (uint32_t)np);
     if (r == WGDNA_OK && cudaMemset(c->d_secq, 0, sizeof(SecRec) * (size_t)c0.max_sec) != cudaSuccess) r = WGDNA_ERR_CUDA;
+    if (r == WGDNA_OK && cudaMallocHost((void**)&c->h_pin, H_PIN) != cudaSuccess) {
+        cudaGetLastError();
+        c->h_pin = nullptr;
+        wg_set_error("wgdna_create: cudaMallocHost(%zu bytes) failed", H_PIN);
+        r = WGDNA_ERR_NOMEM;
+    }
     if (r == WGDNA_OK) r = wgdna_set_dna_target(c, 3000.0, 21, 150.0);
     if (r != WGDNA_OK) { wgdna_destroy(c); return r; }
     wgdna_default_tuning(&c->tune);
@@ -317,7 +329,7 @@ extern "C" void wgdna_destroy(wgdna_ctx* c) {
     void* ptrs[] = {c->d_small, c->d_xcw, c->d_results, c->d_dose, c->d_rad_raw, c->d_key, c->d_rad,
                     c->d_perm, c->d_secq, c->d_st, c->d_Eprim, c->d_pid_cnt, c->d_pid_off, c->d_pid_cur,
                     c->d_red, c->d_err, c->d_fy, c->d_fz, c->d_rbb0, c->d_rbb1, c->d_hits, c->d_alive,
-                    c->sc.info, c->sc.last_brk, c->sc.cnt0, c->sc.cnt1, c->sc.cs_in, c->sc.base, c->sc.u64,
+                    c->sc.list, c->sc.seg, c->sc.u64,
                     c->sc.fib, c->d_px, c->d_py, c->d_pz, c->d_tb, c->d_sp, c->d_alive8, c->d_lst, c->d_lpos, c->d_evt, c->d_evab,
                     c->d_hov_t, c->d_hov_ab, c->d_track, c->d_toff, c->d_irt_cnt, c->d_pf, c->d_rec, c->d_tdel, c->d_curves, c->d_acc_tl, c->d_acc, c->d_maxpid,
                     c->d_dose_in, c->d_lambda, c->d_hits_in, c->d_dres, c->d_cg_pos, c->d_cg_rad, c->d_cg_alive,
@@ -326,6 +338,8 @@ extern "C" void wgdna_destroy(wgdna_ctx* c) {
     if (c->cg_graph) cudaGraphExecDestroy(c->cg_graph);
     if (c->irt_graph.exec) cudaGraphExecDestroy(c->irt_graph.exec);
     for (void* p : ptrs) if (p) cudaFree(p);
+    if (c->h_pin) cudaFreeHost(c->h_pin);
+    if (c->h_fib) cudaFreeHost(c->h_fib);
     for (auto& ev : c->ev) if (ev) cudaEventDestroy(ev);
     if (c->own) cudaStreamDestroy(c->own);
     delete c;
@@ -781,6 +795,13 @@ extern "C" int wgdna_set_dna_target(wgdna_ctx* c, double L_nm, uint32_t grid_N, 
     size_t hb = ((size_t)info.n_bp * 2 + 3) & ~(size_t)3;
     TRY(dalloc(&c->d_hits, hb));
     TRY(dalloc(&c->sc.fib, 3 * (size_t)info.n_fibers));
+    if (info.n_fibers > c->h_fib_cap) {
+        if (c->h_fib) cudaFreeHost(c->h_fib);
+        c->h_fib = nullptr;
+        c->h_fib_cap = 0;
+        WG_CUDA_OK(cudaMallocHost((void**)&c->h_fib, 12 * (size_t)info.n_fibers));
+        c->h_fib_cap = info.n_fibers;
+    }
     WG_CUDA_OK(cudaMemcpy(c->d_fy, fy.data(), fy.size() * 4, cudaMemcpyHostToDevice));
     WG_CUDA_OK(cudaMemcpy(c->d_fz, fz.data(), fz.size() * 4, cudaMemcpyHostToDevice));
     WG_CUDA_OK(cudaMemcpy(c->d_rbb0, r0.data(), r0.size() * 4, cudaMemcpyHostToDevice));
@@ -800,35 +821,42 @@ static DnaDev dna_dev(wgdna_ctx* c) {
 static int score_ensure(wgdna_ctx* c, unsigned long long n) {
     if (n <= c->sc_cap && c->sc.u64) return WGDNA_OK;
     unsigned long long cap = n < (1ull << 20) ? (1ull << 20) : n;
-    unsigned long long nt = (cap + 1023) / 1024;
-    TRY(dalloc(&c->sc.info, cap));
-    TRY(dalloc(&c->sc.last_brk, nt)); TRY(dalloc(&c->sc.cnt0, nt)); TRY(dalloc(&c->sc.cnt1, nt));
-    TRY(dalloc(&c->sc.cs_in, nt)); TRY(dalloc(&c->sc.base, nt));
+    c->sc_cap = 0;                       // until every buffer has its new size
+    TRY(dalloc(&c->sc.list, cap));
+    TRY(dalloc(&c->sc.seg, (cap + wg::SCORE_SEG - 1) / wg::SCORE_SEG));
     if (!c->sc.u64) TRY(dalloc(&c->sc.u64, 8));
     c->sc_cap = cap;
     return WGDNA_OK;
 }
 
-// score n entries of d_in (device) into c->d_hits
-static int score_dev(wgdna_ctx* c, const float4* d_in, const uint32_t* d_alive, unsigned long long n, double p,
-                     int dedupe, uint32_t lcg, wgdna_ssb_result* out) {
+// score n entries of d_in (device) into c->d_hits: launches, then the readback
+static int score_launch(wgdna_ctx* c, const float4* d_in, const uint32_t* d_alive, unsigned long long n, double p,
+                        int dedupe, uint32_t lcg) {
     TRY(score_ensure(c, n));
     cudaStream_t s = c->stream;
     DnaDev d = dna_dev(c);
     WG_CUDA_OK(cudaEventRecord(c->ev[6], s));
     WG_CUDA_OK(launch_score(d_in, d_alive, n, d, 0.29, p, dedupe, lcg, (uint32_t*)c->d_hits, c->sc, s));
     WG_CUDA_OK(cudaEventRecord(c->ev[7], s));
-    unsigned long long u[8];
-    WG_CUDA_OK(cudaMemcpyAsync(u, c->sc.u64, sizeof u, cudaMemcpyDeviceToHost, s));
-    WG_CUDA_OK(cudaStreamSynchronize(s));
-    if (out) {
-        memset(out, 0, sizeof *out);
-        out->ssb = u[0]; out->ssb0 = u[1]; out->ssb1 = u[2]; out->candidates = u[3];
-        unsigned long long draws = n ? u[4] : 0;
-        out->in_reach = draws;
-        out->lcg_state = lcg_jump_host(lcg, draws);
-        out->ms = elapsed_ms(c->ev[6], c->ev[7]);
-    }
+    WG_CUDA_OK(cudaMemcpyAsync(c->h_pin, c->sc.u64, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    return WGDNA_OK;
+}
+// after the stream has reached the end of score_launch
+static void score_result(wgdna_ctx* c, unsigned long long n, uint32_t lcg, wgdna_ssb_result* out) {
+    if (!out) return;
+    const unsigned long long* u = (const unsigned long long*)c->h_pin;
+    memset(out, 0, sizeof *out);
+    out->ssb = u[0]; out->ssb0 = u[1]; out->ssb1 = u[2]; out->candidates = u[3];
+    unsigned long long draws = n ? u[4] : 0;
+    out->in_reach = draws;
+    out->lcg_state = lcg_jump_host(lcg, draws);
+    out->ms = elapsed_ms(c->ev[6], c->ev[7]);
+}
+static int score_dev(wgdna_ctx* c, const float4* d_in, const uint32_t* d_alive, unsigned long long n, double p,
+                     int dedupe, uint32_t lcg, wgdna_ssb_result* out) {
+    TRY(score_launch(c, d_in, d_alive, n, p, dedupe, lcg));
+    WG_CUDA_OK(cudaStreamSynchronize(c->stream));
+    score_result(c, n, lcg, out);
     return WGDNA_OK;
 }
 
@@ -869,25 +897,31 @@ extern "C" int wgdna_score_indirect(wgdna_ctx* c, const float* pos, const uint32
     return WGDNA_OK;
 }
 
-static int cluster_dev(wgdna_ctx* c, wgdna_dsb_result* out) {
+static int cluster_launch(wgdna_ctx* c) {
     cudaStream_t s = c->stream;
     DnaDev d = dna_dev(c);
-    WG_CUDA_OK(cudaEventRecord(c->ev[6], s));
+    WG_CUDA_OK(cudaEventRecord(c->ev[11], s));
     WG_CUDA_OK(launch_cluster(c->d_hits, d, c->dna.n_fibers, c->sc.fib, s));
-    WG_CUDA_OK(cudaEventRecord(c->ev[7], s));
-    std::vector<uint32_t> fib(3 * (size_t)c->dna.n_fibers);
-    WG_CUDA_OK(cudaMemcpyAsync(fib.data(), c->sc.fib, fib.size() * 4, cudaMemcpyDeviceToHost, s));
-    WG_CUDA_OK(cudaStreamSynchronize(s));
-    if (out) {
-        memset(out, 0, sizeof *out);
-        double p_pair = fmin(1, (2.0 * 10 + 1) / c->dna.n_bp_per);
-        for (uint32_t f = 0; f < c->dna.n_fibers; ++f) {
-            uint32_t k0 = fib[3 * f + 1], k1 = fib[3 * f + 2];
-            out->dsb += fib[3 * f]; out->ssb0 += k0; out->ssb1 += k1;
-            if (k0 > 0 && k1 > 0) out->dsb_expected += 1 - pow(1 - p_pair, (double)k0 * (double)k1);
-        }
-        out->ms = elapsed_ms(c->ev[6], c->ev[7]);
+    WG_CUDA_OK(cudaEventRecord(c->ev[12], s));
+    WG_CUDA_OK(cudaMemcpyAsync(c->h_fib, c->sc.fib, 12 * (size_t)c->dna.n_fibers, cudaMemcpyDeviceToHost, s));
+    return WGDNA_OK;
+}
+// after the stream has reached the end of cluster_launch
+static void cluster_result(wgdna_ctx* c, wgdna_dsb_result* out) {
+    if (!out) return;
+    memset(out, 0, sizeof *out);
+    double p_pair = fmin(1, (2.0 * 10 + 1) / c->dna.n_bp_per);
+    for (uint32_t f = 0; f < c->dna.n_fibers; ++f) {
+        uint32_t k0 = c->h_fib[3 * f + 1], k1 = c->h_fib[3 * f + 2];
+        out->dsb += c->h_fib[3 * f]; out->ssb0 += k0; out->ssb1 += k1;
+        if (k0 > 0 && k1 > 0) out->dsb_expected += 1 - pow(1 - p_pair, (double)k0 * (double)k1);
     }
+    out->ms = elapsed_ms(c->ev[11], c->ev[12]);
+}
+static int cluster_dev(wgdna_ctx* c, wgdna_dsb_result* out) {
+    TRY(cluster_launch(c));
+    WG_CUDA_OK(cudaStreamSynchronize(c->stream));
+    cluster_result(c, out);
     return WGDNA_OK;
 }
 
@@ -903,8 +937,12 @@ extern "C" int wgdna_score(wgdna_ctx* c, uint32_t lcg_state, wgdna_ssb_result* s
     if (!c->have_transport) { wg_set_error("wgdna_score: no transport result in the context"); return WGDNA_ERR_STATE; }
     WG_CUDA_OK(cudaSetDevice(c->device));
     TRY(hits_in(c, nullptr));
-    TRY(score_dev(c, c->d_rad, nullptr, c->last_rad_n, 0.15, 1, lcg_state, ssb));
-    return cluster_dev(c, dsb);
+    TRY(score_launch(c, c->d_rad, nullptr, c->last_rad_n, 0.15, 1, lcg_state));
+    TRY(cluster_launch(c));
+    WG_CUDA_OK(cudaStreamSynchronize(c->stream));
+    score_result(c, c->last_rad_n, lcg_state, ssb);
+    cluster_result(c, dsb);
+    return WGDNA_OK;
 }
 
 extern "C" int wgdna_reaction_table(double out[9][6]) {

@@ -17,14 +17,9 @@ namespace wg {
 
 // At most 4,194,304 rad_buf entries per call; 16.1 MB of scratch per device.
 constexpr unsigned long long NOALLOC_MAX_ENTRIES = 1ull << 22;
-constexpr unsigned long long NOALLOC_TILES = NOALLOC_MAX_ENTRIES / 1024;
-constexpr size_t NA_INFO = 0;                                             // u32 per entry
-constexpr size_t NA_LAST = NA_INFO + 4 * NOALLOC_MAX_ENTRIES;              // i64 per tile
-constexpr size_t NA_CNT0 = NA_LAST + 8 * NOALLOC_TILES;                    // u32 per tile
-constexpr size_t NA_CNT1 = NA_CNT0 + 4 * NOALLOC_TILES;                    // u32 per tile
-constexpr size_t NA_CSIN = NA_CNT1 + 4 * NOALLOC_TILES;                    // i64 per tile
-constexpr size_t NA_BASE = NA_CSIN + 8 * NOALLOC_TILES;                    // u64 per tile
-constexpr size_t NA_U64 = NA_BASE + 8 * NOALLOC_TILES;                     // 8 x u64 results
+constexpr size_t NA_LIST = 0;                                             // u32 per entry
+constexpr size_t NA_SEG = NA_LIST + 4 * NOALLOC_MAX_ENTRIES;               // u64 per segment
+constexpr size_t NA_U64 = NA_SEG + 8 * (NOALLOC_MAX_ENTRIES / SCORE_SEG);  // 8 x u64 results
 constexpr size_t NOALLOC_BYTES = NA_U64 + 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
@@ -79,12 +74,8 @@ extern "C" int wgdna_score_direct_noalloc(const float* d_rad, uint64_t rad_n, co
     }
     cudaStream_t s = (cudaStream_t)cuda_stream;
     ScoreScratch sc;
-    sc.info = (uint32_t*)(base + NA_INFO);
-    sc.last_brk = (long long*)(base + NA_LAST);
-    sc.cnt0 = (uint32_t*)(base + NA_CNT0);
-    sc.cnt1 = (uint32_t*)(base + NA_CNT1);
-    sc.cs_in = (long long*)(base + NA_CSIN);
-    sc.base = (unsigned long long*)(base + NA_BASE);
+    sc.list = (uint32_t*)(base + NA_LIST);
+    sc.seg = (unsigned long long*)(base + NA_SEG);
     sc.u64 = (unsigned long long*)(base + NA_U64);
     sc.fib = nullptr;
     DnaDev d;
@@ -92,7 +83,7 @@ extern "C" int wgdna_score_direct_noalloc(const float* d_rad, uint64_t rad_n, co
     d.x0 = dna->x0; d.rise = dna->rise; d.r_bb = dna->r_bb; d.spacing = dna->spacing_nm;
     d.grid_N = dna->grid_N; d.n_bp_per = dna->n_bp_per; d.n_bp = dna->n_bp;
     // launch_score clears the result counters (the only scratch that must start
-    // at zero); the per-entry and per-tile scratch is fully rewritten
+    // at zero); what it reads of the lists and summaries it has written before
     WG_CUDA_OK(launch_score((const float4*)d_rad, nullptr, rad_n, d, 0.29, 0.15, 1, lcg_state, (uint32_t*)d_hits,
                             sc, s));
     unsigned long long u[8];

@@ -5,16 +5,24 @@
 // :348-407, makeSsbRng :421-427) evaluated with JavaScript number semantics.
 // The reference is a sequential loop; here every entry is scored in parallel:
 //
-//  1. k_prep: per entry, the adjacent-duplicate link (same xyz as the next
-//     entry), the in-reach test and the hit-byte index.  The reference's
-//     skip-by-2 walk visits entry i iff (i - start of its run of linked
-//     entries) is even.
-//  2. k_tiles / k_tilescan: per tile of 1024 entries, the last run start and
-//     the number of LCG draws for either parity of an incoming run; one block
-//     scans the tiles (run starts by max-scan, draw counts by sum-scan).
-//  3. k_apply: per entry, its draw index k; the LCG state after k+1 steps is
-//     an affine map (1664525 s + 1013904223 mod 2^32) raised to k+1 by
-//     squaring; a draw below p sets the hit byte (atomicOr, counted once).
+//  1. k_find: a warp per segment of 512 entries, in order.  The reference's
+//     skip-by-2 walk visits entry i iff its distance from the start of its run of
+//     equal positions is even, that is iff i has the parity of that start.  The
+//     entries within reach of a backbone (a few in ten thousand) are listed in
+//     order; those before the segment's first run start wait for the parity
+//     that comes in.
+//  2. k_draw: every block sums the draws of the segments before its own, each
+//     thread then walks one segment's list: the LCG state after k steps is an affine
+//     map (1664525 s + 1013904223 mod 2^32) raised to k by squaring, and one step
+//     per draw from there on; a draw below p sets the hit byte (atomicOr, counted
+//     once).
+//
+// What bounds it: the 16 bytes per entry that k_find reads.  An f32 test of the
+// distance to the nearest fibre axis keeps all but the listed entries out of the
+// f64 geometry, and nothing is written per entry.
+// Measured on 5.3 M entries of 4096 x 10 keV: 203 us with an info word per entry and
+// block-wide scans over 1024-entry tiles (k_prep 33, k_tiles 74, k_tilescan 22,
+// k_apply 70, launches), 45 us now (k_find 29, k_draw 16).
 //
 // clusterDSB: one block per fibre collects the strand-0 / strand-1 hit lists
 // in order and pairs them greedily; the expected-DSB sum uses the host's pow.
@@ -23,7 +31,7 @@
 namespace wg {
 
 
-constexpr int STILE = 1024;
+constexpr int SEG = (int)SCORE_SEG;
 
 __device__ __forceinline__ double js_round(double x) {
     double f = floor(x);
@@ -69,68 +77,92 @@ __device__ __forceinline__ long long near_backbone(const DnaDev& d, double x, do
     return (long long)fiber * d.n_bp_per + best_bp + (long long)best_s * d.n_bp;
 }
 
-// info word: bit31 run start, bit30 in reach, bit29 candidate (near a fibre
-// axis), bits 0..28 hit index.  Candidates are counted by k_apply for the
-// entries the reference's walk visits (ssb-dsb.ts:183).
-__global__ void k_prep(const float4* rad, const uint32_t* alive, unsigned long long n, DnaDev d,
-                       double r_d, int dedupe, uint32_t* info) {
-    unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
-    if (i < n) {
-        float4 e = rad[i];
-        uint32_t brk = 1;
-        if (dedupe && i > 0) {
-            float4 p = rad[i - 1];
-            brk = !(p.x == e.x && p.y == e.y && p.z == e.z);
-        }
-        uint32_t w = brk << 31;
-        bool consider = true;
-        if (alive) consider = alive[i] != 0 && js_round((double)e.w) == 0.0;   // OH only
-        if (consider) {
-            int cand;
-            long long h = near_backbone(d, e.x, e.y, e.z, r_d, &cand);
-            if (cand) w |= 1u << 29;
-            if (h >= 0) w |= (1u << 30) | (uint32_t)h;
-        }
-        info[i] = w;
-    }
+// False only if the entry is certainly beyond reach of every fibre axis: the f32
+// offset from the nearest axis has an error below 0.03 nm for |y|, |z| up to
+// 100 um, `far` adds 0.05 nm to the reach.  A NaN goes on to the f64 geometry.
+__device__ __forceinline__ bool maybe_near(float y, float z, float grid_off, float inv_sp, float sp, float far) {
+    const float u = (y - grid_off) * inv_sp, v = (z - grid_off) * inv_sp;
+    const float dy = fabsf(u - rintf(u)) * sp, dz = fabsf(v - rintf(v)) * sp;
+    return (dy <= far && dz <= far) || !(dy + dz >= 0.0f) || fmaxf(fabsf(y), fabsf(z)) > 1e5f;
 }
 
-// per tile: last run start (or -1) and draw counts for incoming parity 0 / 1
-__global__ void __launch_bounds__(STILE) k_tiles(const uint32_t* info, unsigned long long n,
-                                                 long long* last_brk, uint32_t* cnt0, uint32_t* cnt1) {
-    __shared__ long long s_last;
-    __shared__ uint32_t s_c0, s_c1;
-    unsigned long long a = (unsigned long long)blockIdx.x * STILE;
-    unsigned long long i = a + threadIdx.x;
-    if (threadIdx.x == 0) { s_last = -1; s_c0 = 0; s_c1 = 0; }
-    __syncthreads();
-    uint32_t w = i < n ? info[i] : 0u;
-    bool brk = i < n && (w >> 31);
-    if (brk) atomicMax(&s_last, (long long)i);
-    __syncthreads();
-    // local run start: max brk position <= t within the tile (inclusive max-scan)
-    __shared__ int s_cs[STILE];
-    s_cs[threadIdx.x] = brk ? (int)threadIdx.x : -1;
-    __syncthreads();
-    for (int off = 1; off < STILE; off <<= 1) {
-        int v = s_cs[threadIdx.x];
-        int u = threadIdx.x >= (unsigned)off ? s_cs[threadIdx.x - off] : -1;
-        __syncthreads();
-        s_cs[threadIdx.x] = max(v, u);
-        __syncthreads();
-    }
-    bool inr = i < n && ((w >> 30) & 1u);
-    if (inr) {
-        int cs = s_cs[threadIdx.x];
-        if (cs >= 0) {
-            if (((threadIdx.x - cs) & 1) == 0) { atomicAdd(&s_c0, 1u); atomicAdd(&s_c1, 1u); }
-        } else {
-            // before the tile's first run start: parity relative to the incoming run
-            if ((threadIdx.x & 1) == 0) atomicAdd(&s_c0, 1u); else atomicAdd(&s_c1, 1u);
+// A segment's summary: listed draws (resolved, waiting with even and odd index) and
+// candidates (near a fibre axis, ssb-dsb.ts:183) the same way, ten bits each, then
+// whether a run starts in the segment and the parity of its last run start.
+// List words: bit31 waiting, bit30 parity of the index, bits 0..28 hit index.
+__device__ __forceinline__ uint32_t fld(unsigned long long v, int k) { return (uint32_t)(v >> (10 * k)) & 1023u; }
+
+constexpr int FB = 256;
+__global__ void __launch_bounds__(FB) k_find(const float4* rad, const uint32_t* alive, unsigned long long n, DnaDev d,
+                                             double r_d, int dedupe, uint32_t* list, unsigned long long* seg,
+                                             unsigned long long* cnt) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    if (blockIdx.x == 0 && threadIdx.x < 8) cnt[threadIdx.x] = 0ull;
+    const unsigned long long q = (unsigned long long)blockIdx.x * (FB / 32) + (threadIdx.x >> 5);
+    const unsigned long long a = q * SEG;
+    if (a >= n) return;
+    const float grid_off = (float)(-(((double)d.grid_N - 1) * d.spacing) * 0.5), sp = (float)d.spacing;
+    const float inv_sp = (float)(1 / d.spacing), far = (float)(d.r_bb + r_d) + 0.05f;
+    uint32_t f[6] = {0, 0, 0, 0, 0, 0}, len = 0;
+    bool open = true;                             // no run has started in the segment yet
+    uint32_t par = 0;                             // parity of the last run start
+    float4 last = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (dedupe && a > 0) last = rad[a - 1];
+    constexpr int U = 4;
+    for (int c = 0; c < SEG; c += 32 * U) {
+        if (a + c >= n) break;
+        float4 e[U];
+        uint32_t al[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const unsigned long long i = a + c + 32 * k + lane;
+            e[k] = i < n ? __ldcs(rad + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            al[k] = alive ? (i < n ? alive[i] : 0u) : 1u;
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const unsigned long long i = a + c + 32 * k + lane;
+            const bool in = i < n;
+            unsigned brk = 0xffffffffu;
+            if (dedupe) {
+                float4 p;
+                p.x = __shfl_up_sync(0xffffffffu, e[k].x, 1); p.y = __shfl_up_sync(0xffffffffu, e[k].y, 1);
+                p.z = __shfl_up_sync(0xffffffffu, e[k].z, 1);
+                if (lane == 0) p = last;
+                brk = __ballot_sync(0xffffffffu, in && (i == 0 || !(p.x == e[k].x && p.y == e[k].y && p.z == e[k].z)));
+                last.x = __shfl_sync(0xffffffffu, e[k].x, 31); last.y = __shfl_sync(0xffffffffu, e[k].y, 31);
+                last.z = __shfl_sync(0xffffffffu, e[k].z, 31);
+            }
+            const bool look = in && al[k] != 0u && (!alive || js_round((double)e[k].w) == 0.0) &&      // OH only
+                              maybe_near(e[k].y, e[k].z, grid_off, inv_sp, sp, far);
+            if (__any_sync(0xffffffffu, look)) {
+                int cand = 0;
+                long long h = -1;
+                if (look) h = near_backbone(d, e[k].x, e[k].y, e[k].z, r_d, &cand);
+                const unsigned b = brk & (lt | (1u << lane));      // run starts up to this entry
+                const uint32_t odd = (uint32_t)lane & 1u;          // a, c and 32 k are even
+                const bool wait = open && b == 0u;
+                const uint32_t start = b ? (uint32_t)(31 - __clz(b)) & 1u : par;
+                const bool seen = cand && (wait || start == odd);
+                const bool draw = seen && h >= 0;
+                const unsigned m = __ballot_sync(0xffffffffu, draw);
+                if (draw)
+                    list[a + len + __popc(m & lt)] = (wait ? 0x80000000u | (odd << 30) : 0u) | (uint32_t)h;
+                len += __popc(m);
+                const unsigned w = __ballot_sync(0xffffffffu, wait), s = __ballot_sync(0xffffffffu, seen);
+                f[0] += __popc(m & ~w); f[1] += __popc(m & w & 0x55555555u); f[2] += __popc(m & w & 0xaaaaaaaau);
+                f[3] += __popc(s & ~w); f[4] += __popc(s & w & 0x55555555u); f[5] += __popc(s & w & 0xaaaaaaaau);
+            }
+            if (brk) { open = false; par = (uint32_t)(31 - __clz(brk)) & 1u; }
         }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) { last_brk[blockIdx.x] = s_last; cnt0[blockIdx.x] = s_c0; cnt1[blockIdx.x] = s_c1; }
+    if (lane == 0) {
+        unsigned long long v = 0;
+#pragma unroll
+        for (int k = 5; k >= 0; --k) v = (v << 10) | f[k];
+        seg[q] = v | ((unsigned long long)!open << 60) | ((unsigned long long)par << 61);
+    }
 }
 
 struct Aff { uint32_t a, c; };
@@ -145,128 +177,131 @@ __device__ __forceinline__ uint32_t lcg_jump(uint32_t s, unsigned long long k) {
     return r.a * s + r.c;
 }
 
-// one block: per-tile incoming run start and draw base
-__global__ void k_tilescan(const long long* last_brk, const uint32_t* cnt0, const uint32_t* cnt1,
-                           uint32_t ntiles, long long* cs_in, unsigned long long* base,
-                           unsigned long long* total) {
-    __shared__ long long smax[1024];
-    __shared__ unsigned long long ssum[1024];
-    uint32_t t = threadIdx.x, per = (ntiles + blockDim.x - 1) / blockDim.x;
-    uint32_t lo = min(t * per, ntiles), hi = min(lo + per, ntiles);
-    long long m = -1;
-    for (uint32_t k = lo; k < hi; ++k) m = max(m, last_brk[k]);
-    smax[t] = m;
-    __syncthreads();
-    if (t == 0) {
-        long long acc = -1;
-        for (uint32_t k = 0; k < blockDim.x; ++k) { long long v = smax[k]; smax[k] = acc; acc = max(acc, v); }
+// parity of the run that is open where segment k begins; `known` (>= 0) holds at segment `from`
+__device__ uint32_t run_parity(const unsigned long long* seg, long long k, long long from, uint32_t known) {
+    while (--k >= from) {
+        const unsigned long long v = seg[k];
+        if ((v >> 60) & 1ull) return (uint32_t)(v >> 61) & 1u;
     }
-    __syncthreads();
-    long long run = smax[t];
-    unsigned long long s = 0;
-    for (uint32_t k = lo; k < hi; ++k) {
-        cs_in[k] = run;
-        unsigned long long a = (unsigned long long)k * STILE;
-        uint32_t par = (uint32_t)((a - (unsigned long long)run) & 1ull);   // run >= 0 for k >= 1
-        s += k == 0 ? cnt0[k] : (par ? cnt1[k] : cnt0[k]);
-        run = max(run, last_brk[k]);
-    }
-    ssum[t] = s;
-    __syncthreads();
-    if (t == 0) {
-        unsigned long long acc = 0;
-        for (uint32_t k = 0; k < blockDim.x; ++k) { unsigned long long v = ssum[k]; ssum[k] = acc; acc += v; }
-        *total = acc;
-    }
-    __syncthreads();
-    s = ssum[t];
-    run = smax[t];
-    for (uint32_t k = lo; k < hi; ++k) {
-        base[k] = s;
-        unsigned long long a = (unsigned long long)k * STILE;
-        uint32_t par = (uint32_t)((a - (unsigned long long)run) & 1ull);
-        s += k == 0 ? cnt0[k] : (par ? cnt1[k] : cnt0[k]);
-        run = max(run, last_brk[k]);
-    }
+    return known;
 }
 
-// per entry: visited? draw index, LCG value, hit byte
-__global__ void __launch_bounds__(STILE) k_apply(const uint32_t* info, unsigned long long n, const long long* cs_in,
-                                                 const unsigned long long* base, uint32_t s0, double p,
-                                                 uint32_t n_bp, uint32_t* hits_words, unsigned long long* cnt) {
-    __shared__ int s_cs[STILE];
-    __shared__ uint32_t s_scan[STILE];
-    unsigned long long a = (unsigned long long)blockIdx.x * STILE;
-    unsigned long long i = a + threadIdx.x;
-    uint32_t w = i < n ? info[i] : 0u;
-    bool brk = i < n && (w >> 31);
-    s_cs[threadIdx.x] = brk ? (int)threadIdx.x : -1;
+// the draws of each segment's list, in order; block b takes segments [b per, (b + 1) per)
+constexpr int DB = 256;
+__global__ void __launch_bounds__(DB) k_draw(const uint32_t* list, const unsigned long long* seg, uint32_t nseg, uint32_t per,
+                                             uint32_t s0, double p, uint32_t n_bp, uint32_t* hits_words,
+                                             unsigned long long* cnt) {
+    __shared__ unsigned long long s_sum[DB / 32], s_cand;
+    __shared__ int s_last;
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const uint32_t lo = blockIdx.x * per, hi = min(lo + per, nseg);
+    if (threadIdx.x == 0) { s_last = -1; s_cand = 0; }
     __syncthreads();
-    for (int off = 1; off < STILE; off <<= 1) {
-        int v = s_cs[threadIdx.x];
-        int u = threadIdx.x >= (unsigned)off ? s_cs[threadIdx.x - off] : -1;
-        __syncthreads();
-        s_cs[threadIdx.x] = max(v, u);
-        __syncthreads();
+    // draws before the block's first segment, and the last run start before it
+    unsigned long long sum = 0;
+    int mine = -1;
+    for (uint32_t k = threadIdx.x; k < lo; k += DB) {
+        const unsigned long long v = seg[k];
+        const uint32_t d0 = fld(v, 1), d1 = fld(v, 2);
+        sum += fld(v, 0) + (d0 == d1 ? d0 : run_parity(seg, k, 0, 0u) ? d1 : d0);
+        if ((v >> 60) & 1ull) mine = (int)k;
     }
-    long long cs = s_cs[threadIdx.x] >= 0 ? (long long)(a + s_cs[threadIdx.x]) : cs_in[blockIdx.x];
-    bool visited = i < n && (((unsigned long long)((long long)i - cs) & 1ull) == 0);
-    bool draw = visited && ((w >> 30) & 1u);
-    unsigned cm = __ballot_sync(0xffffffffu, visited && ((w >> 29) & 1u));
-    if ((threadIdx.x & 31) == 0 && cm) atomicAdd(&cnt[3], (unsigned long long)__popc(cm));
-    // exclusive prefix count of draws in the tile
-    s_scan[threadIdx.x] = draw ? 1u : 0u;
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (mine >= 0) atomicMax(&s_last, mine);
+    if (lane == 0) s_sum[wl] = sum;
     __syncthreads();
-    for (int off = 1; off < STILE; off <<= 1) {
-        uint32_t v = s_scan[threadIdx.x];
-        uint32_t u = threadIdx.x >= (unsigned)off ? s_scan[threadIdx.x - off] : 0u;
+    unsigned long long base = 0;
+    for (int k = 0; k < DB / 32; ++k) base += s_sum[k];
+    const uint32_t known = s_last >= 0 ? (uint32_t)(seg[s_last] >> 61) & 1u : 0u;
+    unsigned long long cand = 0;
+    for (uint32_t c = lo; c < hi; c += DB) {
+        const uint32_t k = c + threadIdx.x;
+        const unsigned long long v = k < hi ? seg[k] : 0ull;
+        const uint32_t nres = fld(v, 0), d0 = fld(v, 1), d1 = fld(v, 2), c0 = fld(v, 4), c1 = fld(v, 5);
+        const uint32_t par = (d0 | d1 | c0 | c1) ? run_parity(seg, k, lo, known) : 0u;
+        cand += fld(v, 3) + (par ? c1 : c0);
+        const uint32_t mydraws = nres + (par ? d1 : d0);
+        uint32_t off = mydraws;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t u = __shfl_up_sync(0xffffffffu, off, o); if (lane >= o) off += u; }
         __syncthreads();
-        s_scan[threadIdx.x] = v + u;
+        if (lane == 31) s_sum[wl] = off;
         __syncthreads();
-    }
-    if (!draw) return;
-    unsigned long long k = base[blockIdx.x] + s_scan[threadIdx.x] - 1;   // 0-based draw index
-    uint32_t s = lcg_jump(s0, k + 1);
-    double u = s / 4294967296.0;
-    if (u < p) {
-        uint32_t h = w & 0x1fffffffu;
-        uint32_t shift = (h & 3u) * 8u;
-        uint32_t old = atomicOr(&hits_words[h >> 2], 1u << shift);
-        if (((old >> shift) & 0xffu) == 0u) {
-            atomicAdd(&cnt[0], 1ull);
-            atomicAdd(&cnt[h >= n_bp ? 2 : 1], 1ull);
+        unsigned long long before = base + off - mydraws;
+        for (int q = 0; q < DB / 32; ++q) { if (q < wl) before += s_sum[q]; base += s_sum[q]; }
+        if (!mydraws) continue;
+        uint32_t s = lcg_jump(s0, before);
+        for (uint32_t q = 0; q < nres + d0 + d1; ++q) {
+            const uint32_t w = list[(unsigned long long)k * SEG + q];
+            if ((w >> 31) && ((w >> 30) & 1u) != par) continue;
+            s = 1664525u * s + 1013904223u;
+            if (s / 4294967296.0 < p) {
+                const uint32_t h = w & 0x1fffffffu, shift = (h & 3u) * 8u;
+                const uint32_t old = atomicOr(&hits_words[h >> 2], 1u << shift);
+                if (((old >> shift) & 0xffu) == 0u) {
+                    atomicAdd(&cnt[0], 1ull);
+                    atomicAdd(&cnt[h >= n_bp ? 2 : 1], 1ull);
+                }
+            }
         }
     }
+    if (cand) atomicAdd(&s_cand, cand);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (s_cand) atomicAdd(&cnt[3], s_cand);
+        if (hi == nseg) cnt[4] = base;
+    }
 }
 
-// clusterDSB, one block per fibre
-__global__ void k_cluster(const uint8_t* hits, uint32_t n_per, uint32_t n_bp, uint32_t* out /*3 per fibre*/) {
+// clusterDSB, one block per fibre.  Each thread looks through a run of aligned
+// words of either strand (most are zero), counts its hits, and writes them at
+// its place in the strand's list: two passes and one scan, where 256 bytes at a
+// time with a scan each took three barriers per step (38 us on 441 fibres of 8823
+// bp, 7.4 us now).
+constexpr int CB = 256;
+__global__ void __launch_bounds__(CB) k_cluster(const uint8_t* hits, uint32_t n_per, uint32_t n_bp, uint32_t* out /*3 per fibre*/) {
     extern __shared__ uint32_t lists[];
-    uint32_t* s0 = lists;
-    uint32_t* s1 = lists + n_per;
-    __shared__ uint32_t k0, k1, wcount[2][32];
-    const uint8_t* h0 = hits + (size_t)blockIdx.x * n_per;
-    const uint8_t* h1 = h0 + n_bp;
-    if (threadIdx.x == 0) { k0 = 0; k1 = 0; }
-    __syncthreads();
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (uint32_t c = 0; c < n_per; c += blockDim.x) {
-        uint32_t b = c + threadIdx.x;
-        bool f0 = b < n_per && h0[b] == 1, f1 = b < n_per && h1[b] == 1;
-        unsigned m0 = __ballot_sync(0xffffffffu, f0), m1 = __ballot_sync(0xffffffffu, f1);
-        if (lane == 0) { wcount[0][wid] = __popc(m0); wcount[1][wid] = __popc(m1); }
+    __shared__ uint32_t tot[2][CB / 32];
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    uint32_t k01[2];
+#pragma unroll
+    for (int st = 0; st < 2; ++st) {
+        const unsigned long long h0 = (unsigned long long)blockIdx.x * n_per + (st ? n_bp : 0u), h1 = h0 + n_per;
+        const uint32_t nw = (uint32_t)((h1 + 3) / 4 - h0 / 4), per = (nw + CB - 1) / CB;
+        const uint32_t* W = reinterpret_cast<const uint32_t*>(hits) + h0 / 4;
+        const uint32_t w0 = min(threadIdx.x * per, nw), w1 = min(w0 + per, nw);
+        // bytes equal to 1 inside the fibre, as flags in bit 0 of each byte
+        auto ones = [&](uint32_t w) -> uint32_t {
+            const uint32_t v = W[w];
+            if (v == 0u) return 0u;
+            uint32_t m = 0;
+            for (int b = 0; b < 4; ++b) {
+                const unsigned long long at = (h0 / 4 + w) * 4 + b;
+                if (((v >> (8 * b)) & 0xffu) == 1u && at >= h0 && at < h1) m |= 1u << (8 * b);
+            }
+            return m;
+        };
+        uint32_t c = 0;
+        for (uint32_t w = w0; w < w1; ++w) c += __popc(ones(w));
+        uint32_t off = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t u = __shfl_up_sync(0xffffffffu, off, o); if (lane >= o) off += u; }
+        if (lane == 31) tot[st][wl] = off;
         __syncthreads();
-        uint32_t o0 = k0, o1 = k1;
-        for (int q = 0; q < wid; ++q) { o0 += wcount[0][q]; o1 += wcount[1][q]; }
-        unsigned lt = (1u << lane) - 1u;
-        if (f0) s0[o0 + __popc(m0 & lt)] = b;
-        if (f1) s1[o1 + __popc(m1 & lt)] = b;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int q = 0; q < nw; ++q) { k0 += wcount[0][q]; k1 += wcount[1][q]; }
-        }
-        __syncthreads();
+        uint32_t all = 0;
+        off -= c;
+        for (int q = 0; q < CB / 32; ++q) { if (q < wl) off += tot[st][q]; all += tot[st][q]; }
+        k01[st] = all;
+        uint32_t* L = lists + (st ? n_per : 0u);
+        if (c)
+            for (uint32_t w = w0; w < w1; ++w)
+                for (uint32_t m = ones(w); m; m &= m - 1)
+                    L[off++] = (uint32_t)((h0 / 4 + w) * 4 + (__ffs(m) - 1) / 8 - h0);
     }
+    __syncthreads();
+    const uint32_t* s0 = lists;
+    const uint32_t k0 = k01[0], k1 = k01[1];
+    uint32_t* s1 = lists + n_per;
     if (threadIdx.x == 0) {
         const int W = 10;
         uint32_t dsb = 0, jlo = 0;
@@ -289,16 +324,13 @@ __global__ void k_cluster(const uint8_t* hits, uint32_t n_per, uint32_t n_bp, ui
 cudaError_t launch_score(const float4* rad, const uint32_t* alive, unsigned long long n, const DnaDev& d,
                          double r_d, double p, int dedupe, uint32_t s0, uint32_t* hits_words,
                          const ScoreScratch& sc, cudaStream_t s) {
-    // the result counters must start at zero: a failed clear would leave the
-    // previous call's counts to be read back
-    cudaError_t e = cudaMemsetAsync(sc.u64, 0, 8 * sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
-    if (n == 0) return cudaGetLastError();
-    unsigned long long ntiles = (n + STILE - 1) / STILE;
-    k_prep<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(rad, alive, n, d, r_d, dedupe, sc.info);
-    k_tiles<<<(unsigned)ntiles, STILE, 0, s>>>(sc.info, n, sc.last_brk, sc.cnt0, sc.cnt1);
-    k_tilescan<<<1, 1024, 0, s>>>(sc.last_brk, sc.cnt0, sc.cnt1, (uint32_t)ntiles, sc.cs_in, sc.base, sc.u64 + 4);
-    k_apply<<<(unsigned)ntiles, STILE, 0, s>>>(sc.info, n, sc.cs_in, sc.base, s0, p, d.n_bp, hits_words, sc.u64);
+    if (n == 0) return cudaMemsetAsync(sc.u64, 0, 8 * sizeof(unsigned long long), s);
+    const uint32_t nseg = (uint32_t)((n + SEG - 1) / SEG);
+    // k_find clears the result counters
+    k_find<<<(nseg + FB / 32 - 1) / (FB / 32), FB, 0, s>>>(rad, alive, n, d, r_d, dedupe, sc.list, sc.seg, sc.u64);
+    // at least 64 segments to a block: each block reads all summaries before its own
+    const uint32_t nb = min((nseg + 63) / 64, 148u), per = (nseg + nb - 1) / nb;
+    k_draw<<<(nseg + per - 1) / per, DB, 0, s>>>(sc.list, sc.seg, nseg, per, s0, p, d.n_bp, hits_words, sc.u64);
     return cudaGetLastError();
 }
 
@@ -309,7 +341,7 @@ cudaError_t launch_cluster(const uint8_t* hits, const DnaDev& d, uint32_t n_fibe
         return cudaFuncSetAttribute(k_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     });
     if (e != cudaSuccess) return e;
-    k_cluster<<<n_fibers, 256, sm, s>>>(hits, d.n_bp_per, d.n_bp, out);
+    k_cluster<<<n_fibers, CB, sm, s>>>(hits, d.n_bp_per, d.n_bp, out);
     return cudaGetLastError();
 }
 

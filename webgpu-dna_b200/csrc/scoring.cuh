@@ -10,12 +10,11 @@ struct DnaDev {
     uint32_t grid_N, n_bp_per, n_bp;
 };
 
+constexpr unsigned long long SCORE_SEG = 512;   // entries per segment (scoring.cu k_find)
+
 struct ScoreScratch {
-    uint32_t* info;
-    long long* last_brk;
-    uint32_t *cnt0, *cnt1;
-    long long* cs_in;
-    unsigned long long* base;
+    uint32_t* list;            // one word per entry: each segment's draws
+    unsigned long long* seg;   // one per segment: its summary
     unsigned long long* u64;   // [0] ssb [1] ssb0 [2] ssb1 [3] cand [4] total draws
     uint32_t* fib;             // 3 per fibre
 };
