@@ -4,16 +4,20 @@
 // primary.wgsl:41-663 and secondary.wgsl:17-450 (same statements, same f32
 // evaluation order); the execution model is new:
 //
-// * One persistent kernel runs primaries and secondaries together.  Each warp
-//   iteration advances every lane's electron by one step (the reference's
-//   Phase A loop body for a primary, one Phase B dispatch for a secondary).
-//   Lanes whose electron finished refill at once: first from the global
-//   secondary queue, then from the primary pool, so warps stay full and the
-//   reference's 2000 Phase B dispatches become per-secondary step caps.
+// * One persistent kernel runs primaries and secondaries together.  A CTA holds
+//   256 electrons in shared memory and advances each by one step per iteration
+//   (the reference's Phase A loop body for a primary, one Phase B dispatch for a
+//   secondary), in phases with a barrier between them: move, then the
+//   interactions sorted by kind, then the spurs sorted by kind.  So a warp's
+//   lanes run the same branch, the branches of one step run side by side on
+//   different warps, and the warps of a CTA fetch the same code.
+//   Slots whose electron ended refill from the CTA's stash of secondaries,
+//   the global queue or the primary pool, so the reference's 2000 Phase B
+//   dispatches become per-secondary step caps.
 // * Every particle owns a Philox4x32-10 stream: key = seed, counter =
 //   (block, secondary index, primary id, 1).  Results do not depend on which
 //   lane or SM runs a particle, or when.
-// * rad_buf entries are staged per warp in shared memory and written out in
+// * rad_buf entries are staged per CTA in shared memory and written out in
 //   coalesced bursts with one global atomic per burst; each carries a 64-bit
 //   key (pid << 34 | secondary index << 17 | sequence) from which
 //   canonicalise() rebuilds a deterministic order.
@@ -25,11 +29,16 @@
 
 namespace wg {
 
-constexpr int TB = 256;            // threads per block
+constexpr int TB = 256;            // threads and electron slots per block
 constexpr int TW = TB / 32;        // warps per block
-constexpr int STG = 192;           // staged rad entries per warp
-constexpr int STG_FLUSH = 96;      // flushed at this level: + 32 lanes x at most 3 entries per step <= STG
-constexpr int STASH = (int)TRANSPORT_STASH;   // secondaries a warp keeps in shared memory
+constexpr int STG_FLUSH = 256;     // staged rad entries written out at this level: + 3 per slot and
+constexpr int STG = STG_FLUSH + 3 * TB;   // iteration at most
+constexpr int STASH = TW * (int)TRANSPORT_STASH / 2;   // secondaries a block keeps in shared memory
+constexpr int NREC = 512;          // steps drawn ahead per iteration (few electrons)
+#ifndef WG_HUNGRY
+#define WG_HUNGRY 8
+#endif
+constexpr int HUNGRY_CAP = WG_HUNGRY;     // electrons a block keeps while others have none
 
 __device__ __forceinline__ unsigned long long gtime() {
     unsigned long long t;
@@ -53,23 +62,33 @@ enum { C_OH = 0, C_EAQ = 1, C_H = 2, C_H3O = 3, C_DNA = 4, C_H2 = 5,
        SS_CUT = 9, SS_BOUNDS = 10, SS_STEPS = 11, SS_TERT = 12,
        D_IONS = 16, D_EXC = 17, D_ESC = 18, D_PRIM = 19, D_WSUM = 20, D_DOSE = 21 };
 
-struct Particle {
-    float px, py, pz, E, dx, dy, dz;
-    uint32_t pid, sub, seq, it, nsec;
-    uint32_t blk, ri, b0, b1, b2, b3;
-    float tpath, ppath, maxr, sx, sy, sz;
-    uint32_t nion, nexc;
-    bool prim, active;
+// Electron slots, one array per field.  A primary has secondary index 0.
+struct Slots {
+    float px[TB], py[TB], pz[TB], E[TB], dx[TB], dy[TB], dz[TB];
+    uint32_t pid[TB], sub[TB], seq[TB], it[TB];
+    uint32_t nd[TB];               // draws taken from its stream
+    float tpath[TB], ppath[TB], maxr[TB], sx[TB], sy[TB], sz[TB];   // primaries
+    uint32_t nion[TB], nexc[TB], nsec[TB];
+    float a[TB], b[TB];            // move -> interaction: table position, flags; ionisation -> spur: W_sec, binding
+    float xi[TB], xic[TB], xicv[TB], xicvd[TB], stot[TB], lam[TB], fE[TB];   // cross sections (XS)
+    uint32_t iE[TB];
 };
+// a step drawn ahead: path length, elastic and azimuthal deflection, kind of interaction
+struct StepRec { float dist[NREC], ce[NREC], se[NREC], sp[NREC], cp[NREC]; int kind[NREC]; };
+enum { L_ION = 0, L_EXC = 1, L_VIB = 2, L_TRACKED = 3, L_SPUR = 4, L_MOVE = 5, NLIST = 6 };
 
 struct Blk {
-    const float* T;       // tables in shared memory
-    float4* srad;         // this warp's rad_buf staging
+    const float* T;       // tables
+    Slots* S;
+    StepRec* R;
+    float4* srad;         // rad_buf staging
     unsigned long long* skey;
     int* sn;
     uint32_t* cnt;        // block counters
-    StashRec* stash;      // this warp's secondaries
+    StashRec* stash;      // secondaries
     int* stn;
+    uint16_t (*list)[TB]; // slots by kind (spurs: | kind << 8)
+    uint32_t* ln;         // this iteration's list lengths
 };
 
 // One out-of-line copy each of the step's f32 log, exp, pow and sincos: the
@@ -80,32 +99,39 @@ __device__ __noinline__ float expf_nc(float x) { return expf_(x); }
 __device__ __noinline__ float powf_nc(float x, float y) { return powf_(x, y); }
 __device__ __noinline__ float2 sincosf_nc(float x) { float s, c; sincosf_(x, &s, &c); return make_float2(s, c); }
 
-// Out-of-line Philox block for the transport stream: the generator is drawn
-// from many call sites, and one shared copy keeps the kernel's code small
-// enough for the instruction cache.
-__device__ __noinline__ u4 philox_transport(uint32_t blk, uint32_t sub, uint32_t pid, uint32_t k0, uint32_t k1) {
-    return philox(blk, sub, pid, 1u, k0, k1);
+// Four draws of an electron's stream from draw nd on: the two Philox blocks they can
+// lie in, whatever the position in the first, so that the lanes of a warp generate
+// together (a draw at a time, some lane needed a new block at nearly every one) and
+// nothing but the count is kept between phases.
+__device__ __forceinline__ float4 draw4_of(const u4& a, const u4& b, uint32_t ri) {
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t v[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] = (ri & 1u) ? w[k + 1] : w[k];
+    return make_float4(u01f((ri & 2u) ? v[2] : v[0]), u01f((ri & 2u) ? v[3] : v[1]), u01f((ri & 2u) ? v[4] : v[2]),
+                       u01f((ri & 2u) ? v[5] : v[3]));
+}
+// out of line: one copy for all call sites of the interactions and spurs
+__device__ __noinline__ float4 draw4_nc(uint32_t nd, uint32_t sub, uint32_t pid, uint32_t k0, uint32_t k1) {
+    return draw4_of(philox(nd >> 2, sub, pid, 1u, k0, k1), philox((nd >> 2) + 1u, sub, pid, 1u, k0, k1), nd & 3u);
 }
 
-__device__ __forceinline__ uint32_t rn(Particle& q, uint32_t k0, uint32_t k1) {
-    if (q.ri == 4u) {
-        u4 o = philox_transport(q.blk, q.sub, q.pid, k0, k1);
-        q.blk++;
-        q.b0 = o.x; q.b1 = o.y; q.b2 = o.z; q.b3 = o.w;
-        q.ri = 0;
-    }
-    uint32_t v = q.ri == 0 ? q.b0 : q.ri == 1 ? q.b1 : q.ri == 2 ? q.b2 : q.b3;
-    q.ri++;
-    return v;
-}
-#define RF() u01f(rn(q, A.k0, A.k1))
+// An electron's stream during a phase.
+struct Stream {
+    uint32_t nd, sub, pid;
+    __device__ __forceinline__ void load(const Slots& S, int s) { nd = S.nd[s]; sub = S.sub[s]; pid = S.pid[s]; }
+    __device__ __forceinline__ void store(Slots& S, int s) const { S.nd[s] = nd; }
+    // the next four draws; d of them are taken by nd += d
+    __device__ __forceinline__ float4 peek(const TArgs& A) const { return draw4_nc(nd, sub, pid, A.k0, A.k1); }
+};
 
-__device__ __forceinline__ void put(const TArgs& A, Blk& b, Particle& q, float x, float y, float z, float code) {
+__device__ __forceinline__ void put(const TArgs& A, Blk& b, const Stream& q, uint32_t& seq, float x, float y, float z,
+                                    float code) {
     int s = atomicAdd(b.sn, 1);
     b.srad[s] = make_float4(x, y, z, code + __uint2float_rn(q.pid) * 8.0f);
-    if (q.seq >= (1u << 17)) atomicOr(&A.st->err, DERR_KEY_RANGE);
-    b.skey[s] = ((unsigned long long)(q.pid - A.pid_base) << 34) | ((unsigned long long)q.sub << 17) | q.seq;
-    q.seq++;
+    if (seq >= (1u << 17)) atomicOr(&A.st->err, DERR_KEY_RANGE);
+    b.skey[s] = ((unsigned long long)(q.pid - A.pid_base) << 34) | ((unsigned long long)q.sub << 17) | seq;
+    seq++;
 }
 
 // per-thread deposited energy and number of dose-grid atomics
@@ -186,54 +212,32 @@ __device__ __forceinline__ float meesungnoen_sigma(float k) {   // primary.wgsl:
     return fmaxf(r, 0.0f) * 0.6267f;
 }
 
-// Gaussian 3-D displacement, the mu1..mu4 pattern of primary.wgsl:216-220.
-// Out of line (8 call sites); the particle's generator state travels by value.
-struct G3 { float x, y, z; uint32_t blk, ri, b0, b1, b2, b3; };
-
-__device__ __noinline__ G3 gauss3_nc(uint32_t blk, uint32_t ri, uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3,
-                                     uint32_t sub, uint32_t pid, uint32_t k0, uint32_t k1, float sigma) {
-    // four draws: words ri..3 of the current block, then (unless ri = 0) the
-    // first ri words of the next one (all four of it when ri = 4)
-    G3 g;
-    u4 n = {b0, b1, b2, b3};
-    if (ri != 0u) n = philox_transport(blk, sub, pid, k0, k1);
-    const uint32_t w[8] = {b0, b1, b2, b3, n.x, n.y, n.z, n.w};
-    float u[4];
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-        const uint32_t v = ri == 0u ? w[d] : ri == 1u ? w[d + 1] : ri == 2u ? w[d + 2] : ri == 3u ? w[d + 3] : w[d + 4];
-        u[d] = u01f(v);
-    }
-    if (ri == 0u) { g.blk = blk; g.ri = 4u; g.b0 = b0; g.b1 = b1; g.b2 = b2; g.b3 = b3; }
-    else { g.blk = blk + 1u; g.ri = ri; g.b0 = n.x; g.b1 = n.y; g.b2 = n.z; g.b3 = n.w; }
-    float u1 = fmaxf(u[0], 1e-30f);
-    float rr = sqrtf(-2.0f * logf_pos(u1)) * sigma;
+// Gaussian 3-D displacement from four draws, the mu1..mu4 pattern of primary.wgsl:216-220
+__device__ __noinline__ float3 gauss3_nc(float u0, float u1, float u2, float u3, float sigma) {
+    const float rr = sqrtf(-2.0f * logf_pos(fmaxf(u0, 1e-30f))) * sigma;
     float sn, cs;
-    sincosf_(TWO_PI_F * u[1], &sn, &cs);
-    g.x = rr * cs; g.y = rr * sn;
-    float u3 = fmaxf(u[2], 1e-30f);
-    g.z = sqrtf(-2.0f * logf_pos(u3)) * sigma * cosf_(TWO_PI_F * u[3]);
-    return g;
+    sincosf_(TWO_PI_F * u1, &sn, &cs);
+    const float z = sqrtf(-2.0f * logf_pos(fmaxf(u2, 1e-30f))) * sigma * cosf_(TWO_PI_F * u3);
+    return make_float3(rr * cs, rr * sn, z);
 }
-
-__device__ __forceinline__ float3 gauss3(const TArgs& A, Particle& q, float sigma) {
-    G3 g = gauss3_nc(q.blk, q.ri, q.b0, q.b1, q.b2, q.b3, q.sub, q.pid, A.k0, A.k1, sigma);
-    q.blk = g.blk; q.ri = g.ri; q.b0 = g.b0; q.b1 = g.b1; q.b2 = g.b2; q.b3 = g.b3;
-    return make_float3(g.x, g.y, g.z);
+__device__ __forceinline__ float3 gauss3(const TArgs& A, Stream& q, float sigma) {
+    const float4 p = q.peek(A);
+    q.nd += 4u;
+    return gauss3_nc(p.x, p.y, p.z, p.w, sigma);
 }
 
 // H2O+ + eaq -> H2Ovib dissociation channels (primary.wgsl:246-276)
-__device__ __forceinline__ void h2ovib(const TArgs& A, Blk& b, Particle& q, float x, float y, float z) {
-    float r_vd = RF();
+__device__ __forceinline__ void h2ovib(const TArgs& A, Blk& b, const Stream& q, uint32_t& seq, float r_vd, float x, float y,
+                                       float z) {
     if (r_vd < 0.1365f) {
         atomicAdd(&b.cnt[C_OH], 2u); atomicAdd(&b.cnt[C_H2], 1u);
-        put(A, b, q, x, y, z, 0.0f); put(A, b, q, x, y, z, 0.0f); put(A, b, q, x, y, z, 7.0f);
+        put(A, b, q, seq, x, y, z, 0.0f); put(A, b, q, seq, x, y, z, 0.0f); put(A, b, q, seq, x, y, z, 7.0f);
     } else if (r_vd < 0.494f) {
         atomicAdd(&b.cnt[C_OH], 1u); atomicAdd(&b.cnt[C_H], 1u);
-        put(A, b, q, x, y, z, 0.0f); put(A, b, q, x, y, z, 2.0f);
+        put(A, b, q, seq, x, y, z, 0.0f); put(A, b, q, seq, x, y, z, 2.0f);
     } else if (r_vd < 0.650f) {
         atomicAdd(&b.cnt[C_H], 2u);
-        put(A, b, q, x, y, z, 2.0f); put(A, b, q, x, y, z, 2.0f);
+        put(A, b, q, seq, x, y, z, 2.0f); put(A, b, q, seq, x, y, z, 2.0f);
     }
 }
 
@@ -283,499 +287,671 @@ __device__ __forceinline__ float sample_W_sec(const TArgs& A, const float* T, fl
     return e0 + (e1 - e0) * f;
 }
 
-// Append n stash records to the global queue (one atomic for the batch); the
-// consumer spins on the epoch flag written after the payload.  Records beyond
-// the queue capacity are dropped and counted, as sec_dropped in the reference.
-__device__ void push_global(const TArgs& A, const StashRec* r, int n, int lane_stride) {
-    (void)lane_stride;
-    unsigned long long base = atomicAdd(&A.st->sec_qtail.v, (uint32_t)n);
-    for (int k = 0; k < n; ++k) {
-        unsigned long long slot = base + k;
-        if (slot >= A.max_sec) { atomicAdd(&A.st->sec_drop, 1u); continue; }
-        SecRec* rec = A.secq + slot;
-        rec->pe = make_float4(r[k].x, r[k].y, r[k].z, r[k].E);
-        rec->dir = make_float4(r[k].dx, r[k].dy, r[k].dz, 0.0f);
-        rec->meta.x = r[k].pid;
-        rec->meta.y = r[k].sub;
-        __threadfence();
-        *(volatile uint32_t*)&rec->meta.z = A.pub_epoch;     // publish
-    }
+// Write one record to the global queue; the consumer spins on the epoch flag
+// written after the payload.  Records beyond the queue capacity are dropped and
+// counted, as sec_dropped in the reference.
+__device__ __forceinline__ void push_global(const TArgs& A, unsigned long long slot, const StashRec& r) {
+    if (slot >= A.max_sec) { atomicAdd(&A.st->sec_drop, 1u); return; }
+    SecRec* rec = A.secq + slot;
+    rec->pe = make_float4(r.x, r.y, r.z, r.E);
+    rec->dir = make_float4(r.dx, r.dy, r.dz, 0.0f);
+    rec->meta.x = r.pid;
+    rec->meta.y = r.sub;
+    __threadfence();
+    *(volatile uint32_t*)&rec->meta.z = A.pub_epoch;     // publish
 }
 
-struct XS {
-    float xi, xc, xl, svib, sdea, s_tot, t;
-    int grid;        // -1 below the grid, 1 above, 0 inside (t valid)
-    uint32_t vbin;
-};
+// the lanes of the warp with `on` append their slot to a list; their place in it
+__device__ __forceinline__ int push_list(Blk& b, int k, bool on, uint32_t v, int lane) {
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (!m) return 0;
+    uint32_t base = 0;
+    if (lane == __ffs(m) - 1) base = atomicAdd(&b.ln[k], (uint32_t)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, __ffs(m) - 1);
+    base += __popc(m & ((1u << lane) - 1u));
+    if (on) b.list[k][base] = (uint16_t)v;
+    return (int)base;
+}
 
-// Spurs of interact(): an ionisation whose e-aq thermalises nearby (code 5,
-// displaced from the ionisation site), a primary's ionisation with a tracked
-// secondary (separation estimated from the secondary's range, no e-aq entry),
-// an autoionising excitation (code 1, e-aq displaced from the displaced
-// mother site), and a secondary that thermalises below the cutoff (its e-aq
-// alone, code 5, secondary.wgsl:100-124).  All share one code path so that a
-// warp runs it once.
+// Spurs: an ionisation whose e-aq thermalises nearby (code 5, displaced from the
+// ionisation site), a primary's ionisation with a tracked secondary (separation
+// estimated from the secondary's range, no e-aq entry; its own list), an
+// autoionising excitation (code 1, e-aq displaced from the displaced mother
+// site), and a secondary that thermalises below the cutoff (its e-aq alone, code
+// 5, secondary.wgsl:100-124).
 enum : int { SPUR_NONE = 0, SPUR_LOCAL = 1, SPUR_TRACKED = 2, SPUR_AUTO = 3, SPUR_THERM = 4 };
 
-// the interaction after the move (primary.wgsl:180-649, secondary.wgsl:167-443).
-// First each lane takes its branch (ionisation, excitation, vibration, DEA) up
-// to the point where it needs a spur; then the lanes that need one run it
-// together; then a primary that ionised with W_sec > cutoff emits its
-// secondary.  Every lane still draws in the reference's statement order.
-__device__ __forceinline__ void interact(const TArgs& A, Blk& b, Particle& q, Dep& dep, const XS& x, bool therm) {
+// ---- interactions after the move (primary.wgsl:180-649, secondary.wgsl:167-443);
+// every electron draws in the reference's statement order.
+
+// ionisation; returns the spur it starts
+__device__ __forceinline__ int ionise(const TArgs& A, Blk& b, int s, Dep& dep) {
     const float* T = b.T;
-    float E = q.E;
-    const float px = q.px, py = q.py, pz = q.pz;
-    const bool prim = q.prim;
-    int spur = SPUR_NONE;
-    float W_sec = 0.0f, bind = 0.0f;
-    float r_type = therm ? 0.0f : RF() * x.s_tot;
-    if (therm) {
-        spur = SPUR_THERM;                                       // the lane did not move this step
-    } else if (r_type < x.xi && E > c_SB[0]) {
-        float sf[5];
-        if (x.grid < 0) { for (int k = 0; k < 5; ++k) sf[k] = T[S_XSF + k * XN_]; }
-        else if (x.grid > 0) { for (int k = 0; k < 5; ++k) sf[k] = T[S_XSF + k * XN_ + XN_ - 1]; }
-        else {
-            uint32_t i = (uint32_t)fminf(fmaxf(floorf(x.t), 0.0f), (float)(XN_ - 2));
-            float f = x.t - (float)i;
-            for (int k = 0; k < 5; ++k) {
-                const float* a = T + S_XSF + k * XN_;
-                sf[k] = fmaxf(0.0f, a[i] + (a[i + 1] - a[i]) * f);
-            }
-        }
-        float fsum = fmaxf(sf[0] + sf[1] + sf[2] + sf[3] + sf[4], 1e-12f);
-        float r_sh = RF() * fsum;
-        uint32_t shell;
-        if (r_sh < sf[0]) { bind = c_SB[0]; shell = 0; }
-        else if (r_sh < sf[0] + sf[1]) { bind = c_SB[1]; shell = 1; }
-        else if (r_sh < sf[0] + sf[1] + sf[2]) { bind = c_SB[2]; shell = 2; }
-        else if (r_sh < sf[0] + sf[1] + sf[2] + sf[3]) { bind = c_SB[3]; shell = 3; }
-        else { bind = c_SB[4]; shell = 4; }
-        if (E > bind) {
-            float r_w = RF();
-            float Wmax = (E + bind) * 0.5f;
-            float W = sample_W_sec(A, T, E, shell, r_w);
-            W = fminf(fmaxf(W, bind), Wmax);
-            W_sec = fmaxf(W - bind, 0.0f);
-            E -= W;
-            if (prim) {
-                q.nion++;
-                atomicAdd(&b.cnt[D_WSUM], (uint32_t)(W * 10.0f));
-                deposit(A, dep, px, py, pz, bind);
-                if (W_sec <= A.ce) deposit(A, dep, px, py, pz, W_sec);
-            } else {                                             // secondary.wgsl:192-255
-                atomicAdd(&b.cnt[SS_TERT], 1u);
-                deposit(A, dep, px, py, pz, W);
-            }
-            if (dna_near(A, px, py, pz) == 1u) atomicAdd(&b.cnt[C_DNA], 1u);
-            spur = (!prim || W_sec <= A.ce) ? SPUR_LOCAL : SPUR_TRACKED;
-        }
-    } else if (r_type < x.xi + x.xc) {
-        float ef[5];
-        if (x.grid < 0) { for (int k = 0; k < 5; ++k) ef[k] = T[S_XEF + k * XN_]; }
-        else if (x.grid > 0) { for (int k = 0; k < 5; ++k) ef[k] = T[S_XEF + k * XN_ + 85]; }
-        else {
-            uint32_t i = (uint32_t)fminf(fmaxf(floorf(x.t), 0.0f), (float)(XN_ - 2));
-            if (i > 85u) i = 85u;
-            float f = (i == 85u) ? 0.0f : x.t - (float)i;
-            uint32_t j = i + 1 < 85u ? i + 1 : 85u;
-            for (int k = 0; k < 5; ++k) {
-                const float* a = T + S_XEF + k * XN_;
-                ef[k] = fmaxf(0.0f, a[i] + (a[j] - a[i]) * f);
-            }
-        }
-        float efsum = fmaxf(ef[0] + ef[1] + ef[2] + ef[3] + ef[4], 1e-12f);
-        float r_ex = RF() * efsum;
-        float exc_E; uint32_t lvl;
-        if (r_ex < ef[0]) { exc_E = c_EX[0]; lvl = 0; }
-        else if (r_ex < ef[0] + ef[1]) { exc_E = c_EX[1]; lvl = 1; }
-        else if (r_ex < ef[0] + ef[1] + ef[2]) { exc_E = c_EX[2]; lvl = 2; }
-        else if (r_ex < ef[0] + ef[1] + ef[2] + ef[3]) { exc_E = c_EX[3]; lvl = 3; }
-        else { exc_E = c_EX[4]; lvl = 4; }
-        float d = fminf(exc_E, E);
-        E -= d;
-        deposit(A, dep, px, py, pz, d);
-        if (prim) q.nexc++;
-        float r_ch = RF();
-        if (lvl == 0u) {
-            if (r_ch < 0.65f) {
-                atomicAdd(&b.cnt[C_OH], 1u); atomicAdd(&b.cnt[C_H], 1u);
-                put(A, b, q, px, py, pz, 0.0f); put(A, b, q, px, py, pz, 2.0f);
-            }
-        } else if (lvl == 1u) {
-            if (r_ch < 0.175f) {
-            } else if (r_ch < 0.2075f) {
-                atomicAdd(&b.cnt[C_OH], 2u); atomicAdd(&b.cnt[C_H2], 1u);
-                put(A, b, q, px, py, pz, 0.0f); put(A, b, q, px, py, pz, 0.0f); put(A, b, q, px, py, pz, 7.0f);
-            } else if (r_ch < 0.7075f) {
-                spur = SPUR_AUTO;                                // primary.wgsl:473-536
-            } else if (r_ch < 0.961f) {
-                atomicAdd(&b.cnt[C_OH], 1u); atomicAdd(&b.cnt[C_H], 1u);
-                put(A, b, q, px, py, pz, 0.0f); put(A, b, q, px, py, pz, 2.0f);
-            } else {
-                atomicAdd(&b.cnt[C_H], 2u);
-                put(A, b, q, px, py, pz, 2.0f); put(A, b, q, px, py, pz, 2.0f);
-            }
-        } else {
-            if (r_ch < 0.50f) spur = SPUR_AUTO;                  // primary.wgsl:560-619
-        }
-        if (dna_near(A, px, py, pz) == 1u) atomicAdd(&b.cnt[C_DNA], 1u);
-    } else if (r_type < x.xi + x.xc + x.svib) {
-        // sample_vib_mode (helpers.wgsl:148-170) with the bin found by fly()
-        float r = RF();
-        uint32_t base = x.vbin * 9u;
-        float cumsum = 0.0f, cs[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            float frac = (T[S_VIB + k] > E) ? 0.0f : T[S_XVMF + base + k];
-            cumsum = cumsum + frac;
-            cs[k] = cumsum;
-        }
-        uint32_t mode = 8u;
-        if (cumsum <= 0.0f) mode = 0u;
-        else {
-            float thr = r * cumsum;
-#pragma unroll
-            for (int k = 8; k >= 0; --k) if (thr < cs[k]) mode = (uint32_t)k;
-        }
-        float d = fminf(T[S_VIB + mode], E);
-        E -= d;
-        deposit(A, dep, px, py, pz, d);
-    } else if (r_type < x.xi + x.xc + x.svib + x.sdea) {
-        deposit(A, dep, px, py, pz, E);                          // Melton DEA
-        atomicAdd(&b.cnt[C_OH], 1u); atomicAdd(&b.cnt[C_H2], 1u);
-        put(A, b, q, px, py, pz, 0.0f); put(A, b, q, px, py, pz, 6.0f); put(A, b, q, px, py, pz, 7.0f);
-        E = 0.0f;
-    }
-    if (spur != SPUR_NONE) {
-        // mother (H2O+) displacement, then e-aq displacement and Onsager
-        // recombination (p = 1 - exp(-0.711 / r)) or the tracked-secondary
-        // estimate r = 0.04 W^1.3 + meesungnoen(min(W, 7.4)), then the H2Ovib
-        // channels or the OH + [e-aq] + H3O+ entries (primary.wgsl:216-353)
-        float mpx = px, mpy = py, mpz = pz;
-        if (spur != SPUR_THERM) {
-            const float3 m = gauss3(A, q, 1.1547005f);
-            mpx = px + m.x; mpy = py + m.y; mpz = pz + m.z;
-        }
-        float epx = px, epy = py, epz = pz, p_recomb = 0.0f;
-        if (spur != SPUR_TRACKED) {
-            const bool au = spur == SPUR_AUTO;
-            if (au) { epx = mpx; epy = mpy; epz = mpz; }
-            const float eaq_s = meesungnoen_sigma(au ? 1.7f : spur == SPUR_THERM ? E : W_sec);
-            if (eaq_s > 0.0f) {
-                const float3 g = gauss3(A, q, eaq_s);
-                epx = epx + g.x; epy = epy + g.y; epz = epz + g.z;
-            }
-            const float rdx = epx - mpx, rdy = epy - mpy, rdz = epz - mpz;
-            const float r_sep = fmaxf(sqrtf(rdx * rdx + rdy * rdy + rdz * rdz), 1e-6f);
-            p_recomb = 1.0f - expf_nc(-0.711f / r_sep);
-        } else {
-            const float r_track = 0.04f * powf_nc(W_sec, 1.3f);
-            const float r_tail = meesungnoen_sigma(fminf(W_sec, 7.4f));
-            const float r_sep_est = fmaxf(r_track + r_tail, 1e-3f);
-            p_recomb = 1.0f - expf_nc(-0.711f / r_sep_est);
-        }
-        if (spur == SPUR_THERM) {
-            put(A, b, q, epx, epy, epz, 5.0f);
-        } else if (RF() < p_recomb) {
-            h2ovib(A, b, q, mpx, mpy, mpz);
-        } else {
-            atomicAdd(&b.cnt[C_OH], 1u); atomicAdd(&b.cnt[C_H3O], 1u);
-            put(A, b, q, mpx, mpy, mpz, 0.0f);
-            if (spur != SPUR_TRACKED) {
-                atomicAdd(&b.cnt[C_EAQ], 1u);
-                put(A, b, q, epx, epy, epz, spur == SPUR_AUTO ? 1.0f : 5.0f);
-            }
-            put(A, b, q, mpx, mpy, mpz, 3.0f);
+    Slots& S = *b.S;
+    Stream q;
+    q.load(S, s);
+    float E = S.E[s];
+    const float px = S.px[s], py = S.py[s], pz = S.pz[s], t = S.a[s];
+    const int grid = (int)(__float_as_uint(S.b[s]) & 3u) - 1;
+    const bool prim = q.sub == 0u;
+    const float4 d = q.peek(A);
+    float sf[5];
+    if (grid < 0) { for (int k = 0; k < 5; ++k) sf[k] = T[S_XSF + k * XN_]; }
+    else if (grid > 0) { for (int k = 0; k < 5; ++k) sf[k] = T[S_XSF + k * XN_ + XN_ - 1]; }
+    else {
+        uint32_t i = (uint32_t)fminf(fmaxf(floorf(t), 0.0f), (float)(XN_ - 2));
+        float f = t - (float)i;
+        for (int k = 0; k < 5; ++k) {
+            const float* a = T + S_XSF + k * XN_;
+            sf[k] = fmaxf(0.0f, a[i] + (a[i + 1] - a[i]) * f);
         }
     }
-    if (spur == SPUR_TRACKED) {                                  // primary.wgsl:362-413
-        // every emission takes a sec_buf index (counters[6]); at or beyond
-        // max_sec the secondary is dropped together with its angle draws and
-        // the primary's momentum update (:364)
-        const uint32_t sec_idx = atomicAdd(&A.st->sec_tail.v, 1u);
-        if (sec_idx < A.max_sec) {
-            q.nsec++;
-            float E_before = E + bind + W_sec;
-            float cos_s;
-            if (W_sec < 50.0f) {
-                cos_s = 2.0f * RF() - 1.0f;
-            } else if (W_sec <= 200.0f) {
-                if (RF() <= 0.1f) cos_s = 2.0f * RF() - 1.0f;
-                else cos_s = RF() * 0.70710678f;
-            } else {
-                float sin2 = fminf(fmaxf((1.0f - W_sec / E_before) / (1.0f + W_sec / 1022000.0f), 0.0f), 1.0f);
-                cos_s = sqrtf(fmaxf(0.0f, 1.0f - sin2));
-            }
-            float sin_s = sqrtf(fmaxf(0.0f, 1.0f - cos_s * cos_s));
-            float sps, cps;
-            const float2 sc = sincosf_nc(TWO_PI_F * RF());
-            sps = sc.x; cps = sc.y;
-            float sdx = q.dx, sdy = q.dy, sdz = q.dz;
-            rotate(sdx, sdy, sdz, cos_s, sin_s, cps, sps);
-            float p_inc = sqrtf(E_before), p_sec = sqrtf(W_sec);
-            float pfx = p_inc * q.dx - p_sec * sdx;
-            float pfy = p_inc * q.dy - p_sec * sdy;
-            float pfz = p_inc * q.dz - p_sec * sdz;
-            float pfl = sqrtf(pfx * pfx + pfy * pfy + pfz * pfz);
-            if (pfl > 1e-10f) { q.dx = pfx / pfl; q.dy = pfy / pfl; q.dz = pfz / pfl; }
-            if (q.nsec >= (1u << 17)) atomicOr(&A.st->err, DERR_KEY_RANGE);
-            StashRec r{px, py, pz, W_sec, sdx, sdy, sdz, q.pid, q.nsec};
-            int slot = A.stash_spill ? atomicAdd(b.stn, 1) : STASH;
-            if (slot < STASH) b.stash[slot] = r;
-            else push_global(A, &r, 1, 0);
-        }
+    float fsum = fmaxf(sf[0] + sf[1] + sf[2] + sf[3] + sf[4], 1e-12f);
+    float r_sh = d.x * fsum;
+    uint32_t shell;
+    float bind;
+    if (r_sh < sf[0]) { bind = c_SB[0]; shell = 0; }
+    else if (r_sh < sf[0] + sf[1]) { bind = c_SB[1]; shell = 1; }
+    else if (r_sh < sf[0] + sf[1] + sf[2]) { bind = c_SB[2]; shell = 2; }
+    else if (r_sh < sf[0] + sf[1] + sf[2] + sf[3]) { bind = c_SB[3]; shell = 3; }
+    else { bind = c_SB[4]; shell = 4; }
+    if (!(E > bind)) {
+        S.nd[s] = q.nd + 1u;
+        return SPUR_NONE;
     }
-    q.E = E;
+    S.nd[s] = q.nd + 2u;
+    float Wmax = (E + bind) * 0.5f;
+    float W = sample_W_sec(A, T, E, shell, d.y);
+    W = fminf(fmaxf(W, bind), Wmax);
+    const float W_sec = fmaxf(W - bind, 0.0f);
+    E -= W;
+    if (prim) {
+        S.nion[s]++;
+        atomicAdd(&b.cnt[D_WSUM], (uint32_t)(W * 10.0f));
+        deposit(A, dep, px, py, pz, bind);
+        if (W_sec <= A.ce) deposit(A, dep, px, py, pz, W_sec);
+    } else {                                             // secondary.wgsl:192-255
+        atomicAdd(&b.cnt[SS_TERT], 1u);
+        deposit(A, dep, px, py, pz, W);
+    }
+    if (dna_near(A, px, py, pz) == 1u) atomicAdd(&b.cnt[C_DNA], 1u);
+    S.E[s] = E;
+    S.a[s] = W_sec;
+    S.b[s] = bind;
+    return (!prim || W_sec <= A.ce) ? SPUR_LOCAL : SPUR_TRACKED;
 }
 
-// Cross sections, free flight and elastic deflection (primary.wgsl:155-172)
-__device__ __forceinline__ bool fly(const TArgs& A, Blk& b, Particle& q, XS& x, float& dist) {
+// excitation; returns the spur it starts
+__device__ __forceinline__ int excite(const TArgs& A, Blk& b, int s, Dep& dep) {
     const float* T = b.T;
-    float E = q.E;
-    float lE = logf_nc(E);
-    if (E <= T[S_XE]) { x.grid = -1; x.xi = 0.0f; x.xc = 0.0f; x.xl = T[S_XL]; x.t = 0.0f; }
-    else if (E >= T[S_XE + XN_ - 1]) {
-        x.grid = 1; x.xi = T[S_XI + XN_ - 1]; x.xc = T[S_XC + XN_ - 1]; x.xl = T[S_XL + XN_ - 1]; x.t = 0.0f;
+    Slots& S = *b.S;
+    Stream q;
+    q.load(S, s);
+    const float E = S.E[s], px = S.px[s], py = S.py[s], pz = S.pz[s], t = S.a[s];
+    const int grid = (int)(__float_as_uint(S.b[s]) & 3u) - 1;
+    const float4 p = q.peek(A);
+    S.nd[s] = q.nd + 2u;
+    float ef[5];
+    if (grid < 0) { for (int k = 0; k < 5; ++k) ef[k] = T[S_XEF + k * XN_]; }
+    else if (grid > 0) { for (int k = 0; k < 5; ++k) ef[k] = T[S_XEF + k * XN_ + 85]; }
+    else {
+        uint32_t i = (uint32_t)fminf(fmaxf(floorf(t), 0.0f), (float)(XN_ - 2));
+        if (i > 85u) i = 85u;
+        float f = (i == 85u) ? 0.0f : t - (float)i;
+        uint32_t j = i + 1 < 85u ? i + 1 : 85u;
+        for (int k = 0; k < 5; ++k) {
+            const float* a = T + S_XEF + k * XN_;
+            ef[k] = fmaxf(0.0f, a[i] + (a[j] - a[i]) * f);
+        }
+    }
+    float efsum = fmaxf(ef[0] + ef[1] + ef[2] + ef[3] + ef[4], 1e-12f);
+    float r_ex = p.x * efsum;
+    float exc_E; uint32_t lvl;
+    if (r_ex < ef[0]) { exc_E = c_EX[0]; lvl = 0; }
+    else if (r_ex < ef[0] + ef[1]) { exc_E = c_EX[1]; lvl = 1; }
+    else if (r_ex < ef[0] + ef[1] + ef[2]) { exc_E = c_EX[2]; lvl = 2; }
+    else if (r_ex < ef[0] + ef[1] + ef[2] + ef[3]) { exc_E = c_EX[3]; lvl = 3; }
+    else { exc_E = c_EX[4]; lvl = 4; }
+    float d = fminf(exc_E, E);
+    S.E[s] = E - d;
+    deposit(A, dep, px, py, pz, d);
+    if (q.sub == 0u) S.nexc[s]++;
+    const float r_ch = p.y;
+    int spur = SPUR_NONE;
+    // channel: 1 OH + H, 2 2 OH + H2, 3 2 H
+    int ch = 0;
+    if (lvl == 0u) {
+        if (r_ch < 0.65f) ch = 1;
+    } else if (lvl == 1u) {
+        if (r_ch < 0.175f) {
+        } else if (r_ch < 0.2075f) ch = 2;
+        else if (r_ch < 0.7075f) spur = SPUR_AUTO;           // primary.wgsl:473-536
+        else if (r_ch < 0.961f) ch = 1;
+        else ch = 3;
     } else {
-        x.grid = 0;
+        if (r_ch < 0.50f) spur = SPUR_AUTO;                  // primary.wgsl:560-619
+    }
+    if (ch) {
+        uint32_t seq = S.seq[s];
+        if (ch != 3) put(A, b, q, seq, px, py, pz, 0.0f);
+        if (ch == 2) put(A, b, q, seq, px, py, pz, 0.0f);
+        if (ch == 2) put(A, b, q, seq, px, py, pz, 7.0f);
+        else put(A, b, q, seq, px, py, pz, 2.0f);
+        if (ch == 3) put(A, b, q, seq, px, py, pz, 2.0f);
+        S.seq[s] = seq;
+        if (ch != 3) atomicAdd(&b.cnt[C_OH], (uint32_t)ch);
+        if (ch == 2) atomicAdd(&b.cnt[C_H2], 1u);
+        else atomicAdd(&b.cnt[C_H], ch == 3 ? 2u : 1u);
+    }
+    if (dna_near(A, px, py, pz) == 1u) atomicAdd(&b.cnt[C_DNA], 1u);
+    return spur;
+}
+
+// vibrational excitation, or dissociative attachment
+__device__ __forceinline__ void vibrate(const TArgs& A, Blk& b, int s, Dep& dep) {
+    const float* T = b.T;
+    Slots& S = *b.S;
+    Stream q;
+    q.load(S, s);
+    const float E = S.E[s], px = S.px[s], py = S.py[s], pz = S.pz[s];
+    const uint32_t meta = __float_as_uint(S.b[s]);
+    if (meta & 4u) {                                             // Melton DEA
+        deposit(A, dep, px, py, pz, E);
+        atomicAdd(&b.cnt[C_OH], 1u); atomicAdd(&b.cnt[C_H2], 1u);
+        uint32_t seq = S.seq[s];
+        put(A, b, q, seq, px, py, pz, 0.0f); put(A, b, q, seq, px, py, pz, 6.0f); put(A, b, q, seq, px, py, pz, 7.0f);
+        S.seq[s] = seq;
+        S.E[s] = 0.0f;
+        return;
+    }
+    // sample_vib_mode (helpers.wgsl:148-170) with the bin found by the move
+    const float4 p = q.peek(A);
+    S.nd[s] = q.nd + 1u;
+    const uint32_t base = (meta >> 3) * 9u;
+    float cumsum = 0.0f, cs[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        float frac = (T[S_VIB + k] > E) ? 0.0f : T[S_XVMF + base + k];
+        cumsum = cumsum + frac;
+        cs[k] = cumsum;
+    }
+    uint32_t mode = 8u;
+    if (cumsum <= 0.0f) mode = 0u;
+    else {
+        float thr = p.x * cumsum;
+#pragma unroll
+        for (int k = 8; k >= 0; --k) if (thr < cs[k]) mode = (uint32_t)k;
+    }
+    float d = fminf(T[S_VIB + mode], E);
+    S.E[s] = E - d;
+    deposit(A, dep, px, py, pz, d);
+}
+
+// ---- spurs: mother (H2O+) displacement, then e-aq displacement and Onsager
+// recombination (p = 1 - exp(-0.711 / r)) or the tracked-secondary estimate
+// r = 0.04 W^1.3 + meesungnoen(min(W, 7.4)), then the H2Ovib channels or the
+// OH + [e-aq] + H3O+ entries (primary.wgsl:216-353)
+__device__ __forceinline__ void spur(const TArgs& A, Blk& b, int s, int kind) {
+    Slots& S = *b.S;
+    Stream q;
+    q.load(S, s);
+    uint32_t seq = S.seq[s];
+    const float px = S.px[s], py = S.py[s], pz = S.pz[s];
+    float mpx = px, mpy = py, mpz = pz;
+    if (kind != SPUR_THERM) {
+        const float3 m = gauss3(A, q, 1.1547005f);
+        mpx = px + m.x; mpy = py + m.y; mpz = pz + m.z;
+    }
+    float epx = px, epy = py, epz = pz;
+    if (kind == SPUR_AUTO) { epx = mpx; epy = mpy; epz = mpz; }
+    const float eaq_s = meesungnoen_sigma(kind == SPUR_AUTO ? 1.7f : kind == SPUR_THERM ? S.E[s] : S.a[s]);
+    if (eaq_s > 0.0f) {
+        const float3 g = gauss3(A, q, eaq_s);
+        epx = epx + g.x; epy = epy + g.y; epz = epz + g.z;
+    }
+    if (kind == SPUR_THERM) {
+        put(A, b, q, seq, epx, epy, epz, 5.0f);
+        return;                                                  // the slot is free
+    }
+    const float4 p = q.peek(A);
+    const float rdx = epx - mpx, rdy = epy - mpy, rdz = epz - mpz;
+    const float r_sep = fmaxf(sqrtf(rdx * rdx + rdy * rdy + rdz * rdz), 1e-6f);
+    const float p_recomb = 1.0f - expf_nc(-0.711f / r_sep);
+    if (p.x < p_recomb) {
+        q.nd += 2u;
+        h2ovib(A, b, q, seq, p.y, mpx, mpy, mpz);
+    } else {
+        q.nd += 1u;
+        atomicAdd(&b.cnt[C_OH], 1u); atomicAdd(&b.cnt[C_H3O], 1u); atomicAdd(&b.cnt[C_EAQ], 1u);
+        put(A, b, q, seq, mpx, mpy, mpz, 0.0f);
+        put(A, b, q, seq, epx, epy, epz, kind == SPUR_AUTO ? 1.0f : 5.0f);
+        put(A, b, q, seq, mpx, mpy, mpz, 3.0f);
+    }
+    S.seq[s] = seq;
+    q.store(S, s);
+}
+
+// the spur of a primary's ionisation above the cutoff, and its secondary
+__device__ __forceinline__ void spur_tracked(const TArgs& A, Blk& b, int s, uint32_t sec_idx) {
+    Slots& S = *b.S;
+    Stream q;
+    q.load(S, s);
+    uint32_t seq = S.seq[s];
+    const float px = S.px[s], py = S.py[s], pz = S.pz[s], W_sec = S.a[s], bind = S.b[s];
+    const float3 m = gauss3(A, q, 1.1547005f);
+    const float mpx = px + m.x, mpy = py + m.y, mpz = pz + m.z;
+    const float r_track = 0.04f * powf_nc(W_sec, 1.3f);
+    const float r_tail = meesungnoen_sigma(fminf(W_sec, 7.4f));
+    const float r_sep_est = fmaxf(r_track + r_tail, 1e-3f);
+    const float p_recomb = 1.0f - expf_nc(-0.711f / r_sep_est);
+    {
+        const float4 p = q.peek(A);
+        if (p.x < p_recomb) {
+            q.nd += 2u;
+            h2ovib(A, b, q, seq, p.y, mpx, mpy, mpz);
+        } else {
+            q.nd += 1u;
+            atomicAdd(&b.cnt[C_OH], 1u); atomicAdd(&b.cnt[C_H3O], 1u);
+            put(A, b, q, seq, mpx, mpy, mpz, 0.0f);
+            put(A, b, q, seq, mpx, mpy, mpz, 3.0f);
+        }
+    }
+    S.seq[s] = seq;
+    // primary.wgsl:362-413: at or beyond max_sec the secondary is dropped
+    // together with its angle draws and the primary's momentum update (:364)
+    if (sec_idx < A.max_sec) {
+        const uint32_t nsec = S.nsec[s] + 1u;
+        S.nsec[s] = nsec;
+        const float E_before = S.E[s] + bind + W_sec;
+        const float4 p = q.peek(A);
+        uint32_t nd = 0;
+        float cos_s;
+        if (W_sec < 50.0f) {
+            cos_s = 2.0f * p.x - 1.0f;
+            nd = 1;
+        } else if (W_sec <= 200.0f) {
+            cos_s = p.x <= 0.1f ? 2.0f * p.y - 1.0f : p.y * 0.70710678f;
+            nd = 2;
+        } else {
+            float sin2 = fminf(fmaxf((1.0f - W_sec / E_before) / (1.0f + W_sec / 1022000.0f), 0.0f), 1.0f);
+            cos_s = sqrtf(fmaxf(0.0f, 1.0f - sin2));
+        }
+        const float sin_s = sqrtf(fmaxf(0.0f, 1.0f - cos_s * cos_s));
+        const float2 sc = sincosf_nc(TWO_PI_F * (nd == 0u ? p.x : nd == 1u ? p.y : p.z));
+        q.nd += nd + 1u;
+        const float qx = S.dx[s], qy = S.dy[s], qz = S.dz[s];
+        float sdx = qx, sdy = qy, sdz = qz;
+        rotate(sdx, sdy, sdz, cos_s, sin_s, sc.y, sc.x);
+        const float p_inc = sqrtf(E_before), p_sec = sqrtf(W_sec);
+        const float pfx = p_inc * qx - p_sec * sdx;
+        const float pfy = p_inc * qy - p_sec * sdy;
+        const float pfz = p_inc * qz - p_sec * sdz;
+        const float pfl = sqrtf(pfx * pfx + pfy * pfy + pfz * pfz);
+        if (pfl > 1e-10f) { S.dx[s] = pfx / pfl; S.dy[s] = pfy / pfl; S.dz[s] = pfz / pfl; }
+        if (nsec >= (1u << 17)) atomicOr(&A.st->err, DERR_KEY_RANGE);
+        const StashRec r{px, py, pz, W_sec, sdx, sdy, sdz, q.pid, nsec};
+        const int slot = A.stash_spill ? atomicAdd(b.stn, 1) : STASH;
+        if (slot < STASH) b.stash[slot] = r;
+        else push_global(A, atomicAdd(&A.st->sec_qtail.v, 1u), r);
+    }
+    q.store(S, s);
+}
+
+// ---- cross sections at the electron's energy (helpers.wgsl:15-66, 134-186).  They
+// hold until an interaction changes the energy, so a run of elastic steps
+// shares them.
+struct XS {
+    float xi, xic, xicv, xicvd;    // running sums of ionisation, excitation, vibration, attachment
+    float s_tot, lambda, fE;       // total, mean free path; place in the elastic table
+    uint32_t iE;
+    float t;                       // place in the energy grid
+    uint32_t meta;                 // grid + 1 | vibrational bin << 3
+};
+__device__ __forceinline__ bool cross_sections(const TArgs& A, const float* T, float E, XS& x) {
+    float xi, xc, xl;
+    int grid;
+    x.t = 0.0f;
+    const float lE = logf_nc(E);
+    if (E <= T[S_XE]) { grid = -1; xi = 0.0f; xc = 0.0f; xl = T[S_XL]; }
+    else if (E >= T[S_XE + XN_ - 1]) { grid = 1; xi = T[S_XI + XN_ - 1]; xc = T[S_XC + XN_ - 1]; xl = T[S_XL + XN_ - 1]; }
+    else {
+        grid = 0;
         x.t = (lE - A.tab.log_xe0) * A.tab.inv_log_xe_step;
         uint32_t i = (uint32_t)fminf(fmaxf(floorf(x.t), 0.0f), (float)(XN_ - 2));
         float f = x.t - (float)i;
-        x.xi = fmaxf(0.0f, T[S_XI + i] + (T[S_XI + i + 1] - T[S_XI + i]) * f);
-        x.xc = fmaxf(0.0f, T[S_XC + i] + (T[S_XC + i + 1] - T[S_XC + i]) * f);
-        x.xl = fmaxf(0.0f, T[S_XL + i] + (T[S_XL + i + 1] - T[S_XL + i]) * f);
+        xi = fmaxf(0.0f, T[S_XI + i] + (T[S_XI + i + 1] - T[S_XI + i]) * f);
+        xc = fmaxf(0.0f, T[S_XC + i] + (T[S_XC + i + 1] - T[S_XC + i]) * f);
+        xl = fmaxf(0.0f, T[S_XL + i] + (T[S_XL + i + 1] - T[S_XL + i]) * f);
     }
-    x.svib = 0.0f;
-    x.vbin = 0;
+    float svib = 0.0f;
+    uint32_t vbin = 0;
     if (E >= 2.0f && E < 100.0f) {                               // xs_vib_total
         uint32_t lo = 0, hi = NVIB_ - 1;
         while (hi - lo > 1u) { uint32_t mid = (lo + hi) >> 1; if (T[S_XVE + mid] <= E) lo = mid; else hi = mid; }
-        x.vbin = lo;
+        vbin = lo;
         float f = (E - T[S_XVE + lo]) / (T[S_XVE + lo + 1] - T[S_XVE + lo]);
-        x.svib = fmaxf(0.0f, T[S_XVS + lo] + (T[S_XVS + lo + 1] - T[S_XVS + lo]) * f);
+        svib = fmaxf(0.0f, T[S_XVS + lo] + (T[S_XVS + lo + 1] - T[S_XVS + lo]) * f);
     }
-    x.sdea = 0.0f;
+    float sdea = 0.0f;
     if (E >= 4.0f && E <= 13.0f) {                               // xs_dea
-        // rolled: thirteen unrolled copies cost more in instruction fetch than the loop
-#pragma unroll 1
-        for (int i = 0; i < 13; ++i) {
-            if (E >= c_DEA_E[i] && E < c_DEA_E[i + 1]) {
-                float f = (E - c_DEA_E[i]) / (c_DEA_E[i + 1] - c_DEA_E[i]);
-                x.sdea = fmaxf(0.0f, c_DEA_S[i] + (c_DEA_S[i + 1] - c_DEA_S[i]) * f);
-                break;
-            }
+        int i = 0;                                               // last breakpoint <= E
+#pragma unroll
+        for (int k = 1; k < 14; ++k) i += E >= c_DEA_E[k] ? 1 : 0;
+        if (i < 13) {
+            float f = (E - c_DEA_E[i]) / (c_DEA_E[i + 1] - c_DEA_E[i]);
+            sdea = fmaxf(0.0f, c_DEA_S[i] + (c_DEA_S[i + 1] - c_DEA_S[i]) * f);
         }
     }
-    x.s_tot = x.xi + x.xc + x.xl + x.svib + x.sdea;
+    x.s_tot = xi + xc + xl + svib + sdea;
     if (x.s_tot <= 0.0f) return false;
-    float lambda = 1.0f / (NWf * x.s_tot);
-    dist = -logf_nc(fmaxf(RF(), 1e-10f)) * lambda;
-    // xs_el_cos (helpers.wgsl:66-82)
-    float r = RF();
-    float rr = fminf(fmaxf(r, 0.0f), 1.0f);
-    float jf = rr * (float)(NAC_ - 1);
-    uint32_t jlo = (uint32_t)floorf(jf);
-    uint32_t jhi = jlo + 1 < NAC_ - 1 ? jlo + 1 : NAC_ - 1;
-    float fj = jf - (float)jlo;
-    float lEa = (E >= T[S_XAE]) ? lE : logf_nc(T[S_XAE]);
-    float tE = (lEa - A.tab.log_xae0) * A.tab.inv_log_xae_step;
-    uint32_t iE = (uint32_t)fminf(fmaxf(floorf(tE), 0.0f), (float)(NAE_ - 2));
-    float fE = fminf(fmaxf(tE - (float)iE, 0.0f), 1.0f);
-    const float* a0 = T + S_XAC + iE * NAC_;
-    const float* a1 = a0 + NAC_;
-    float cE0 = a0[jlo] + (a0[jhi] - a0[jlo]) * fj;
-    float cE1 = a1[jlo] + (a1[jhi] - a1[jlo]) * fj;
-    float cos_el = fminf(fmaxf(cE0 + (cE1 - cE0) * fE, -1.0f), 1.0f);
-    float sin_el = sqrtf(fmaxf(0.0f, 1.0f - cos_el * cos_el));
-    const float2 sc = sincosf_nc(TWO_PI_F * RF());
-    const float sp = sc.x, cp = sc.y;
-    rotate(q.dx, q.dy, q.dz, cos_el, sin_el, cp, sp);
-    q.px += q.dx * dist; q.py += q.dy * dist; q.pz += q.dz * dist;
+    x.xi = E > c_SB[0] ? xi : -1.0f;                             // no ionisation below the first shell
+    x.xic = xi + xc;
+    x.xicv = x.xic + svib;
+    x.xicvd = x.xicv + sdea;
+    x.lambda = 1.0f / (NWf * x.s_tot);
+    const float lEa = (E >= T[S_XAE]) ? lE : logf_nc(T[S_XAE]);
+    const float tE = (lEa - A.tab.log_xae0) * A.tab.inv_log_xae_step;
+    x.iE = (uint32_t)fminf(fmaxf(floorf(tE), 0.0f), (float)(NAE_ - 2));
+    x.fE = fminf(fmaxf(tE - (float)x.iE, 0.0f), 1.0f);
+    x.meta = (uint32_t)(grid + 1) | (vbin << 3);
     return true;
 }
 
-__device__ __forceinline__ void start_primary(const TArgs& A, Particle& q, uint32_t idx) {
-    q.pid = A.pid_base + idx; q.sub = 0; q.seq = 0; q.it = 0; q.nsec = 0;
-    q.blk = 0; q.ri = 4;
-    q.prim = true; q.active = true;
-    q.E = A.E_prim ? A.E_prim[idx] : A.be;
-    q.px = 0.0f; q.py = 0.0f; q.pz = 0.0f;
-    float sh = A.start_half;
+__device__ __forceinline__ void start_primary(const TArgs& A, Slots& S, int s, uint32_t idx) {
+    Stream q;
+    q.nd = 0; q.sub = 0; q.pid = A.pid_base + idx;
+    float px = 0.0f, py = 0.0f, pz = 0.0f;
+    const float sh = A.start_half;
     if (sh > 0.0f) {
-        q.px = (RF() * 2.0f - 1.0f) * sh;
-        q.py = (RF() * 2.0f - 1.0f) * sh;
-        q.pz = (RF() * 2.0f - 1.0f) * sh;
+        const float4 p = q.peek(A);
+        q.nd += 3u;
+        px = (p.x * 2.0f - 1.0f) * sh;
+        py = (p.y * 2.0f - 1.0f) * sh;
+        pz = (p.z * 2.0f - 1.0f) * sh;
     }
-    q.sx = q.px; q.sy = q.py; q.sz = q.pz;
-    float u1 = fmaxf(RF(), 1e-10f);
-    float u2 = RF();
-    float cos_i = 1.0f - 2.0f * u1;
-    float sin_i = sqrtf(fmaxf(0.0f, 1.0f - cos_i * cos_i));
+    const float4 p = q.peek(A);
+    q.nd += 2u;
+    const float u1 = fmaxf(p.x, 1e-10f);
+    const float cos_i = 1.0f - 2.0f * u1;
+    const float sin_i = sqrtf(fmaxf(0.0f, 1.0f - cos_i * cos_i));
     float spi, cpi;
-    sincosf_(TWO_PI_F * u2, &spi, &cpi);
-    q.dx = sin_i * cpi; q.dy = sin_i * spi; q.dz = cos_i;
-    q.tpath = 0.0f; q.ppath = 0.0f; q.maxr = 0.0f; q.nion = 0; q.nexc = 0;
+    sincosf_(TWO_PI_F * p.y, &spi, &cpi);
+    S.px[s] = px; S.py[s] = py; S.pz[s] = pz;
+    S.sx[s] = px; S.sy[s] = py; S.sz[s] = pz;
+    S.E[s] = A.E_prim ? A.E_prim[idx] : A.be;
+    S.dx[s] = sin_i * cpi; S.dy[s] = sin_i * spi; S.dz[s] = cos_i;
+    S.pid[s] = q.pid; S.sub[s] = 0; S.seq[s] = 0; S.it[s] = 0; S.nsec[s] = 0;
+    S.tpath[s] = 0.0f; S.ppath[s] = 0.0f; S.maxr[s] = 0.0f; S.nion[s] = 0; S.nexc[s] = 0;
+    q.store(S, s);
 }
 
-__device__ __forceinline__ void finish_primary(const TArgs& A, Blk& b, Particle& q, Dep& dep, uint32_t esc) {
-    if (esc == 0u && q.E > 0.0f) deposit(A, dep, q.px, q.py, q.pz, q.E);
-    float4* r = reinterpret_cast<float4*>(A.results + 8ull * (q.pid - A.pid_base));
-    r[0] = make_float4(q.tpath, q.ppath, q.E, __uint_as_float(q.nion));
-    r[1] = make_float4(__uint_as_float(q.nexc), __uint_as_float(esc), q.maxr, 0.0f);
-    atomicAdd(&b.cnt[D_IONS], q.nion); atomicAdd(&b.cnt[D_EXC], q.nexc);
+__device__ __forceinline__ void load_secondary(Slots& S, int s, const StashRec& r) {
+    S.px[s] = r.x; S.py[s] = r.y; S.pz[s] = r.z; S.E[s] = r.E;
+    S.dx[s] = r.dx; S.dy[s] = r.dy; S.dz[s] = r.dz;
+    S.pid[s] = r.pid; S.sub[s] = r.sub; S.seq[s] = 0; S.it[s] = 0; S.nd[s] = 0;
+}
+
+__device__ __forceinline__ void finish_primary(const TArgs& A, Blk& b, int s, Dep& dep, float px, float py, float pz,
+                                               uint32_t esc) {
+    const Slots& S = *b.S;
+    const float E = S.E[s];
+    if (esc == 0u && E > 0.0f) deposit(A, dep, px, py, pz, E);
+    float4* r = reinterpret_cast<float4*>(A.results + 8ull * (S.pid[s] - A.pid_base));
+    r[0] = make_float4(S.tpath[s], S.ppath[s], E, __uint_as_float(S.nion[s]));
+    r[1] = make_float4(__uint_as_float(S.nexc[s]), __uint_as_float(esc), S.maxr[s], 0.0f);
+    atomicAdd(&b.cnt[D_IONS], S.nion[s]); atomicAdd(&b.cnt[D_EXC], S.nexc[s]);
     atomicAdd(&b.cnt[D_ESC], esc); atomicAdd(&b.cnt[D_PRIM], 1u);
-    q.active = false;
 }
 
-// one warp-iteration of a lane's electron.  Primaries and secondaries share
-// one fly + interact call site, so a warp holding both kinds runs the step
-// code once instead of once per kind; the lanes of `act` (those that entered)
-// meet again before the interaction, so its branches run once per warp step.
-__device__ __forceinline__ void lane_step(const TArgs& A, Blk& b, Particle& q, Dep& dep,
-                                          unsigned long long& nsteps, unsigned act) {
-    const float box = A.box;
-    const bool prim = q.prim;
-    const bool out = fabsf(q.px) >= box || fabsf(q.py) >= box || fabsf(q.pz) >= box;
-    bool go = true, therm = false;
-    if (prim) {
-        if (q.it >= A.ms || q.E < A.ce) { finish_primary(A, b, q, dep, 0u); go = false; }
-        else if (out) { finish_primary(A, b, q, dep, 1u); go = false; }
-    } else {
-        if (q.it >= A.sec_steps) { q.active = false; go = false; }
-        else if (q.E < A.ce) {                                   // secondary.wgsl:100-124
-            // thermalised: its e-aq is placed in interact()'s spur block
-            deposit(A, dep, q.px, q.py, q.pz, q.E);
-            atomicAdd(&b.cnt[C_EAQ], 1u);
-            atomicAdd(&b.cnt[SS_CUT], 1u);
-            therm = true;
-            go = false;
-        } else if (out) {
-            atomicAdd(&b.cnt[SS_BOUNDS], 1u);
-            q.active = false;
-            go = false;
-        }
+// ---- the move: steps (primary.wgsl:155-172: free flight, elastic deflection, kind of
+// interaction, four draws) until one interacts.  Five of six steps are elastic
+// only; they leave the energy and so the cross sections alone, and need no other
+// phase, so an iteration takes a run of them.
+
+// a step's draws: all of it that does not depend on where the electron is
+struct Step { float dist, ce, se, sp, cp; int kind; };
+__device__ __forceinline__ Step draw_step(const float* T, const float4& u, float lambda, uint32_t iE, float fE, float s_tot,
+                                          float xi, float xic, float xicv, float xicvd) {
+    Step r;
+    r.dist = -logf_nc(fmaxf(u.x, 1e-10f)) * lambda;
+    // xs_el_cos (helpers.wgsl:66-82)
+    const float* a0 = T + S_XAC + iE * NAC_;
+    const float* a1 = a0 + NAC_;
+    const float rr = fminf(fmaxf(u.y, 0.0f), 1.0f);
+    const float jf = rr * (float)(NAC_ - 1);
+    const uint32_t jlo = (uint32_t)floorf(jf);
+    const uint32_t jhi = jlo + 1 < NAC_ - 1 ? jlo + 1 : NAC_ - 1;
+    const float fj = jf - (float)jlo;
+    const float cE0 = a0[jlo] + (a0[jhi] - a0[jlo]) * fj;
+    const float cE1 = a1[jlo] + (a1[jhi] - a1[jlo]) * fj;
+    r.ce = fminf(fmaxf(cE0 + (cE1 - cE0) * fE, -1.0f), 1.0f);
+    r.se = sqrtf(fmaxf(0.0f, 1.0f - r.ce * r.ce));
+    const float2 sc = sincosf_nc(TWO_PI_F * u.z);
+    r.sp = sc.x;
+    r.cp = sc.y;
+    const float r_type = u.w * s_tot;
+    // list | attachment << 8, or -1: elastic only
+    r.kind = r_type < xi ? L_ION : r_type < xic ? L_EXC : r_type < xicv ? L_VIB : r_type < xicvd ? L_VIB | 256 : -1;
+    return r;
+}
+
+// an electron between steps
+struct Flight {
+    float px, py, pz, dx, dy, dz, tpath, ppath, maxr, sx, sy, sz;
+    uint32_t it, it_max, n;
+    bool prim, productive;
+    __device__ __forceinline__ void load(const Slots& S, int s, const TArgs& A) {
+        px = S.px[s]; py = S.py[s]; pz = S.pz[s]; dx = S.dx[s]; dy = S.dy[s]; dz = S.dz[s];
+        tpath = S.tpath[s]; ppath = S.ppath[s]; maxr = S.maxr[s]; sx = S.sx[s]; sy = S.sy[s]; sz = S.sz[s];
+        it = S.it[s]; n = 0;
+        prim = S.sub[s] == 0u;
+        productive = S.E[s] > 12.0f;
+        it_max = prim ? A.ms : A.sec_steps;
     }
+    // takes a step; true: the run ends here (what the step drew, the box, the step cap)
+    __device__ __forceinline__ bool step(const Step& r, float box, int& kind, bool& esc) {
+        rotate(dx, dy, dz, r.ce, r.se, r.cp, r.sp);
+        px += dx * r.dist; py += dy * r.dist; pz += dz * r.dist;
+        ++n;
+        ++it;
+        const bool out = fabsf(px) >= box || fabsf(py) >= box || fabsf(pz) >= box;
+        if (prim) {
+            tpath += r.dist;
+            if (productive) ppath += r.dist;
+            const float rdx = px - sx, rdy = py - sy, rdz = pz - sz;
+            const float rad = sqrtf(rdx * rdx + rdy * rdy + rdz * rdz);
+            if (rad > maxr) maxr = rad;
+            if (out) { esc = true; return true; }
+        }
+        kind = r.kind;
+        // a secondary that leaves the box or reaches the cap still interacts
+        return kind >= 0 || out || it >= it_max;
+    }
+    __device__ __forceinline__ void store(Slots& S, int s) const {
+        S.px[s] = px; S.py[s] = py; S.pz[s] = pz; S.dx[s] = dx; S.dy[s] = dy; S.dz[s] = dz;
+        if (prim) { S.tpath[s] = tpath; S.ppath[s] = ppath; S.maxr[s] = maxr; }
+        S.it[s] = it;
+    }
+};
+
+// What comes before a run of steps: the reference's checks and the cross
+// sections.  0: go; 1: ended; 2: thermalised (a spur follows).
+__device__ __forceinline__ int begin_move(const TArgs& A, Blk& b, int s, Dep& dep, XS& x) {
+    Slots& S = *b.S;
+    const float box = A.box, E = S.E[s], px = S.px[s], py = S.py[s], pz = S.pz[s];
+    const bool prim = S.sub[s] == 0u;
+    const bool capped = S.it[s] >= (prim ? A.ms : A.sec_steps);
+    int esc = -1;                                                // a primary's end (1: left the box)
+    if (capped || (prim && E < A.ce)) esc = 0;
+    else if (E < A.ce) {                                         // secondary.wgsl:100-124
+        deposit(A, dep, px, py, pz, E);
+        atomicAdd(&b.cnt[C_EAQ], 1u);
+        atomicAdd(&b.cnt[SS_CUT], 1u);
+        return 2;
+    } else if (fabsf(px) >= box || fabsf(py) >= box || fabsf(pz) >= box) {
+        if (!prim) atomicAdd(&b.cnt[SS_BOUNDS], 1u);
+        esc = 1;
+    } else if (!cross_sections(A, b.T, E, x)) esc = 0;
+    if (esc < 0) return 0;
+    if (prim) finish_primary(A, b, s, dep, px, py, pz, (uint32_t)esc);
+    return 1;
+}
+
+// What comes after it; the list that follows, or -1
+__device__ __forceinline__ int end_move(const TArgs& A, Blk& b, int s, Dep& dep, unsigned long long& nsteps, const Flight& f,
+                                        float t, uint32_t meta, int kind, bool esc, bool& active) {
+    Slots& S = *b.S;
+    nsteps += f.n;
+    if (!f.prim) atomicAdd(&b.cnt[SS_STEPS], f.n);
+    f.store(S, s);
+    S.nd[s] += 4u * f.n;
+    if (esc) {
+        finish_primary(A, b, s, dep, f.px, f.py, f.pz, 1u);
+        active = false;
+        return -1;
+    }
+    S.a[s] = t;
+    S.b[s] = __uint_as_float(kind >= 256 ? meta | 4u : meta);
+    return kind < 0 ? -1 : kind & 255;
+}
+
+// Many electrons: a lane draws and takes its own steps, at most `most` (a warp
+// waits for its longest run).  Returns the list that follows (-1: none) and clears
+// `active` when the electron ends.
+#ifndef WG_MOVE_STEPS
+#define WG_MOVE_STEPS 12
+#endif
+constexpr uint32_t MOVE_STEPS = WG_MOVE_STEPS;
+__device__ __forceinline__ int move(const TArgs& A, Blk& b, int s, Dep& dep, unsigned long long& nsteps, bool& active,
+                                    uint32_t most) {
+    Slots& S = *b.S;
     XS x;
-    if (go) {
-        const bool productive = q.E > 12.0f;
-        float dist;
-        if (!fly(A, b, q, x, dist)) {
-            if (prim) finish_primary(A, b, q, dep, 0u);
-            else q.active = false;
-            go = false;
-        } else {
-            nsteps++;
-            if (prim) {
-                q.tpath += dist;
-                if (productive) q.ppath += dist;
-                float rdx = q.px - q.sx, rdy = q.py - q.sy, rdz = q.pz - q.sz;
-                float r = sqrtf(rdx * rdx + rdy * rdy + rdz * rdz);
-                if (r > q.maxr) q.maxr = r;
-                if (fabsf(q.px) >= box || fabsf(q.py) >= box || fabsf(q.pz) >= box) { finish_primary(A, b, q, dep, 1u); go = false; }
-            } else {
-                atomicAdd(&b.cnt[SS_STEPS], 1u);
-            }
-        }
+    const int go = begin_move(A, b, s, dep, x);
+    if (go) { active = false; return go == 2 ? L_SPUR : -1; }
+    Flight f;
+    f.load(S, s, A);
+    const uint32_t nd = S.nd[s], sub = S.sub[s], pid = S.pid[s];
+    u4 cur = philox(nd >> 2, sub, pid, 1u, A.k0, A.k1);
+    int kind = -1;
+    bool esc = false;
+#pragma unroll 1
+    for (uint32_t k = 1; k <= most; ++k) {
+        const u4 nxt = philox((nd >> 2) + k, sub, pid, 1u, A.k0, A.k1);
+        const Step r = draw_step(b.T, draw4_of(cur, nxt, nd & 3u), x.lambda, x.iE, x.fE, x.s_tot, x.xi, x.xic, x.xicv, x.xicvd);
+        cur = nxt;
+        if (f.step(r, A.box, kind, esc)) break;
     }
-    __syncwarp(act);
-    if (go || therm) {
-        interact(A, b, q, dep, x, therm);
-        if (go) q.it++;
-        else q.active = false;
-    }
+    return end_move(A, b, s, dep, nsteps, f, x.t, x.meta, kind, esc, active);
 }
 
-__device__ __forceinline__ void flush_staging(const TArgs& A, Blk& b, int lane) {
-    __syncwarp();
-    int n = *b.sn;
-    if (n == 0) return;
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(&A.st->rad_next.v, (unsigned long long)n);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    int ndrop = 0;
-    for (int i = lane; i < n; i += 32) {
-        unsigned long long slot = base + (unsigned long long)i;
-        if (slot < A.max_rad) { A.rad[slot] = b.srad[i]; A.key[slot] = b.skey[i]; }
-        else ndrop++;
-    }
-    if (ndrop) atomicAdd(&A.st->rad_drop, (unsigned long long)ndrop);
-    __syncwarp();
-    if (lane == 0) *b.sn = 0;
-    __syncwarp();
-}
-
-__device__ __forceinline__ void load_secondary(Particle& q, const StashRec& r) {
-    q.px = r.x; q.py = r.y; q.pz = r.z; q.E = r.E;
-    q.dx = r.dx; q.dy = r.dy; q.dz = r.dz;
-    q.pid = r.pid; q.sub = r.sub; q.seq = 0; q.it = 0; q.nsec = 0;
-    q.blk = 0; q.ri = 4; q.prim = false; q.active = true;
-}
-
-// 2 CTAs per SM: 3 (80 registers, less staging) measured 15 % slower
+// What bounds it: the chain of a primary's steps (650 at 10 keV), each as long as
+// an iteration takes.  2 CTAs per SM hold 512 electrons; at 4096 x 10 keV about 325
+// are alive at a time, so an iteration costs little more than its longest
+// phase path, and with more electrons the issue slots bind.
+// Measured at 4096 x 10 keV: 14.9 ms with one warp per 32 electrons taking all
+// branches one after another (7.8 lanes per instruction, 16 % issue), TR_MS now.
 __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     float* T = reinterpret_cast<float*>(smem);
     float4* stg_rad = reinterpret_cast<float4*>(smem + S_TOTAL_PAD * 4);
-    unsigned long long* stg_key = reinterpret_cast<unsigned long long*>(stg_rad + TW * STG);
-    StashRec* stash = reinterpret_cast<StashRec*>(stg_key + TW * STG);
-    int* stg_n = reinterpret_cast<int*>(stash + TW * STASH);
-    int* stn = stg_n + TW;
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(stn + TW);
-    for (int i = threadIdx.x; i < S_TOTAL; i += TB) T[i] = A.tab.small[i];
-    if (threadIdx.x < TW) { stg_n[threadIdx.x] = 0; stn[threadIdx.x] = 0; }
-    if (threadIdx.x < 24) cnt[threadIdx.x] = 0;
-    __syncthreads();
-
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned long long* stg_key = reinterpret_cast<unsigned long long*>(stg_rad + STG);
+    Slots* SL = reinterpret_cast<Slots*>(stg_key + STG);
+    StepRec* SR = reinterpret_cast<StepRec*>(SL + 1);
+    StashRec* stash = reinterpret_cast<StashRec*>(SR + 1);
+    uint16_t (*lists)[TB] = reinterpret_cast<uint16_t (*)[TB]>(stash + STASH);
+    // What decides a barrier is read by every thread at the top of an iteration and
+    // written only where a barrier lies on either side: s_want, s_hungry and s_done
+    // below, s_free and s_ln by turns (par).
+    __shared__ int s_sn, s_stn, s_nprim, s_done, s_hungry, s_want;
+    __shared__ uint32_t s_ln[2][NLIST], s_free[2][TW], cnt[24], s_got[4];
+    __shared__ unsigned long long s_flush, s_spill;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    Blk b{T, stg_rad + w * STG, stg_key + w * STG, stg_n + w, cnt, stash + w * STASH, stn + w};
+    for (int i = tid; i < S_TOTAL; i += TB) T[i] = A.tab.small[i];
+    if (tid < 24) cnt[tid] = 0;
+    if (tid < 2 * NLIST) s_ln[tid / NLIST][tid % NLIST] = 0;
+    if (tid < TW) s_free[0][tid] = 32u;
+    if (tid == 0) { s_sn = 0; s_stn = 0; s_nprim = 0; s_done = 0; s_hungry = 0; s_want = 1; }
     DevState* S = A.st;
-    Particle q;
-    q.active = false;
+    Blk b{T, SL, SR, stg_rad, stg_key, &s_sn, cnt, stash, &s_stn, lists, nullptr};
+    // primaries a block holds at a time: its share, at most half its slots
+    const int quota = (int)min((uint32_t)TB / 2, (A.np + gridDim.x - 1) / gridDim.x);
     Dep dep{0.0, 0u};
     unsigned long long nsteps = 0;
-    bool busy = false;
+    bool active = false, busy = false, left = true;              // busy, left: thread 0
+    uint32_t par = 0;
     unsigned sleep_ns = 64;
     unsigned long long idle_since = 0;
+    __syncthreads();
 
     for (uint32_t it = 0;; ++it) {
-        unsigned need = __ballot_sync(0xffffffffu, !q.active);
-        // 1) this warp's stash (LIFO)
-        if (need) {
-            int sn = *(volatile int*)b.stn;
-            if (sn > 0) {
-                uint32_t take = min((uint32_t)__popc(need), (uint32_t)sn);
-                uint32_t rank = __popc(need & lt);
-                if (!q.active && rank < take) load_secondary(q, b.stash[sn - 1 - rank]);
-                __syncwarp();
-                if (lane == 0) *b.stn = sn - (int)take;
-                __syncwarp();
-                need = __ballot_sync(0xffffffffu, !q.active);
+        // 0) here all of the last iteration is done: staging, stash and free slots
+        //    are at rest until the interaction phase
+        int rn = s_sn, stn = min(s_stn, STASH);
+        if (rn >= STG_FLUSH || s_done) {
+            if (tid == 0) s_flush = atomicAdd(&S->rad_next.v, (unsigned long long)rn);
+            __syncthreads();
+            if (tid == 0) s_sn = 0;                              // all have read it
+            const unsigned long long base = s_flush;
+            int ndrop = 0;
+            for (int i = tid; i < rn; i += TB) {
+                const unsigned long long slot = base + (unsigned long long)i;
+                if (slot < A.max_rad) { A.rad[slot] = stg_rad[i]; A.key[slot] = stg_key[i]; }
+                else ndrop++;
             }
+            if (ndrop) atomicAdd(&S->rad_drop, (unsigned long long)ndrop);
+            if (s_done) break;
         }
-        const bool idle_warp = need == 0xffffffffu;
-        const bool poll = idle_warp || (it & A.poll_mask) == 0u;
-        // 2) the global queue
-        if (need && poll) {
-            uint32_t base = 0, got = 0;
-            if (lane == 0) {
-                uint32_t lim = min(*(volatile uint32_t*)&S->sec_qtail.v, A.max_sec);
-                uint32_t h = *(volatile uint32_t*)&S->sec_head.v;
-                uint32_t k = __popc(need);
-                while (h < lim) {
-                    uint32_t take = min(k, lim - h);
-                    uint32_t old = atomicCAS(&S->sec_head.v, h, h + take);
-                    if (old == h) { base = h; got = take; break; }
-                    h = old;
+        // refill: 1) the stash (LIFO)
+        int nfree = 0, rank = 0;
+#pragma unroll
+        for (int k = 0; k < TW; ++k) { const int f = (int)s_free[par][k]; if (k < w) rank += f; nfree += f; }
+        rank += __popc(__ballot_sync(0xffffffffu, !active) & lt);
+        const int hungry = s_hungry;
+        const int room = hungry ? max(0, HUNGRY_CAP - (TB - nfree)) : nfree;
+        const int take = min(min(nfree, room), stn);
+        if (!active && rank < take) { load_secondary(*SL, tid, stash[stn - 1 - rank]); active = true; }
+        stn -= take;
+        // a stash above its level, or with other blocks idle, goes to the queue
+        const int keep = hungry ? 0 : TW / 2 * (int)A.stash_keep;
+        if (stn > 0 && (hungry || (A.stash_spill && stn >= TW / 2 * (int)A.stash_spill))) {
+            const int n = stn - min(keep, stn);
+            if (tid == 0) s_spill = atomicAdd(&S->sec_qtail.v, (uint32_t)n);
+            __syncthreads();
+            for (int k = tid; k < n; k += TB) push_global(A, s_spill + k, stash[stn - n + k]);
+            stn -= n;
+        }
+        int nact = TB - nfree + take;
+        // 2) the global queue and 3) new primaries
+        const bool poll = nact == 0 || (it & A.poll_mask) == 0u;
+        const bool want = s_want != 0;
+        if (nfree > take && (poll || want)) {
+            if (tid == 0) {
+                uint32_t base = 0, got = 0, pb = 0, pg = 0;
+                const uint32_t k = (uint32_t)(nfree - take);
+                if (poll) {
+                    uint32_t lim = min(*(volatile uint32_t*)&S->sec_qtail.v, A.max_sec);
+                    uint32_t h = *(volatile uint32_t*)&S->sec_head.v;
+                    while (h < lim) {
+                        uint32_t n = min(min(k, lim - h), (uint32_t)HUNGRY_CAP);
+                        uint32_t old = atomicCAS(&S->sec_head.v, h, h + n);
+                        if (old == h) { base = h; got = n; break; }
+                        h = old;
+                    }
                 }
+                if (want && k > got) {
+                    const uint32_t n = min(min(k - got, A.prim_take * TW), (uint32_t)(quota - s_nprim));
+                    const uint32_t old = atomicAdd(&S->prim_next.v, n);
+                    if (old < A.np) { pg = min(n, A.np - old); pb = old; }
+                    if (old + n >= A.np) left = false;
+                    s_nprim += (int)pg;                          // read by this thread alone until phase C
+                }
+                s_got[0] = base; s_got[1] = got; s_got[2] = pb; s_got[3] = pg;
             }
-            base = __shfl_sync(0xffffffffu, base, 0);
-            got = __shfl_sync(0xffffffffu, got, 0);
-            uint32_t rank = __popc(need & lt);
-            if (!q.active && rank < got) {
-                const SecRec* rec = A.secq + base + rank;
+            __syncthreads();
+            const int got = (int)s_got[1], pg = (int)s_got[3], r2 = rank - take;
+            if (!active && r2 >= 0 && r2 < got) {
+                const SecRec* rec = A.secq + s_got[0] + r2;
                 unsigned long long t0 = gtime();
                 bool ok = true;
                 // bounded wait for the record's publication; once one wait has
@@ -793,62 +969,140 @@ __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
                     float4 pe = __ldcg(&rec->pe);
                     float4 dr = __ldcg(&rec->dir);
                     uint4 mt = __ldcg(&rec->meta);
-                    StashRec r{pe.x, pe.y, pe.z, pe.w, dr.x, dr.y, dr.z, mt.x, mt.y};
-                    load_secondary(q, r);
+                    load_secondary(*SL, tid, StashRec{pe.x, pe.y, pe.z, pe.w, dr.x, dr.y, dr.z, mt.x, mt.y});
+                    active = true;
                 }
+            } else if (!active && r2 >= got && r2 < got + pg) {
+                start_primary(A, *SL, tid, s_got[2] + (uint32_t)(r2 - got));
+                active = true;
             }
-            need = __ballot_sync(0xffffffffu, !q.active);
+            nact += got + pg;                                    // (records that never came count until the next refill)
         }
-        // 3) new primaries
-        if (need && poll && *(volatile uint32_t*)&S->prim_next.v < A.np) {
-            uint32_t pb = 0, pg = 0;
-            if (lane == 0) {
-                uint32_t take = min((uint32_t)__popc(need), A.prim_take);
-                uint32_t old = atomicAdd(&S->prim_next.v, take);
-                if (old < A.np) { pg = min(take, A.np - old); pb = old; }
-            }
-            pb = __shfl_sync(0xffffffffu, pb, 0);
-            pg = __shfl_sync(0xffffffffu, pg, 0);
-            uint32_t r2 = __popc(need & lt);
-            if (!q.active && r2 < pg) start_primary(A, q, pb + r2);
-        }
-        unsigned act = __ballot_sync(0xffffffffu, q.active);
-        if (act && !busy) { busy = true; if (lane == 0) atomicAdd(&S->busy.v, 1u); }
-        if (!act) {
-            // no lanes and an empty stash: idle
-            if (busy) { busy = false; if (lane == 0) atomicSub(&S->busy.v, 1u); idle_since = gtime(); }
-            int done = 0;
-            if (lane == 0) {
+        if (nact == 0) {
+            // nothing to do and an empty stash: idle
+            if (tid == 0) {
+                if (busy) { busy = false; atomicSub(&S->busy.v, 1u); idle_since = gtime(); }
                 uint32_t lim = min(*(volatile uint32_t*)&S->sec_qtail.v, A.max_sec);
-                done = *(volatile uint32_t*)&S->prim_next.v >= A.np &&
-                       *(volatile uint32_t*)&S->sec_head.v >= lim && *(volatile uint32_t*)&S->busy.v == 0u;
+                bool done = *(volatile uint32_t*)&S->prim_next.v >= A.np && *(volatile uint32_t*)&S->sec_head.v >= lim &&
+                            *(volatile uint32_t*)&S->busy.v == 0u;
+                if (idle_since == 0) idle_since = gtime();
+                if (!done && gtime() - idle_since > A.idle_ns) { atomicOr(&S->err, DERR_IDLE_WAIT); done = true; }
+                if (done) s_done = 1;
+                else { __nanosleep(sleep_ns); sleep_ns = min(sleep_ns * 2, 8192u); }
+                s_stn = 0;
+                s_want = left && s_nprim < quota;
             }
-            done = __shfl_sync(0xffffffffu, done, 0);
-            if (done) break;
-            if (idle_since == 0) idle_since = gtime();
-            if (gtime() - idle_since > A.idle_ns) { if (lane == 0) atomicOr(&S->err, DERR_IDLE_WAIT); break; }
-            __nanosleep(sleep_ns);
-            sleep_ns = min(sleep_ns * 2, 8192u);
+            __syncthreads();
             continue;
         }
-        sleep_ns = 64;
-        idle_since = 0;
-        if (q.active) lane_step(A, b, q, dep, nsteps, act);
-        __syncwarp();
-        // stash overflow went straight to the global queue; spill a full stash
-        if (lane == 0) {
-            int sn = *b.stn;
-            if (sn > STASH) sn = STASH;
-            if (A.stash_spill && sn >= (int)A.stash_spill) {
-                push_global(A, b.stash + A.stash_keep, sn - (int)A.stash_keep, 0);
-                sn = (int)A.stash_keep;
-            }
-            *b.stn = sn;
+        if (tid == 0) {
+            if (!busy) { busy = true; atomicAdd(&S->busy.v, 1u); }
+            sleep_ns = 64;
+            idle_since = 0;
         }
-        __syncwarp();
-        if (*b.sn >= STG_FLUSH) flush_staging(A, b, lane);
+        // A) move
+        b.ln = s_ln[par];
+        {
+            int k = -1;
+            const bool was = active;
+            if (nact > NREC / 4) {
+                // with secondaries waiting the run may be long, else its length is latency
+                if (active) k = move(A, b, tid, dep, nsteps, active, stn > 0 ? MOVE_STEPS : 4u);
+            } else {
+                // Few electrons, most warps idle: the draws of a run do not depend on the flight,
+                // so all threads draw the next 4, 8 or 16 steps of every electron side by
+                // side, and the electron's own thread is left with the rotations.
+                XS x;
+                const int go = active ? begin_move(A, b, tid, dep, x) : 1;
+                if (go) active = false;
+                if (go == 2) k = L_SPUR;
+                if (go == 0) {
+                    SL->xi[tid] = x.xi; SL->xic[tid] = x.xic; SL->xicv[tid] = x.xicv; SL->xicvd[tid] = x.xicvd;
+                    SL->stot[tid] = x.s_tot; SL->lam[tid] = x.lambda; SL->fE[tid] = x.fE; SL->iE[tid] = x.iE;
+                }
+                __syncwarp();
+                const int at = push_list(b, L_MOVE, go == 0, (uint32_t)tid, lane);
+                __syncthreads();
+                const int na = (int)b.ln[L_MOVE], lg = na <= NREC / 16 ? 4 : na <= NREC / 8 ? 3 : 2;
+                for (int t = tid; t < na << lg; t += TB) {
+                    const int s = b.list[L_MOVE][t >> lg];
+                    const uint32_t nd = SL->nd[s];
+                    const float4 u = draw4_nc(nd + 4u * (uint32_t)(t & ((1 << lg) - 1)), SL->sub[s], SL->pid[s], A.k0, A.k1);
+                    const Step r = draw_step(T, u, SL->lam[s], SL->iE[s], SL->fE[s], SL->stot[s], SL->xi[s], SL->xic[s],
+                                             SL->xicv[s], SL->xicvd[s]);
+                    SR->dist[t] = r.dist; SR->ce[t] = r.ce; SR->se[t] = r.se; SR->sp[t] = r.sp; SR->cp[t] = r.cp;
+                    SR->kind[t] = r.kind;
+                }
+                __syncthreads();
+                if (go == 0) {
+                    Flight f;
+                    f.load(*SL, tid, A);
+                    bool esc = false;
+                    for (int t = at << lg; t < (at + 1) << lg; ++t) {
+                        const Step r{SR->dist[t], SR->ce[t], SR->se[t], SR->sp[t], SR->cp[t], SR->kind[t]};
+                        if (f.step(r, A.box, k, esc)) break;
+                    }
+                    k = end_move(A, b, tid, dep, nsteps, f, x.t, x.meta, k, esc, active);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 3; ++q) push_list(b, q, k == q, (uint32_t)tid, lane);
+            push_list(b, L_SPUR, k == L_SPUR, (uint32_t)tid | (SPUR_THERM << 8), lane);
+            const unsigned ended = __ballot_sync(0xffffffffu, was && !active && SL->sub[tid] == 0u);
+            const unsigned fm = __ballot_sync(0xffffffffu, !active);
+            if (lane == 0) {
+                s_free[par ^ 1u][w] = (uint32_t)__popc(fm);
+                if (ended) atomicSub(&s_nprim, __popc(ended));
+            }
+        }
+        __syncthreads();
+        if (tid == 0) s_stn = stn;
+        if (tid < NLIST) s_ln[par ^ 1u][tid] = 0;                // the next iteration's
+        // B) interactions: chunks of 32 of one kind
+        {
+            const int n0 = (int)(b.ln[L_ION] + 31u) / 32, n1 = n0 + (int)(b.ln[L_EXC] + 31u) / 32;
+            const int n2 = n1 + (int)(b.ln[L_VIB] + 31u) / 32;
+            for (int c = w; c < n2; c += TW) {
+                const int kind = c < n0 ? L_ION : c < n1 ? L_EXC : L_VIB;
+                const uint32_t at = (uint32_t)(c - (kind == L_ION ? 0 : kind == L_EXC ? n0 : n1)) * 32u + lane;
+                const bool on = at < b.ln[kind];
+                const int s = on ? b.list[kind][at] : 0;
+                int sp = SPUR_NONE;
+                if (kind == L_VIB) { if (on) vibrate(A, b, s, dep); continue; }
+                if (on) sp = kind == L_ION ? ionise(A, b, s, dep) : excite(A, b, s, dep);
+                __syncwarp();
+                push_list(b, L_TRACKED, sp == SPUR_TRACKED, (uint32_t)s, lane);
+                push_list(b, L_SPUR, sp == SPUR_LOCAL || sp == SPUR_AUTO, (uint32_t)s | ((uint32_t)sp << 8), lane);
+            }
+        }
+        __syncthreads();
+        // C) spurs, the tracked ones with their secondary
+        if (tid == TB - 1) s_hungry = *(volatile uint32_t*)&S->busy.v < gridDim.x;
+        if (tid == 0) s_want = left && s_nprim < quota;
+        {
+            const uint32_t nt = b.ln[L_TRACKED], ns = b.ln[L_SPUR];
+            const int n0 = (int)(nt + 31u) / 32, n1 = n0 + (int)(ns + 31u) / 32;
+            for (int c = w; c < n1; c += TW) {
+                if (c < n0) {
+                    const uint32_t at = (uint32_t)c * 32u + lane;
+                    const bool on = at < nt;
+                    const unsigned m = __ballot_sync(0xffffffffu, on);
+                    // every emission takes a sec_buf index (counters[6]); asked for
+                    // before the spur, which hides the round trip
+                    uint32_t base = 0;
+                    if (lane == 0) base = atomicAdd(&S->sec_tail.v, (uint32_t)__popc(m));
+                    base = __shfl_sync(0xffffffffu, base, 0);
+                    if (on) spur_tracked(A, b, b.list[L_TRACKED][at], base + __popc(m & lt));
+                } else {
+                    const uint32_t at = (uint32_t)(c - n0) * 32u + lane;
+                    if (at < ns) { const uint32_t v = b.list[L_SPUR][at]; spur(A, b, (int)(v & 255u), (int)(v >> 8)); }
+                }
+            }
+        }
+        par ^= 1u;
+        __syncthreads();
     }
-    flush_staging(A, b, lane);
     for (int o = 16; o; o >>= 1) {
         dep.e += __shfl_xor_sync(0xffffffffu, dep.e, o);
         dep.n += __shfl_xor_sync(0xffffffffu, dep.n, o);
@@ -860,11 +1114,11 @@ __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
         atomicAdd(&cnt[D_DOSE], dep.n);
     }
     __syncthreads();
-    if (threadIdx.x < 24 && cnt[threadIdx.x]) {
-        uint32_t v = cnt[threadIdx.x];
-        if (threadIdx.x < 8) atomicAdd(&S->counters[threadIdx.x], v);
-        else if (threadIdx.x < 16) atomicAdd(&S->sec_stats[threadIdx.x - 8], v);
-        else atomicAdd(&S->dbg[threadIdx.x - 16], v);
+    if (tid < 24 && cnt[tid]) {
+        uint32_t v = cnt[tid];
+        if (tid < 8) atomicAdd(&S->counters[tid], v);
+        else if (tid < 16) atomicAdd(&S->sec_stats[tid - 8], v);
+        else atomicAdd(&S->dbg[tid - 16], v);
     }
 }
 
@@ -960,7 +1214,7 @@ __global__ void k_reduce(const float* results, uint32_t np, const uint32_t* dose
 
 // ------------------------------------------------------------------ host side
 size_t transport_smem_bytes() {
-    return S_TOTAL_PAD * 4 + TW * STG * 16 + TW * STG * 8 + TW * STASH * sizeof(StashRec) + 2 * TW * 4 + 24 * 4;
+    return S_TOTAL_PAD * 4 + STG * 24 + sizeof(Slots) + sizeof(StepRec) + STASH * sizeof(StashRec) + NLIST * TB * 2;
 }
 
 // resident CTAs of k_transport on `device` (the current device); the shared
