@@ -74,7 +74,8 @@ struct DevState {
     Line32 sec_qtail;              // secondaries placed in the global queue
     Line32 sec_head;               // queued secondaries taken
     Line32 prim_next;              // primaries taken
-    Line32 busy;                   // warps holding work
+    Line32 busy;                   // blocks holding work
+    Line32 idle;                   // blocks that found none
 };
 
 // One queued secondary (the Particle struct of primary.wgsl:14, with the

@@ -35,10 +35,11 @@ constexpr int STG_FLUSH = 256;     // staged rad entries written out at this lev
 constexpr int STG = STG_FLUSH + 3 * TB;   // iteration at most
 constexpr int STASH = TW * (int)TRANSPORT_STASH / 2;   // secondaries a block keeps in shared memory
 constexpr int NREC = 512;          // steps drawn ahead per iteration (few electrons)
-#ifndef WG_HUNGRY
-#define WG_HUNGRY 8
+#ifndef WG_SHARE
+#define WG_SHARE 8
 #endif
-constexpr int HUNGRY_CAP = WG_HUNGRY;     // electrons a block keeps while others have none
+constexpr int SHARE = WG_SHARE;    // secondaries a block gives away per iteration while others have no work
+constexpr int QTAKE = 64;          // and takes from the queue at a time
 
 __device__ __forceinline__ unsigned long long gtime() {
     unsigned long long t;
@@ -878,7 +879,7 @@ __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
     const int quota = (int)min((uint32_t)TB / 2, (A.np + gridDim.x - 1) / gridDim.x);
     Dep dep{0.0, 0u};
     unsigned long long nsteps = 0;
-    bool active = false, busy = false, left = true;              // busy, left: thread 0
+    bool active = false, busy = false, idle = false, left = true;    // all but active: thread 0
     uint32_t par = 0;
     unsigned sleep_ns = 64;
     unsigned long long idle_since = 0;
@@ -907,19 +908,18 @@ __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
 #pragma unroll
         for (int k = 0; k < TW; ++k) { const int f = (int)s_free[par][k]; if (k < w) rank += f; nfree += f; }
         rank += __popc(__ballot_sync(0xffffffffu, !active) & lt);
-        const int hungry = s_hungry;
-        const int room = hungry ? max(0, HUNGRY_CAP - (TB - nfree)) : nfree;
-        const int take = min(min(nfree, room), stn);
+        const int share = s_hungry && TB - nfree >= SHARE ? min(SHARE, stn) : 0;
+        const int take = min(nfree, stn - share);
         if (!active && rank < take) { load_secondary(*SL, tid, stash[stn - 1 - rank]); active = true; }
         stn -= take;
-        // a stash above its level, or with other blocks idle, goes to the queue
-        const int keep = hungry ? 0 : TW / 2 * (int)A.stash_keep;
-        if (stn > 0 && (hungry || (A.stash_spill && stn >= TW / 2 * (int)A.stash_spill))) {
-            const int n = stn - min(keep, stn);
-            if (tid == 0) s_spill = atomicAdd(&S->sec_qtail.v, (uint32_t)n);
+        // to the queue: a share for idle blocks, or a stash above its level
+        int n_out = share;
+        if (A.stash_spill && stn >= TW / 2 * (int)A.stash_spill) n_out = max(n_out, stn - TW / 2 * (int)A.stash_keep);
+        if (n_out > 0) {
+            if (tid == 0) s_spill = atomicAdd(&S->sec_qtail.v, (uint32_t)n_out);
             __syncthreads();
-            for (int k = tid; k < n; k += TB) push_global(A, s_spill + k, stash[stn - n + k]);
-            stn -= n;
+            for (int k = tid; k < n_out; k += TB) push_global(A, s_spill + k, stash[stn - n_out + k]);
+            stn -= n_out;
         }
         int nact = TB - nfree + take;
         // 2) the global queue and 3) new primaries
@@ -933,7 +933,7 @@ __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
                     uint32_t lim = min(*(volatile uint32_t*)&S->sec_qtail.v, A.max_sec);
                     uint32_t h = *(volatile uint32_t*)&S->sec_head.v;
                     while (h < lim) {
-                        uint32_t n = min(min(k, lim - h), (uint32_t)HUNGRY_CAP);
+                        uint32_t n = min(min(k, lim - h), (uint32_t)QTAKE);
                         uint32_t old = atomicCAS(&S->sec_head.v, h, h + n);
                         if (old == h) { base = h; got = n; break; }
                         h = old;
@@ -982,12 +982,13 @@ __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
             // nothing to do and an empty stash: idle
             if (tid == 0) {
                 if (busy) { busy = false; atomicSub(&S->busy.v, 1u); idle_since = gtime(); }
+                if (!idle) { idle = true; atomicAdd(&S->idle.v, 1u); }
                 uint32_t lim = min(*(volatile uint32_t*)&S->sec_qtail.v, A.max_sec);
                 bool done = *(volatile uint32_t*)&S->prim_next.v >= A.np && *(volatile uint32_t*)&S->sec_head.v >= lim &&
                             *(volatile uint32_t*)&S->busy.v == 0u;
                 if (idle_since == 0) idle_since = gtime();
                 if (!done && gtime() - idle_since > A.idle_ns) { atomicOr(&S->err, DERR_IDLE_WAIT); done = true; }
-                if (done) s_done = 1;
+                if (done) { s_done = 1; atomicSub(&S->idle.v, 1u); }
                 else { __nanosleep(sleep_ns); sleep_ns = min(sleep_ns * 2, 8192u); }
                 s_stn = 0;
                 s_want = left && s_nprim < quota;
@@ -997,6 +998,7 @@ __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
         }
         if (tid == 0) {
             if (!busy) { busy = true; atomicAdd(&S->busy.v, 1u); }
+            if (idle) { idle = false; atomicSub(&S->idle.v, 1u); }
             sleep_ns = 64;
             idle_since = 0;
         }
@@ -1078,7 +1080,7 @@ __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
         }
         __syncthreads();
         // C) spurs, the tracked ones with their secondary
-        if (tid == TB - 1) s_hungry = *(volatile uint32_t*)&S->busy.v < gridDim.x;
+        if (tid == TB - 1) s_hungry = *(volatile uint32_t*)&S->idle.v != 0u;
         if (tid == 0) s_want = left && s_nprim < quota;
         {
             const uint32_t nt = b.ln[L_TRACKED], ns = b.ln[L_SPUR];
@@ -1222,6 +1224,11 @@ size_t transport_smem_bytes() {
 int transport_blocks(int device, uint32_t ctas_per_sm) {
     static DeviceOnce attr;
     attr.run([] {
+        // all of the SM's memory as shared memory: with the split the previous
+        // kernel left, a second CTA may not fit beside the first
+        cudaError_t e = cudaFuncSetAttribute(k_transport, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                             cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return e;
         return cudaFuncSetAttribute(k_transport, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)transport_smem_bytes());
     });
