@@ -55,6 +55,8 @@ struct wgdna_ctx {
     unsigned long long* d_pid_off = nullptr;
     uint32_t* d_pid_cur = nullptr;
     unsigned long long* d_red = nullptr;  // [0] dose sum [1] n_therm [2] seg max
+    uint32_t *d_nsec = nullptr, *d_first = nullptr, *d_part = nullptr, *d_share = nullptr;   // canonical order
+    size_t part_cap = 0;
     uint32_t* d_err = nullptr;            // canonicalisation / IRT / scoring error word
     uint32_t epoch = 0;
     int tblocks = 0;
@@ -84,7 +86,7 @@ struct wgdna_ctx {
     size_t cg_cap = 0, cg_rad_cap = 0;
     cudaGraphExec_t cg_graph = nullptr;
     wg::CgGraphKey cg_key{};
-    unsigned long long last_rad_n = 0;
+    unsigned long long last_rad_n = 0, last_seg_max = 0;
     // DNA target + scoring
     wgdna_dna_info dna{};
     float *d_fy = nullptr, *d_fz = nullptr, *d_rbb0 = nullptr, *d_rbb1 = nullptr;
@@ -274,6 +276,11 @@ extern "C" int wgdna_create(const wgdna_cfg* cfg, wgdna_ctx** out) {
     if (r == WGDNA_OK) r = dalloc(&c->d_Eprim, np);
     if (r == WGDNA_OK) r = dalloc(&c->d_red, 4);
     if (r == WGDNA_OK) r = dalloc(&c->d_err, 1);
+    c->part_cap = np + (size_t)c0.max_sec < 0xffffffffull ? np + (size_t)c0.max_sec : 0xffffffffull;
+    if (r == WGDNA_OK) r = dalloc(&c->d_nsec, np);
+    if (r == WGDNA_OK) r = dalloc(&c->d_first, np + 1);
+    if (r == WGDNA_OK) r = dalloc(&c->d_part, c->part_cap);
+    if (r == WGDNA_OK) r = dalloc(&c->d_share, 592);
     if (r == WGDNA_OK) r = ensure_segments(c, (uint32_t)np);
     if (r == WGDNA_OK && cudaMemset(c->d_secq, 0, sizeof(SecRec) * (size_t)c0.max_sec) != cudaSuccess) r = WGDNA_ERR_CUDA;
     if (r == WGDNA_OK && cudaMallocHost((void**)&c->h_pin, H_PIN) != cudaSuccess) {
@@ -328,7 +335,7 @@ extern "C" void wgdna_destroy(wgdna_ctx* c) {
     wg::sg_free(c->sg);
     void* ptrs[] = {c->d_small, c->d_xcw, c->d_results, c->d_dose, c->d_rad_raw, c->d_key, c->d_rad,
                     c->d_perm, c->d_secq, c->d_st, c->d_Eprim, c->d_pid_cnt, c->d_pid_off, c->d_pid_cur,
-                    c->d_red, c->d_err, c->d_fy, c->d_fz, c->d_rbb0, c->d_rbb1, c->d_hits, c->d_alive,
+                    c->d_red, c->d_nsec, c->d_first, c->d_part, c->d_share, c->d_err, c->d_fy, c->d_fz, c->d_rbb0, c->d_rbb1, c->d_hits, c->d_alive,
                     c->sc.list, c->sc.seg, c->sc.u64,
                     c->sc.fib, c->d_px, c->d_py, c->d_pz, c->d_tb, c->d_sp, c->d_alive8, c->d_lst, c->d_lpos, c->d_evt, c->d_evab,
                     c->d_hov_t, c->d_hov_ab, c->d_track, c->d_toff, c->d_irt_cnt, c->d_pf, c->d_rec, c->d_tdel, c->d_curves, c->d_acc_tl, c->d_acc, c->d_maxpid,
@@ -363,7 +370,7 @@ static TArgs make_targs(wgdna_ctx* c, const wgdna_transport_params* p) {
     a.poll_mask = c->tune.queue_poll - 1;
     a.tab = c->tab;
     a.E_prim = p->E_per_primary ? c->d_Eprim : nullptr;
-    a.results = c->d_results; a.dose = c->d_dose; a.rad = c->d_rad_raw; a.key = c->d_key;
+    a.results = c->d_results; a.nsec = c->d_nsec; a.dose = c->d_dose; a.rad = c->d_rad_raw; a.key = c->d_key;
     a.secq = c->d_secq; a.st = c->d_st;
     return a;
 }
@@ -415,9 +422,7 @@ extern "C" int wgdna_transport(wgdna_ctx* c, const wgdna_transport_params* p, wg
     cudaStream_t s = c->stream;
     c->have_transport = false;
     size_t nv = (size_t)c->cfg.vc * c->cfg.vc * c->cfg.vc;
-    WG_CUDA_OK(cudaMemsetAsync(c->d_st, 0, sizeof(DevState), s));
-    WG_CUDA_OK(cudaMemsetAsync(c->d_dose, 0, nv * 4, s));
-    WG_CUDA_OK(cudaMemsetAsync(c->d_err, 0, 4, s));
+    WG_CUDA_OK(launch_clear(ClearArgs{c->d_dose, nv, c->d_part, c->part_cap, c->d_nsec, p->np, c->d_st, c->d_red, c->d_err}, s));
     if (p->E_per_primary)
         WG_CUDA_OK(cudaMemcpyAsync(c->d_Eprim, p->E_per_primary, (size_t)p->np * 4, cudaMemcpyHostToDevice, s));
     c->epoch++;
@@ -426,20 +431,38 @@ extern "C" int wgdna_transport(wgdna_ctx* c, const wgdna_transport_params* p, wg
     WG_CUDA_OK(cudaEventRecord(c->ev[0], s));
     WG_CUDA_OK(launch_transport(a, c->tblocks, s));
     WG_CUDA_OK(cudaEventRecord(c->ev[1], s));
-    DevState hs;
-    WG_CUDA_OK(cudaMemcpyAsync(&hs, c->d_st, sizeof hs, cudaMemcpyDeviceToHost, s));
-    WG_CUDA_OK(cudaStreamSynchronize(s));
-    unsigned long long stored = hs.rad_next.v < c->cfg.max_rad ? hs.rad_next.v : c->cfg.max_rad;
-    WG_CUDA_OK(cudaEventRecord(c->ev[2], s));
-    WG_CUDA_OK(launch_canon(c->d_key, c->d_rad_raw, stored, p->np, c->d_pid_cnt, c->d_pid_off, c->d_pid_cur,
-                            c->d_perm, c->d_rad, c->d_err, s));
+    // canonical order and sums follow without a look at the counts; what is read
+    // back lands in page-locked memory with one synchronisation
+    WG_CUDA_OK(launch_place(CanonArgs{c->d_key, c->d_rad_raw, c->d_st, c->cfg.max_rad, p->np, (uint32_t)c->part_cap, c->d_nsec,
+                                      c->d_first, c->d_part, c->d_share, c->d_pid_off, c->d_rad, c->d_red, c->d_err}, s));
     WG_CUDA_OK(launch_reduce(c->d_results, p->np, c->d_dose, (uint32_t)nv, c->d_red, s));
     WG_CUDA_OK(cudaEventRecord(c->ev[3], s));
-    unsigned long long red[2];
-    uint32_t err2 = 0;
-    WG_CUDA_OK(cudaMemcpyAsync(red, c->d_red, 16, cudaMemcpyDeviceToHost, s));
-    WG_CUDA_OK(cudaMemcpyAsync(&err2, c->d_err, 4, cudaMemcpyDeviceToHost, s));
+    constexpr size_t AT_RED = 2048, AT_ERR = AT_RED + 32;
+    static_assert(sizeof(DevState) <= AT_RED && AT_ERR + 4 <= H_PIN, "the readback's place");
+    WG_CUDA_OK(cudaMemcpyAsync(c->h_pin, c->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
+    WG_CUDA_OK(cudaMemcpyAsync(c->h_pin + AT_RED, c->d_red, 32, cudaMemcpyDeviceToHost, s));
+    WG_CUDA_OK(cudaMemcpyAsync(c->h_pin + AT_ERR, c->d_err, 4, cudaMemcpyDeviceToHost, s));
     WG_CUDA_OK(cudaStreamSynchronize(s));
+    DevState hs;
+    unsigned long long red[4];
+    uint32_t err2 = 0;
+    memcpy(&hs, c->h_pin, sizeof hs);
+    memcpy(red, c->h_pin + AT_RED, 32);
+    memcpy(&err2, c->h_pin + AT_ERR, 4);
+    unsigned long long stored = hs.rad_next.v < c->cfg.max_rad ? hs.rad_next.v : c->cfg.max_rad;
+    if (hs.rad_next.v > stored) {
+        // entries were dropped: the places are not those of the counts
+        WG_CUDA_OK(cudaMemsetAsync(c->d_err, 0, 4, s));
+        WG_CUDA_OK(launch_canon(c->d_key, c->d_rad_raw, stored, p->np, c->d_pid_cnt, c->d_pid_off, c->d_pid_cur,
+                                c->d_perm, c->d_rad, c->d_err, s));
+        WG_CUDA_OK(cudaEventRecord(c->ev[3], s));
+        WG_CUDA_OK(launch_seg_max(c->d_pid_off, p->np, c->d_red + 2, s));
+        WG_CUDA_OK(cudaMemcpyAsync(c->h_pin, c->d_red + 2, 8, cudaMemcpyDeviceToHost, s));
+        WG_CUDA_OK(cudaMemcpyAsync(c->h_pin + 8, c->d_err, 4, cudaMemcpyDeviceToHost, s));
+        WG_CUDA_OK(cudaStreamSynchronize(s));
+        memcpy(&red[2], c->h_pin, 8);
+        memcpy(&err2, c->h_pin + 8, 4);
+    }
     if (st) {
         memset(st, 0, sizeof *st);
         memcpy(st->counters, hs.counters, sizeof st->counters);
@@ -461,7 +484,7 @@ extern "C" int wgdna_transport(wgdna_ctx* c, const wgdna_transport_params* p, wg
         st->steps = hs.steps;
         st->n_therm = (uint32_t)red[1];
         st->ms_transport = elapsed_ms(c->ev[0], c->ev[1]);
-        st->ms_canon = elapsed_ms(c->ev[2], c->ev[3]);
+        st->ms_canon = elapsed_ms(c->ev[1], c->ev[3]);
         st->device_error = hs.err | err2;
     }
     if (hs.err | err2) {
@@ -473,6 +496,7 @@ extern "C" int wgdna_transport(wgdna_ctx* c, const wgdna_transport_params* p, wg
     c->last_nseg = p->np;
     c->last_pid_base = p->pid_base;
     c->last_rad_n = stored;
+    c->last_seg_max = red[2];
     c->last_E = p->E_eV;
     c->last_has_eprim = p->E_per_primary != nullptr;
     return WGDNA_OK;
@@ -552,13 +576,9 @@ static int irt_ensure(wgdna_ctx* c, uint32_t nseg, uint64_t rad_n, uint32_t cap)
 }
 
 // run the IRT over nseg segments of c->d_rad (segment offsets in c->d_pid_off)
-static int irt_run(wgdna_ctx* c, uint32_t nseg, uint32_t n_therm, double E_eV, uint64_t seed, uint64_t chem_n,
-                   wgdna_irt_result* out) {
+static int irt_run(wgdna_ctx* c, uint32_t nseg, unsigned long long maxseg, uint32_t n_therm, double E_eV, uint64_t seed,
+                   uint64_t chem_n, wgdna_irt_result* out) {
     cudaStream_t s = c->stream;
-    WG_CUDA_OK(launch_seg_max(c->d_pid_off, nseg, c->d_red + 2, s));
-    unsigned long long maxseg = 0;
-    WG_CUDA_OK(cudaMemcpyAsync(&maxseg, c->d_red + 2, 8, cudaMemcpyDeviceToHost, s));
-    WG_CUDA_OK(cudaStreamSynchronize(s));
     if (maxseg > (1ull << 24)) { wg_set_error("wgdna_irt: track of %llu entries is too large", maxseg); return WGDNA_ERR_CAPACITY; }
     uint32_t cap = (uint32_t)(2 * maxseg + 64);
     if (cap > 65535u) {
@@ -587,10 +607,13 @@ static int irt_run(wgdna_ctx* c, uint32_t nseg, uint32_t n_therm, double E_eV, u
     double tl[35];
     unsigned long long acc[16];
     uint32_t err = 0;
-    WG_CUDA_OK(cudaMemcpyAsync(tl, c->d_acc_tl, sizeof tl, cudaMemcpyDeviceToHost, s));
-    WG_CUDA_OK(cudaMemcpyAsync(acc, c->d_acc, sizeof acc, cudaMemcpyDeviceToHost, s));
-    WG_CUDA_OK(cudaMemcpyAsync(&err, c->d_err, 4, cudaMemcpyDeviceToHost, s));
+    WG_CUDA_OK(cudaMemcpyAsync(c->h_pin, c->d_acc_tl, sizeof tl, cudaMemcpyDeviceToHost, s));
+    WG_CUDA_OK(cudaMemcpyAsync(c->h_pin + sizeof tl, c->d_acc, sizeof acc, cudaMemcpyDeviceToHost, s));
+    WG_CUDA_OK(cudaMemcpyAsync(c->h_pin + sizeof tl + sizeof acc, c->d_err, 4, cudaMemcpyDeviceToHost, s));
     WG_CUDA_OK(cudaStreamSynchronize(s));
+    memcpy(tl, c->h_pin, sizeof tl);
+    memcpy(acc, c->h_pin + sizeof tl, sizeof acc);
+    memcpy(&err, c->h_pin + sizeof tl + sizeof acc, 4);
     if (out) {
         memset(out, 0, sizeof *out);
         double per100 = ((double)n_therm * E_eV) / 100;
@@ -645,7 +668,7 @@ extern "C" int wgdna_irt(wgdna_ctx* c, uint32_t n_therm, double E_eV, uint64_t s
     if (!c->have_transport) { wg_set_error("wgdna_irt: no transport result in the context"); return WGDNA_ERR_STATE; }
     WG_CUDA_OK(cudaSetDevice(c->device));
     c->irt_pid_base = c->last_pid_base;
-    return irt_run(c, c->last_nseg, n_therm, E_eV, seed, c->last_rad_n, out);
+    return irt_run(c, c->last_nseg, c->last_seg_max, n_therm, E_eV, seed, c->last_rad_n, out);
 }
 
 extern "C" int wgdna_run_irt(wgdna_ctx* c, const float* rad_buf, uint64_t rad_n, uint32_t n_therm, double E_eV,
@@ -670,12 +693,17 @@ extern "C" int wgdna_run_irt(wgdna_ctx* c, const float* rad_buf, uint64_t rad_n,
     WG_CUDA_OK(cudaMemsetAsync(c->d_err, 0, 4, s));
     WG_CUDA_OK(launch_canon(c->d_key, c->d_rad_raw, rad_n, nseg, c->d_pid_cnt, c->d_pid_off, c->d_pid_cur,
                             c->d_perm, c->d_rad, c->d_err, s));
-    uint32_t err = 0;
-    WG_CUDA_OK(cudaMemcpyAsync(&err, c->d_err, 4, cudaMemcpyDeviceToHost, s));
+    WG_CUDA_OK(launch_seg_max(c->d_pid_off, nseg, c->d_red + 2, s));
+    WG_CUDA_OK(cudaMemcpyAsync(c->h_pin, c->d_red + 2, 8, cudaMemcpyDeviceToHost, s));
+    WG_CUDA_OK(cudaMemcpyAsync(c->h_pin + 8, c->d_err, 4, cudaMemcpyDeviceToHost, s));
     WG_CUDA_OK(cudaStreamSynchronize(s));
+    unsigned long long maxseg = 0;
+    uint32_t err = 0;
+    memcpy(&maxseg, c->h_pin, 8);
+    memcpy(&err, c->h_pin + 8, 4);
     if (err) { wg_set_error("wgdna_run_irt: grouping error flags 0x%x", err); return WGDNA_ERR_DEVICE; }
     c->irt_pid_base = 0;
-    return irt_run(c, nseg, n_therm, E_eV, seed, rad_n, out);
+    return irt_run(c, nseg, maxseg, n_therm, E_eV, seed, rad_n, out);
 }
 
 // IRT per-reaction constants, irt-worker.js:191-286 (C library functions,

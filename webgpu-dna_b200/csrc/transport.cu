@@ -700,6 +700,7 @@ __device__ __forceinline__ void finish_primary(const TArgs& A, Blk& b, int s, De
     float4* r = reinterpret_cast<float4*>(A.results + 8ull * (S.pid[s] - A.pid_base));
     r[0] = make_float4(S.tpath[s], S.ppath[s], E, __uint_as_float(S.nion[s]));
     r[1] = make_float4(__uint_as_float(S.nexc[s]), __uint_as_float(esc), S.maxr[s], 0.0f);
+    A.nsec[S.pid[s] - A.pid_base] = S.nsec[s];
     atomicAdd(&b.cnt[D_IONS], S.nion[s]); atomicAdd(&b.cnt[D_EXC], S.nexc[s]);
     atomicAdd(&b.cnt[D_ESC], esc); atomicAdd(&b.cnt[D_PRIM], 1u);
 }
@@ -850,7 +851,7 @@ __device__ __forceinline__ int move(const TArgs& A, Blk& b, int s, Dep& dep, uns
 // are alive at a time, so an iteration costs little more than its longest
 // phase path, and with more electrons the issue slots bind.
 // Measured at 4096 x 10 keV: 14.9 ms with one warp per 32 electrons taking all
-// branches one after another (7.8 lanes per instruction, 16 % issue), TR_MS now.
+// branches one after another (7.8 lanes per instruction, 16 % issue), 4.5 ms now.
 __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     float* T = reinterpret_cast<float*>(smem);
@@ -1132,23 +1133,154 @@ __global__ void k_pid_hist(const unsigned long long* key, unsigned long long n, 
     for (; i < n; i += stride) atomicAdd(&cnt[(uint32_t)(key[i] >> 34)], 1u);
 }
 
-// Exclusive scan of n counts into off[0..n] with one block (chunked per thread).
-__global__ void k_scan(const uint32_t* cnt, uint32_t n, unsigned long long* off) {
-    __shared__ unsigned long long part[1024];
-    uint32_t t = threadIdx.x, per = (n + blockDim.x - 1) / blockDim.x;
-    uint32_t lo = min(t * per, n), hi = min(lo + per, n);
-    unsigned long long s = 0;
-    for (uint32_t i = lo; i < hi; ++i) s += cnt[i];
-    part[t] = s;
-    __syncthreads();
-    if (t == 0) {
-        unsigned long long acc = 0;
-        for (uint32_t i = 0; i < blockDim.x; ++i) { unsigned long long v = part[i]; part[i] = acc; acc += v; }
-        off[n] = acc;
+// Exclusive scan of n counts (+ add each) into off[0..n], one block: 4096 at a time,
+// four consecutive ones per thread (9 us for 65,536; with a run of counts per thread and
+// one thread adding the runs up, 128 us).
+template <class T>
+__device__ __forceinline__ void scan_block(const uint32_t* cnt, uint32_t n, uint32_t add, T* off) {
+    __shared__ unsigned long long wsum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned long long carry = 0;
+    for (uint32_t base = 0; base < n; base += 4096) {
+        const uint32_t i = base + 4 * threadIdx.x;
+        unsigned long long v[4], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { v[k] = i + k < n ? (unsigned long long)cnt[i + k] + add : 0ull; sum += v[k]; }
+        unsigned long long x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const unsigned long long u = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += u; }
+        __syncthreads();
+        if (lane == 31) wsum[w] = x;
+        __syncthreads();
+        unsigned long long before = carry + x - sum;
+        for (int q = 0; q < 32; ++q) { if (q < w) before += wsum[q]; carry += wsum[q]; }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (i + k < n) off[i + k] = (T)before;
+            before += v[k];
+        }
     }
+    if (threadIdx.x == 0) off[n] = (T)carry;
+}
+__global__ void __launch_bounds__(1024) k_scan(const uint32_t* cnt, uint32_t n, unsigned long long* off) {
+    scan_block(cnt, n, 0u, off);
+}
+
+// ---- canonical order without a sort.  A particle numbers its entries from 0, so an
+// entry's place is the number of entries of the particles before its own plus
+// its number: count per (primary, secondary), scan, scatter.  Needs every entry
+// stored; a run that dropped some sorts (launch_canon).
+// Measured on 5.3 M entries of 4096 x 10 keV: 910 us by per-primary bitonic
+// sorts (691 of them the sorts), 140 us now; 65,536 mixed: 7.1 -> 1.4 ms.
+
+// first particle of each primary: scan of (secondaries + 1)
+__global__ void __launch_bounds__(1024) k_particles(const uint32_t* nsec, uint32_t np, uint32_t* first) {
+    scan_block(nsec, np, 1u, first);
+}
+
+__device__ __forceinline__ unsigned long long stored_of(const CanonArgs& c) {
+    const unsigned long long n = c.st->rad_next.v;
+    return n < c.max_rad ? n : c.max_rad;
+}
+__device__ __forceinline__ uint32_t particle_of(const CanonArgs& c, unsigned long long key) {
+    return c.first[(uint32_t)(key >> 34)] + ((uint32_t)(key >> 17) & 0x1ffffu);
+}
+
+__global__ void k_count(CanonArgs c) {
+    const unsigned long long n = stored_of(c);
+    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
+         i += (unsigned long long)gridDim.x * blockDim.x) {
+        const uint32_t q = particle_of(c, c.key[i]);
+        if (q < c.cap) atomicAdd(&c.cnt[q], 1u);
+    }
+}
+
+// sums of CB equal shares of the counts, then the scan of each share from the sums before it
+constexpr int CBLK = 592, CTHR = 256;
+__global__ void __launch_bounds__(CTHR) k_share_sum(CanonArgs c) {
+    __shared__ uint32_t s[CTHR / 32];
+    const uint32_t m = min(c.first[c.np], c.cap), per = (m + CBLK - 1) / CBLK;
+    const uint32_t lo = min(blockIdx.x * per, m), hi = min(lo + per, m);
+    uint32_t v = 0;
+    for (uint32_t i = lo + threadIdx.x; i < hi; i += CTHR) v += c.cnt[i];
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
     __syncthreads();
-    s = part[t];
-    for (uint32_t i = lo; i < hi; ++i) { off[i] = s; s += cnt[i]; }
+    if (threadIdx.x == 0) {
+        uint32_t t = 0;
+        for (int k = 0; k < CTHR / 32; ++k) t += s[k];
+        c.share[blockIdx.x] = t;
+    }
+}
+__global__ void __launch_bounds__(CTHR) k_share_scan(CanonArgs c) {
+    __shared__ uint32_t s[CTHR / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t m = min(c.first[c.np], c.cap), per = (m + CBLK - 1) / CBLK;
+    const uint32_t lo = min(blockIdx.x * per, m), hi = min(lo + per, m);
+    uint32_t before = 0;
+    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += CTHR) before += c.share[k];
+    for (int o = 16; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (lane == 0) s[w] = before;
+    __syncthreads();
+    before = 0;
+    for (int k = 0; k < CTHR / 32; ++k) before += s[k];
+    for (uint32_t b = lo; b < hi; b += CTHR) {
+        const uint32_t i = b + threadIdx.x, own = i < hi ? c.cnt[i] : 0u;
+        uint32_t x = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t u = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += u; }
+        __syncthreads();
+        if (lane == 31) s[w] = x;
+        __syncthreads();
+        uint32_t at = before + x - own;
+        for (int k = 0; k < CTHR / 32; ++k) { if (k < w) at += s[k]; before += s[k]; }
+        if (i < hi) c.cnt[i] = at;                               // in place: counts become offsets
+    }
+}
+
+constexpr int SEG_MAX = 8192;
+// entries to their places; the primaries' offsets and the longest segment
+__global__ void k_place(CanonArgs c) {
+    const unsigned long long n = stored_of(c), stride = (unsigned long long)gridDim.x * blockDim.x;
+    const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+    for (unsigned long long i = t; i < n; i += stride) {
+        const unsigned long long key = c.key[i];
+        const uint32_t q = particle_of(c, key);
+        if (q >= c.cap) continue;
+        const unsigned long long at = (unsigned long long)c.cnt[q] + (key & 0x1ffffull);
+        if (at < n) c.out[at] = c.rad[i];
+    }
+    uint32_t longest = 0;
+    for (unsigned long long p = t; p <= c.np; p += stride) {
+        auto off = [&](uint32_t k) -> unsigned long long {
+            const uint32_t q = c.first[k];
+            return k == c.np || q >= c.cap ? n : c.cnt[q];
+        };
+        const unsigned long long a = off((uint32_t)p);
+        c.off[p] = a;
+        if (p < c.np) longest = max(longest, (uint32_t)(off((uint32_t)p + 1) - a));
+    }
+    for (int o = 16; o; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+    if ((threadIdx.x & 31) == 0 && longest) {
+        atomicMax(&c.red[2], (unsigned long long)longest);
+        if (longest > (uint32_t)SEG_MAX) atomicOr(c.err, DERR_SEG_SORT);
+    }
+}
+
+// everything a transport starts from at zero, in one launch
+__global__ void k_clear(ClearArgs c) {
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    uint4* d = reinterpret_cast<uint4*>(c.dose);
+    for (size_t i = t; i < c.nvox / 4; i += stride) d[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (size_t i = c.nvox / 4 * 4 + t; i < c.nvox; i += stride) c.dose[i] = 0u;
+    uint4* q = reinterpret_cast<uint4*>(c.cnt);
+    for (size_t i = t; i < c.cap / 4; i += stride) q[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (size_t i = c.cap / 4 * 4 + t; i < c.cap; i += stride) c.cnt[i] = 0u;
+    for (size_t i = t; i < c.np; i += stride) c.nsec[i] = 0u;
+    uint32_t* st = reinterpret_cast<uint32_t*>(c.st);
+    for (size_t i = t; i < sizeof(DevState) / 4; i += stride) st[i] = 0u;
+    if (t < 4) c.red[t] = 0ull;
+    if (t == 4) *c.err = 0u;
 }
 
 __global__ void k_scatter(const unsigned long long* key, unsigned long long n, const unsigned long long* off,
@@ -1160,8 +1292,6 @@ __global__ void k_scatter(const unsigned long long* key, unsigned long long n, c
         perm[off[p] + atomicAdd(&cur[p], 1u)] = (uint32_t)i;
     }
 }
-
-constexpr int SEG_MAX = 8192;
 
 // One block per primary: sort its entries by key (bitonic, shared memory) and
 // write them to the canonical buffer.
@@ -1205,7 +1335,12 @@ __global__ void k_reduce(const float* results, uint32_t np, const uint32_t* dose
     unsigned long long sd = 0;
     uint32_t nt = 0;
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-    for (uint32_t v = i; v < nvox; v += stride) sd += dose[v];
+    const uint4* d4 = reinterpret_cast<const uint4*>(dose);
+    for (uint32_t v = i; v < nvox / 4; v += stride) {
+        const uint4 q = d4[v];
+        sd += (unsigned long long)q.x + q.y + q.z + q.w;
+    }
+    for (uint32_t v = nvox / 4 * 4 + i; v < nvox; v += stride) sd += dose[v];
     for (uint32_t v = i; v < np; v += stride) nt += (__float_as_uint(results[8ull * v + 5]) == 0u);
     for (int o = 16; o; o >>= 1) {
         sd += __shfl_xor_sync(0xffffffffu, sd, o);
@@ -1272,8 +1407,21 @@ cudaError_t launch_scan_u32(const uint32_t* cnt, uint32_t n, unsigned long long*
 
 cudaError_t launch_reduce(const float* results, uint32_t np, const uint32_t* dose, uint32_t nvox,
                           unsigned long long* out, cudaStream_t s) {
-    { cudaError_t me_ = cudaMemsetAsync(out, 0, 16, s); if (me_ != cudaSuccess) return me_; }
     k_reduce<<<592, 256, 0, s>>>(results, np, dose, nvox, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_clear(const ClearArgs& c, cudaStream_t s) {
+    k_clear<<<592, 256, 0, s>>>(c);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_place(const CanonArgs& c, cudaStream_t s) {
+    k_particles<<<1, 1024, 0, s>>>(c.nsec, c.np, c.first);
+    k_count<<<1184, 256, 0, s>>>(c);
+    k_share_sum<<<CBLK, CTHR, 0, s>>>(c);
+    k_share_scan<<<CBLK, CTHR, 0, s>>>(c);
+    k_place<<<1184, 256, 0, s>>>(c);
     return cudaGetLastError();
 }
 
