@@ -103,7 +103,7 @@ struct wgdna_ctx {
     float4* d_pf = nullptr;
     float4* d_rec = nullptr;
     float* d_tdel = nullptr;
-    uint32_t irt_tracks = 0, irt_hcap = 0;
+    uint32_t irt_tracks = 0, irt_hcap = 0, irt_pcap = 0;
     double *d_px = nullptr, *d_py = nullptr, *d_pz = nullptr, *d_tb = nullptr;
     int8_t* d_sp = nullptr;
     uint8_t* d_alive8 = nullptr;
@@ -390,7 +390,7 @@ static IArgs make_iargs(wgdna_ctx* c, uint32_t nseg, uint64_t seed) {
     a.order = c->d_track + 10 * T;
     a.toff = c->d_toff;
     a.pf = c->d_pf; a.rec = c->d_rec; a.tdel = c->d_tdel;
-    a.hov_t = c->d_hov_t; a.hov_ab = c->d_hov_ab; a.hcap = c->irt_hcap;
+    a.hov_t = c->d_hov_t; a.hov_ab = c->d_hov_ab; a.hcap = c->irt_hcap; a.pcap = c->irt_pcap;
     a.counters = c->d_irt_cnt;
     a.acc_tl = c->d_acc_tl; a.acc = c->d_acc; a.err = c->d_err;
     return a;
@@ -528,14 +528,16 @@ extern "C" int wgdna_run_transport(wgdna_ctx* c, const wgdna_transport_params* p
 static void irt_constants(IrtConst* C);
 
 // Per-track particle slots 2*len + 64 and event slots 16*len + 2048 (the
-// kernels' tbase / ebase), per-warp heap overflow hcap = 8*cap + 4096 with
-// cap = 2*maxlen + 64 the largest track's particle slots.
+// kernels' tbase / ebase), per track in flight heap overflow hcap = 8*pcap + 4352
+// and pcap partners, pcap at least the largest track's particle slots
+// 2*maxlen + 64.
 static int irt_ensure(wgdna_ctx* c, uint32_t nseg, uint64_t rad_n, uint32_t cap) {
     size_t slots = 2 * (size_t)rad_n + 64 * (size_t)nseg;
     size_t evslots = 16 * (size_t)rad_n + 2048 * (size_t)nseg;
-    uint32_t hcap = cap * 8u + 4096u;
+    // (rounded up, so that tracks of about the same size keep the captured launch sequence)
+    const uint32_t pcap = (cap + 1023u) & ~1023u, hcap = pcap * 8u + 4352u;
     const IrtShape shape{c->tune.irt_init_blocks_per_sm, c->tune.irt_loop_blocks_per_sm};
-    size_t hov = (size_t)irt_warps(c->device, shape) * hcap;
+    size_t hov = (size_t)irt_warps(c->device, shape, nseg) * (hcap + (size_t)pcap);
     if (slots > c->irt_slots) {
         TRY(dalloc(&c->d_px, slots)); TRY(dalloc(&c->d_py, slots)); TRY(dalloc(&c->d_pz, slots));
         TRY(dalloc(&c->d_tb, slots)); TRY(dalloc(&c->d_sp, slots)); TRY(dalloc(&c->d_alive8, slots));
@@ -550,7 +552,8 @@ static int irt_ensure(wgdna_ctx* c, uint32_t nseg, uint64_t rad_n, uint32_t cap)
         TRY(dalloc(&c->d_hov_t, hov)); TRY(dalloc(&c->d_hov_ab, hov));
         c->irt_hov = hov;
     }
-    c->irt_hcap = (uint32_t)(hov / irt_warps(c->device, shape));
+    c->irt_hcap = hcap;
+    c->irt_pcap = pcap;
     if (slots > c->irt_pf_slots) {
         TRY(dalloc(&c->d_pf, slots));
         TRY(dalloc(&c->d_rec, 6 * slots));

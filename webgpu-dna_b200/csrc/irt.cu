@@ -4,8 +4,8 @@
 // reaction tables :191-286, sampleIRT :116-184 with SamplePDC :91-113, erfcinv
 // :31-39, erfcx :53-88, the per-primary event loop :470-667 and pairWithAlive
 // :430-465).  The reference runs the primaries one after another on one CPU
-// thread; here one warp owns one track (primary) at a time and the warps of a
-// persistent grid pull tracks from a counter:
+// thread; here a warp, or several where there are few tracks, owns one track (primary)
+// at a time and the warps of a persistent grid pull tracks from a counter:
 //
 // * load: entries of the track (codes 4/7 skipped, 7 counted as initial H2)
 //   are displaced in f64 with the thermalisation Gaussians, 32 at a time;
@@ -14,9 +14,9 @@
 //   four consecutive partners;
 // * sort: the initial events of a track in (t, i, j) order, one block per
 //   track, in shared memory;
-// * events: the sorted initial events merged with a binary heap of product
-//   events ordered by (t, i, j), kept by lane 0; the product re-pairing
-//   (pairWithAlive) is spread over the 32 lanes.
+// * events: the sorted initial events merged with a heap of product events
+//   ordered by (t, i, j); the product re-pairing (pairWithAlive) is spread over
+//   the lanes of the track's warps.
 //
 // Random draws are keyed by what they are for (track, particle, pair), so the
 // result does not depend on scheduling; the CPU oracle uses the same streams:
@@ -28,6 +28,8 @@
 //                                  Box-Muller angles.
 #include <cstring>
 
+#include <algorithm>
+
 #include "irt.cuh"
 #include "dmath.cuh"
 
@@ -37,6 +39,7 @@ namespace wg {
 __constant__ IrtConst c_irt;
 
 
+constexpr uint32_t FULL = 0xffffffffu;
 constexpr int IB = 128;                  // threads per block (4 warps)
 
 __device__ __forceinline__ double erfcinv_(double x) {                       // :31-39
@@ -58,15 +61,19 @@ __constant__ double c_erfcx[28] = {
     3.13092e-13, -1.12708e-13, 3.81e-16, 7.106e-15,
     -1.523e-15, -9.4e-17, 1.21e-16, -2.8e-17};
 
-__device__ double erfcx_pos(double x) {                                      // :53-88, x >= 0
+// (out of line and rolled: the undecided trials that need it are rare, and the kernels'
+// instructions have to stay in the SM's cache)
+__device__ __noinline__ double erfcx_pos(double x) {                                      // :53-88, x >= 0
     if (x >= 6) {
         double f = 0;
+#pragma unroll 1
         for (int n = 30; n >= 1; --n) f = (0.5 * n) / (x + f);
         return 0.5641895835477563 / (x + f);
     }
     double t = 2.0 / (2.0 + x);
     double ty = 4 * t - 2;
     double d = 0, dd = 0;
+#pragma unroll 1
     for (int j = 27; j > 0; --j) { double tmp = d; d = ty * d - dd + c_erfcx[j]; dd = tmp; }
     return t * exp_(0.5 * (c_erfcx[0] + ty * d) - dd);
 }
@@ -179,6 +186,7 @@ __device__ __forceinline__ uint64_t pdc_find(int src, uint32_t i, uint32_t j, ui
     const float bbf = __shfl_sync(0xffffffffu, P.bbf, src), af = __shfl_sync(0xffffffffu, P.af, src);
     const float bf = __shfl_sync(0xffffffffu, P.bf, src);
     const float hpq = 0.5f * pqf, qpq = __fdividef(0.5f * pqf, Mf);
+#pragma unroll 1
     for (uint32_t t0 = 0; t0 < 10000; t0 += 32) {
         const uint32_t trial = t0 + lane;
         const u4 w = philox_pdc(qi, qj, pid, 4u | (trial << 4));
@@ -262,13 +270,6 @@ __device__ __forceinline__ uint64_t pdc_find(int src, uint32_t i, uint32_t j, ui
     return ~0ull;
 }
 
-// the event kernel's copy, out of line (its two call sites in one place)
-__device__ __noinline__ uint64_t pdc_find_nc(int src, uint32_t i, uint32_t j, uint32_t pid, uint32_t k0, uint32_t k1,
-                                             const PdcPair P, double a, double b, int lane) {
-    return pdc_find(src, i, j, pid, P, a, b, lane,
-                    [k0, k1](uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) { return philox(c0, c1, c2, c3, k0, k1); });
-}
-
 // sampleIRT (:116-184) with the acceptance draw U supplied.  Returns the
 // reaction time t >= 0, -1 for no reaction, or -2 when SamplePDC must be run
 // with (*pa, *pb); the caller then uses X / D for X > 0.
@@ -315,8 +316,11 @@ __device__ __forceinline__ double r_acc(const IrtConst& C, int ri, double U) {
     return R * (1.0 + 1e-6) + 1e-6;
 }
 
-// event heap on (t, packed a<<16|b); nodes [0, HS) in shared memory, the rest in global memory
-constexpr uint32_t HS = 512;
+// Event heap on (t, packed a<<16|b): 32 children to a node, so that a warp takes a level
+// in one load and a vote.  Nodes [0, HS) in shared memory, the rest in global memory.
+// A binary heap of one lane took 3100 cycles per pop on a track with 2500 product events
+// (9 levels, the lower ones in L2); this one 1400.
+template <int HS>
 struct Heap {
     double* st; uint32_t* sab; double* gt; uint32_t* gab;
     __device__ __forceinline__ double t(uint32_t k) const { return k < HS ? st[k] : gt[k - HS]; }
@@ -328,43 +332,58 @@ struct Heap {
 __device__ __forceinline__ bool ev_less(double t1, uint32_t x, double t2, uint32_t y) {
     return t1 != t2 ? t1 < t2 : x < y;
 }
-__device__ void heap_push(const Heap& H, uint32_t& n, double t, uint32_t ab) {
-    uint32_t c = n++;
+// node c, the last one, moves up to its place
+template <int HS>
+__device__ __forceinline__ void heap_up(const Heap<HS>& H, uint32_t c) {
+    if (c == 0) return;
+    const double t = H.t(c);
+    const uint32_t ab = H.ab(c);
+#pragma unroll 1
     while (c > 0) {
-        uint32_t p = (c - 1) >> 1;
-        double tp = H.t(p);
-        uint32_t ap = H.ab(p);
+        const uint32_t p = (c - 1) >> 5;
+        const double tp = H.t(p);
+        const uint32_t ap = H.ab(p);
         if (!ev_less(t, ab, tp, ap)) break;
         H.set(c, tp, ap);
         c = p;
     }
     H.set(c, t, ab);
 }
-__device__ void heap_pop(const Heap& H, uint32_t& n) {
+// by the whole warp; times are not negative, so their bit patterns are in order
+template <int HS>
+__device__ __forceinline__ void heap_pop(const Heap<HS>& H, uint32_t& n, int lane) {
     n--;
     if (n == 0) return;
-    double tp = H.t(n);
-    uint32_t ap = H.ab(n);
+    const double tp = H.t(n);
+    const uint32_t ap = H.ab(n);
     uint32_t p = 0;
+#pragma unroll 1
     for (;;) {
-        uint32_t l = 2 * p + 1;
-        if (l >= n) break;
-        uint32_t s = l;
-        double ts = H.t(l);
-        uint32_t as = H.ab(l);
-        if (l + 1 < n) {
-            double tr = H.t(l + 1);
-            uint32_t ar = H.ab(l + 1);
-            if (ev_less(tr, ar, ts, as)) { s = l + 1; ts = tr; as = ar; }
+        const uint32_t c = 32 * p + 1 + lane;
+        if (32 * p + 1 >= n) break;
+        const bool in = c < n;
+        const double tc = in ? H.t(c) : 0.0;
+        const uint32_t ac = in ? H.ab(c) : 0u;
+        const uint32_t hi = in ? (uint32_t)__double2hiint(tc) : 0xffffffffu, lo = (uint32_t)__double2loint(tc);
+        unsigned m = __ballot_sync(FULL, hi == __reduce_min_sync(FULL, hi));
+        if (m & (m - 1)) {                               // equal upper words: the lower ones, then a and b
+            const bool s1 = m >> lane & 1;
+            const uint32_t l1 = __reduce_min_sync(FULL, s1 ? lo : 0xffffffffu);
+            const bool s2 = s1 && lo == l1;
+            const uint32_t a1 = __reduce_min_sync(FULL, s2 ? ac : 0xffffffffu);
+            m = __ballot_sync(FULL, s2 && ac == a1);
         }
-        if (!ev_less(ts, as, tp, ap)) break;
-        H.set(p, ts, as);
-        p = s;
+        const int w = __ffs(m) - 1;
+        const double tm = __shfl_sync(FULL, tc, w);
+        const uint32_t am = __shfl_sync(FULL, ac, w);
+        if (!ev_less(tm, am, tp, ap)) break;
+        if (lane == 0) H.set(p, tm, am);
+        p = 32 * p + 1 + w;
     }
-    H.set(p, tp, ap);
+    if (lane == 0) H.set(p, tp, ap);
+    __syncwarp();
 }
 
-constexpr uint32_t FULL = 0xffffffffu;
 // checkpoint times of the reference timeline (:566-580), ns
 __constant__ double c_cp[7] = {0.001, 0.01, 0.1, 1, 10, 100, 1000};
 
@@ -526,10 +545,10 @@ __device__ __forceinline__ u4 philox_accept(uint32_t blk, uint32_t i, uint32_t p
 //    arithmetic.  Each lane keeps its candidates in its own column of shared memory
 //    (no vote per pair); a full column makes the warp pack all columns and
 //    evaluate them exactly in f64, 32 at a time, one per lane.
-//    Measured at 4096 x 10 keV: 10.5 ms; 14.9 ms with tiles in index order, one
+//    Measured at 4096 x 10 keV: 9.5 ms; 10.5 ms with the rare f64 erfcx inline (the
+//    instruction cache, as in the event kernel), 14.9 ms with tiles in index order, one
 //    table gather per pair and queue votes per partner (5, 6, 7 blocks per SM:
 //    10.8, 10.5, 10.5 ms).
-constexpr int IQ = 64;                   // partner queue per warp of the event kernel
 constexpr int QCAP = 16;                 // candidates per lane
 constexpr float FAR = 1e18f;             // shadow coordinate of a partner that cannot react
 
@@ -763,108 +782,6 @@ __global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(const __grid_cons
     if (lane == 0 && n_pairs) atomicAdd(&A.acc[10], n_pairs);
 }
 
-__device__ __forceinline__ u4 philox_pair(uint32_t id, uint32_t jj, uint32_t pid, uint32_t k0, uint32_t k1) {
-    return philox(id, jj, pid, 5u, k0, k1);
-}
-__device__ __forceinline__ u4 philox_pair_ang(uint32_t id, uint32_t jj, uint32_t pid, uint32_t k0, uint32_t k1) {
-    return philox(id, jj, pid, 5u | (1u << 4), k0, k1);
-}
-
-__device__ __noinline__ double gauss_axis(uint32_t wa, uint32_t wb) {
-    return sqrt(-2 * log_(u01d32(wa) + 1e-30)) * cos_(6.2831853 * u01d32(wb));
-}
-
-// the product being re-paired (uniform over the warp); its position and
-// birth time are read back from its slot when a batch needs them
-struct ProdCtx {
-    const double *px, *py, *pz, *tb;
-    double Di;
-    uint32_t id, pid, k0, k1;
-};
-
-// Exact pairWithAlive step (:430-465) for queued partners [0, cnt), one per
-// lane: Brownian sync of the partner by sqrt(2 D_j dt) (skipped when the
-// Box-Muller radius bound shows it cannot come within r_acc), R_CUT, then
-// sampleIRT; accepted events go to the warp's heap.  Returns true when the
-// heap overflowed.
-__device__ __forceinline__ bool prod_batch(const IrtConst& C, const ProdCtx& P, const uint32_t* pq, int cnt, int lane,
-                                        const Heap& H, uint32_t& hn, uint32_t hcap) {
-    bool acc = false, pdcq = false, over = false;
-    double ta = 0, pa = 1, pb = 1, pD = 1;
-    uint32_t jj = 0;
-    const double pnx = P.px[P.id], pny = P.py[P.id], pnz = P.pz[P.id], pet = P.tb[P.id];
-    if (lane < cnt) {
-        const uint32_t e = pq[lane];
-        jj = e & 0xffffu;
-        const int r2i = (int)((e >> 16) & 15u), s2 = (int)(e >> 20);
-        const double Dj = C.D[s2];
-        const double dt = pet - P.tb[jj];
-        double xj = P.px[jj], yj = P.py[jj], zj = P.pz[jj];
-        const u4 q0 = philox(P.id, jj, P.pid, 5u, P.k0, P.k1);
-        const double U = u01d32(q0.w);
-        const double R = r_acc(C, r2i, U);
-        bool need = true;
-        if (dt > 0) {
-            double sig = sqrt(2.0 * Dj * dt);
-            // |gaussian 3-vector| <= sqrt(sum -2 ln u1_k) (Box-Muller radius), with margin
-            float l0 = -2.0f * __logf(u01f32(q0.x));
-            float l1 = -2.0f * __logf(u01f32(q0.y));
-            float l2 = -2.0f * __logf(u01f32(q0.z));
-            double B = (double)sqrtf((l0 + l1 + l2) * 1.0001f) + 1e-4;
-            double ex = pnx - xj, ey = pny - yj, ez = pnz - zj;
-            double dist = sqrt(ex * ex + ey * ey + ez * ez);
-            if (dist - sig * B > R) need = false;
-            if (need) {
-                u4 q1 = philox(P.id, jj, P.pid, 5u | (1u << 4), P.k0, P.k1);
-                double g0 = gauss_axis(q0.x, q1.x);
-                double g1 = gauss_axis(q0.y, q1.y);
-                double g2 = gauss_axis(q0.z, q1.z);
-                xj += g0 * sig; yj += g1 * sig; zj += g2 * sig;
-            }
-        }
-        if (need) {
-            double dx = pnx - xj, dy = pny - yj, dz = pnz - zj;
-            double r2 = dx * dx + dy * dy + dz * dz;
-            if (r2 <= C.r_cut2) {
-                double D = P.Di + Dj;
-                double t = sample_pre(C, sqrt(r2), r2i, D, U, &pa, &pb);
-                if (t == -2.0) { pdcq = true; pD = D; }
-                else if (t >= 0) { ta = pet + t; acc = ta < 1000; }
-            }
-        }
-    }
-    unsigned pm = __ballot_sync(FULL, pdcq);
-    if (pm) {
-        const PdcPair PP = pdc_pair(pa, pb);
-        uint64_t words = ~0ull;
-        while (pm) {
-            const int src = __ffs(pm) - 1;
-            pm &= pm - 1;
-            const uint64_t wd = pdc_find_nc(src, P.id, jj, P.pid, P.k0, P.k1, PP, pa, pb, lane);
-            if (lane == src) words = wd;
-        }
-        if (pdcq && words != ~0ull) {
-            const double X = pdc_x(pa, pb, PP.pq, PP.M, (uint32_t)(words >> 32), (uint32_t)words);
-            if (X > 0) { ta = pet + X / pD; acc = ta < 1000; }
-        }
-    }
-    unsigned m = __ballot_sync(FULL, acc);
-    while (m) {
-        int src = __ffs(m) - 1;
-        m &= m - 1;
-        double tt = __shfl_sync(FULL, ta, src);
-        uint32_t pj = __shfl_sync(FULL, jj, src);
-        if (lane == 0) {
-            if (hn < HS + hcap) {
-                uint32_t a = pj < P.id ? pj : P.id, bq = pj < P.id ? P.id : pj;
-                heap_push(H, hn, tt, (a << 16) | bq);
-            } else over = true;
-        }
-    }
-    hn = __shfl_sync(FULL, hn, 0);
-    return __any_sync(FULL, over);
-}
-
 // 3) the initial events of each track in (t, i, j) order (:566): a block-wide
 //     bitonic sort, in shared memory up to SORT_SM events (padded to a power
 //     of two), in the track's own event slots beyond that (they hold 2 ecap).
@@ -907,287 +824,548 @@ __global__ void __launch_bounds__(SB) k_irt_sort(IArgs A) {
     }
 }
 
-// 4) events (:566-660): pop the sorted initial events in (t, i, j) order
-//    merged with a heap of product events; one warp per track
-#ifndef WG_LOOP_MINB
-#define WG_LOOP_MINB 4
-#endif
-__global__ void __launch_bounds__(IB, WG_LOOP_MINB) k_irt_loop(IArgs A) {
-    __shared__ double s_tl[IB / 32][35];
-    __shared__ double s_ht[IB / 32][HS];
-    __shared__ uint32_t s_hab[IB / 32][HS];
-    __shared__ int s_lc[IB / 32][6];
-    __shared__ uint32_t s_pq[IB / 32][IQ];
+__device__ __forceinline__ double gauss_axis(uint32_t wa, uint32_t wb) {
+    return sqrt(-2 * log_(u01d32(wa) + 1e-30)) * cos_(6.2831853 * u01d32(wb));
+}
+__device__ __forceinline__ float sqrt_fast(float x) {                // 2^-22 relative; 0 below 2^-126
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float log2_fast(float x) {                // 2^-22 absolute in [1/2, 2], relative outside
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+template <int B>
+__device__ __forceinline__ void cp_async(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "n"(B)
+                 : "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_wait() {                          // this lane's copies but the last N, seen by the warp
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+    __syncwarp();
+}
+
+// 4) events (:566-660): pop the sorted initial events in (t, i, j) order merged
+//    with a heap of product events; W warps per track.  The first warp pops
+//    (stale events and reactions without products change nothing the others work on);
+//    a product is re-paired with the alive partners of the species that react
+//    with it (pairWithAlive, :430-465) in three steps over all lanes of the W warps:
+//    an f32 scan that lists the partners it cannot rule out, their exact f64
+//    evaluation, and the accepted events' way into the heap.
+//
+// What bounds it: with few tracks, a track's chain of events, one after another, so W
+// grows as the tracks get fewer (loop_width).  With many, fetching instructions: the
+// kernel's code is far larger than the SM's instruction cache and the warps are at
+// different places in it (a third of the fetches missed; at 16 warps per SM 5.6 of 11.5
+// cycles between a warp's instructions were that, and 28 warps were no faster).  So
+// the rare f64 paths are out of line and rolled, one copy of the scan serves all species,
+// and at W = 1 the four tracks of a block go from one re-pairing to the next together.
+// The rest keeps work off the chain:
+// * initial events come in windows of 32, copied to shared memory ahead; a window's events
+//   whose species are dead are dropped at once, and a reaction drops those of its two;
+// * kind and life of each species are in shared memory (state), 4 bits each;
+// * the scan's first test bounds the partner's displacement from the product of its
+//   three radius draws (one logarithm); the second runs on full warps of what is left;
+// * in the exact step the three axes of a partner's Gaussian (the longest f64
+//   chains) run on three lanes;
+// * accepted events are written behind the heap's last node by all lanes.
+// Measured (ms, before and after): 4096 tracks of 10 keV 20.0 -> 14.6, 64 of them 6.7 ->
+// 2.7, 4096 of 1 keV 2.2 -> 1.65, one track of 3060 species 17.5 -> 6.2.  Before: one
+// warp per track, events popped by one lane against states in global memory, a binary heap,
+// batches of 64 listed partners.
+constexpr int WN = 4;                    // windows of initial events in shared memory
+constexpr int CQ = 128;                  // listed partners in shared memory, the rest in global
+// heap nodes and species whose state is in shared memory
+template <int W>
+constexpr int HS = W >= 4 ? 1024 : 256 * W;
+template <int W>
+constexpr uint32_t SN = W >= 8 ? 16640 : 4096 * W;
+template <int W>
+struct EvGroup {
+    double tl[35], ht[HS<W>], wt[WN][32], et;
+    unsigned long long cnt[12];          // reactions 0..8, reacted, events, initial events
+    uint32_t hab[HS<W>], cq[CQ], wab[WN][32], eab, track, ncand, nacc, hn;
+    int lc[6], have, si, sj, ri;
+    uint32_t state[SN<W> / 8];           // 4 bits per species: kind, and 8 while it is alive
+    uint32_t nq[W][64];                  // per warp: partners the first test leaves (place in the list | reaction | species)
+    uint8_t src[W][32];                  // per warp: lanes that need a Gaussian
+    uint8_t wsp[32];                     // kinds of a window's species
+};
+
+// The scan's f32 tests of a partner (list record q): false only if the exact step
+// would reject it.
+struct ScanP {
+    float x, y, z, del, et, dtm, rcut;   // the product's shadow and birth time
+    uint32_t id, pid;
+};
+// First without draws: the displacement is at most the largest Box-Muller radius of
+// 32-bit draws (sqrt(3 * 2 ln 2^33) = 11.72) times sqrt(2 D dt), and a partner beyond
+// R_CUT after it is rejected by the exact path too (a quarter of them, 10 keV).  Then
+// with the radius of the three draws, against R of the acceptance draw: one in 18 is
+// left.  dth: upper bound of dt = et - t_birth from the f32 birth time (error < dtm).
+__device__ __forceinline__ bool scan_near(const ScanP& P, const float4& q, uint32_t jj, float Djf2, float fs, float fsc,
+                                          float fadd, const uint32_t* rk) {
+    const float ex = P.x - q.x, ey = P.y - q.y, ez = P.z - q.z;
+    const float dlo = (sqrt_fast(fmaf(ez, ez, fmaf(ey, ey, ex * ex))) - P.del) * 0.999997f;
+    const float dth = fmaxf(P.et - q.w + P.dtm, 0.0f);
+    const float sg = sqrt_fast(Djf2 * dth) * 1.00001f;
+    if (dlo - sg * 11.8f > P.rcut) return false;
+    const u4 q0 = philox_rk(P.id, jj, P.pid, 5u, rk);
+    // -2 ln u summed over the axes is -2 ln of the product (>= 2^-99; the sum to 1.4e-6
+    // absolute, so its root to 2e-3)
+    const float u0 = u01f32(q0.x), u1 = u01f32(q0.y), u2 = u01f32(q0.z);
+    const float Bm = sqrt_fast(fmaxf(-1.3864330f * log2_fast(u0 * u1 * u2), 0.0f)) + 2e-3f;
+    // beyond R = max(fs, fsc / U) + fadd of r_acc, for U >= uf, times 1.00002 plus 1e-6
+    const float uf = __uint2float_rd(q0.w) * 2.3283064365386963e-10f;
+    const float d = fmaf(-sg, Bm, dlo) * 0.99998f - fadd - 1e-6f;
+    return !(d > fs && d * uf > fsc);
+}
+// Second: the partner displaced by the same draws in f32.
+__device__ __forceinline__ bool scan_maybe(const ScanP& P, const float4& q, uint32_t jj, float Djf2, float fs, float fsc,
+                                           float fadd, const uint32_t* rk) {
+    const float ex = P.x - q.x, ey = P.y - q.y, ez = P.z - q.z;
+    const float dth = P.et - q.w + P.dtm;
+    const float sg = dth > 0.0f ? sqrt_fast(Djf2 * dth) * 1.00001f : 0.0f;
+    const u4 q0 = philox_rk(P.id, jj, P.pid, 5u, rk), q1 = philox_rk(P.id, jj, P.pid, 5u | (1u << 4), rk);
+    const float uf = __uint2float_rd(q0.w) * 2.3283064365386963e-10f;
+    const float rhi = (fmaxf(fs, __fdividef(fsc, uf)) + fadd) * 1.00002f + 1e-6f;
+    // per axis |g_f - g| <= 2e-3 + 2e-5 |g| (sqrt of the log near 0, fast log and cos, 2
+    // ulp each), sigma within [sl, sg]
+    const float dtl = fmaxf(P.et - q.w - P.dtm, 0.0f);
+    const float sl = sqrt_fast(Djf2 * dtl) * 0.99999f, sm = 0.5f * (sg + sl);
+    const float r0 = fmaxf(-2.0f * __logf(u01f32(q0.x)), 0.0f), r1 = fmaxf(-2.0f * __logf(u01f32(q0.y)), 0.0f),
+                r2 = fmaxf(-2.0f * __logf(u01f32(q0.z)), 0.0f);
+    const float Bm = sqrt_fast(r0 + r1 + r2) * 1.0001f + 2e-3f;
+    // cos(2 pi u) = -cos(2 pi (u - 1/2)): the argument stays in [-pi, pi]
+    const float g0 = -sqrt_fast(r0) * __cosf(6.2831853f * (u01f32(q1.x) - 0.5f));
+    const float g1 = -sqrt_fast(r1) * __cosf(6.2831853f * (u01f32(q1.y) - 0.5f));
+    const float g2 = -sqrt_fast(r2) * __cosf(6.2831853f * (u01f32(q1.z) - 0.5f));
+    const float fx = ex - g0 * sm, fy = ey - g1 * sm, fz = ez - g2 * sm;
+    const float d2 = sqrt_fast(fmaf(fz, fz, fmaf(fy, fy, fx * fx)));
+    const float eg = 2e-3f + 2e-5f * Bm;
+    const float err = 1.7320508f * (sg * eg + 0.5f * (Bm + eg) * (sg - sl)) + P.del;
+    return !(dth > 0.0f) || !((d2 - err) * 0.99999f > rhi);
+}
+
+// Exact pairWithAlive step (:430-465) for listed partners, at most one per lane (e; on:
+// this lane has one): Brownian sync of the partner by sqrt(2 D_j dt), R_CUT, then
+// sampleIRT.  Returns whether the pair reacts, at *ta.
+__device__ __forceinline__ bool pair_exact(const IArgs& A, const IrtConst& C, unsigned long long tb0, uint32_t id, uint32_t pid,
+                                double Di, uint32_t e, bool on, int lane, uint8_t* src, double* ta) {
+    const uint32_t* rk = A.rk;
+    bool acc = false, pdcq = false, gs = false;
+    double pa = 1, pb = 1, pD = 1, sig = 0, xj = 0, yj = 0, zj = 0, Dj = 0;
+    const double pet = A.tb[tb0 + id];
+    const uint32_t jj = e & 0xffffu;
+    const int r2i = (int)((e >> 16) & 15u), s2 = (int)(e >> 20);
+    u4 q0 = {0, 0, 0, 0}, q1 = {0, 0, 0, 0};
+    if (on) {
+        Dj = C.D[s2];
+        const double dt = pet - A.tb[tb0 + jj];
+        xj = A.px[tb0 + jj]; yj = A.py[tb0 + jj]; zj = A.pz[tb0 + jj];
+        q0 = philox_rk(id, jj, pid, 5u, rk);
+        q1 = philox_rk(id, jj, pid, 5u | (1u << 4), rk);
+        gs = dt > 0;
+        if (gs) sig = sqrt(2.0 * Dj * dt);
+    }
+    const double U = u01d32(q0.w);
+    // the Gaussians: ten partners at a time, lane 3 k + a takes axis a of the k-th
+    const unsigned gm = __ballot_sync(FULL, gs);
+    if (gm) {
+        const int rank = __popc(gm & ((1u << lane) - 1u)), ng = __popc(gm), a = lane % 3;
+        if (gs) src[rank] = (uint8_t)lane;
+        __syncwarp();
+#pragma unroll 1
+        for (int b = 0; b < ng; b += 10) {
+            const int k = b + lane / 3, from = src[min(k, ng - 1)];
+            const uint32_t w0 = __shfl_sync(FULL, q0.x, from), w1 = __shfl_sync(FULL, q0.y, from), w2 = __shfl_sync(FULL, q0.z, from);
+            const uint32_t v0 = __shfl_sync(FULL, q1.x, from), v1 = __shfl_sync(FULL, q1.y, from), v2 = __shfl_sync(FULL, q1.z, from);
+            double g = 0;
+            if (k < ng && lane < 30) g = gauss_axis(a == 0 ? w0 : a == 1 ? w1 : w2, a == 0 ? v0 : a == 1 ? v1 : v2);
+            const int at = 3 * (rank - b);
+            const bool mine = gs && rank >= b && rank < b + 10;
+            const double g0 = __shfl_sync(FULL, g, mine ? at : 0), g1 = __shfl_sync(FULL, g, mine ? at + 1 : 0);
+            const double g2 = __shfl_sync(FULL, g, mine ? at + 2 : 0);
+            if (mine) { xj += g0 * sig; yj += g1 * sig; zj += g2 * sig; }
+        }
+        __syncwarp();
+    }
+    if (on) {
+        const double dx = A.px[tb0 + id] - xj, dy = A.py[tb0 + id] - yj, dz = A.pz[tb0 + id] - zj;
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        if (r2 <= C.r_cut2) {
+            const double D = Di + Dj;
+            const double t = sample_pre(C, sqrt(r2), r2i, D, U, &pa, &pb);
+            if (t == -2.0) { pdcq = true; pD = D; }
+            else if (t >= 0) { *ta = pet + t; acc = *ta < 1000; }
+        }
+    }
+    unsigned pm = __ballot_sync(FULL, pdcq);
+    if (pm) {
+        const PdcPair PP = pdc_pair(pa, pb);
+        uint64_t words = ~0ull;
+        while (pm) {
+            const int s = __ffs(pm) - 1;
+            pm &= pm - 1;
+            const uint64_t wd = pdc_find(s, id, jj, pid, PP, pa, pb, lane,
+                                         [rk](uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) { return philox_rk(c0, c1, c2, c3, rk); });
+            if (lane == s) words = wd;
+        }
+        if (pdcq && words != ~0ull) {
+            const double X = pdc_x(pa, pb, PP.pq, PP.M, (uint32_t)(words >> 32), (uint32_t)words);
+            if (X > 0) { *ta = pet + X / pD; acc = *ta < 1000; }
+        }
+    }
+    return acc;
+}
+
+template <int W>
+constexpr int LT = W <= 4 ? IB : 32 * W;    // 16 warps per SM
+
+template <int W>
+__global__ void __launch_bounds__(LT<W>, 512 / LT<W>) k_irt_loop(const __grid_constant__ IArgs A) {
+    constexpr int G = LT<W> / 32 / W;            // tracks per block
+    __shared__ EvGroup<W> s_g[G];
     __shared__ IrtConst s_c;
     __shared__ uint32_t s_row[6];
     load_consts(&s_c, s_row);
     const IrtConst& C = s_c;
-    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const uint32_t gw = blockIdx.x * (IB / 32) + wl;
-    uint32_t* pq = s_pq[wl];
+    const int lane = threadIdx.x & 31, wg = (threadIdx.x >> 5) % W, g = (threadIdx.x >> 5) / W;
+    const bool lead = wg == 0 && lane == 0;
+    EvGroup<W>& S = s_g[g];
+    auto gsync = [g]() {
+        __syncwarp();
+        if (W > 1) asm volatile("barrier.sync %0, %1;" ::"r"(1 + g), "n"(32 * W) : "memory");
+    };
+    const uint32_t gw = blockIdx.x * G + g;
     // CAP of the reference worker (:405): twice the largest track's species, plus 512
     const uint32_t capref = 2u * A.counters[3] + 512u;
-    const uint32_t k0 = A.k0, k1 = A.k1;
-    for (int k = lane; k < 35; k += 32) s_tl[wl][k] = 0.0;
-    int* lc = s_lc[wl];
-    Heap H{s_ht[wl], s_hab[wl], A.hov_t + (size_t)gw * A.hcap, A.hov_ab + (size_t)gw * A.hcap};
-    // per-warp tallies in shared memory (lane 0): reactions 0..8, reacted, events, initial events
-    __shared__ unsigned long long s_cnt[IB / 32][12];
-    unsigned long long* tally = s_cnt[wl];
-    for (int k = lane; k < 12; k += 32) tally[k] = 0;
+    for (int k = lane + 32 * wg; k < 35; k += 32 * W) S.tl[k] = 0.0;
+    for (int k = lane + 32 * wg; k < 12; k += 32 * W) S.cnt[k] = 0;
+    // global storage of the group: heap beyond HS, partners beyond CQ
+    uint32_t* gab = A.hov_ab + (size_t)gw * (A.hcap + A.pcap);
+    uint32_t* gcq = gab + A.hcap;
+    Heap<HS<W>> H{S.ht, S.hab, A.hov_t + (size_t)gw * A.hcap, gab};
     unsigned long long n_pairs = 0;
-    __syncwarp();
     for (;;) {
-        uint32_t k = 0;
-        if (lane == 0) k = atomicAdd(&A.counters[2], 1u);
-        k = __shfl_sync(FULL, k, 0);
+        if (lead) S.track = atomicAdd(&A.counters[2], 1u);
+        gsync();
+        const uint32_t k = S.track;
+        gsync();
         if (k >= A.nseg) break;
         const uint32_t p = A.order[k];                 // largest tracks first
         const uint32_t n = A.tn[p];
         if (n == 0) continue;
         const uint32_t pid = A.pid_base + p;
         const uint32_t cap = tcap(A, p);
-        const unsigned long long tb0 = tbase(A, p);
-        double* px = A.px + tb0; double* py = A.py + tb0; double* pz = A.pz + tb0; double* tb = A.tb + tb0;
-        int8_t* sp = A.sp + tb0; uint8_t* alive = A.alive + tb0;
-        uint16_t* lst = A.lst + 6 * tb0; uint16_t* lpos = A.lpos + tb0;
-        float4* rec = A.rec + 6 * tb0;
-        double* ET = A.ev_t + ebase(A, p);
-        uint32_t* EAB = A.ev_ab + ebase(A, p);
+        const unsigned long long tb0 = tbase(A, p), eb0 = ebase(A, p);
         const uint32_t nev = A.tev[p];
         const float del = A.tdel[p];
         const float4 org = A.rad[A.seg_off[p]];
-        const double ox = org.x, oy = org.y, oz = org.z;
-        if (lane < 6) lc[lane] = (int)A.tlc[6 * p + lane];     // alive species of each kind
-        if (nev > ecap(A, p)) { if (lane == 0) atomicOr(A.err, DERR_HEAP); continue; }
-        if (lane == 0) tally[11] += nev;
+        if (nev > ecap(A, p)) { if (lead) atomicOr(A.err, DERR_HEAP); continue; }
+        if (wg == 0 && lane < 6) S.lc[lane] = (int)A.tlc[6 * p + lane];     // alive species of each kind
+        if (lead) { S.cnt[11] += nev; S.cnt[10] += nev; }
+        // the state of each species in shared memory, or in global memory in tracks too large for it
+        const bool insm = cap <= SN<W>;
+        if (insm) {
+            for (uint32_t k8 = lane + 32 * wg; k8 < (cap + 7) / 8; k8 += 32 * W) {
+                uint32_t v = 0;
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q) {
+                    const uint32_t k1 = 8 * k8 + q;
+                    if (k1 < n) v |= (uint32_t)(A.sp[tb0 + k1] | 8) << (4 * q);
+                }
+                S.state[k8] = v;
+            }
+            gsync();
+        }
+        auto state = [&](uint32_t k1) -> uint32_t {
+            return insm ? S.state[k1 >> 3] >> (4 * (k1 & 7)) & 15u
+                        : (uint32_t)A.sp[tb0 + k1] | (A.alive[tb0 + k1] ? 8u : 0u);
+        };
         __syncwarp();
-        uint32_t ip = 0, hn = 0;
-        uint32_t ntot = n;
+        // the first warp takes the initial events by windows of 32; wlive marks those whose
+        // two species are alive, and the next windows are copied to shared memory ahead
+        uint32_t ip = 0, hn = 0, ntot = n, wlive = 0;
+        auto window = [&](uint32_t at) {
+            if (at + lane < nev) {
+                cp_async<8>(&S.wt[at / 32 % WN][lane], A.ev_t + eb0 + at + lane);
+                cp_async<4>(&S.wab[at / 32 % WN][lane], A.ev_ab + eb0 + at + lane);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        if (wg == 0)
+#pragma unroll 1
+            for (int w = 0; w < WN - 1; ++w) window(32 * w);
         double h2c = (double)A.th2[p];
         int cp = 0, c16 = 0;
         float* curve = A.curves ? A.curves + 80ull * p : nullptr;
         bool heap_over = false;
         for (;;) {
-            double et = 0;
-            uint32_t eab = 0;
-            int have = 0, si = 0, sj = 0, ri = -1;
-            if (lane == 0) {
-                // pop until a reaction with products: stale events and reactions
-                // without products change nothing the other lanes work on
+            if (wg == 0) {
+                // pop until a reaction with products
+                int have = 0;
                 for (;;) {
-                    const bool hi_ = ip < nev, hh = hn > 0;
+                    while (!wlive && ip < nev) {           // the next window: its live events
+                        cp_wait<WN - 2>();
+                        const bool in = ip + lane < nev;
+                        const uint32_t wab = S.wab[ip / 32 % WN][lane], wi = wab >> 16, wj = wab & 0xffffu;
+                        const uint32_t ws = in ? state(wi) | state(wj) << 4 : 0u;
+                        S.wsp[lane] = (uint8_t)(ws & 0x77u);
+                        wlive = __ballot_sync(FULL, (ws & 0x88u) == 0x88u);
+                        ip += 32;
+                        window(ip + 32 * (WN - 2));
+                        __syncwarp();
+                    }
+                    const bool hi_ = wlive != 0, hh = hn > 0;
                     if (!hi_ && !hh) break;
-                    double ti = hi_ ? ET[ip] : 0.0, th = hh ? H.t(0) : 0.0;
-                    uint32_t ai = hi_ ? EAB[ip] : 0u, ah = hh ? H.ab(0) : 0u;
-                    if (hi_ && (!hh || ev_less(ti, ai, th, ah))) { et = ti; eab = ai; ip++; }
-                    else { et = th; eab = ah; heap_pop(H, hn); }
-                    tally[10]++;
+                    const int w = hi_ ? __ffs(wlive) - 1 : 0;
+                    const int wb = (ip / 32 + WN - 1) % WN;
+                    const double ti = S.wt[wb][w], th = hh ? S.ht[0] : 0.0;
+                    const uint32_t ai = S.wab[wb][w], ah = hh ? S.hab[0] : 0u;
+                    const int spi = S.wsp[w];
+                    const bool init = hi_ && (!hh || ev_less(ti, ai, th, ah));
+                    const double et = init ? ti : th;
+                    const uint32_t eab = init ? ai : ah;
+                    const int ei = (int)(eab >> 16), ej = (int)(eab & 0xffffu);
+                    int a = spi & 15, b2 = spi >> 4;
+                    if (init) wlive &= wlive - 1;
+                    else {
+                        const uint32_t s0 = state(ei), s1 = state(ej);
+                        a = (int)(s0 & 7u); b2 = (int)(s1 & 7u);
+                        heap_pop(H, hn, lane);
+                        if (!(s0 & s1 & 8u)) continue;
+                    }
                     while (cp < 7 && et >= c_cp[cp]) {
-                        s_tl[wl][cp * 5 + 0] += lc[0]; s_tl[wl][cp * 5 + 1] += lc[1];
-                        s_tl[wl][cp * 5 + 2] += lc[2]; s_tl[wl][cp * 5 + 3] += lc[4];
-                        s_tl[wl][cp * 5 + 4] += h2c;
+                        if (lane < 5) S.tl[cp * 5 + lane] += lane == 4 ? h2c : (double)S.lc[lane == 3 ? 4 : lane];
                         cp++;
                     }
                     while (curve && c16 < 16 && et >= C.t16[c16]) {
-                        float* c = curve + 5 * c16;
-                        c[0] = (float)lc[0]; c[1] = (float)lc[1]; c[2] = (float)lc[2]; c[3] = (float)lc[4];
-                        c[4] = (float)h2c;
+                        if (lane < 5) curve[5 * c16 + lane] = lane == 4 ? (float)h2c : (float)S.lc[lane == 3 ? 4 : lane];
                         c16++;
                     }
-                    const int ei = (int)(eab >> 16), ej = (int)(eab & 0xffffu);
-                    if (!(alive[ei] && alive[ej])) continue;
-                    const int a = sp[ei], b2 = sp[ej];
                     const int r = C.map[(a < b2 ? a : b2) * 6 + (a < b2 ? b2 : a)];
                     if (r < 0) continue;
-                    alive[ei] = 0; alive[ej] = 0;
-                    // rolled: one copy of the list update (fewer spills in the event kernel)
-#pragma unroll 1
-                    for (int w2 = 0; w2 < 2; ++w2) {
-                        int k = w2 == 0 ? ei : ej, q = w2 == 0 ? a : b2;
-                        uint32_t at = lpos[k];
-                        uint16_t last = lst[q * cap + lc[q] - 1];
-                        lst[q * cap + at] = last;
-                        rec[q * cap + at] = rec[q * cap + lc[q] - 1];
-                        lpos[last] = (uint16_t)at;
-                        lc[q]--;
+                    __syncwarp();
+                    if (lane < 6) {                        // where the products will be
+                        const double* at = (lane < 2 ? A.px : lane < 4 ? A.py : A.pz) + tb0 + (lane & 1 ? ej : ei);
+                        asm volatile("prefetch.global.L1 [%0];" ::"l"(at));
                     }
-                    tally[9]++;
-                    tally[r]++;
+                    // both leave their species' list (its last entry takes the place)
+                    const int st = a == b2 ? 1 : 2;
+                    if (lane < st) {
+#pragma unroll 1
+                        for (int w2 = lane; w2 < 2; w2 += st) {
+                            const int k2 = w2 == 0 ? ei : ej, q = w2 == 0 ? a : b2;
+                            if (insm) atomicAnd(&S.state[k2 >> 3], ~(8u << (4 * (k2 & 7))));
+                            else A.alive[tb0 + k2] = 0;
+                            const uint32_t at = A.lpos[tb0 + k2], end = (uint32_t)S.lc[q] - 1;
+                            const uint16_t last = A.lst[6 * tb0 + q * cap + end];
+                            A.rec[6 * tb0 + q * cap + at] = A.rec[6 * tb0 + q * cap + end];
+                            A.lst[6 * tb0 + q * cap + at] = last;
+                            A.lpos[tb0 + last] = (uint16_t)at;
+                            S.lc[q] = (int)end;
+                        }
+                    }
+                    if (lane == 0) { S.cnt[9]++; S.cnt[r]++; }
+                    const uint32_t wab = S.wab[wb][lane];
+                    const int wi = (int)(wab >> 16), wj = (int)(wab & 0xffffu);
+                    wlive &= ~__ballot_sync(FULL, wi == ei || wi == ej || wj == ei || wj == ej);
+                    __syncwarp();
                     if (r == 3 || r == 4 || r == 6) h2c += 1;
                     if (C.nprod[r] == 0) continue;
-                    have = 1; si = a; sj = b2; ri = r;
+                    have = 1;
+                    if (lane == 0) { S.et = et; S.eab = eab; S.si = a; S.sj = b2; S.ri = r; }
                     break;
                 }
+                if (lane == 0) S.have = have;
             }
-            if (!__shfl_sync(FULL, have, 0)) break;
-            et = __shfl_sync(FULL, et, 0);
-            eab = __shfl_sync(FULL, eab, 0);
+            gsync();
+            if (!S.have) break;
+            const double et = S.et;
+            const uint32_t eab = S.eab;
             const int ei = (int)(eab >> 16), ej = (int)(eab & 0xffffu);
-            si = __shfl_sync(FULL, si, 0);
-            sj = __shfl_sync(FULL, sj, 0);
-            ri = __shfl_sync(FULL, ri, 0);
+            const int si = S.si, sj = S.sj, ri = S.ri;
             const int np_ = C.nprod[ri];
+            if (W > 1) gsync();                            // all have read the event
+            else __syncthreads_count(1);                   // the block's tracks go on together
+#pragma unroll 1
             for (int pp = 0; pp < np_; ++pp) {
-                int nsp = pp == 0 ? C.prod0[ri] : C.prod1[ri];
-                uint32_t id = ntot;
-                if (id >= capref) break;                 // the reference's CAP (:405, :621)
-                if (id >= cap) { if (lane == 0) atomicOr(A.err, DERR_TRACK_SIZE); break; }
+                const int nsp = pp == 0 ? C.prod0[ri] : C.prod1[ri];
+                const uint32_t id = ntot;
+                if (id >= capref) break;                   // the reference's CAP (:405, :621)
+                if (id >= cap) { if (lead) atomicOr(A.err, DERR_TRACK_SIZE); break; }
+                ntot++;
                 double nx, ny, nz;
-                if (np_ == 1) {                          // at the diffusion-weighted centre
+                if (np_ == 1) {                            // at the diffusion-weighted centre
                     const double sqDi = sqrt(C.D[si]), sqDj = sqrt(C.D[sj]);
                     const double ww = sqDi + sqDj;
-                    const double xa = px[ei], ya = py[ei], za = pz[ei];
-                    const double xb = px[ej], yb = py[ej], zb = pz[ej];
+                    const double xa = A.px[tb0 + ei], ya = A.py[tb0 + ei], za = A.pz[tb0 + ei];
+                    const double xb = A.px[tb0 + ej], yb = A.py[tb0 + ej], zb = A.pz[tb0 + ej];
                     nx = (sqDj * xa + sqDi * xb) / ww;
                     ny = (sqDj * ya + sqDi * yb) / ww;
                     nz = (sqDj * za + sqDi * zb) / ww;
-                } else {                                 // at the two reactants
+                } else {                                   // at the two reactants
                     const int e = pp == 0 ? ei : ej;
-                    nx = px[e]; ny = py[e]; nz = pz[e];
+                    nx = A.px[tb0 + e]; ny = A.py[tb0 + e]; nz = A.pz[tb0 + e];
                 }
-                const float nsx = (float)(nx - ox), nsy = (float)(ny - oy), nsz = (float)(nz - oz);
-                if (lane == 0) {
-                    px[id] = nx; py[id] = ny; pz[id] = nz; tb[id] = et;
-                    sp[id] = (int8_t)nsp; alive[id] = 1;
-                    lst[nsp * cap + lc[nsp]] = (uint16_t)id;
-                    rec[nsp * cap + lc[nsp]] = make_float4(nsx, nsy, nsz, (float)et);
-                    lpos[id] = (uint16_t)lc[nsp];
-                    lc[nsp]++;
+                ScanP P;
+                P.x = (float)(nx - (double)org.x); P.y = (float)(ny - (double)org.y); P.z = (float)(nz - (double)org.z);
+                P.del = del; P.et = (float)et; P.dtm = 1e-4f + 1e-6f * P.et;
+                P.rcut = (float)sqrt(C.r_cut2) * 1.00001f;
+                P.id = id; P.pid = pid;
+                if (lead) {
+                    const int at = S.lc[nsp];
+                    A.px[tb0 + id] = nx; A.py[tb0 + id] = ny; A.pz[tb0 + id] = nz; A.tb[tb0 + id] = et;
+                    if (insm) atomicOr(&S.state[id >> 3], (8u | (uint32_t)nsp) << (4 * (id & 7)));
+                    else { A.sp[tb0 + id] = (int8_t)nsp; A.alive[tb0 + id] = 1; }
+                    A.lst[6 * tb0 + nsp * cap + at] = (uint16_t)id;
+                    A.rec[6 * tb0 + nsp * cap + at] = make_float4(P.x, P.y, P.z, P.et);
+                    A.lpos[tb0 + id] = (uint16_t)at;
+                    S.lc[nsp] = at + 1;
+                    S.ncand = 0; S.nacc = 0; S.hn = hn;
                 }
-                ntot++;
-                __syncwarp();
-                __threadfence_block();
-                // pairWithAlive (:430-465) over the alive particles of the species that react with nsp.
-                // f32 prefilter per partner; the partners it cannot rule out are queued and
-                // evaluated exactly (ProdPair), 32 at a time, one per lane.
-                const double Di = C.D[nsp];
+                gsync();
                 const uint32_t rowp = s_row[nsp];
-                int qn = 0;
-                const ProdCtx P{px, py, pz, tb, Di, id, pid, k0, k1};
-                const float etf = (float)et, dtm = 1e-4f + 1e-6f * etf;
-                const float rcut_hi = (float)sqrt(C.r_cut2) * 1.00001f;
-                for (int s2 = 0; s2 < 6; ++s2) {
-                    const int r2i = (int)((rowp >> (4 * s2)) & 15u);
-                    if (r2i == 15) continue;
-                    const uint32_t len = (uint32_t)lc[s2];
-                    const float Djf2 = (float)(2.0 * C.D[s2]);
-                    const float fs = C.fs[r2i], fsc = C.fsc[r2i], fadd = C.fadd[r2i];
-                    const uint16_t* L2 = lst + s2 * cap;
-                    const float4* R2 = rec + s2 * cap;
-                    // chunks of 32 partners; the next chunk's list entry and record are
-                    // loaded before this chunk is tested (the lists do not change here)
-                    uint32_t jnext = lane < len ? L2[lane] : 0xffffu;
-                    float4 rnext = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (lane < len) rnext = R2[lane];
-                    for (uint32_t c0 = 0; c0 < len; c0 += 32) {
-                        const uint32_t jj = jnext;
-                        const float4 q = rnext;
-                        {
-                            const uint32_t li = c0 + 32u + lane;
-                            jnext = li < len ? L2[li] : 0xffffu;
-                            if (li < len) rnext = R2[li];
+                // Chunks of 32 partners, over the lists of all species that react with the product;
+                // the next chunk's list entries and records are loaded before this chunk is
+                // tested (the lists do not change here).  What the first test leaves waits in nq
+                // until 32 can take the second.  One copy of the code serves all species and
+                // the rest at the end: see the kernel's comment.
+                uint32_t qn = 0, nli = 0, nlen = 0, njj = 0, ntag = 0;
+                int ns2 = -1;
+                float4 nrec = make_float4(0.f, 0.f, 0.f, 0.f);
+                auto advance = [&]() {
+#pragma unroll 1
+                    while (nli - lane >= nlen) {
+                        if (++ns2 == 6) return;
+                        const uint32_t r2i = (rowp >> (4 * ns2)) & 15u;
+                        if (r2i == 15u) continue;
+                        // the product itself is the last of its own list
+                        nlen = (uint32_t)S.lc[ns2] - (ns2 == nsp ? 1u : 0u);
+                        nli = 32u * wg + lane;
+                        ntag = (r2i << 16) | ((uint32_t)ns2 << 20);
+                        if (wg == 0) n_pairs += nlen;          // (as many on every lane)
+                    }
+                    if (nli < nlen) {
+                        const size_t at = 6 * tb0 + (uint32_t)ns2 * cap + nli;
+                        nrec = A.rec[at];
+                        njj = A.lst[at];
+                    }
+                };
+                nli = lane;
+                advance();
+#pragma unroll 1
+                for (;;) {
+                    const int s2 = ns2;
+                    if (s2 < 6) {
+                        const float4 q = nrec;
+                        const uint32_t jj = njj, at = nli, tag = ntag;
+                        const bool in = at < nlen;
+                        nli += 32u * W;
+                        advance();
+                        bool nr = false;
+                        if (in) {
+                            const int r2i = (int)(tag >> 16 & 15u);
+                            nr = scan_near(P, q, jj, (float)(2.0 * C.D[s2]), C.fs[r2i], C.fsc[r2i], C.fadd[r2i], A.rk);
                         }
+                        const unsigned m = __ballot_sync(FULL, nr);
+                        if (!m) continue;
+                        if (nr) S.nq[wg][qn + __popc(m & ((1u << lane) - 1u))] = at | tag;
+                        qn += __popc(m);
+                        __syncwarp();
+                        if (qn < 32) continue;
+                    }
+                    if (qn) {
+                        const uint32_t from = qn >= 32 ? qn - 32 : 0;
                         bool mv = false;
-                        {
-                            if (jj != 0xffffu && jj != id) {
-                                n_pairs++;
-                                const float ex = nsx - q.x, ey = nsy - q.y, ez = nsz - q.z;
-                                const float dlo = (sqrtf(fmaf(ez, ez, fmaf(ey, ey, ex * ex))) - del) * 0.999998f;
-                                // draw-free bound first: the displacement is at most the largest
-                                // Box-Muller radius of 32-bit draws (sqrt(3 * 2 ln 2^33) = 11.72)
-                                // times sqrt(2 D dt), and a partner beyond R_CUT after it is
-                                // rejected by the exact path too
-                                const float dth = etf - q.w + dtm;
-                                if (dlo - (dth > 0.0f ? sqrtf(Djf2 * dth) * 11.8f : 0.0f) > rcut_hi) goto scored;
-                                const u4 q0 = philox_pair(id, jj, pid, k0, k1);
-                                // R of r_acc for U >= uf, rounded up
-                                const float uf = __uint2float_rd(q0.w) * 2.3283064365386963e-10f;
-                                const float rhi = (fmaxf(fs, __fdividef(fsc, uf)) + fadd) * 1.00002f + 1e-6f;
-                                // dth: upper bound of dt = et - t_birth from the f32 birth time (error < dtm)
-                                float reach = 0.0f, l0 = 0.0f, l1 = 0.0f, l2 = 0.0f, Bf = 0.0f;
-                                if (dth > 0.0f) {
-                                    l0 = -2.0f * __logf(u01f32(q0.x));
-                                    l1 = -2.0f * __logf(u01f32(q0.y));
-                                    l2 = -2.0f * __logf(u01f32(q0.z));
-                                    Bf = sqrtf((l0 + l1 + l2) * 1.0001f);
-                                    reach = sqrtf(Djf2 * dth) * 1.00001f * (Bf + 1e-4f);
-                                }
-                                mv = !(dlo - reach > rhi);
-                                if (mv && dth > 0.0f) {
-                                    // second stage: the partner displaced by the same Box-Muller draws in
-                                    // f32.  Per axis |g_f - g| <= 2e-3 + 2e-5 |g| (sqrt of the log near 0,
-                                    // fast log and cos, 2 ulp each), sigma within [sl, sh].
-                                    const u4 q1 = philox_pair_ang(id, jj, pid, k0, k1);
-                                    const float dtl = fmaxf(etf - q.w - dtm, 0.0f);
-                                    const float sh = sqrtf(Djf2 * dth) * 1.00001f, sl = sqrtf(Djf2 * dtl) * 0.99999f;
-                                    const float sm = 0.5f * (sh + sl), Bm = Bf + 1e-4f;
-                                    // cos(2 pi u) = -cos(2 pi (u - 1/2)): the argument stays in [-pi, pi]
-                                    const float g0 = -sqrtf(l0) * __cosf(6.2831853f * (u01f32(q1.x) - 0.5f));
-                                    const float g1 = -sqrtf(l1) * __cosf(6.2831853f * (u01f32(q1.y) - 0.5f));
-                                    const float g2 = -sqrtf(l2) * __cosf(6.2831853f * (u01f32(q1.z) - 0.5f));
-                                    const float fx = ex - g0 * sm, fy = ey - g1 * sm, fz = ez - g2 * sm;
-                                    const float d2 = sqrtf(fmaf(fz, fz, fmaf(fy, fy, fx * fx)));
-                                    const float eg = 2e-3f + 2e-5f * Bm;
-                                    const float err = 1.7320508f * (sh * eg + 0.5f * (Bm + eg) * (sh - sl)) + del;
-                                    mv = !((d2 - err) * 0.99999f > rhi);
-                                }
+                        uint32_t v = 0;
+                        if (from + lane < qn) {
+                            const uint32_t e = S.nq[wg][from + lane];
+                            const int ri2 = (int)((e >> 16) & 15u), sj2 = (int)(e >> 20);
+                            const size_t at = (size_t)sj2 * cap + (e & 0xffffu);
+                            const uint32_t jj = A.lst[6 * tb0 + at];
+                            mv = scan_maybe(P, A.rec[6 * tb0 + at], jj, (float)(2.0 * C.D[sj2]), C.fs[ri2], C.fsc[ri2], C.fadd[ri2], A.rk);
+                            v = (e & ~0xffffu) | jj;
+                        }
+                        qn = from;
+                        const unsigned m = __ballot_sync(FULL, mv);
+                        if (m) {
+                            uint32_t base = 0;
+                            if (lane == 0) base = atomicAdd(&S.ncand, (uint32_t)__popc(m));
+                            base = __shfl_sync(FULL, base, 0);
+                            if (mv) {
+                                base += __popc(m & ((1u << lane) - 1u));
+                                if (base < CQ) S.cq[base] = v; else gcq[base - CQ] = v;
                             }
                         }
-                    scored:
-                        {
-                            const unsigned m = __ballot_sync(FULL, mv);
-                            if (m) {
-                                if (mv) pq[qn + __popc(m & ((1u << lane) - 1u))] = jj | ((uint32_t)r2i << 16) | ((uint32_t)s2 << 20);
-                                qn += __popc(m);
-                                if (qn >= 32) {
-                                    __syncwarp();
-                                    heap_over |= prod_batch(C, P, pq, 32, lane, H, hn, A.hcap);
-                                    __syncwarp();
-                                    if (lane < qn - 32) pq[lane] = pq[32 + lane];
-                                    qn -= 32;
-                                    __syncwarp();
-                                }
-                            }
+                        __syncwarp();
+                    }
+                    if (s2 == 6) break;
+                }
+                gsync();
+                const uint32_t nc = S.ncand;
+                if (nc == 0) continue;
+                // few partners per warp when there are several warps: their chains run side by side
+                constexpr uint32_t BL = W == 1 ? 32u : 8u;
+#pragma unroll 1
+                for (uint32_t b = BL * wg; b < nc; b += BL * W) {
+                    const bool on = (uint32_t)lane < BL && b + lane < nc;
+                    const uint32_t at = b + lane;
+                    const uint32_t e = on ? (at < CQ ? S.cq[at] : gcq[at - CQ]) : 0u;
+                    double ta = 0;
+                    const bool acc = pair_exact(A, C, tb0, id, pid, C.D[nsp], e, on, lane, S.src[wg], &ta);
+                    const unsigned m = __ballot_sync(FULL, acc);
+                    if (m) {
+                        uint32_t base = 0;
+                        if (lane == 0) base = atomicAdd(&S.nacc, (uint32_t)__popc(m));
+                        base = __shfl_sync(FULL, base, 0);
+                        if (acc) {
+                            base += __popc(m & ((1u << lane) - 1u));
+                            const uint32_t pj = e & 0xffffu;
+                            base += S.hn;                  // the heap's next free nodes
+                            if (base < HS<W> + A.hcap) H.set(base, ta, pj < id ? (pj << 16) | id : (id << 16) | pj);
                         }
                     }
                 }
-                if (qn) {
+                gsync();
+                if (wg == 0) {
+                    const uint32_t na = S.nacc;
+                    if (lane == 0) {
+                        S.cnt[10] += na;
+#pragma unroll 1
+                        for (uint32_t q = hn; q < min(hn + na, HS<W> + A.hcap); ++q) heap_up(H, q);
+                    }
+                    heap_over |= hn + na > HS<W> + A.hcap;
+                    hn = min(hn + na, HS<W> + A.hcap);
                     __syncwarp();
-                    heap_over |= prod_batch(C, P, pq, qn, lane, H, hn, A.hcap);
                 }
-                __syncwarp();
-                __threadfence_block();
             }
         }
-        if (lane == 0) {
-            if (heap_over) atomicOr(A.err, DERR_HEAP);
-            while (cp < 7) {
-                s_tl[wl][cp * 5 + 0] += lc[0]; s_tl[wl][cp * 5 + 1] += lc[1];
-                s_tl[wl][cp * 5 + 2] += lc[2]; s_tl[wl][cp * 5 + 3] += lc[4];
-                s_tl[wl][cp * 5 + 4] += h2c;
-                cp++;
+        if (wg == 0) {
+            if (heap_over && lane == 0) atomicOr(A.err, DERR_HEAP);
+            if (lane < 5) {
+                const double v = lane == 4 ? h2c : (double)S.lc[lane == 3 ? 4 : lane];
+                for (; cp < 7; cp++) S.tl[cp * 5 + lane] += v;
+                for (; curve && c16 < 16; c16++) curve[5 * c16 + lane] = (float)v;
             }
-            while (curve && c16 < 16) {
-                float* c = curve + 5 * c16;
-                c[0] = (float)lc[0]; c[1] = (float)lc[1]; c[2] = (float)lc[2]; c[3] = (float)lc[4];
-                c[4] = (float)h2c;
-                c16++;
-            }
+            __syncwarp();
         }
-        __syncwarp();
     }
-    for (int o = 16; o; o >>= 1) n_pairs += __shfl_xor_sync(FULL, n_pairs, o);
-    __syncwarp();
-    if (lane == 0) {
-        for (int k = 0; k < 9; ++k) if (tally[k]) atomicAdd(&A.acc[k], tally[k]);
-        if (tally[9]) atomicAdd(&A.acc[9], tally[9]);
-        if (n_pairs) atomicAdd(&A.acc[10], n_pairs);
-        if (tally[10]) atomicAdd(&A.acc[11], tally[10]);
-        if (tally[11]) atomicAdd(&A.acc[14], tally[11]);
+    if (W == 1) while (__syncthreads_count(0)) {}          // until the block's last track has ended
+    if (lane == 0 && n_pairs) atomicAdd(&A.acc[10], n_pairs);
+    gsync();
+    if (lead) {
+        for (int k = 0; k < 10; ++k) if (S.cnt[k]) atomicAdd(&A.acc[k], S.cnt[k]);
+        if (S.cnt[10]) atomicAdd(&A.acc[11], S.cnt[10]);
+        if (S.cnt[11]) atomicAdd(&A.acc[14], S.cnt[11]);
     }
-    for (int k = lane; k < 35; k += 32)
-        if (s_tl[wl][k] != 0.0) atomicAdd(&A.acc_tl[k], s_tl[wl][k]);
+    for (int k = lane + 32 * wg; k < 35; k += 32 * W)
+        if (S.tl[k] != 0.0) atomicAdd(&A.acc_tl[k], S.tl[k]);
 }
 
 // codes -> grouping keys (pid << 34 | original index) for a caller's rad_buf
@@ -1254,8 +1432,54 @@ __global__ void __launch_bounds__(1024) k_track_order(const uint32_t* tn, uint32
     }
 }
 
-int irt_warps(int device, const IrtShape& shape) {
-    return blocks_for((const void*)k_irt_loop, device, shape.loop_per_sm) * (IB / 32);
+// Warps per track of the event kernel: two while all tracks are resident at once at 16 warps
+// per SM, more while they are at 8 per SM.  Measured (10 keV tracks on 148 SMs, ms with
+// W = 1, 2, 4, 8, 16): 64 tracks 5.96 3.46 3.13 3.02 3.07, 150: 6.34 3.90 3.56 3.47 3.83,
+// 300: 6.38 3.91 3.66 4.02 6.65, 600: 6.61 4.38 4.85 7.09 -, 1200: 6.98 6.28 8.07 - -,
+// 1800: 7.97 8.95 11.2 - -; one track of 3060 species 10.3 9.2 9.0 9.0 8.7.
+static int loop_width(int device, uint32_t nseg) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const unsigned long long warps = 16ull * (unsigned long long)sms;
+    int w = 16;
+    while (w > 1 && (unsigned long long)nseg * (unsigned long long)w > (w > 2 ? warps / 2 : warps)) w >>= 1;
+    return w;
+}
+
+// resident blocks of the event kernel with W warps per track; the shape's limit is in
+// blocks of 4 warps
+template <int W>
+static int loop_blocks(int device, const IrtShape& shape) {
+    int sms = 0, per = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k_irt_loop<W>, LT<W>, 0);
+    if (per < 1) per = 1;
+    const int limit = (int)shape.loop_per_sm * IB / LT<W>;
+    if (shape.loop_per_sm && limit < per) per = limit > 0 ? limit : 1;
+    return sms * per;
+}
+template <int W>
+static int loop_groups(int device, const IrtShape& shape) {
+    return loop_blocks<W>(device, shape) * (LT<W> / 32 / W);
+}
+
+// tracks of the event kernel in flight at once, at most: each has its own scratch
+// (blocks hold up to 4 tracks, of which the last may be without one)
+int irt_warps(int device, const IrtShape& shape, uint32_t nseg) {
+    int n = loop_groups<1>(device, shape);
+    n = std::max(n, loop_groups<2>(device, shape));
+    n = std::max(n, loop_groups<4>(device, shape));
+    n = std::max(n, loop_groups<8>(device, shape));
+    n = std::max(n, loop_groups<16>(device, shape));
+    return (int)std::min((unsigned long long)n, ((unsigned long long)nseg + 3) & ~3ull);
+}
+
+template <int W>
+static cudaError_t launch_loop(const IArgs& a, int device, const IrtShape& shape, cudaStream_t s) {
+    const unsigned groups = LT<W> / 32 / W, fit = (unsigned)loop_blocks<W>(device, shape);
+    const unsigned want = (a.nseg + groups - 1) / groups;
+    k_irt_loop<W><<<want < fit ? (want ? want : 1) : fit, LT<W>, 0, s>>>(a);
+    return cudaGetLastError();
 }
 
 // tile prefix: the scan of transport.cu
@@ -1286,8 +1510,13 @@ cudaError_t launch_irt(const IArgs& a, int device, const IrtShape& shape, cudaSt
     const unsigned long long sgrid = (unsigned long long)sms * (unsigned long long)(per > 0 ? per : 1);
     k_irt_sort<<<(unsigned)(a.nseg < sgrid ? (a.nseg > 0 ? a.nseg : 1) : sgrid), SB, 0, s>>>(a);
     if (ev && (e = irt_mark(ev[2], s)) != cudaSuccess) return e;
-    k_irt_loop<<<blocks_for((const void*)k_irt_loop, device, shape.loop_per_sm), IB, 0, s>>>(a);
-    return cudaGetLastError();
+    switch (loop_width(device, a.nseg)) {
+    case 16: return launch_loop<16>(a, device, shape, s);
+    case 8: return launch_loop<8>(a, device, shape, s);
+    case 4: return launch_loop<4>(a, device, shape, s);
+    case 2: return launch_loop<2>(a, device, shape, s);
+    default: return launch_loop<1>(a, device, shape, s);
+    }
 }
 
 // The IRT launch sequence as one CUDA graph, captured on a private stream and

@@ -45,10 +45,11 @@ struct IArgs {
     uint32_t *tn, *th2, *ttiles, *tev, *tlc;   // per track: particles, H2 markers, tiles, events, 6 list lengths
     unsigned long long* toff;            // nseg + 1: prefix of ttiles
     uint32_t* order;                     // nseg: tracks in the order the event kernel takes them
-    // per-warp heap overflow of the event kernel
+    // per track in flight of the event kernel: hcap heap nodes beyond the shared ones and,
+    // in hov_ab, pcap listed partners beyond those
     double* hov_t;
     uint32_t* hov_ab;
-    uint32_t hcap;
+    uint32_t hcap, pcap;
     uint32_t* counters;                  // [0] load, [1] init items, [2] loop tracks, [3] largest track
     double* acc_tl;                      // 35
     unsigned long long* acc;             // [0..8] rxn, 9 reacted, 10 pairs, 11 events, 12 tracks
@@ -58,10 +59,11 @@ struct IArgs {
 
 cudaError_t irt_set_constants(const IrtConst& c);
 // Resident blocks per SM of the pairing and event kernels: as many as fit, at
-// most the given number (0 = no limit).  The heap overflow is sized per event
-// warp, so irt_warps and launch_irt must see the same limits.
+// most the given number (0 = no limit; of the event kernel in blocks of 4 warps).  The heap
+// overflow is sized per track in flight, so irt_warps and launch_irt must see the
+// same limits.
 struct IrtShape { uint32_t init_per_sm, loop_per_sm; };
-int irt_warps(int device, const IrtShape& shape);
+int irt_warps(int device, const IrtShape& shape, uint32_t nseg);
 // ev (optional, 3 events): recorded after the load, the initial pairing and the sort
 cudaError_t launch_irt(const IArgs& a, int device, const IrtShape& shape, cudaStream_t s, cudaEvent_t* ev = nullptr);
 // A captured IRT launch sequence and what it was captured for (irt.cu irt_graph_run).
