@@ -10,6 +10,7 @@
 
 #include "chemgrid.cuh"
 #include "dose.cuh"
+#include "hostcopy.cuh"
 #include "irt.cuh"
 #include "scoring.cuh"
 #include "surrogate_api.cuh"
@@ -122,6 +123,7 @@ struct wgdna_ctx {
     cudaEvent_t ev[13]{};
     // small results land here (page-locked, so that a readback is a stream operation)
     unsigned char* h_pin = nullptr;       // H_PIN bytes
+    wg::HostCopy hc;                      // slots of large copies to and from the host
     uint32_t* h_fib = nullptr;            // 3 per fibre
     size_t h_fib_cap = 0;
 };
@@ -345,6 +347,7 @@ extern "C" void wgdna_destroy(wgdna_ctx* c) {
     if (c->cg_graph) cudaGraphExecDestroy(c->cg_graph);
     if (c->irt_graph.exec) cudaGraphExecDestroy(c->irt_graph.exec);
     for (void* p : ptrs) if (p) cudaFree(p);
+    wg::host_copy_free(&c->hc);
     if (c->h_pin) cudaFreeHost(c->h_pin);
     if (c->h_fib) cudaFreeHost(c->h_fib);
     for (auto& ev : c->ev) if (ev) cudaEventDestroy(ev);
@@ -508,10 +511,10 @@ extern "C" int wgdna_transport_copy_out(wgdna_ctx* c, float* results, uint32_t* 
     if (!c->have_transport) { wg_set_error("wgdna_transport_copy_out: no transport result"); return WGDNA_ERR_STATE; }
     cudaStream_t s = c->stream;
     size_t nv = (size_t)c->cfg.vc * c->cfg.vc * c->cfg.vc;
-    if (results) WG_CUDA_OK(cudaMemcpyAsync(results, c->d_results, (size_t)c->last_np * 32, cudaMemcpyDeviceToHost, s));
-    if (dose) WG_CUDA_OK(cudaMemcpyAsync(dose, c->d_dose, nv * 4, cudaMemcpyDeviceToHost, s));
+    if (results) WG_CUDA_OK(host_copy(&c->hc, c->device, results, c->d_results, (size_t)c->last_np * 32, cudaMemcpyDeviceToHost, s));
+    if (dose) WG_CUDA_OK(host_copy(&c->hc, c->device, dose, c->d_dose, nv * 4, cudaMemcpyDeviceToHost, s));
     unsigned long long n = c->last_rad_n < rad_cap ? c->last_rad_n : rad_cap;
-    if (rad && n) WG_CUDA_OK(cudaMemcpyAsync(rad, c->d_rad, n * 16, cudaMemcpyDeviceToHost, s));
+    if (rad && n) WG_CUDA_OK(host_copy(&c->hc, c->device, rad, c->d_rad, n * 16, cudaMemcpyDeviceToHost, s));
     if (rad_n) *rad_n = c->last_rad_n;
     WG_CUDA_OK(cudaStreamSynchronize(s));
     return WGDNA_OK;
@@ -685,7 +688,7 @@ extern "C" int wgdna_run_irt(wgdna_ctx* c, const float* rad_buf, uint64_t rad_n,
         if (out) { memset(out, 0, sizeof *out); }
         return WGDNA_OK;
     }
-    WG_CUDA_OK(cudaMemcpyAsync(c->d_rad_raw, rad_buf, rad_n * 16, cudaMemcpyHostToDevice, s));
+    WG_CUDA_OK(host_copy(&c->hc, c->device, c->d_rad_raw, rad_buf, rad_n * 16, cudaMemcpyHostToDevice, s));
     if (!c->d_maxpid) TRY(dalloc(&c->d_maxpid, 1));
     WG_CUDA_OK(launch_group_keys(c->d_rad_raw, rad_n, c->d_key, c->d_maxpid, s));
     uint32_t maxpid = 0;
@@ -893,8 +896,14 @@ static int score_dev(wgdna_ctx* c, const float4* d_in, const uint32_t* d_alive, 
 
 static int hits_in(wgdna_ctx* c, const uint8_t* hits) {
     size_t hb = (size_t)c->dna.n_bp * 2;
-    if (hits) WG_CUDA_OK(cudaMemcpyAsync(c->d_hits, hits, hb, cudaMemcpyHostToDevice, c->stream));
+    if (hits) WG_CUDA_OK(host_copy(&c->hc, c->device, c->d_hits, hits, hb, cudaMemcpyHostToDevice, c->stream));
     else WG_CUDA_OK(cudaMemsetAsync(c->d_hits, 0, (hb + 3) & ~(size_t)3, c->stream));
+    return WGDNA_OK;
+}
+
+static int hits_out(wgdna_ctx* c, uint8_t* hits) {
+    WG_CUDA_OK(host_copy(&c->hc, c->device, hits, c->d_hits, (size_t)c->dna.n_bp * 2, cudaMemcpyDeviceToHost, c->stream));
+    WG_CUDA_OK(cudaStreamSynchronize(c->stream));
     return WGDNA_OK;
 }
 
@@ -905,9 +914,9 @@ extern "C" int wgdna_score_direct(wgdna_ctx* c, const float* rad, uint64_t rad_n
     WG_CUDA_OK(cudaSetDevice(c->device));
     c->have_transport = false;
     TRY(hits_in(c, hits));
-    if (rad_n) WG_CUDA_OK(cudaMemcpyAsync(c->d_rad_raw, rad, rad_n * 16, cudaMemcpyHostToDevice, c->stream));
+    if (rad_n) WG_CUDA_OK(host_copy(&c->hc, c->device, c->d_rad_raw, rad, rad_n * 16, cudaMemcpyHostToDevice, c->stream));
     TRY(score_dev(c, c->d_rad_raw, nullptr, rad_n, 0.15, 1, lcg_state, out));
-    if (hits) WG_CUDA_OK(cudaMemcpy(hits, c->d_hits, (size_t)c->dna.n_bp * 2, cudaMemcpyDeviceToHost));
+    if (hits) TRY(hits_out(c, hits));
     return WGDNA_OK;
 }
 
@@ -920,11 +929,11 @@ extern "C" int wgdna_score_indirect(wgdna_ctx* c, const float* pos, const uint32
     TRY(hits_in(c, hits));
     if (n > c->alive_cap) { TRY(dalloc(&c->d_alive, n)); c->alive_cap = n; }
     if (n) {
-        WG_CUDA_OK(cudaMemcpyAsync(c->d_rad_raw, pos, n * 16, cudaMemcpyHostToDevice, c->stream));
-        WG_CUDA_OK(cudaMemcpyAsync(c->d_alive, alive, n * 4, cudaMemcpyHostToDevice, c->stream));
+        WG_CUDA_OK(host_copy(&c->hc, c->device, c->d_rad_raw, pos, n * 16, cudaMemcpyHostToDevice, c->stream));
+        WG_CUDA_OK(host_copy(&c->hc, c->device, c->d_alive, alive, n * 4, cudaMemcpyHostToDevice, c->stream));
     }
     TRY(score_dev(c, c->d_rad_raw, c->d_alive, n, 0.4, 0, lcg_state, out));
-    if (hits) WG_CUDA_OK(cudaMemcpy(hits, c->d_hits, (size_t)c->dna.n_bp * 2, cudaMemcpyDeviceToHost));
+    if (hits) TRY(hits_out(c, hits));
     return WGDNA_OK;
 }
 
@@ -993,7 +1002,7 @@ static int dose_source(wgdna_ctx* c, const uint32_t* dose, const uint32_t** out)
     const size_t nv = (size_t)c->cfg.vc * c->cfg.vc * c->cfg.vc;
     if (dose) {
         if (!c->d_dose_in) TRY(dalloc(&c->d_dose_in, nv));
-        WG_CUDA_OK(cudaMemcpyAsync(c->d_dose_in, dose, nv * 4, cudaMemcpyHostToDevice, c->stream));
+        WG_CUDA_OK(host_copy(&c->hc, c->device, c->d_dose_in, dose, nv * 4, cudaMemcpyHostToDevice, c->stream));
         *out = c->d_dose_in;
         return WGDNA_OK;
     }
@@ -1089,7 +1098,7 @@ extern "C" int wgdna_chem_grid(wgdna_ctx* c, const float* rad, uint64_t rad_n, u
     if (rad) {
         n_all = rad_n;
         if (rad_n > c->cg_rad_cap) { TRY(dalloc(&c->d_cg_rad, rad_n)); c->cg_rad_cap = rad_n; }
-        WG_CUDA_OK(cudaMemcpyAsync(c->d_cg_rad, rad, rad_n * 16, cudaMemcpyHostToDevice, s));
+        WG_CUDA_OK(host_copy(&c->hc, c->device, c->d_cg_rad, rad, rad_n * 16, cudaMemcpyHostToDevice, s));
         src = c->d_cg_rad;
     } else {
         if (!c->have_transport) { wg_set_error("wgdna_chem_grid: no rad_buf (pass one or run wgdna_transport)"); return WGDNA_ERR_STATE; }
@@ -1118,8 +1127,8 @@ extern "C" int wgdna_chem_grid(wgdna_ctx* c, const float* rad, uint64_t rad_n, u
     WG_CUDA_OK(cudaEventRecord(c->ev[5], s));
     uint32_t counts[40];
     WG_CUDA_OK(cudaMemcpyAsync(counts, c->d_cg_counts, sizeof counts, cudaMemcpyDeviceToHost, s));
-    if (pos && cap >= n) WG_CUDA_OK(cudaMemcpyAsync(pos, c->d_cg_pos, (size_t)n * 16, cudaMemcpyDeviceToHost, s));
-    if (alive && cap >= n) WG_CUDA_OK(cudaMemcpyAsync(alive, c->d_cg_alive, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
+    if (pos && cap >= n) WG_CUDA_OK(host_copy(&c->hc, c->device, pos, c->d_cg_pos, (size_t)n * 16, cudaMemcpyDeviceToHost, s));
+    if (alive && cap >= n) WG_CUDA_OK(host_copy(&c->hc, c->device, alive, c->d_cg_alive, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
     WG_CUDA_OK(cudaStreamSynchronize(s));
     out->ms = elapsed_ms(c->ev[4], c->ev[5]);
     out->chem_n = n;
