@@ -147,9 +147,10 @@ __device__ __forceinline__ double pdc_x(double a, double b, double pq, double M,
 //   Its draws are the upper words alone (U1 and 1 - U1 within 2^-27, so X to 2.2e-4
 //   and e to 2.2e-4 b^2/X relative when both exceed 1.2e-4, else the trial goes on;
 //   U2 rounded down); 3 % + 1e-3 b^2/X covers that.
-// Only a warp with a trial left evaluates the bracket (54 % of the rounds).
-// Measured in the pairing kernel (4096 x 10 keV, 6.5 M calls): 4.5 ms; 5.1 ms
-// with the bracket in every round and 6 ms with the f64 set-up in every lane.
+// Only what is left meets the bracket.  Measured in the pairing kernel (4096 x 10 keV,
+// 6.5 M calls): 2.8 ms with a pair to a lane (pdc_queue), 3.7 ms by whole warps
+// (pdc_find), there 5.1 ms with the bracket in every round and 6 ms with the f64
+// set-up in every lane.
 //
 // A trial is accepted when U2 <= lambdax (X <= 2b/a) or U2 M / X <= lambdax
 // (X >= 2b/a), lambdax = e (1 - Q), e = exp(-b^2/X), Q = a sqrt(pi X)
@@ -175,11 +176,88 @@ __device__ __forceinline__ double pdc_x(double a, double b, double pq, double M,
 // itself widened by 2e-6 relative and 1e-30, with a further margin of 1e-6
 // (5e-6).  Trials inside the bracket, near X = 2b/a, z < 0, or with a zero draw
 // are evaluated exactly in f64.
-__device__ __forceinline__ float rcp_fast(float x) { return __fdividef(1.0f, x); }
+__device__ __forceinline__ float rcp_fast(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float exp_fast(float x) {                 // 0 below 2^-126
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.4426950f));
+    return r;
+}
 
-template <class Philox>
+// the upper bound: false when the trial is surely rejected
+__device__ __forceinline__ bool pdc_maybe(const u4& w, float thr, float hpq, float qpq, float Mf, float t2f, float af, float bf) {
+    const float u = __uint2float_rd(w.x) * 0x1p-32f, v = 1.0f - u;
+    const bool ca = u < thr;
+    const float q = ca ? u * hpq : v * qpq;             // sqrt(X), or its reciprocal
+    const float r = rcp_fast(q);
+    const float hx = ca ? q : r, rs = ca ? r : q;
+    const float y = bf * rs, arg = y * y, iz = rcp_fast(fmaf(af, hx, y));
+    const float lam = fmaxf(exp_fast(-arg), 1e-30f) * iz * fmaf(0.5f, iz, y) * fmaf(1e-3f, arg, 1.03f);
+    const float mult = hx * hx < t2f * 1.001f ? 1.0f : Mf * rs * rs;
+    const bool rej = __uint2float_rd(w.z) * 0x1p-32f * mult > lam;
+    return !(rej && fminf(u, v) > 1.2e-4f && bf >= 0.0f);
+}
+// the bracket: 0 rejected, 1 accepted, 2 undecided
+__device__ __forceinline__ int pdc_bracket(const u4& w, float thr, float pqf, float Mf, float t2f, float bbf, float af, float bf) {
+    const uint32_t ah = w.x >> 5, al = w.y >> 6;
+    const float u1 = fmaf((float)ah, 0x1p-27f, (float)al * 0x1p-53f);
+    const float v1 = fmaf((float)(0x7ffffffu - ah), 0x1p-27f, (float)(0x4000000u - al) * 0x1p-53f);   // 1 - U1
+    const float u2 = fmaf((float)(w.z >> 5), 0x1p-27f, (float)(w.w >> 6) * 0x1p-53f);
+    const float hx = u1 < thr ? u1 * pqf * 0.5f : __fdividef(2.0f * Mf, v1 * pqf);
+    const float xf = hx * hx;
+    const bool ca = xf < t2f * 0.99999f, cb = xf > t2f * 1.00001f;
+    if (!(u2 > 0.0f && xf > 1e-30f && xf < 1.0e30f && (ca || cb) && fabsf(u1 - thr) > thr * 1e-6f)) return 2;
+    const float rs = rsqrtf(xf);
+    const float argf = bbf * rs * rs;
+    float elo = 0.0f, ehi = 1e-30f;
+    if (argf <= 80.0f) {
+        const float ef = __expf(-argf), re = argf * 4e-6f + 2e-6f;
+        elo = ef * (1.0f - re); ehi = ef * (1.0f + re);
+    }
+    const float sx = xf * rs;
+    const float zf = bf * rs + af * sx;
+    if (!(zf >= 0.0f)) return 2;
+    float flo, fhi;
+    if (zf >= 6.0f && bf >= 0.0f) {
+        const float iz = __frcp_rn(zf), h = 0.5f * iz * iz;
+        float s = 1.0f - 13.0f * h;
+        s = 1.0f - 11.0f * h * s; s = 1.0f - 9.0f * h * s; s = 1.0f - 7.0f * h * s;
+        s = 1.0f - 5.0f * h * s; s = 1.0f - 3.0f * h * s;
+        const float omq = fmaf(af * sx * iz, h * s, bf * rs * iz);
+        flo = omq * 0.99998f - 1e-14f; fhi = omq * 1.00002f + 1e-14f;
+    } else {
+        const float Q = af * 1.7724539f * sx * erfcx_f(zf);
+        flo = 1.0f - Q * 1.00002f - 1e-6f; fhi = 1.0f - Q * 0.99998f + 1e-6f;
+    }
+    const float Llo = elo * fmaxf(flo, 0.0f) * (1.0f - 2e-6f) - 1e-30f;
+    const float Lhi = ehi * fmaxf(fhi, 0.0f) * (1.0f + 2e-6f) + 1e-30f;
+    if (ca) return u2 <= Llo * (1.0f - 1e-6f) ? 1 : (u2 > Lhi * (1.0f + 1e-6f) ? 0 : 2);
+    const float lhs = u2 * Mf;
+    return lhs <= Llo * xf * (1.0f - 5e-6f) ? 1 : (lhs > Lhi * xf * (1.0f + 5e-6f) ? 0 : 2);
+}
+// the trial in f64 (:97-110)
+__device__ __forceinline__ bool pdc_exact(const u4& w, double da, double db) {
+    const double t2 = 2.0 * db / da, r = sqrt(t2), M = fmax(1.0 / (da * da), 3.0 * db / da);
+    const double pq = 2.0 * r + 2.0 / r * M;
+    const double X = pdc_x(da, db, pq, M, w.x, w.y), U2 = u01d(w.z, w.w);
+    // lambdax <= e: a trial that fails against e alone is rejected
+    // without evaluating erfcx (same decision as the full test)
+    const double e = exp_(-db * db / X);
+    const double v = U2 * M / X;
+    if (!((X <= t2 && U2 <= e) || (X >= t2 && v <= e))) return false;
+    const double sqX = sqrt(X);
+    const double lambdax = e * (1.0 - da * sqrt(3.141592653589793 * X) * erfcx_(db / sqX + da * sqX));
+    return (X <= t2 && U2 <= lambdax) || (X >= t2 && v <= lambdax);
+}
+
+// One pair by the whole warp, 32 trials at a time from trial `first` on; all 32 lanes
+// call.  What a pair costs this way: 59 evaluated trials (42 up to the accepted
+// one), and the bracket in 54 % of the rounds, for one lane or two.
 __device__ __forceinline__ uint64_t pdc_find(int src, uint32_t i, uint32_t j, uint32_t pid, const PdcPair& P, double a,
-                                             double b, int lane, Philox philox_pdc) {
+                                             double b, int lane, const uint32_t* rk, uint32_t first = 0) {
     const uint32_t qi = __shfl_sync(0xffffffffu, i, src), qj = __shfl_sync(0xffffffffu, j, src);
     const float thr = __shfl_sync(0xffffffffu, P.thr, src), pqf = __shfl_sync(0xffffffffu, P.pqf, src);
     const float Mf = __shfl_sync(0xffffffffu, P.Mf, src), t2f = __shfl_sync(0xffffffffu, P.t2f, src);
@@ -187,79 +265,15 @@ __device__ __forceinline__ uint64_t pdc_find(int src, uint32_t i, uint32_t j, ui
     const float bf = __shfl_sync(0xffffffffu, P.bf, src);
     const float hpq = 0.5f * pqf, qpq = __fdividef(0.5f * pqf, Mf);
 #pragma unroll 1
-    for (uint32_t t0 = 0; t0 < 10000; t0 += 32) {
+    for (uint32_t t0 = first; t0 < 10000; t0 += 32) {
         const uint32_t trial = t0 + lane;
-        const u4 w = philox_pdc(qi, qj, pid, 4u | (trial << 4));
-        int st = 0;                               // 0 rejected, 1 accepted, 2 undecided
-        {
-            const float u = __uint2float_rd(w.x) * 0x1p-32f, v = 1.0f - u;
-            const bool ca = u < thr;
-            const float q = ca ? u * hpq : v * qpq;             // sqrt(X), or its reciprocal
-            const float r = rcp_fast(q);
-            const float hx = ca ? q : r, rs = ca ? r : q;
-            const float y = bf * rs, arg = y * y, iz = rcp_fast(fmaf(af, hx, y));
-            const float lam = fmaxf(__expf(-arg), 1e-30f) * iz * fmaf(0.5f, iz, y) * fmaf(1e-3f, arg, 1.03f);
-            const float mult = hx * hx < t2f * 1.001f ? 1.0f : Mf * rs * rs;
-            const bool rej = __uint2float_rd(w.z) * 0x1p-32f * mult > lam;
-            if (trial < 10000 && !(rej && fminf(u, v) > 1.2e-4f && bf >= 0.0f)) st = 2;
-        }
+        const u4 w = philox_rk(qi, qj, pid, 4u | (trial << 4), rk);
+        int st = trial < 10000 && pdc_maybe(w, thr, hpq, qpq, Mf, t2f, af, bf) ? 2 : 0;
         if (!__any_sync(0xffffffffu, st != 0)) continue;
-        const uint32_t ah = w.x >> 5, al = w.y >> 6;
-        const float u1 = fmaf((float)ah, 0x1p-27f, (float)al * 0x1p-53f);
-        const float v1 = fmaf((float)(0x7ffffffu - ah), 0x1p-27f, (float)(0x4000000u - al) * 0x1p-53f);   // 1 - U1
-        const float u2 = fmaf((float)(w.z >> 5), 0x1p-27f, (float)(w.w >> 6) * 0x1p-53f);
-        const float hx = u1 < thr ? u1 * pqf * 0.5f : __fdividef(2.0f * Mf, v1 * pqf);
-        const float xf = hx * hx;
-        const bool ca = xf < t2f * 0.99999f, cb = xf > t2f * 1.00001f;
-        if (st != 0 && u2 > 0.0f && xf > 1e-30f && xf < 1.0e30f && (ca || cb) && fabsf(u1 - thr) > thr * 1e-6f) {
-            const float rs = rsqrtf(xf);
-            const float argf = bbf * rs * rs;
-            float elo = 0.0f, ehi = 1e-30f;
-            if (argf <= 80.0f) {
-                const float ef = __expf(-argf), re = argf * 4e-6f + 2e-6f;
-                elo = ef * (1.0f - re); ehi = ef * (1.0f + re);
-            }
-            const float sx = xf * rs;
-            const float zf = bf * rs + af * sx;
-            if (zf >= 0.0f) {
-                float flo, fhi;
-                if (zf >= 6.0f && bf >= 0.0f) {
-                    const float iz = __frcp_rn(zf), h = 0.5f * iz * iz;
-                    float s = 1.0f - 13.0f * h;
-                    s = 1.0f - 11.0f * h * s; s = 1.0f - 9.0f * h * s; s = 1.0f - 7.0f * h * s;
-                    s = 1.0f - 5.0f * h * s; s = 1.0f - 3.0f * h * s;
-                    const float omq = fmaf(af * sx * iz, h * s, bf * rs * iz);
-                    flo = omq * 0.99998f - 1e-14f; fhi = omq * 1.00002f + 1e-14f;
-                } else {
-                    const float Q = af * 1.7724539f * sx * erfcx_f(zf);
-                    flo = 1.0f - Q * 1.00002f - 1e-6f; fhi = 1.0f - Q * 0.99998f + 1e-6f;
-                }
-                const float Llo = elo * fmaxf(flo, 0.0f) * (1.0f - 2e-6f) - 1e-30f;
-                const float Lhi = ehi * fmaxf(fhi, 0.0f) * (1.0f + 2e-6f) + 1e-30f;
-                if (ca) st = u2 <= Llo * (1.0f - 1e-6f) ? 1 : (u2 > Lhi * (1.0f + 1e-6f) ? 0 : 2);
-                else {
-                    const float lhs = u2 * Mf;
-                    st = lhs <= Llo * xf * (1.0f - 5e-6f) ? 1 : (lhs > Lhi * xf * (1.0f + 5e-6f) ? 0 : 2);
-                }
-            }
-        }
+        if (st != 0) st = pdc_bracket(w, thr, pqf, Mf, t2f, bbf, af, bf);
         if (__any_sync(0xffffffffu, st == 2)) {
             const double da = __shfl_sync(0xffffffffu, a, src), db = __shfl_sync(0xffffffffu, b, src);
-            if (st == 2) {
-                const double t2 = 2.0 * db / da, r = sqrt(t2), M = fmax(1.0 / (da * da), 3.0 * db / da);
-                const double pq = 2.0 * r + 2.0 / r * M;
-                const double X = pdc_x(da, db, pq, M, w.x, w.y), U2 = u01d(w.z, w.w);
-                // lambdax <= e: a trial that fails against e alone is rejected
-                // without evaluating erfcx (same decision as the full test)
-                const double e = exp_(-db * db / X);
-                const double v = U2 * M / X;
-                st = 0;
-                if ((X <= t2 && U2 <= e) || (X >= t2 && v <= e)) {
-                    const double sqX = sqrt(X);
-                    const double lambdax = e * (1.0 - da * sqrt(3.141592653589793 * X) * erfcx_(db / sqX + da * sqX));
-                    st = ((X <= t2 && U2 <= lambdax) || (X >= t2 && v <= lambdax)) ? 1 : 0;
-                }
-            }
+            if (st == 2) st = pdc_exact(w, da, db) ? 1 : 0;
         }
         const unsigned m = __ballot_sync(0xffffffffu, st == 1);
         if (m) {
@@ -545,12 +559,39 @@ __device__ __forceinline__ u4 philox_accept(uint32_t blk, uint32_t i, uint32_t p
 //    arithmetic.  Each lane keeps its candidates in its own column of shared memory
 //    (no vote per pair); a full column makes the warp pack all columns and
 //    evaluate them exactly in f64, 32 at a time, one per lane.
-//    Measured at 4096 x 10 keV: 9.5 ms; 10.5 ms with the rare f64 erfcx inline (the
-//    instruction cache, as in the event kernel), 14.9 ms with tiles in index order, one
-//    table gather per pair and queue votes per partner (5, 6, 7 blocks per SM:
-//    10.8, 10.5, 10.5 ms).
+//    The distances, the bound's products and the counts' sums run two to an
+//    instruction (f32x2: one issue slot for both).
+//    Measured at 4096 x 10 keV: 8.2 ms, of which the scan is 4.7, SamplePDC 2.8; 9.1 ms
+//    with every SamplePDC pair through pdc_find at once, 9.5 ms also without f32x2,
+//    10.5 ms also with the rare f64 erfcx inline (the instruction cache, as in the event
+//    kernel), 14.9 ms also with tiles in index order, one table gather per pair and
+//    queue votes per partner (4, 5, 6, 7 blocks per SM: 9.0, 8.2, 8.2, 8.4 ms).
 constexpr int QCAP = 16;                 // candidates per lane
 constexpr float FAR = 1e18f;             // shadow coordinate of a partner that cannot react
+
+// two f32 values in a register pair; the packed instructions take one issue slot for both
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 
 struct InitTrack {
     const double *px, *py, *pz;
@@ -559,18 +600,27 @@ struct InitTrack {
     double* ET;
     uint32_t* EAB;
     uint32_t* tev;
-    uint32_t ecp, pid;
+    uint32_t ecp, pid, p;
     float lo2;                           // shadow distance^2 below which a pair is certainly inside R_CUT
 };
 
+// a warp's SamplePDC pairs: b, (i, j), track, and reaction | kinds | trial
+constexpr int PDC_WAIT = 12, PDC_KEEP = 26, PDC_FEW = 20;
+constexpr uint32_t PDC_Q = 96;
+struct PdcQueue {
+    double b[PDC_Q], lb[32];             // lb: of the pairs in the lanes
+    uint32_t ij[PDC_Q], p[PDC_Q], kt[PDC_Q];
+};
+
 // exact evaluation of queued candidates [0, cnt), one per lane; returns the
-// reactive pairs inside R_CUT found among those within rounding of it
+// reactive pairs inside R_CUT found among those within rounding of it.  SamplePDC's pairs
+// join the warp's queue Q (room for 32).
 __device__ __forceinline__ uint32_t init_batch(const IrtConst& C, const InitTrack& T, const uint32_t* qij, int cnt,
-                                               int lane, const uint32_t* rk, bool& ev_over) {
+                                               int lane, const uint32_t* rk, bool& ev_over, PdcQueue& Q, uint32_t& qn) {
     const unsigned lt = (1u << lane) - 1u;
     bool acc = false, pdcq = false;
-    double t = 0, pa = 1, pb = 1, pD = 1;
-    uint32_t i = 0, j = 0, np = 0;
+    double t = 0, pa = 1, pb = 1;
+    uint32_t i = 0, j = 0, np = 0, kinds = 0;
     if (lane < cnt) {
         const uint32_t ij = qij[lane];
         i = ij >> 16; j = ij & 0xffffu;
@@ -590,26 +640,19 @@ __device__ __forceinline__ uint32_t init_batch(const IrtConst& C, const InitTrac
             if (r2 <= R * R) {
                 const double D = C.D[si] + C.D[sj];
                 t = sample_pre(C, sqrt(r2), ri, D, U, &pa, &pb);
-                if (t == -2.0) { pdcq = true; pD = D; }
+                if (t == -2.0) { pdcq = true; kinds = (uint32_t)(ri | si << 4 | sj << 8); }
                 else acc = (t >= 0 && t < 1000);
             }
         }
     }
-    unsigned pm = __ballot_sync(FULL, pdcq);
+    const unsigned pm = __ballot_sync(FULL, pdcq);
     if (pm) {
-        const PdcPair P = pdc_pair(pa, pb);
-        uint64_t words = ~0ull;
-        while (pm) {
-            const int src = __ffs(pm) - 1;
-            pm &= pm - 1;
-            const uint64_t wd = pdc_find(src, i, j, T.pid, P, pa, pb, lane,
-                                         [rk](uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) { return philox_rk(c0, c1, c2, c3, rk); });
-            if (lane == src) words = wd;
+        if (pdcq) {
+            const uint32_t at = qn + __popc(pm & lt);
+            Q.b[at] = pb; Q.ij[at] = (i << 16) | j; Q.p[at] = T.p; Q.kt[at] = kinds;
         }
-        if (pdcq && words != ~0ull) {
-            const double X = pdc_x(pa, pb, P.pq, P.M, (uint32_t)(words >> 32), (uint32_t)words);
-            if (X > 0) { t = X / pD; acc = t < 1000; }
-        }
+        qn += __popc(pm);
+        __syncwarp();
     }
     const unsigned m = __ballot_sync(FULL, acc);
     if (m) {
@@ -625,16 +668,103 @@ __device__ __forceinline__ uint32_t init_batch(const IrtConst& C, const InitTrac
     return np;
 }
 
-#ifndef WG_INIT_MINB
-#define WG_INIT_MINB 6
-#endif
-__global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(const __grid_constant__ IArgs A) {
+// SamplePDC of the queued pairs, a pair to a lane: every lane goes through its own
+// pair's trials in order, all of them needed (pdc_find evaluates 42 % more), until
+// PDC_WAIT lanes have one that passes the upper bound; these take the bracket and their
+// pair's end together, and idle lanes take the next pairs.  The queue must not be empty.
+// With `all` false, what is left when the queue is empty and less than PDC_KEEP lanes have a
+// pair goes back to the queue, with its place in the trials; otherwise the last PDC_FEW
+// pairs go through pdc_find, whose rounds are 32 trials of one pair: a few pairs need
+// thousands of trials.
+// Measured (pairing kernel, ms, every pair through pdc_find and this): 4096 tracks of 10 keV
+// 9.05 and 8.24, 4096 of 1 keV 0.78 and 0.61, 64 of 10 keV 0.42 and 0.31; PDC_WAIT 8, 12,
+// 16: 8.30, 8.24, 8.33; PDC_FEW 6, 12, 20: 64 tracks 0.64, 0.40, 0.36.
+__device__ __forceinline__ void pdc_queue(const IArgs& A, const IrtConst& C, PdcQueue& Q, uint32_t& qn, bool all, int lane,
+                                          bool& ev_over) {
+    const unsigned lt = (1u << lane) - 1u;
+    bool act = false, pend = false;
+    uint32_t ij = 0, p = 0, kinds = 0, trial = 0;
+    PdcPair P = {};
+    u4 w = {0, 0, 0, 0};
+    float hpq = 0, qpq = 0;
+    auto event = [&](uint32_t wx, uint32_t wy) {
+        const double X = pdc_x(C.a_pdc[kinds & 15u], Q.lb[lane], P.pq, P.M, wx, wy);
+        if (!(X > 0)) return;
+        const double t = X / (C.D[kinds >> 4 & 15u] + C.D[kinds >> 8]);
+        if (!(t < 1000)) return;
+        const uint32_t slot = atomicAdd(&A.tev[p], 1u);
+        if (slot < ecap(A, p)) { A.ev_t[ebase(A, p) + slot] = t; A.ev_ab[ebase(A, p) + slot] = ij; }
+        else ev_over = true;
+    };
+    for (;;) {
+        const unsigned idle = __ballot_sync(FULL, !act);
+        if (idle && qn) {
+            const uint32_t take = min((uint32_t)__popc(idle), qn), rank = __popc(idle & lt);
+            if (!act && rank < take) {
+                const uint32_t at = qn - 1 - rank;
+                ij = Q.ij[at]; p = Q.p[at];
+                kinds = Q.kt[at] & 0xfffu; trial = Q.kt[at] >> 12;
+                const double b = Q.b[at];
+                Q.lb[lane] = b;
+                P = pdc_pair(C.a_pdc[kinds & 15u], b);
+                hpq = 0.5f * P.pqf; qpq = __fdividef(0.5f * P.pqf, P.Mf);
+                act = true;
+            }
+            qn -= take;
+            __syncwarp();
+        }
+        unsigned run = __ballot_sync(FULL, act);
+        if (!run) break;
+        if (qn == 0 && !all && __popc(run) < PDC_KEEP) {
+            if (act) {
+                const uint32_t at = __popc(run & lt);
+                Q.b[at] = Q.lb[lane]; Q.ij[at] = ij; Q.p[at] = p; Q.kt[at] = kinds | trial << 12;
+            }
+            qn = __popc(run);
+            __syncwarp();
+            break;
+        }
+        if (qn == 0 && __popc(run) <= PDC_FEW) {
+            do {
+                const int src = __ffs(run) - 1;
+                run &= run - 1;
+                const uint32_t pid = A.pid_base + __shfl_sync(FULL, p, src);
+                const double a = C.a_pdc[kinds & 15u], b = Q.lb[lane];
+                const uint64_t wd = pdc_find(src, ij >> 16, ij & 0xffffu, pid, P, a, b, lane, A.rk, __shfl_sync(FULL, trial, src));
+                if (lane == src && wd != ~0ull) event((uint32_t)(wd >> 32), (uint32_t)wd);
+            } while (run);
+            break;
+        }
+        // trials until enough lanes wait
+        int waiting = 0;
+#pragma unroll 1
+        do {
+            if (act && !pend) {
+                w = philox_rk(ij >> 16, ij & 0xffffu, A.pid_base + p, 4u | (trial << 4), A.rk);
+                pend = pdc_maybe(w, P.thr, hpq, qpq, P.Mf, P.t2f, P.af, P.bf);
+                if (!pend && ++trial == 10000) act = false;
+            }
+            waiting = __popc(__ballot_sync(FULL, pend));
+            run = __ballot_sync(FULL, act && !pend);
+        } while (run && waiting < PDC_WAIT && waiting + __popc(run) > PDC_FEW);
+        if (pend) {
+            int st = pdc_bracket(w, P.thr, P.pqf, P.Mf, P.t2f, P.bbf, P.af, P.bf);
+            if (st == 2) st = pdc_exact(w, C.a_pdc[kinds & 15u], Q.lb[lane]) ? 1 : 0;
+            if (st == 1) { event(w.x, w.y); act = false; }
+            else if (++trial == 10000) act = false;
+            pend = false;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(IB, 5) k_irt_init(const __grid_constant__ IArgs A) {
     __shared__ IrtConst s_c;
     __shared__ uint32_t s_row[6];
-    // partners of a chunk: shadow x, y, z and the bound's kb and fk (scaled to 16-bit U)
+    // partners of a chunk: negated shadow x, y, z and the bound's kb and fk (scaled to 16-bit U)
     __shared__ __align__(16) float s_p[IB / 32][5][32];
     __shared__ uint16_t s_q[IB / 32][QCAP][32];
     __shared__ uint32_t s_d[IB / 32][QCAP * 32 + 32];
+    __shared__ PdcQueue s_pdc[IB / 32];
     load_consts(&s_c, s_row);
     const IrtConst& C = s_c;
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -643,6 +773,7 @@ __global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(const __grid_cons
     float (*sp)[32] = s_p[wl];
     uint32_t* dq = s_d[wl];
     unsigned long long n_pairs = 0;
+    uint32_t qn = 0;
     bool ev_over = false;
     for (;;) {
         unsigned long long item = 0;
@@ -671,12 +802,13 @@ __global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(const __grid_cons
         const float clo = (rcut - del) * 0.99999f, chi = (rcut + del) * 1.00001f;
         const float lo2 = clo * clo, hi2 = chi * chi, lo2s = lo2 * 0x1p100f, hi2s = hi2 * 0x1p100f;
         const InitTrack T{A.px + tb0, A.py + tb0, A.pz + tb0, pf, A.sp + tb0, A.ev_t + ebase(A, p), A.ev_ab + ebase(A, p),
-                          &A.tev[p], ecap(A, p), A.pid_base + p, lo2};
+                          &A.tev[p], ecap(A, p), A.pid_base + p, p, lo2};
         const uint32_t at = 32u * tile + lane;
         const bool have = at < len;
         const uint32_t i = have ? A.lst[6 * tb0 + (size_t)s * cap + at] : 0xffffu;
         float4 me = make_float4(-3.0f * FAR, 0.f, 0.f, 0.f);
         if (have) me = A.rec[6 * tb0 + (size_t)s * cap + at];
+        const f32x2 mx = pack2(me.x, me.x), my = pack2(me.y, me.y), mz = pack2(me.z, me.z);
         float ta2 = 0.0f;                             // (r_acc's radius for U -> 1)^2, over the row's reactions
         for (int q = 0; q < 6; ++q) {
             const int r = (int)((row >> (4 * q)) & 15u);
@@ -699,20 +831,18 @@ __global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(const __grid_cons
                     if (r == 15) q.x = FAR;
                     else { kb = (C.fkb0[r] + del) * 1.00006f; fk = C.fk[r] * (65536.0f * 1.00006f); }
                 }
-                sp[0][lane] = q.x; sp[1][lane] = q.y; sp[2][lane] = q.z; sp[3][lane] = kb; sp[4][lane] = fk;
+                sp[0][lane] = -q.x; sp[1][lane] = -q.y; sp[2][lane] = -q.z; sp[3][lane] = kb; sp[4][lane] = fk;
                 __syncwarp();
             }
             const uint32_t k = (g & 7u) * 4u;
-            const float4 X = *reinterpret_cast<const float4*>(&sp[0][k]), Y = *reinterpret_cast<const float4*>(&sp[1][k]);
-            const float4 Z = *reinterpret_cast<const float4*>(&sp[2][k]);
+            const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(&sp[0][k]), Y = *reinterpret_cast<const ulonglong2*>(&sp[1][k]);
+            const ulonglong2 Z = *reinterpret_cast<const ulonglong2*>(&sp[2][k]);
             float r2[4];
             {
-                const float qx[4] = {X.x, X.y, X.z, X.w}, qy[4] = {Y.x, Y.y, Y.z, Y.w}, qz[4] = {Z.x, Z.y, Z.z, Z.w};
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const float dx = me.x - qx[u], dy = me.y - qy[u], dz = me.z - qz[u];
-                    r2[u] = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                }
+                const f32x2 x0 = add2(mx, X.x), y0 = add2(my, Y.x), z0 = add2(mz, Z.x);
+                const f32x2 x1 = add2(mx, X.y), y1 = add2(my, Y.y), z1 = add2(mz, Z.y);
+                unpack2(fma2(z0, z0, fma2(y0, y0, mul2(x0, x0))), r2[0], r2[1]);
+                unpack2(fma2(z1, z1, fma2(y1, y1, mul2(x1, x1))), r2[2], r2[3]);
             }
             if (4 * g <= imax) {                      // partners not after i do not count
 #pragma unroll
@@ -721,25 +851,33 @@ __global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(const __grid_cons
             // pairs surely inside R_CUT, and those that may be: sums of saturated
             // differences (the sign decides, 2^100 makes any difference 1), which run on the
             // FP32 pipe; a compare and a count would each take two cycles of the integer one
-            float nlo = 0.0f, nhi = 0.0f;
+            float lo4[4], hi4[4], nlo, nhi, nl1, nh1;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                nlo += __saturatef(fmaf(r2[u], -0x1p100f, lo2s));
-                nhi += __saturatef(fmaf(r2[u], -0x1p100f, hi2s));
+                lo4[u] = __saturatef(fmaf(r2[u], -0x1p100f, lo2s));
+                hi4[u] = __saturatef(fmaf(r2[u], -0x1p100f, hi2s));
             }
+            unpack2(add2(pack2(lo4[0], lo4[1]), pack2(lo4[2], lo4[3])), nlo, nl1);
+            unpack2(add2(pack2(hi4[0], hi4[1]), pack2(hi4[2], hi4[3])), nhi, nh1);
+            nlo += nl1;
+            nhi += nh1;
             if (nhi > 0.0f) {
-                const float4 KB = *reinterpret_cast<const float4*>(&sp[3][k]), FK = *reinterpret_cast<const float4*>(&sp[4][k]);
-                const float kb[4] = {KB.x, KB.y, KB.z, KB.w}, fk[4] = {FK.x, FK.y, FK.z, FK.w};
+                const ulonglong2 KB = *reinterpret_cast<const ulonglong2*>(&sp[3][k]), FK = *reinterpret_cast<const ulonglong2*>(&sp[4][k]);
                 const u4 cw = philox_accept(g, i, T.pid, A.rk);
                 const uint32_t wd[4] = {cw.x, cw.y, cw.z, cw.w};
                 np += nlo;
-                float v[4];
+                float v[4], uw[4];
+                // 2^23 + the word's upper 16 bits, minus 2^23
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    // 2^23 + the word's upper 16 bits, minus 2^23
-                    const float uf = __uint_as_float(__byte_perm(wd[u], 0x4B000000u, 0x7632)) - 8388608.0f;
-                    const float rhs = fmaf(kb[u], uf, fk[u]);
-                    v[u] = fmaf(rhs, rhs, -(r2[u] * (uf * uf)));
+                for (int u = 0; u < 4; ++u) uw[u] = __uint_as_float(__byte_perm(wd[u], 0x4B000000u, 0x7632));
+#pragma unroll
+                for (int u = 0; u < 4; u += 2) {
+                    const f32x2 uf = add2(pack2(uw[u], uw[u + 1]), pack2(-8388608.0f, -8388608.0f));
+                    float ra, rb, wa, wb;
+                    unpack2(fma2(u ? KB.y : KB.x, uf, u ? FK.y : FK.x), ra, rb);
+                    unpack2(mul2(pack2(r2[u], r2[u + 1]), mul2(uf, uf)), wa, wb);
+                    v[u] = fmaf(ra, ra, -wa);
+                    v[u + 1] = fmaf(rb, rb, -wb);
                 }
                 const float mn = fminf(fminf(fminf(r2[0], r2[1]), r2[2]), r2[3]);
                 if (fmaxf(fmaxf(fmaxf(v[0], v[1]), v[2]), v[3]) >= 0.0f || nhi != nlo || mn <= ta2) {
@@ -763,8 +901,10 @@ __global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(const __grid_cons
                 cnt = 0;
                 __syncwarp();
                 uint32_t b = 0;
-                for (; b + (last ? 1u : 32u) <= total; b += 32)
-                    n_pairs += init_batch(C, T, dq + b, (int)min(32u, total - b), lane, A.rk, ev_over);
+                for (; b + (last ? 1u : 32u) <= total; b += 32) {
+                    n_pairs += init_batch(C, T, dq + b, (int)min(32u, total - b), lane, A.rk, ev_over, s_pdc[wl], qn);
+                    if (qn > PDC_Q - 32) pdc_queue(A, C, s_pdc[wl], qn, false, lane, ev_over);
+                }
                 rem = 0;
                 if (b < total) {
                     rem = total - b;
@@ -777,6 +917,7 @@ __global__ void __launch_bounds__(IB, WG_INIT_MINB) k_irt_init(const __grid_cons
         }
         n_pairs += (unsigned long long)np;
     }
+    if (qn) pdc_queue(A, C, s_pdc[wl], qn, true, lane, ev_over);
     if (__any_sync(FULL, ev_over) && lane == 0) atomicOr(A.err, DERR_HEAP);
     for (int o = 16; o; o >>= 1) n_pairs += __shfl_xor_sync(FULL, n_pairs, o);
     if (lane == 0 && n_pairs) atomicAdd(&A.acc[10], n_pairs);
@@ -1011,8 +1152,7 @@ __device__ __forceinline__ bool pair_exact(const IArgs& A, const IrtConst& C, un
         while (pm) {
             const int s = __ffs(pm) - 1;
             pm &= pm - 1;
-            const uint64_t wd = pdc_find(s, id, jj, pid, PP, pa, pb, lane,
-                                         [rk](uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) { return philox_rk(c0, c1, c2, c3, rk); });
+            const uint64_t wd = pdc_find(s, id, jj, pid, PP, pa, pb, lane, rk);
             if (lane == s) words = wd;
         }
         if (pdcq && words != ~0ull) {
@@ -1463,14 +1603,18 @@ static int loop_groups(int device, const IrtShape& shape) {
     return loop_blocks<W>(device, shape) * (LT<W> / 32 / W);
 }
 
-// tracks of the event kernel in flight at once, at most: each has its own scratch
+// tracks of the event kernel in flight at once, at most: each has its own scratch (asking for
+// the width in use alone keeps the other widths' code from being loaded)
 // (blocks hold up to 4 tracks, of which the last may be without one)
 int irt_warps(int device, const IrtShape& shape, uint32_t nseg) {
-    int n = loop_groups<1>(device, shape);
-    n = std::max(n, loop_groups<2>(device, shape));
-    n = std::max(n, loop_groups<4>(device, shape));
-    n = std::max(n, loop_groups<8>(device, shape));
-    n = std::max(n, loop_groups<16>(device, shape));
+    int n = 1;
+    switch (loop_width(device, nseg)) {
+    case 16: n = loop_groups<16>(device, shape); break;
+    case 8: n = loop_groups<8>(device, shape); break;
+    case 4: n = loop_groups<4>(device, shape); break;
+    case 2: n = loop_groups<2>(device, shape); break;
+    default: n = loop_groups<1>(device, shape);
+    }
     return (int)std::min((unsigned long long)n, ((unsigned long long)nseg + 3) & ~3ull);
 }
 
