@@ -105,6 +105,8 @@ struct wgdna_ctx {
     float4* d_rec = nullptr;
     float* d_tdel = nullptr;
     uint32_t irt_tracks = 0, irt_hcap = 0, irt_pcap = 0;
+    size_t irt_big = 0;
+    unsigned long long* d_irt_big = nullptr;
     double *d_px = nullptr, *d_py = nullptr, *d_pz = nullptr, *d_tb = nullptr;
     int8_t* d_sp = nullptr;
     uint8_t* d_alive8 = nullptr;
@@ -340,7 +342,7 @@ extern "C" void wgdna_destroy(wgdna_ctx* c) {
                     c->d_red, c->d_nsec, c->d_first, c->d_part, c->d_share, c->d_err, c->d_fy, c->d_fz, c->d_rbb0, c->d_rbb1, c->d_hits, c->d_alive,
                     c->sc.list, c->sc.seg, c->sc.u64,
                     c->sc.fib, c->d_px, c->d_py, c->d_pz, c->d_tb, c->d_sp, c->d_alive8, c->d_lst, c->d_lpos, c->d_evt, c->d_evab,
-                    c->d_hov_t, c->d_hov_ab, c->d_track, c->d_toff, c->d_irt_cnt, c->d_pf, c->d_rec, c->d_tdel, c->d_curves, c->d_acc_tl, c->d_acc, c->d_maxpid,
+                    c->d_hov_t, c->d_hov_ab, c->d_track, c->d_toff, c->d_irt_cnt, c->d_irt_big, c->d_pf, c->d_rec, c->d_tdel, c->d_curves, c->d_acc_tl, c->d_acc, c->d_maxpid,
                     c->d_dose_in, c->d_lambda, c->d_hits_in, c->d_dres, c->d_cg_pos, c->d_cg_rad, c->d_cg_alive,
                     c->d_cg_prod, c->d_cg_counts, c->d_cg_head, c->d_cg_next, c->d_cg_tab,
                     c->d_cg_cell, c->d_cg_rank, c->d_cg_sorted, c->d_cg_state};
@@ -395,6 +397,7 @@ static IArgs make_iargs(wgdna_ctx* c, uint32_t nseg, uint64_t seed) {
     a.pf = c->d_pf; a.rec = c->d_rec; a.tdel = c->d_tdel;
     a.hov_t = c->d_hov_t; a.hov_ab = c->d_hov_ab; a.hcap = c->irt_hcap; a.pcap = c->irt_pcap;
     a.counters = c->d_irt_cnt;
+    a.big = c->d_irt_big;
     a.acc_tl = c->d_acc_tl; a.acc = c->d_acc; a.err = c->d_err;
     return a;
 }
@@ -538,6 +541,7 @@ static int irt_ensure(wgdna_ctx* c, uint32_t nseg, uint64_t rad_n, uint32_t cap)
     size_t slots = 2 * (size_t)rad_n + 64 * (size_t)nseg;
     size_t evslots = 16 * (size_t)rad_n + 2048 * (size_t)nseg;
     // (rounded up, so that tracks of about the same size keep the captured launch sequence)
+    static_assert(IRT_PCAP_MIN == 1024, "");
     const uint32_t pcap = (cap + 1023u) & ~1023u, hcap = pcap * 8u + 4352u;
     const IrtShape shape{c->tune.irt_init_blocks_per_sm, c->tune.irt_loop_blocks_per_sm};
     size_t hov = (size_t)irt_warps(c->device, shape, nseg) * (hcap + (size_t)pcap);
@@ -567,7 +571,12 @@ static int irt_ensure(wgdna_ctx* c, uint32_t nseg, uint64_t rad_n, uint32_t cap)
         TRY(dalloc(&c->d_tdel, (size_t)nseg));
         c->irt_tracks = nseg;
     }
-    if (!c->d_irt_cnt) TRY(dalloc(&c->d_irt_cnt, 4));
+    if (!c->d_irt_cnt) TRY(dalloc(&c->d_irt_cnt, 8));
+    // a track of n entries has up to 8 n + 1024 events, in chunks of 2048 from 4097 on
+    if (rad_n / 128 + 64 > c->irt_big) {
+        TRY(dalloc(&c->d_irt_big, rad_n / 128 + 64));
+        c->irt_big = rad_n / 128 + 64;
+    }
     if (!c->d_acc_tl) TRY(dalloc(&c->d_acc_tl, 35));
     if (!c->d_acc) TRY(dalloc(&c->d_acc, 16));
     // the reaction constants live in __constant__ memory, which every device

@@ -925,10 +925,19 @@ __global__ void __launch_bounds__(IB, 5) k_irt_init(const __grid_constant__ IArg
 
 // 3) the initial events of each track in (t, i, j) order (:566): a block-wide
 //     bitonic sort, in shared memory up to SORT_SM events (padded to a power
-//     of two), in the track's own event slots beyond that (they hold 2 ecap).
+//     of two).  A larger track is cut into chunks that blocks of their own sort
+//     (k_irt_sort_chunks) and merge by rank into the second half of the track's event slots
+//     (they hold 2 ecap; k_irt_sort_merge): one block's bitonic sort of 16,626 events in
+//     global memory took 2.2 ms, bound by one SM's latency, this 0.06 ms.  These two
+//     kernels cost a launch each even when no track needs them, so they run only when
+//     tracks are long enough to have that many events as a rule (sort_chunked); a dense
+//     track below that is sorted in its slots by its one block.
 //     Keys are unique, so the order is that of any other sort.
 constexpr int SB = 256;
 constexpr uint32_t SORT_SM = 4096;
+constexpr int SCB = 512;
+constexpr uint32_t SORT_CH = 2048;       // events per chunk
+__device__ __forceinline__ bool sort_chunked(const IArgs& A, uint32_t nev) { return nev > SORT_SM && A.pcap > IRT_PCAP_MIN; }
 __global__ void __launch_bounds__(SB) k_irt_sort(IArgs A) {
     __shared__ double st[SORT_SM];
     __shared__ uint32_t sab[SORT_SM];
@@ -940,6 +949,14 @@ __global__ void __launch_bounds__(SB) k_irt_sort(IArgs A) {
         uint32_t* AB = A.ev_ab + ebase(A, p);
         uint32_t n2 = 2;
         while (n2 < nev) n2 <<= 1;
+        if (sort_chunked(A, nev)) {
+            const uint32_t nch = (nev + SORT_CH - 1) / SORT_CH;
+            if (threadIdx.x == 0) {
+                const uint32_t at = atomicAdd(&A.counters[4], nch);
+                for (uint32_t c = 0; c < nch; ++c) A.big[at + c] = (unsigned long long)p << 32 | c;
+            }
+            continue;
+        }
         const bool sm = n2 <= SORT_SM;
         double* t = sm ? st : T;
         uint32_t* ab = sm ? sab : AB;
@@ -962,6 +979,71 @@ __global__ void __launch_bounds__(SB) k_irt_sort(IArgs A) {
         }
         if (sm)
             for (uint32_t i = threadIdx.x; i < nev; i += SB) { T[i] = st[i]; AB[i] = sab[i]; }
+    }
+}
+
+__global__ void __launch_bounds__(SCB) k_irt_sort_chunks(const __grid_constant__ IArgs A) {
+    __shared__ double st[SORT_CH];
+    __shared__ uint32_t sab[SORT_CH];
+    const uint32_t n = A.counters[4];
+    for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) {
+        const uint32_t p = (uint32_t)(A.big[k] >> 32), c = (uint32_t)A.big[k];
+        double* T = A.ev_t + ebase(A, p) + c * SORT_CH;
+        uint32_t* AB = A.ev_ab + ebase(A, p) + c * SORT_CH;
+        const uint32_t len = min(SORT_CH, A.tev[p] - c * SORT_CH);
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < SORT_CH; i += SCB) {
+            st[i] = i < len ? T[i] : 1e300;
+            sab[i] = i < len ? AB[i] : 0xffffffffu;
+        }
+        __syncthreads();
+        for (uint32_t kk = 2; kk <= SORT_CH; kk <<= 1)
+            for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
+#pragma unroll
+                for (uint32_t q0 = 0; q0 < SORT_CH / 2; q0 += SCB) {
+                    const uint32_t q = q0 + threadIdx.x;
+                    const uint32_t i = ((q & ~(j - 1)) << 1) | (q & (j - 1)), l = i | j;   // bit j of i clear
+                    const double ti = st[i], tl = st[l];
+                    const uint32_t ai = sab[i], al = sab[l];
+                    if (ev_less(tl, al, ti, ai) == ((i & kk) == 0)) { st[i] = tl; st[l] = ti; sab[i] = al; sab[l] = ai; }
+                }
+                __syncthreads();
+            }
+        for (uint32_t i = threadIdx.x; i < len; i += SCB) { T[i] = st[i]; AB[i] = sab[i]; }
+    }
+}
+
+// an event's place: its place in its chunk plus the events before it in the track's others
+__global__ void __launch_bounds__(SB) k_irt_sort_merge(const __grid_constant__ IArgs A) {
+    __shared__ double st[SORT_CH];
+    __shared__ uint32_t sab[SORT_CH];
+    constexpr uint32_t PARTS = SORT_CH / SB;
+    const uint32_t n = A.counters[4] * PARTS;
+    for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) {
+        const unsigned long long e = A.big[k / PARTS];
+        const uint32_t p = (uint32_t)(e >> 32), c = (uint32_t)e, nev = A.tev[p];
+        double* T = A.ev_t + ebase(A, p);
+        uint32_t* AB = A.ev_ab + ebase(A, p);
+        const uint32_t i = c * SORT_CH + k % PARTS * SB + threadIdx.x;
+        if (i - threadIdx.x >= nev) continue;
+        const bool have = i < nev;
+        const double t = have ? T[i] : 0.0;
+        const uint32_t ab = have ? AB[i] : 0u;
+        uint32_t pos = i - c * SORT_CH;
+        for (uint32_t d = 0; d * SORT_CH < nev; ++d) {
+            if (d == c) continue;
+            const uint32_t len = min(SORT_CH, nev - d * SORT_CH);
+            __syncthreads();
+            for (uint32_t q = threadIdx.x; q < len; q += SB) { st[q] = T[d * SORT_CH + q]; sab[q] = AB[d * SORT_CH + q]; }
+            __syncthreads();
+            uint32_t lo = 0, hi = len;
+            while (lo < hi) {
+                const uint32_t m = (lo + hi) >> 1;
+                if (ev_less(st[m], sab[m], t, ab)) lo = m + 1; else hi = m;
+            }
+            pos += lo;
+        }
+        if (have) { T[ecap(A, p) + pos] = t; AB[ecap(A, p) + pos] = ab; }
     }
 }
 
@@ -1202,7 +1284,7 @@ __global__ void __launch_bounds__(LT<W>, 512 / LT<W>) k_irt_loop(const __grid_co
         if (n == 0) continue;
         const uint32_t pid = A.pid_base + p;
         const uint32_t cap = tcap(A, p);
-        const unsigned long long tb0 = tbase(A, p), eb0 = ebase(A, p);
+        const unsigned long long tb0 = tbase(A, p), eb0 = ebase(A, p) + (sort_chunked(A, A.tev[p]) ? ecap(A, p) : 0u);
         const uint32_t nev = A.tev[p];
         const float del = A.tdel[p];
         const float4 org = A.rad[A.seg_off[p]];
@@ -1640,7 +1722,7 @@ static cudaError_t irt_mark(cudaEvent_t e, cudaStream_t s) {
 }
 
 cudaError_t launch_irt(const IArgs& a, int device, const IrtShape& shape, cudaStream_t s, cudaEvent_t* ev) {
-    { cudaError_t me_ = cudaMemsetAsync(a.counters, 0, 4 * sizeof(uint32_t), s); if (me_ != cudaSuccess) return me_; }
+    { cudaError_t me_ = cudaMemsetAsync(a.counters, 0, 8 * sizeof(uint32_t), s); if (me_ != cudaSuccess) return me_; }
     k_irt_load<<<blocks_for((const void*)k_irt_load, device), IB, 0, s>>>(a);
     cudaError_t e = launch_scan_u32(a.ttiles, a.nseg, a.toff, s);
     if (e != cudaSuccess) return e;
@@ -1653,6 +1735,10 @@ cudaError_t launch_irt(const IArgs& a, int device, const IrtShape& shape, cudaSt
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k_irt_sort, SB, 0);
     const unsigned long long sgrid = (unsigned long long)sms * (unsigned long long)(per > 0 ? per : 1);
     k_irt_sort<<<(unsigned)(a.nseg < sgrid ? (a.nseg > 0 ? a.nseg : 1) : sgrid), SB, 0, s>>>(a);
+    if (a.pcap > IRT_PCAP_MIN) {
+        k_irt_sort_chunks<<<2 * sms, SCB, 0, s>>>(a);
+        k_irt_sort_merge<<<4 * sms, SB, 0, s>>>(a);
+    }
     if (ev && (e = irt_mark(ev[2], s)) != cudaSuccess) return e;
     switch (loop_width(device, a.nseg)) {
     case 16: return launch_loop<16>(a, device, shape, s);

@@ -50,12 +50,15 @@ struct IArgs {
     double* hov_t;
     uint32_t* hov_ab;
     uint32_t hcap, pcap;
-    uint32_t* counters;                  // [0] load, [1] init items, [2] loop tracks, [3] largest track
+    uint32_t* counters;                  // [0] load, [1] init items, [2] loop tracks, [3] largest track, [4] chunks
+    unsigned long long* big;             // chunks of the tracks with more events than one block sorts
     double* acc_tl;                      // 35
     unsigned long long* acc;             // [0..8] rxn, 9 reacted, 10 pairs, 11 events, 12 tracks
     float* curves;                       // optional: per track 16 x 5 counts (OH, eaq, H, H2O2, H2)
     uint32_t* err;
 };
+
+constexpr uint32_t IRT_PCAP_MIN = 1024;  // pcap of tracks of up to 480 entries
 
 cudaError_t irt_set_constants(const IrtConst& c);
 // Resident blocks per SM of the pairing and event kernels: as many as fit, at
