@@ -1096,8 +1096,8 @@ __device__ __forceinline__ void cp_wait() {                          // this lan
 // * in the exact step the three axes of a partner's Gaussian (the longest f64
 //   chains) run on three lanes;
 // * accepted events are written behind the heap's last node by all lanes.
-// Measured (ms, before and after): 4096 tracks of 10 keV 20.0 -> 14.6, 64 of them 6.7 ->
-// 2.7, 4096 of 1 keV 2.2 -> 1.65, one track of 3060 species 17.5 -> 6.2.  Before: one
+// Measured (ms, before and after): 4096 tracks of 10 keV 20.0 -> 14.0, 64 of them 6.7 ->
+// 2.7, 4096 of 1 keV 2.2 -> 1.53, one track of 3060 species 17.5 -> 6.1.  Before: one
 // warp per track, events popped by one lane against states in global memory, a binary heap,
 // batches of 64 listed partners.
 constexpr int WN = 4;                    // windows of initial events in shared memory
@@ -1136,7 +1136,7 @@ __device__ __forceinline__ bool scan_near(const ScanP& P, const float4& q, uint3
     const float dlo = (sqrt_fast(fmaf(ez, ez, fmaf(ey, ey, ex * ex))) - P.del) * 0.999997f;
     const float dth = fmaxf(P.et - q.w + P.dtm, 0.0f);
     const float sg = sqrt_fast(Djf2 * dth) * 1.00001f;
-    if (dlo - sg * 11.8f > P.rcut) return false;
+    const bool far = dlo - sg * 11.8f > P.rcut;             // (no branch: some lane goes on in 9 of 10 chunks)
     const u4 q0 = philox_rk(P.id, jj, P.pid, 5u, rk);
     // -2 ln u summed over the axes is -2 ln of the product (>= 2^-99; the sum to 1.4e-6
     // absolute, so its root to 2e-3)
@@ -1145,7 +1145,7 @@ __device__ __forceinline__ bool scan_near(const ScanP& P, const float4& q, uint3
     // beyond R = max(fs, fsc / U) + fadd of r_acc, for U >= uf, times 1.00002 plus 1e-6
     const float uf = __uint2float_rd(q0.w) * 2.3283064365386963e-10f;
     const float d = fmaf(-sg, Bm, dlo) * 0.99998f - fadd - 1e-6f;
-    return !(d > fs && d * uf > fsc);
+    return !(far || (d > fs && d * uf > fsc));
 }
 // Second: the partner displaced by the same draws in f32.
 __device__ __forceinline__ bool scan_maybe(const ScanP& P, const float4& q, uint32_t jj, float Djf2, float fs, float fsc,
@@ -1422,19 +1422,18 @@ __global__ void __launch_bounds__(LT<W>, 512 / LT<W>) k_irt_loop(const __grid_co
                 if (id >= capref) break;                   // the reference's CAP (:405, :621)
                 if (id >= cap) { if (lead) atomicOr(A.err, DERR_TRACK_SIZE); break; }
                 ntot++;
-                double nx, ny, nz;
+                // an axis per lane: one copy of the division
+                const int ax = lane % 3;
+                double* pa = (ax == 0 ? A.px : ax == 1 ? A.py : A.pz) + tb0;
+                double v;
                 if (np_ == 1) {                            // at the diffusion-weighted centre
-                    const double sqDi = sqrt(C.D[si]), sqDj = sqrt(C.D[sj]);
-                    const double ww = sqDi + sqDj;
-                    const double xa = A.px[tb0 + ei], ya = A.py[tb0 + ei], za = A.pz[tb0 + ei];
-                    const double xb = A.px[tb0 + ej], yb = A.py[tb0 + ej], zb = A.pz[tb0 + ej];
-                    nx = (sqDj * xa + sqDi * xb) / ww;
-                    ny = (sqDj * ya + sqDi * yb) / ww;
-                    nz = (sqDj * za + sqDi * zb) / ww;
+                    const double sqDi = C.sqD[si], sqDj = C.sqD[sj];
+                    v = (sqDj * pa[ei] + sqDi * pa[ej]) / (sqDi + sqDj);
                 } else {                                   // at the two reactants
-                    const int e = pp == 0 ? ei : ej;
-                    nx = A.px[tb0 + e]; ny = A.py[tb0 + e]; nz = A.pz[tb0 + e];
+                    v = pa[pp == 0 ? ei : ej];
                 }
+                const double nx = __shfl_sync(FULL, v, 0), ny = __shfl_sync(FULL, v, 1), nz = __shfl_sync(FULL, v, 2);
+                if (wg == 0 && lane < 3) pa[id] = v;
                 ScanP P;
                 P.x = (float)(nx - (double)org.x); P.y = (float)(ny - (double)org.y); P.z = (float)(nz - (double)org.z);
                 P.del = del; P.et = (float)et; P.dtm = 1e-4f + 1e-6f * P.et;
@@ -1442,7 +1441,7 @@ __global__ void __launch_bounds__(LT<W>, 512 / LT<W>) k_irt_loop(const __grid_co
                 P.id = id; P.pid = pid;
                 if (lead) {
                     const int at = S.lc[nsp];
-                    A.px[tb0 + id] = nx; A.py[tb0 + id] = ny; A.pz[tb0 + id] = nz; A.tb[tb0 + id] = et;
+                    A.tb[tb0 + id] = et;
                     if (insm) atomicOr(&S.state[id >> 3], (8u | (uint32_t)nsp) << (4 * (id & 7)));
                     else { A.sp[tb0 + id] = (int8_t)nsp; A.alive[tb0 + id] = 1; }
                     A.lst[6 * tb0 + nsp * cap + at] = (uint16_t)id;

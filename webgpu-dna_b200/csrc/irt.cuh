@@ -10,7 +10,7 @@ struct IrtConst {
     double kact[9];
     int type[9], nprod[9], prod0[9], prod1[9];
     int map[36];
-    double D[6];
+    double D[6], sqD[6];                 // and their square roots
     double sig_oh, sig_h, sig_eaq, r_cut2;
     // f32 prefilter bounds of r_acc (irt.cu pair_maybe): (s + add)(1+1e-6) + 1e-6,
     // add(1+1e-6) + 1e-6 and s c (1+1e-6)^2
