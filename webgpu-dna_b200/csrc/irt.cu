@@ -424,32 +424,74 @@ __device__ __forceinline__ void load_consts(IrtConst* dst, uint32_t* row) {
     __syncthreads();
 }
 
-// 1) load + thermalisation displacement (:475-537) and species lists; one warp per track
-__global__ void __launch_bounds__(IB) k_irt_load(IArgs A) {
+// 1) load + thermalisation displacement (:475-537) and species lists; W warps per track,
+//    each taking a contiguous part of its entries.  What bounds it is the chain of
+//    Philox blocks and f64 sums of an entry's displacement (18 draws), one chunk of 32 after
+//    another; with several warps a first look at the codes alone tells where each warp's
+//    particles and list entries go.
+//    One warp per track took 0.37 ms for a track of 3060 entries and 0.53 ms for 4096
+//    tracks of 10 keV, 8 warps 0.05 and 0.43.
+template <int W>
+__global__ void __launch_bounds__(W == 1 ? IB : 32 * W) k_irt_load(const __grid_constant__ IArgs A) {
     __shared__ IrtConst s_c;
-    __shared__ uint32_t s_row[6];
+    __shared__ uint32_t s_row[6], s_cnt[W][8], s_track, s_ext;
     load_consts(&s_c, s_row);
     const IrtConst& C = s_c;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, wg = W == 1 ? 0 : threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
     const uint32_t k0 = A.k0, k1 = A.k1;
     unsigned long long n_tracks = 0, n_part = 0;
     for (;;) {
         uint32_t p = 0;
-        if (lane == 0) p = atomicAdd(&A.counters[0], 1u);
-        p = __shfl_sync(FULL, p, 0);
+        if (W == 1) {
+            if (lane == 0) p = atomicAdd(&A.counters[0], 1u);
+            p = __shfl_sync(FULL, p, 0);
+        } else {
+            if (threadIdx.x == 0) { s_track = atomicAdd(&A.counters[0], 1u); s_ext = 0; }
+            __syncthreads();
+            p = s_track;
+        }
         if (p >= A.nseg) break;
-        unsigned long long s = A.seg_off[p], e = A.seg_off[p + 1];
+        const unsigned long long s0 = A.seg_off[p], e0 = A.seg_off[p + 1];
         const uint32_t pid = A.pid_base + p;
         const uint32_t cap = tcap(A, p);
         const unsigned long long tb0 = tbase(A, p);
         double* px = A.px + tb0; double* py = A.py + tb0; double* pz = A.pz + tb0; double* tb = A.tb + tb0;
         int8_t* sp = A.sp + tb0; uint8_t* alive = A.alive + tb0;
         uint16_t* lst = A.lst + 6 * tb0; uint16_t* lpos = A.lpos + tb0;
-        uint32_t n = 0, h2 = 0;
+        float4* rec = A.rec + 6 * tb0;
         float4* pf = A.pf + tb0;
+        // particles, H2 markers and list entries before this warp's
+        uint32_t n = 0, h2 = 0, cnt[6] = {0, 0, 0, 0, 0, 0};
+        unsigned long long s = s0, e = e0;
+        if (W > 1) {
+            const unsigned long long part = (e0 - s0 + 32 * W - 1) / (32 * W) * 32;
+            s = min(e0, s0 + wg * part);
+            e = min(e0, s + part);
+            for (unsigned long long c = s; c < e; c += 32) {
+                const int code = c + lane < e ? (int)rintf(A.rad[c + lane].w) % 8 : -1;
+                n += __popc(__ballot_sync(FULL, code >= 0 && code != 4 && code != 7));
+                h2 += __popc(__ballot_sync(FULL, code == 7));
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    cnt[q] += __popc(__ballot_sync(FULL, q == 1 ? code == 1 || code == 5 : q == 5 ? code == 6 : q != 4 && code == q));
+            }
+            if (lane == 0) {
+                s_cnt[wg][6] = n; s_cnt[wg][7] = h2;
+#pragma unroll
+                for (int q = 0; q < 6; ++q) s_cnt[wg][q] = cnt[q];
+            }
+            __syncthreads();
+            uint32_t before = 0;
+            if (lane < 8)
+                for (int w = 0; w < wg; ++w) before += s_cnt[w][lane];
+            n = __shfl_sync(FULL, before, 6);
+            h2 = __shfl_sync(FULL, before, 7);
+#pragma unroll
+            for (int q = 0; q < 6; ++q) cnt[q] = __shfl_sync(FULL, before, q);
+        }
         // origin of the track's f32 shadow coordinates: its first rad_buf entry
-        const float4 r0 = A.rad[s];
+        const float4 r0 = s0 < e0 ? A.rad[s0] : make_float4(0.f, 0.f, 0.f, 0.f);
         const double ox = r0.x, oy = r0.y, oz = r0.z;
         float mext = 0.0f;
         for (unsigned long long c = s; c < e; c += 32) {
@@ -462,9 +504,11 @@ __global__ void __launch_bounds__(IB) k_irt_load(IArgs A) {
             h2 += __popc(__ballot_sync(FULL, valid && code == 7));
             unsigned m = __ballot_sync(FULL, keep);
             uint32_t k = n + __popc(m & lt);
+            int spc = -1;
+            float4 sh = make_float4(0.f, 0.f, 0.f, 0.f);           // shadow and birth time 0
             if (keep) {
                 double x = r.x, y = r.y, z = r.z;
-                int spc = code;
+                spc = code;
                 double sigma = 0;
                 int disp = 0;
                 uint32_t blk = 0, wi = 4;
@@ -493,39 +537,38 @@ __global__ void __launch_bounds__(IB) k_irt_load(IArgs A) {
                 sp[k] = (int8_t)spc; alive[k] = 1;
                 float fx = (float)(x - ox), fy = (float)(y - oy), fz = (float)(z - oz);
                 pf[k] = make_float4(fx, fy, fz, __int_as_float(spc));
+                sh = make_float4(fx, fy, fz, 0.0f);
                 mext = fmaxf(mext, fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))));
             }
             n += __popc(m);
-        }
-        for (int o = 16; o; o >>= 1) mext = fmaxf(mext, __shfl_xor_sync(FULL, mext, o));
-        __syncwarp();
-        __threadfence_block();
-        uint32_t cnt[6] = {0, 0, 0, 0, 0, 0};
-        float4* rec = A.rec + 6 * tb0;
-        for (uint32_t c = 0; c < n; c += 32) {
-            uint32_t k = c + lane;
-            int spc = k < n ? sp[k] : -1;
-            float4 sh = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (k < n) { sh = pf[k]; sh.w = 0.0f; }               // shadow and birth time 0
+#pragma unroll
             for (int q = 0; q < 6; ++q) {
-                unsigned m = __ballot_sync(FULL, spc == q);
+                const unsigned mq = __ballot_sync(FULL, spc == q);
                 if (spc == q) {
-                    uint32_t at = cnt[q] + __popc(m & lt);
+                    const uint32_t at = cnt[q] + __popc(mq & lt);
                     lst[q * cap + at] = (uint16_t)k;
                     rec[q * cap + at] = sh;
                     lpos[k] = (uint16_t)at;
                 }
-                cnt[q] += __popc(m);
+                cnt[q] += __popc(mq);
             }
         }
-        if (lane < 6) A.tlc[6 * p + lane] = cnt[lane];
+        for (int o = 16; o; o >>= 1) mext = fmaxf(mext, __shfl_xor_sync(FULL, mext, o));
+        if (W > 1) {
+            if (lane == 0) atomicMax(&s_ext, __float_as_uint(mext));
+            __syncthreads();
+            mext = __uint_as_float(s_ext);
+            __syncthreads();                               // read by all
+            if (wg != W - 1) continue;                     // the last warp's counts are the track's
+        }
         if (lane == 0) {
             A.tn[p] = n;
             A.th2[p] = h2;
             // |f32 shadow distance - f64 distance| <= 3.1e-7 * extent; 1e-6 * extent + 1e-4 nm bounds it
             A.tdel[p] = mext * 1e-6f + 1e-4f;
             uint32_t tiles = 0;                    // the pairing kernel's tiles: 32 particles of one species
-            for (int q = 0; q < 6; ++q) tiles += (cnt[q] + 31) / 32;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) { A.tlc[6 * p + q] = cnt[q]; tiles += (cnt[q] + 31) / 32; }
             A.ttiles[p] = tiles;
             A.tev[p] = 0;
         }
@@ -1653,6 +1696,18 @@ __global__ void __launch_bounds__(1024) k_track_order(const uint32_t* tn, uint32
     }
 }
 
+// Warps per track of the load: several where there are few tracks for the SMs, of long
+// ones (over 480 entries) also with more; many tracks fill the warps by themselves.
+// Measured (us, 1 and 8): 16 tracks of 10 keV 186 and 30, 592: 265 and 90, 4096: 529 and
+// 430; 64 of 1 keV 40 and 18, 592: 50 and 26, 4096: 91 and 98, 16384: 221 and 370; 65,536
+// of 0.1 to 30 keV 3097 and 3523.
+constexpr int LOAD_W = 8;
+static bool load_wide(int device, const IArgs& a) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return a.nseg <= (a.pcap > IRT_PCAP_MIN ? 64u : 4u) * (unsigned)sms;
+}
+
 // Warps per track of the event kernel: two while all tracks are resident at once at 16 warps
 // per SM, more while they are at 8 per SM.  Measured (10 keV tracks on 148 SMs, ms with
 // W = 1, 2, 4, 8, 16): 64 tracks 5.96 3.46 3.13 3.02 3.07, 150: 6.34 3.90 3.56 3.47 3.83,
@@ -1722,7 +1777,14 @@ static cudaError_t irt_mark(cudaEvent_t e, cudaStream_t s) {
 
 cudaError_t launch_irt(const IArgs& a, int device, const IrtShape& shape, cudaStream_t s, cudaEvent_t* ev) {
     { cudaError_t me_ = cudaMemsetAsync(a.counters, 0, 8 * sizeof(uint32_t), s); if (me_ != cudaSuccess) return me_; }
-    k_irt_load<<<blocks_for((const void*)k_irt_load, device), IB, 0, s>>>(a);
+    if (load_wide(device, a)) {
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        const unsigned fit = 8u * (unsigned)sms;           // at most 8 blocks of 8 warps per SM; they take tracks in turn
+        k_irt_load<LOAD_W><<<a.nseg < fit ? (a.nseg ? a.nseg : 1) : fit, 32 * LOAD_W, 0, s>>>(a);
+    } else {
+        k_irt_load<1><<<blocks_for((const void*)k_irt_load<1>, device), IB, 0, s>>>(a);
+    }
     cudaError_t e = launch_scan_u32(a.ttiles, a.nseg, a.toff, s);
     if (e != cudaSuccess) return e;
     if (ev && (e = irt_mark(ev[0], s)) != cudaSuccess) return e;
