@@ -24,6 +24,7 @@ from wgdna import _lib
     (900, 4200, 250.0),
     (2500, 0, 15.0),
     (2400, 2300, 150.0),
+    (2400, 4200, 250.0),
 ])
 def test_event_widths_bit_exact(ctx, n_tracks, large, spread):
     g = np.random.default_rng(n_tracks)

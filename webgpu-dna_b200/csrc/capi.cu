@@ -733,7 +733,7 @@ static void irt_constants(IrtConst* C) {
                             {1, 1, 0.636e10, 5, 5, 2, 0}, {1, 2, 2.50e10, 5, 0, 1, 0}, {1, 3, 2.11e10, 2, 0, 1, 1},
                             {2, 2, 0.503e10, 0, 0, 0, 0}, {1, 4, 1.10e10, 5, 0, 2, 1}, {3, 5, 1.13e11, 0, 0, 0, 0}};
     const double ONS = 1.44 / (0.02527 * 80.1), Rs = 0.29, KC = 1e24 / (6.022e23 * 1e9);
-    for (int i = 0; i < 6; ++i) { C->D[i] = D[i]; C->sqD[i] = sqrt(D[i]); }
+    for (int i = 0; i < 6; ++i) { C->D[i] = D[i]; C->sqD[i] = sqrt(D[i]); C->D2f[i] = (float)(2.0 * D[i]); }
     for (int r = 0; r < 9; ++r) {
         int a = RX[r].a, b = RX[r].b;
         double Ds = D[a] + D[b];

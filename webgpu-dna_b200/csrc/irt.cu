@@ -1149,7 +1149,7 @@ constexpr int CQ = 128;                  // listed partners in shared memory, th
 template <int W>
 constexpr int HS = W >= 4 ? 1024 : 256 * W;
 template <int W>
-constexpr uint32_t SN = W >= 8 ? 16640 : 4096 * W;
+constexpr uint32_t SN = W >= 8 ? 16640 : 8192;
 template <int W>
 struct EvGroup {
     double tl[35], ht[HS<W>], wt[WN][32], et;
@@ -1535,7 +1535,7 @@ __global__ void __launch_bounds__(LT<W>, 512 / LT<W>) k_irt_loop(const __grid_co
                         bool nr = false;
                         if (in) {
                             const int r2i = (int)(tag >> 16 & 15u);
-                            nr = scan_near(P, q, jj, (float)(2.0 * C.D[s2]), C.fs[r2i], C.fsc[r2i], C.fadd[r2i], A.rk);
+                            nr = scan_near(P, q, jj, C.D2f[s2], C.fs[r2i], C.fsc[r2i], C.fadd[r2i], A.rk);
                         }
                         const unsigned m = __ballot_sync(FULL, nr);
                         if (!m) continue;
@@ -1553,7 +1553,7 @@ __global__ void __launch_bounds__(LT<W>, 512 / LT<W>) k_irt_loop(const __grid_co
                             const int ri2 = (int)((e >> 16) & 15u), sj2 = (int)(e >> 20);
                             const size_t at = (size_t)sj2 * cap + (e & 0xffffu);
                             const uint32_t jj = A.lst[6 * tb0 + at];
-                            mv = scan_maybe(P, A.rec[6 * tb0 + at], jj, (float)(2.0 * C.D[sj2]), C.fs[ri2], C.fsc[ri2], C.fadd[ri2], A.rk);
+                            mv = scan_maybe(P, A.rec[6 * tb0 + at], jj, C.D2f[sj2], C.fs[ri2], C.fsc[ri2], C.fadd[ri2], A.rk);
                             v = (e & ~0xffffu) | jj;
                         }
                         qn = from;
