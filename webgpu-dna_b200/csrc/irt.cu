@@ -604,11 +604,14 @@ __device__ __forceinline__ u4 philox_accept(uint32_t blk, uint32_t i, uint32_t p
 //    evaluate them exactly in f64, 32 at a time, one per lane.
 //    The distances, the bound's products and the counts' sums run two to an
 //    instruction (f32x2: one issue slot for both).
-//    Measured at 4096 x 10 keV: 8.2 ms, of which the scan is 4.7, SamplePDC 2.8; 9.1 ms
-//    with every SamplePDC pair through pdc_find at once, 9.5 ms also without f32x2,
-//    10.5 ms also with the rare f64 erfcx inline (the instruction cache, as in the event
-//    kernel), 14.9 ms also with tiles in index order, one table gather per pair and
-//    queue votes per partner (4, 5, 6, 7 blocks per SM: 9.0, 8.2, 8.2, 8.4 ms).
+//    In a track wider than R_CUT, chunks of 32 partners whose box lies beyond it
+//    from the tile's are passed by before their first pair.
+//    Measured at 4096 x 10 keV: 8.1 ms, of which the scan is 4.6, SamplePDC 2.8; 8.2 ms
+//    without the boxes (2048 x 30 keV 15.4 without them, 10.6 with), 9.1 ms also with
+//    every SamplePDC pair through pdc_find at once, 9.5 ms also without f32x2, 10.5 ms also
+//    with the rare f64 erfcx inline (the instruction cache, as in the event kernel), 14.9 ms
+//    also with tiles in index order, one table gather per pair and queue votes per
+//    partner (5, 6 blocks per SM: 8.5, 8.1 ms; 4, 7 were slower before the boxes).
 constexpr int QCAP = 16;                 // candidates per lane
 constexpr float FAR = 1e18f;             // shadow coordinate of a partner that cannot react
 
@@ -633,6 +636,17 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     f32x2 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
     return r;
 }
 
@@ -800,11 +814,12 @@ __device__ __forceinline__ void pdc_queue(const IArgs& A, const IrtConst& C, Pdc
     }
 }
 
-__global__ void __launch_bounds__(IB, 5) k_irt_init(const __grid_constant__ IArgs A) {
+__global__ void __launch_bounds__(IB, 6) k_irt_init(const __grid_constant__ IArgs A) {
     __shared__ IrtConst s_c;
     __shared__ uint32_t s_row[6];
     // partners of a chunk: negated shadow x, y, z and the bound's kb and fk (scaled to 16-bit U)
     __shared__ __align__(16) float s_p[IB / 32][5][32];
+    __shared__ float s_box[IB / 32][6];
     __shared__ uint16_t s_q[IB / 32][QCAP][32];
     __shared__ uint32_t s_d[IB / 32][QCAP * 32 + 32];
     __shared__ PdcQueue s_pdc[IB / 32];
@@ -814,6 +829,7 @@ __global__ void __launch_bounds__(IB, 5) k_irt_init(const __grid_constant__ IArg
     const unsigned long long nitems = A.toff[A.nseg];
     const float rcut = (float)sqrt(C.r_cut2);
     float (*sp)[32] = s_p[wl];
+    float* box = s_box[wl];
     uint32_t* dq = s_d[wl];
     unsigned long long n_pairs = 0;
     uint32_t qn = 0;
@@ -859,23 +875,47 @@ __global__ void __launch_bounds__(IB, 5) k_irt_init(const __grid_constant__ IArg
         }
         const uint32_t imin = __shfl_sync(FULL, i, 0);
         const uint32_t imax = __shfl_sync(FULL, i, min(31u, len - 32u * tile - 1u));
+        // a track that fits into R_CUT needs no boxes (del bounds its extent)
+        const bool wide = (del - 1e-4f) * 3.5e6f > rcut;
+        if (wide) {                                   // the tile's box
+            const float x0 = warp_min(have ? me.x : FAR), x1 = warp_max(have ? me.x : -FAR);
+            const float y0 = warp_min(have ? me.y : FAR), y1 = warp_max(have ? me.y : -FAR);
+            const float z0 = warp_min(have ? me.z : FAR), z1 = warp_max(have ? me.z : -FAR);
+            if (lane == 0) { box[0] = x0; box[1] = x1; box[2] = y0; box[3] = y1; box[4] = z0; box[5] = z1; }
+        }
         uint32_t cnt = 0, rem = 0;
         float np = 0.0f;                              // at most 32,735 partners: exact
         const uint32_t gend = (n + 3) >> 2;           // groups of 4 partners = one Philox block
         for (uint32_t g = (imin >> 5) << 3; g < gend; ++g) {
             if ((g & 7u) == 0) {
-                __syncwarp();
-                const uint32_t j = 4 * g + lane;
-                float4 q = make_float4(FAR, 0.f, 0.f, 0.f);
-                float kb = 0.0f, fk = 0.0f;
-                if (j < n) {
-                    q = pf[j];
-                    const int r = (int)((row >> (4 * __float_as_int(q.w))) & 15u);
-                    if (r == 15) q.x = FAR;
-                    else { kb = (C.fkb0[r] + del) * 1.00006f; fk = C.fk[r] * (65536.0f * 1.00006f); }
+                for (;;) {
+                    __syncwarp();
+                    const uint32_t j = 4 * g + lane;
+                    float4 q = make_float4(FAR, 0.f, 0.f, 0.f);
+                    float kb = 0.0f, fk = 0.0f;
+                    bool re = false;
+                    if (j < n) {
+                        q = pf[j];
+                        const int r = (int)((row >> (4 * __float_as_int(q.w))) & 15u);
+                        re = r != 15;
+                        if (!re) q.x = FAR;
+                        else { kb = (C.fkb0[r] + del) * 1.00006f; fk = C.fk[r] * (65536.0f * 1.00006f); }
+                    }
+                    // in a track wider than R_CUT, chunks of which no pair is inside it are passed by
+                    // (but for the last, of which nothing comes)
+                    if (wide && g + 8 < gend) {
+                        // the chunk's box against the tile's: with the pairs' own operations in
+                        // their order (each is monotonic), so that it holds for every pair's r2
+                        const float gx = fmaxf(warp_min(re ? q.x : FAR) - box[1], box[0] - warp_max(re ? q.x : -FAR));
+                        const float gy = fmaxf(warp_min(re ? q.y : FAR) - box[3], box[2] - warp_max(re ? q.y : -FAR));
+                        const float gz = fmaxf(warp_min(re ? q.z : FAR) - box[5], box[4] - warp_max(re ? q.z : -FAR));
+                        const float cx = fmaxf(gx, 0.0f), cy = fmaxf(gy, 0.0f), cz = fmaxf(gz, 0.0f);
+                        if (fmaf(cz, cz, fmaf(cy, cy, cx * cx)) > hi2) { g += 8; continue; }
+                    }
+                    sp[0][lane] = -q.x; sp[1][lane] = -q.y; sp[2][lane] = -q.z; sp[3][lane] = kb; sp[4][lane] = fk;
+                    __syncwarp();
+                    break;
                 }
-                sp[0][lane] = -q.x; sp[1][lane] = -q.y; sp[2][lane] = -q.z; sp[3][lane] = kb; sp[4][lane] = fk;
-                __syncwarp();
             }
             const uint32_t k = (g & 7u) * 4u;
             const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(&sp[0][k]), Y = *reinterpret_cast<const ulonglong2*>(&sp[1][k]);
