@@ -281,10 +281,9 @@ extern "C" int wgdna_create(const wgdna_cfg* cfg, wgdna_ctx** out) {
     if (r == WGDNA_OK) r = dalloc(&c->d_red, 4);
     if (r == WGDNA_OK) r = dalloc(&c->d_err, 1);
     c->part_cap = np + (size_t)c0.max_sec < 0xffffffffull ? np + (size_t)c0.max_sec : 0xffffffffull;
-    if (r == WGDNA_OK) r = dalloc(&c->d_nsec, np);
-    if (r == WGDNA_OK) r = dalloc(&c->d_first, np + 1);
-    if (r == WGDNA_OK) r = dalloc(&c->d_part, c->part_cap);
-    if (r == WGDNA_OK) r = dalloc(&c->d_share, 592);
+    // the canonical order's arrays in one allocation (d_part first: it is cleared 16 bytes at a time)
+    if (r == WGDNA_OK) r = dalloc(&c->d_part, c->part_cap + np + (np + 1) + 592);
+    if (r == WGDNA_OK) { c->d_nsec = c->d_part + c->part_cap; c->d_first = c->d_nsec + np; c->d_share = c->d_first + np + 1; }
     if (r == WGDNA_OK) r = ensure_segments(c, (uint32_t)np);
     if (r == WGDNA_OK && cudaMemset(c->d_secq, 0, sizeof(SecRec) * (size_t)c0.max_sec) != cudaSuccess) r = WGDNA_ERR_CUDA;
     if (r == WGDNA_OK && cudaMallocHost((void**)&c->h_pin, H_PIN) != cudaSuccess) {
@@ -339,7 +338,7 @@ extern "C" void wgdna_destroy(wgdna_ctx* c) {
     wg::sg_free(c->sg);
     void* ptrs[] = {c->d_small, c->d_xcw, c->d_results, c->d_dose, c->d_rad_raw, c->d_key, c->d_rad,
                     c->d_perm, c->d_secq, c->d_st, c->d_Eprim, c->d_pid_cnt, c->d_pid_off, c->d_pid_cur,
-                    c->d_red, c->d_nsec, c->d_first, c->d_part, c->d_share, c->d_err, c->d_fy, c->d_fz, c->d_rbb0, c->d_rbb1, c->d_hits, c->d_alive,
+                    c->d_red, c->d_part, c->d_err, c->d_fy, c->d_fz, c->d_rbb0, c->d_rbb1, c->d_hits, c->d_alive,
                     c->sc.list, c->sc.seg, c->sc.u64,
                     c->sc.fib, c->d_px, c->d_py, c->d_pz, c->d_tb, c->d_sp, c->d_alive8, c->d_lst, c->d_lpos, c->d_evt, c->d_evab,
                     c->d_hov_t, c->d_hov_ab, c->d_track, c->d_toff, c->d_irt_cnt, c->d_irt_big, c->d_pf, c->d_rec, c->d_tdel, c->d_curves, c->d_acc_tl, c->d_acc, c->d_maxpid,
