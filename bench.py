@@ -42,11 +42,11 @@ E_EV = 10000.0
 WORKLOAD = ("4096 x 10 keV e- in liquid water, box +-15 um, cutoff 7.5 eV, Philox seed 0 -> "
             "IRT to 1 us -> direct SSB + DSB on 21x21 B-DNA fibres")
 CPU_SAMPLE_PRIMARIES = 512
-# library kernels per step: transport 1, rad_buf canonical order 5 (histogram,
-# scan, scatter, segment sort, reduce), IRT 7 (segment max, load, scan,
-# pairing, order, initial-event sort, events), scoring 5 (prep, tiles, tile
-# scan, apply, cluster)
-LAUNCHES_PER_STEP = 18
+# library kernels per step: transport 2 (clear, transport), rad_buf canonical order
+# and sums 6 (particles, count, share sums, their scan, place, reduce), IRT 8 (load,
+# scan, pairing, order, initial-event sort, its chunks and merge, events), scoring 3
+# (find, draw, cluster)
+LAUNCHES_PER_STEP = 19
 
 
 def peaks():
@@ -585,7 +585,7 @@ def run_track(args):
                        "species": synthetic.tracked_species(rad), "l2": "input far below L2 (one track)"},
             "e2e": {"value": args.steps / wall, "unit": "tracks/s", "h2d_bytes_per_step": int(rad.nbytes),
                     "d2h_bytes_per_step": C.sizeof(ir)},
-            "gpu_launches": 9 * (args.steps),
+            "gpu_launches": 14 * (args.steps),
             "roofline": {"bound": "hbm", "kernel": name, "achieved": alg / (kms / 1000.0) / 1e9,
                          "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": alg / (kms / 1000.0) / 1e9 / pk["hbm_gbs"],
                          "traffic": None},

@@ -59,11 +59,11 @@ int wgdna_set_stream(wgdna_ctx *ctx, void *cuda_stream);
  * "key value" line per field below), else uses the defaults shown. */
 typedef struct {
     uint32_t transport_ctas_per_sm;  /* resident transport CTAs per SM, 0 = as many as fit (2) */
-    uint32_t prim_take;              /* primaries a transport warp may start per iteration (2), 1..32 */
-    uint32_t stash_keep;             /* secondaries a warp keeps when its stash spills (16) */
-    uint32_t stash_spill;            /* stash level that spills to the global queue (32), <= 48;
+    uint32_t prim_take;              /* primaries a transport CTA may start per iteration, over its 8 warps (2), 1..32 */
+    uint32_t stash_keep;             /* a quarter of the secondaries a CTA keeps when its stash spills (16) */
+    uint32_t stash_spill;            /* a quarter of the stash level that spills to the global queue (32), <= 48;
                                       * 0 = no stash: every secondary goes to the global queue */
-    uint32_t queue_poll;             /* a busy warp polls the global queue every queue_poll iterations (8),
+    uint32_t queue_poll;             /* a busy CTA polls the global queue every queue_poll iterations (8),
                                       * a power of two <= 1024 */
     uint32_t irt_init_blocks_per_sm; /* resident blocks of the IRT pairing kernel per SM, 0 = as many as fit */
     uint32_t irt_loop_blocks_per_sm; /* resident blocks of the IRT event kernel per SM, 0 = as many as fit */
@@ -76,7 +76,7 @@ int wgdna_set_tuning(wgdna_ctx *ctx, const wgdna_tuning *t);
  * WebGPU queue has no device-side waits); for hosts that want a shorter
  * watchdog and for failure-detection tests.  queue_ns: a transport lane's wait
  * for a queued secondary to be published (default 2 s); idle_ns: a transport
- * warp's wait without work before the run ends (default 30 s); mma_ns: a
+ * CTA's wait without work before the run ends (default 30 s); mma_ns: a
  * surrogate kernel's wait for its tensor-core step (default 1 s).  0 keeps the
  * default.  A wait that runs out sets a bit of the stage's device_error and the
  * call returns WGDNA_ERR_DEVICE; the context stays usable.  test_flags is 0 in

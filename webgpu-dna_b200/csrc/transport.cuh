@@ -64,7 +64,7 @@ cudaError_t launch_clear(const ClearArgs& c, cudaStream_t s);
 // resident CTAs of the transport kernel on `device`: per SM as many as fit,
 // at most ctas_per_sm (0 = no limit)
 int transport_blocks(int device, uint32_t ctas_per_sm);
-constexpr uint32_t TRANSPORT_STASH = 48;   // stash capacity per warp (records)
+constexpr uint32_t TRANSPORT_STASH = 48;   // a quarter of a CTA's stash (records); the tuning's levels are in quarters
 cudaError_t launch_transport(const TArgs& a, int blocks, cudaStream_t s);
 cudaError_t launch_canon(const unsigned long long* key, const float4* rad, unsigned long long n, uint32_t np,
                          uint32_t* cnt, unsigned long long* off, uint32_t* cur, uint32_t* perm, float4* out,
