@@ -820,10 +820,11 @@ __device__ __forceinline__ int end_move(const TArgs& A, Blk& b, int s, Dep& dep,
 // Many electrons: a lane draws and takes its own steps, at most `most` (a warp
 // waits for its longest run).  Returns the list that follows (-1: none) and clears
 // `active` when the electron ends.
-#ifndef WG_MOVE_STEPS
-#define WG_MOVE_STEPS 12
-#endif
-constexpr uint32_t MOVE_STEPS = WG_MOVE_STEPS;
+// With secondaries waiting, work is what counts: MOVE_STEPS; else the run's length
+// is latency: MOVE_STEPS_FEW.  Measured (ms at 4096 x 10 keV; 4096 x 1 keV; 16,384 of 0.1 to
+// 30 keV): 12 and 4 4.51, 1.05, 10.62; 6 and 4 4.48, 1.04, 10.28; 6 and 3 4.35, 1.06,
+// 10.20; 5 and 2 4.54, 1.10, 10.17; 12 and 1 5.4, 1.24, 11.6.
+constexpr uint32_t MOVE_STEPS = 6, MOVE_STEPS_FEW = 3;
 __device__ __forceinline__ int move(const TArgs& A, Blk& b, int s, Dep& dep, unsigned long long& nsteps, bool& active,
                                     uint32_t most) {
     Slots& S = *b.S;
@@ -851,7 +852,7 @@ __device__ __forceinline__ int move(const TArgs& A, Blk& b, int s, Dep& dep, uns
 // are alive at a time, so an iteration costs little more than its longest
 // phase path, and with more electrons the issue slots bind.
 // Measured at 4096 x 10 keV: 14.9 ms with one warp per 32 electrons taking all
-// branches one after another (7.8 lanes per instruction, 16 % issue), 4.5 ms now.
+// branches one after another (7.8 lanes per instruction, 16 % issue), 4.35 ms now.
 __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     float* T = reinterpret_cast<float*>(smem);
@@ -1009,8 +1010,7 @@ __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
             int k = -1;
             const bool was = active;
             if (nact > NREC / 4) {
-                // with secondaries waiting the run may be long, else its length is latency
-                if (active) k = move(A, b, tid, dep, nsteps, active, stn > 0 ? MOVE_STEPS : 4u);
+                if (active) k = move(A, b, tid, dep, nsteps, active, stn > 0 ? MOVE_STEPS : MOVE_STEPS_FEW);
             } else {
                 // Few electrons, most warps idle: the draws of a run do not depend on the flight,
                 // so all threads draw the next 4, 8 or 16 steps of every electron side by
