@@ -57,3 +57,26 @@ def test_cluster_at_fibre_edges(ctx, every):
     hits[dna.n_bp + edge - 1] = 1
     got, ref = wgdna.cluster_dsb(ctx, dna, hits), oracle.cluster_dsb(od, hits)
     assert (got["dsb"], got["ssb0"], got["ssb1"]) == (ref["dsb"], ref["ssb0"], ref["ssb1"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 512, 513, 1537])
+def test_scoring_scratch_of_a_full_context(n):
+    """As many entries as the context holds, every one near a site and drawn once: lists and summaries
+    at their largest in the keys' buffer."""
+    dna, od = wgdna.build_dna_target(), oracle.DnaTarget()
+    ctx = wgdna.Context(max_primaries=4, max_rad=n, max_sec=1000)
+    try:
+        g = np.random.default_rng(n)
+        b, f = g.integers(dna.n_bp_per, size=n), g.integers(dna.n_fibers, size=n)
+        off = dna.rbb0.reshape(-1, 2)[b]
+        rad = np.stack([dna.x0 + b * dna.rise, dna.fy[f] + off[:, 0], dna.fz[f] + off[:, 1], np.zeros(n)], 1).astype(np.float32)
+        for _ in range(2):
+            rng = wgdna.make_ssb_rng()
+            got = wgdna.score_direct_ssb_events(ctx, dna, rad, n, rng)
+            ref = oracle.score_direct(od, rad, 0x12345678)
+            assert (got["ssb_count"], got["candidates"], got["in_reach"]) == (ref["ssb"], ref["candidates"], ref["in_reach"])
+            assert rng.state == ref["lcg_state"]
+            np.testing.assert_array_equal(got["hits"], ref["hits"])
+    finally:
+        ctx.close()

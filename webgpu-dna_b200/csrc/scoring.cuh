@@ -19,6 +19,10 @@ struct ScoreScratch {
     uint32_t* fib;             // 3 per fibre
 };
 
+// 64-bit words that hold u64, seg and list for up to n entries, or n keys (score_scratch
+// in capi.cu): 16 for u64, at most n / 512 + 16 for seg and (n + 1) / 2 for list
+constexpr unsigned long long score_scratch_words(unsigned long long n) { return n + 64; }
+
 cudaError_t launch_score(const float4* rad, const uint32_t* alive, unsigned long long n, const DnaDev& d,
                          double r_d, double p, int dedupe, uint32_t s0, uint32_t* hits_words,
                          const ScoreScratch& sc, cudaStream_t s);
