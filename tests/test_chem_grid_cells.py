@@ -35,3 +35,18 @@ def test_yields_against_oracle(ctx, n, k, sigma):
     got, ref = np.array(r.counts).astype(float), ref.astype(float)
     np.testing.assert_array_equal(got[0], ref[0])
     assert np.all(np.abs(got - ref) <= 0.02 * ref + 4 * np.sqrt(ref + 1)), (got, ref)
+
+
+@pytest.mark.gpu
+def test_captured_schedule_serves_other_sizes_and_keys(ctx):
+    """Calls of 4097 to 4350 radicals share one grid size (4352), 255 does not: each
+    gives its own n and key's yields, with buffers that still hold the call before."""
+    for n, seed in ((4350, 3), (4097, 3), (4350, 4), (255, 5), (4200, 6)):
+        rad = clusters(n, 40, 1.0, n)
+        ref, _, _ = oracle.chem_grid(rad, seed=seed)
+        r = _lib.ChemGridResult()
+        _lib.check("grid", _lib.lib().wgdna_chem_grid(ctx.h, _lib.ptr(rad), n, 16, 1000.0, seed, C.byref(r), None, None, 0))
+        got, want = np.array(r.counts).astype(float), ref.astype(float)
+        assert r.chem_n == n
+        np.testing.assert_array_equal(got[0], want[0])
+        assert np.all(np.abs(got - want) <= 0.02 * want + 4 * np.sqrt(want + 1)), (n, seed, got, want)

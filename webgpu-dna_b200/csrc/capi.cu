@@ -1116,16 +1116,17 @@ extern "C" int wgdna_chem_grid(wgdna_ctx* c, const float* rad, uint64_t rad_n, u
     if (n == 0) return WGDNA_OK;
     if (n > c->cg_cap) {
         c->cg_cap = 0;                   // until every buffer has its new size
-        TRY(dalloc(&c->d_cg_pos, n)); TRY(dalloc(&c->d_cg_alive, n)); TRY(dalloc(&c->d_cg_next, n));
-        TRY(dalloc(&c->d_cg_cell, 2 * (size_t)n)); TRY(dalloc(&c->d_cg_rank, n)); TRY(dalloc(&c->d_cg_sorted, n));
-        c->cg_cap = n;
+        const size_t cap = 256 * (size_t)wg::cg_blocks(n);
+        TRY(dalloc(&c->d_cg_pos, cap)); TRY(dalloc(&c->d_cg_alive, cap)); TRY(dalloc(&c->d_cg_next, cap));
+        TRY(dalloc(&c->d_cg_cell, 2 * cap)); TRY(dalloc(&c->d_cg_rank, cap)); TRY(dalloc(&c->d_cg_sorted, cap));
+        c->cg_cap = cap;
     }
     if (!c->d_cg_tab) {                  // the last of them
         TRY(dalloc(&c->d_cg_head, wg::CG_HASH_SIZE)); TRY(dalloc(&c->d_cg_prod, 2));
         TRY(dalloc(&c->d_cg_counts, 40)); TRY(dalloc(&c->d_cg_state, 1));
         TRY(dalloc(&c->d_cg_tab, 2 * (size_t)wg::CG_HASH_SIZE));
     }
-    wg::CgArgs a{src, n, (uint32_t)seed, (uint32_t)(seed >> 32), c->d_cg_pos, c->d_cg_alive, c->d_cg_tab,
+    wg::CgArgs a{src, n, (uint32_t)seed, (uint32_t)(seed >> 32), (uint32_t)c->cg_cap, c->d_cg_pos, c->d_cg_alive, c->d_cg_tab,
                  c->d_cg_cell, c->d_cg_rank, c->d_cg_sorted, c->d_cg_head, c->d_cg_next, c->d_cg_prod, c->d_cg_counts,
                  c->d_cg_state};
     WG_CUDA_OK(cudaEventRecord(c->ev[4], s));

@@ -6,7 +6,11 @@
 // compare-and-swap (so, as in the reference, which of several competing
 // pairs reacts depends on thread timing).  The 7-stage schedule (133 steps of
 // diffuse / place / sort / react, plus the counts at each checkpoint) is
-// captured once into a CUDA graph and replayed with one launch.
+// captured once into a CUDA graph and replayed with one launch: the number of radicals
+// and the key are read from memory (CgState), so calls of about the same size share it
+// (a new batch of 20,000 radicals 5.7 -> 3.3 ms, of 530,000 15.1 -> 12.8; with each size and key
+// captured anew, 2.2 ms of each call were the capture).  Without a graph the 133 steps'
+// launches take 2 ms more than with one at every size.
 //
 // What bounds a step: 27 table lookups per radical, and at the common start of all
 // tracks, where a reference cell holds hundreds of radicals, the pair tests.  The
@@ -82,8 +86,10 @@ __device__ __forceinline__ float2 cg_gauss2(float u1, float u2) {
 }
 
 // sample_init + init_thermal (chemistry.wgsl:92-101, 286-334)
-__global__ void k_cg_init(const float4* rad, uint32_t n, uint32_t k0, uint32_t k1, float4* pos, uint32_t* alive) {
+__global__ void k_cg_init(const float4* rad, uint32_t n, uint32_t k0, uint32_t k1, float4* pos, uint32_t* alive,
+                          CgState* st) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) { st->n = n; st->k0 = k0; st->k1 = k1; st->dense[0] = st->dense[1] = 0u; }
     if (i >= n) return;
     const float4 r = rad[i];
     int kind = (int)(__float2uint_rn(r.w) % 8u);
@@ -115,12 +121,17 @@ constexpr uint32_t CG_NONE = 0xffffffffu;
 constexpr uint32_t CG_WALK = 1024;               // the reference's bound on a walk through a cell
 __device__ __forceinline__ int cg_fine(float x) { return (int)floorf(x / CG_FINE); }
 
-// 1) diffuse (chemistry.wgsl:32-56) and take a place in the fine cell's bucket
-__global__ void k_cg_diffuse(float4* pos, const uint32_t* alive, uint32_t n, float dt, uint32_t step, uint32_t k0,
-                             uint32_t k1, uint32_t* tab, uint32_t* cell, uint32_t* rank, CgState* st) {
+__device__ __forceinline__ int cg_cell(float x) { return (int)floorf(x / CG_CELL); }
+__device__ __forceinline__ uint32_t cg_list(float4 p) { return cg_hash(cg_cell(p.x), cg_cell(p.y), cg_cell(p.z)); }
+
+// 1) diffuse (chemistry.wgsl:32-56) and take a place in the fine cell's bucket.  After a
+//    step with lists, each radical empties the one it was in (it has not moved since).
+__global__ void k_cg_diffuse(float4* pos, const uint32_t* alive, float dt, uint32_t step, uint32_t* tab, uint32_t* cell,
+                             uint32_t* rank, CgState* st, int* head) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) { st->placed = 0u; st->dense = 0u; }
-    if (i >= n) return;
+    if (i == 0) { st->placed = 0u; st->dense[step & 1u] = 0u; }
+    if (i >= st->n) return;
+    if (st->dense[(step + 1) & 1u]) head[cg_list(pos[i])] = -1;
     if (alive[i] == 0u) { cell[i] = CG_NONE; return; }
     float4 p = pos[i];
     const int kind = (int)rintf(p.w);
@@ -131,7 +142,7 @@ __global__ void k_cg_diffuse(float4* pos, const uint32_t* alive, uint32_t n, flo
     else if (kind == 3) D = 9.0f;
     if (kind >= 0 && kind <= 3) {
         const float sigma = sqrtf(2.0f * D * dt);
-        const u4 w = philox(i, step, 0u, 6u, k0, k1);
+        const u4 w = philox(i, step, 0u, 6u, st->k0, st->k1);
         const float2 g01 = cg_gauss2(u01f(w.x), u01f(w.y));
         const float2 g23 = cg_gauss2(u01f(w.z), u01f(w.w));
         p.x += sigma * g01.x;
@@ -152,12 +163,12 @@ __device__ __forceinline__ uint32_t cg_count(uint32_t v) { return (v >> 23) ? v 
 //    first entry | count << 23.  A fine cell with more than an eighth of CG_WALK has
 //    its coarse cell counted.
 constexpr int CG_RB = 512;
-__global__ void __launch_bounds__(CG_RB) k_cg_reserve(const float4* pos, uint32_t n, uint32_t* tab, const uint32_t* cell,
-                                                      const uint32_t* rank, CgState* st) {
+__global__ void __launch_bounds__(CG_RB) k_cg_reserve(const float4* pos, uint32_t* tab, const uint32_t* cell,
+                                                      const uint32_t* rank, CgState* st, uint32_t step) {
     __shared__ uint32_t wsum[CG_RB / 32], s_base;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const uint32_t h = i < n ? cell[i] : CG_NONE;
+    const uint32_t h = i < st->n ? cell[i] : CG_NONE;
     const bool lead = h != CG_NONE && rank[i] == 0u;
     const uint32_t c = lead ? tab[h] : 0u;
     uint32_t off = c;
@@ -184,19 +195,24 @@ __global__ void __launch_bounds__(CG_RB) k_cg_reserve(const float4* pos, uint32_
             sum += cg_count(*(volatile uint32_t*)&tab[cg_hash(ix + (o & 1), iy + ((o >> 1) & 1), iz + (o >> 2))]);
         dense = sum > CG_WALK;
     }
-    if (dense) st->dense = 1u;
+    if (dense) st->dense[step & 1u] = 1u;
     tab[h] = (s_base + wsum[wl] + off - c) | (min(c, 511u) << 23);
 }
 
-// 3) radicals in bucket order; the other table is emptied for the next step
-__global__ void k_cg_sort(const float4* pos, uint32_t n, const uint32_t* tab, const uint32_t* cell, const uint32_t* rank,
-                          float4* sorted, uint32_t* tab_old, const uint32_t* cell_old) {
+// 3) radicals in bucket order; the other table is emptied for the next step.  A step with
+//    an overfull cell also builds the reference's lists (build_hash, chemistry.wgsl:111-122).
+//    Clearing the heads and building the lists in launches of their own cost every ordinary
+//    step two that return at once, and building them in k_cg_react slowed that kernel (530,000
+//    radicals, a call: 12.4 ms with the launches, 14.2 with k_cg_react, 12.3 so).
+__global__ void k_cg_sort(const float4* pos, const uint32_t* tab, const uint32_t* cell, const uint32_t* rank, float4* sorted,
+                          uint32_t* tab_old, const uint32_t* cell_old, const CgState* st, uint32_t step, int* head, int* next) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= st->n) return;
     if (cell_old) { const uint32_t o = cell_old[i]; if (o != CG_NONE) tab_old[o] = 0u; }
     const uint32_t h = cell[i];
-    if (h == CG_NONE) return;
+    if (h == CG_NONE) return;                        // dead: no list leads to it
     const float4 p = pos[i];
+    if (st->dense[step & 1u]) next[i] = atomicExch(&head[cg_list(p)], (int)i);
     const uint32_t kind = (uint32_t)(int)rintf(p.w) & 7u;
     sorted[(tab[h] & 0x7fffffu) + rank[i]] = make_float4(p.x, p.y, p.z, __uint_as_float(i | (kind << 23)));
 }
@@ -205,13 +221,13 @@ __global__ void k_cg_sort(const float4* pos, uint32_t n, const uint32_t* tab, co
 // of now, as the reference reads them), the roll, the claim.  0: go on, 1: radical i is
 // done with this step
 __device__ __forceinline__ int cg_contact(float4* pos, uint32_t* alive, uint32_t i, int ki, uint32_t j, float d2, uint32_t step,
-                                          uint32_t k0, uint32_t k1, uint32_t& draw, u4& w, uint32_t* prod) {
+                                          const CgState* st, uint32_t& draw, u4& w, uint32_t* prod) {
     if (alive[j] == 0u) return 0;
     const int kj = (int)rintf(pos[j].w);
     if (kj < 0 || kj > 3) return 0;
     const float R = cg_sigma_react(ki, kj);
     if (R <= 0.0f || d2 > R * R) return 0;
-    if ((draw & 3u) == 0u) w = philox(i, step, 1u + (draw >> 2), 6u, k0, k1);
+    if ((draw & 3u) == 0u) w = philox(i, step, 1u + (draw >> 2), 6u, st->k0, st->k1);
     const uint32_t word = (draw & 3u) == 0u ? w.x : (draw & 3u) == 1u ? w.y : (draw & 3u) == 2u ? w.z : w.w;
     draw++;
     if (u01f(word) >= cg_pcontact(ki, kj)) return 0;
@@ -234,10 +250,10 @@ __device__ __forceinline__ int cg_contact(float4* pos, uint32_t* alive, uint32_t
 //    take the radicals in index order: which of several contacts is claimed
 //    depends on when threads run, and cell order shifts the yields of a crowded
 //    origin by 0.1 % for 5 % of the time.
-__global__ void k_cg_react(float4* pos, uint32_t* alive, uint32_t n, const uint32_t* tab, const float4* sorted,
-                           const CgState* st, uint32_t step, uint32_t k0, uint32_t k1, uint32_t* prod) {
+__global__ void k_cg_react(float4* pos, uint32_t* alive, const uint32_t* tab, const float4* sorted, const CgState* st,
+                           uint32_t step, uint32_t* prod) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || st->dense || alive[i] == 0u) return;
+    if (i >= st->n || st->dense[step & 1u] || alive[i] == 0u) return;
     const float4 me = pos[i];
     const int ki = (int)rintf(me.w);
     if (ki < 0 || ki > 3) return;
@@ -268,34 +284,19 @@ __global__ void k_cg_react(float4* pos, uint32_t* alive, uint32_t n, const uint3
                     if (fminf(fminf(d2[0], d2[1]), fminf(d2[2], d2[3])) > R2_MAX) continue;
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
-                        if (d2[u] <= R2_MAX && j[u] > i && cg_contact(pos, alive, i, ki, j[u], d2[u], step, k0, k1, draw, w, prod))
+                        if (d2[u] <= R2_MAX && j[u] > i && cg_contact(pos, alive, i, ki, j[u], d2[u], step, st, draw, w, prod))
                             return;
                 }
             }
         }
 }
 
-// Steps with an overfull cell: the reference's lists (build_hash and react,
-// chemistry.wgsl:111-122, 194-266) over 1.5 nm cells, walked at most 1024 deep.
-__global__ void k_cg_clear(const CgState* st, int* head) {
-    if (!st->dense) return;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < CG_HASH; i += gridDim.x * blockDim.x) head[i] = -1;
-}
-
-__device__ __forceinline__ int cg_cell(float x) { return (int)floorf(x / CG_CELL); }
-
-__global__ void k_cg_list(const CgState* st, const float4* pos, const uint32_t* alive, uint32_t n, int* head, int* next) {
-    if (!st->dense) return;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (alive[i] == 0u) { next[i] = -1; continue; }
-        const float4 p = pos[i];
-        next[i] = atomicExch(&head[cg_hash(cg_cell(p.x), cg_cell(p.y), cg_cell(p.z))], (int)i);
-    }
-}
-
-__global__ void k_cg_react_list(const CgState* st, float4* pos, uint32_t* alive, uint32_t n, const int* head,
-                                const int* next, uint32_t step, uint32_t k0, uint32_t k1, uint32_t* prod) {
-    if (!st->dense) return;
+// Steps with an overfull cell: the reference's walk (chemistry.wgsl:194-266), at most
+// 1024 entries of a list deep.
+__global__ void k_cg_react_list(const CgState* st, float4* pos, uint32_t* alive, const int* head, const int* next,
+                                uint32_t step, uint32_t* prod) {
+    if (!st->dense[step & 1u]) return;
+    const uint32_t n = st->n;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (alive[i] == 0u) continue;
         const float4 pi = pos[i];
@@ -313,7 +314,7 @@ __global__ void k_cg_react_list(const CgState* st, float4* pos, uint32_t* alive,
                 if (ju <= i) continue;
                 const float4 pj = pos[ju];
                 const float ddx = pi.x - pj.x, ddy = pi.y - pj.y, ddz = pi.z - pj.z;
-                done = cg_contact(pos, alive, i, ki, ju, ddx * ddx + ddy * ddy + ddz * ddz, step, k0, k1, draw, w, prod) != 0;
+                done = cg_contact(pos, alive, i, ki, ju, ddx * ddx + ddy * ddy + ddz * ddz, step, st, draw, w, prod) != 0;
             }
         }
     }
@@ -321,9 +322,10 @@ __global__ void k_cg_react_list(const CgState* st, float4* pos, uint32_t* alive,
 
 // count_alive (chemistry.wgsl:270-281) into checkpoint slot k: OH, e-aq, H
 // alive, then the running H2O2 and H2 product counts
-__global__ void k_cg_count(const float4* pos, const uint32_t* alive, uint32_t n, const uint32_t* prod,
+__global__ void k_cg_count(const float4* pos, const uint32_t* alive, const CgState* st, const uint32_t* prod,
                            uint32_t* out) {
     __shared__ uint32_t s[3];
+    const uint32_t n = st->n;
     if (threadIdx.x < 3) s[threadIdx.x] = 0;
     __syncthreads();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -340,21 +342,31 @@ __global__ void k_cg_count(const float4* pos, const uint32_t* alive, uint32_t n,
 static const float CG_DT[7] = {0.0001f, 0.001f, 0.005f, 0.05f, 0.5f, 3.0f, 30.0f};
 static const int CG_NS[7] = {10, 9, 18, 18, 18, 30, 30};
 
+// Blocks of 256 for n radicals, rounded up to one of eight sizes per factor of two, so that
+// batches of about the same size (a spectrum's next seed) find their schedule captured.
+uint32_t cg_blocks(uint32_t n) {
+    const uint32_t nb = (n + 255) / 256;
+    uint32_t unit = 1;
+    while (unit * 16 <= nb) unit *= 2;
+    return (nb + unit - 1) / unit * unit;
+}
+
 cudaError_t cg_run(const CgArgs& a, cudaStream_t s, cudaGraphExec_t* cache, CgGraphKey* key) {
     const uint32_t n = a.n;
-    const unsigned nb = (n + 255) / 256;
+    const unsigned nb = cg_blocks(n);
     cudaError_t e;
-    k_cg_init<<<nb, 256, 0, s>>>(a.rad, n, a.k0, a.k1, a.pos, a.alive);
+    k_cg_init<<<nb, 256, 0, s>>>(a.rad, n, a.k0, a.k1, a.pos, a.alive, a.st);
     { cudaError_t me_ = cudaMemsetAsync(a.counts, 0, 8 * 5 * sizeof(uint32_t), s); if (me_ != cudaSuccess) return me_; }
     { cudaError_t me_ = cudaMemsetAsync(a.prod, 0, 2 * sizeof(uint32_t), s); if (me_ != cudaSuccess) return me_; }
-    k_cg_count<<<296, 256, 0, s>>>(a.pos, a.alive, n, a.prod, a.counts);
+    k_cg_count<<<296, 256, 0, s>>>(a.pos, a.alive, a.st, a.prod, a.counts);
     if ((e = cudaMemsetAsync(a.tab, 0, 2 * (size_t)CG_HASH * sizeof(uint32_t), s)) != cudaSuccess) return e;
-    // the schedule as one graph; rebuilt when the buffers or sizes change
+    if ((e = cudaMemsetAsync(a.head, 0xff, (size_t)CG_HASH * sizeof(int), s)) != cudaSuccess) return e;
+    // the schedule as one graph; rebuilt when the buffers or the grid sizes change
     CgGraphKey want;
     memset(&want, 0, sizeof want);
     want.pos = a.pos; want.sorted = a.sorted; want.alive = a.alive; want.tab = a.tab; want.cell = a.cell;
     want.rank = a.rank; want.prod = a.prod; want.counts = a.counts; want.head = a.head; want.next = a.next;
-    want.st = a.st; want.n = n; want.k0 = a.k0; want.k1 = a.k1;
+    want.st = a.st; want.nb = nb; want.cap = a.cap;
     if (!*cache || memcmp(key, &want, sizeof want) != 0) {
         if (*cache) { cudaGraphExecDestroy(*cache); *cache = nullptr; }
         cudaStream_t cs;
@@ -366,16 +378,15 @@ cudaError_t cg_run(const CgArgs& a, cudaStream_t s, cudaGraphExec_t* cache, CgGr
             for (int k = 0; k < CG_NS[stage]; ++k) {
                 ++step;
                 uint32_t *tab = a.tab + (size_t)(step & 1u) * CG_HASH, *tab_old = a.tab + (size_t)((step + 1) & 1u) * CG_HASH;
-                uint32_t *cell = a.cell + (size_t)(step & 1u) * n, *cell_old = a.cell + (size_t)((step + 1) & 1u) * n;
-                k_cg_diffuse<<<nb, 256, 0, cs>>>(a.pos, a.alive, n, CG_DT[stage], step, a.k0, a.k1, tab, cell, a.rank, a.st);
-                k_cg_reserve<<<(n + CG_RB - 1) / CG_RB, CG_RB, 0, cs>>>(a.pos, n, tab, cell, a.rank, a.st);
-                k_cg_sort<<<nb, 256, 0, cs>>>(a.pos, n, tab, cell, a.rank, a.sorted, tab_old, step > 1 ? cell_old : nullptr);
-                k_cg_react<<<nb, 256, 0, cs>>>(a.pos, a.alive, n, tab, a.sorted, a.st, step, a.k0, a.k1, a.prod);
-                k_cg_clear<<<592, 256, 0, cs>>>(a.st, a.head);
-                k_cg_list<<<592, 256, 0, cs>>>(a.st, a.pos, a.alive, n, a.head, a.next);
-                k_cg_react_list<<<592, 256, 0, cs>>>(a.st, a.pos, a.alive, n, a.head, a.next, step, a.k0, a.k1, a.prod);
+                uint32_t *cell = a.cell + (size_t)(step & 1u) * a.cap, *cell_old = a.cell + (size_t)((step + 1) & 1u) * a.cap;
+                k_cg_diffuse<<<nb, 256, 0, cs>>>(a.pos, a.alive, CG_DT[stage], step, tab, cell, a.rank, a.st, a.head);
+                k_cg_reserve<<<(nb * 256 + CG_RB - 1) / CG_RB, CG_RB, 0, cs>>>(a.pos, tab, cell, a.rank, a.st, step);
+                k_cg_sort<<<nb, 256, 0, cs>>>(a.pos, tab, cell, a.rank, a.sorted, tab_old, step > 1 ? cell_old : nullptr,
+                                              a.st, step, a.head, a.next);
+                k_cg_react<<<nb, 256, 0, cs>>>(a.pos, a.alive, tab, a.sorted, a.st, step, a.prod);
+                k_cg_react_list<<<592, 256, 0, cs>>>(a.st, a.pos, a.alive, a.head, a.next, step, a.prod);
             }
-            k_cg_count<<<296, 256, 0, cs>>>(a.pos, a.alive, n, a.prod, a.counts + 5 * (stage + 1));
+            k_cg_count<<<296, 256, 0, cs>>>(a.pos, a.alive, a.st, a.prod, a.counts + 5 * (stage + 1));
         }
         e = cudaStreamEndCapture(cs, &g);
         cudaStreamDestroy(cs);
