@@ -70,11 +70,12 @@ struct IrtShape { uint32_t init_per_sm, loop_per_sm; };
 int irt_warps(int device, const IrtShape& shape, uint32_t nseg);
 // ev (optional, 3 events): recorded after the load, the initial pairing and the sort
 cudaError_t launch_irt(const IArgs& a, int device, const IrtShape& shape, cudaStream_t s, cudaEvent_t* ev = nullptr);
-// A captured IRT launch sequence and what it was captured for (irt.cu irt_graph_run).
+// The last call's arguments and, once they were repeated, its captured launch sequence
+// (irt.cu irt_graph_run).
 struct IrtGraphKey { IArgs a; IrtShape shape; int device; cudaEvent_t* ev; };
 struct IrtGraph {
     cudaGraphExec_t exec = nullptr;
-    IrtGraphKey key;
+    IrtGraphKey key{};                   // no call's (its pointers are null)
     bool off = false;                    // capturing failed once: plain launches from then on
 };
 cudaError_t irt_graph_run(const IArgs& a, int device, const IrtShape& shape, cudaStream_t s, cudaEvent_t* ev,
