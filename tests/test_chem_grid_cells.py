@@ -26,14 +26,18 @@ def clusters(n, k, sigma, seed):
     (30_000, 15, 0.4),         # 2000 per cluster within a nanometre: overfull until they spread
 ])
 def test_yields_against_oracle(ctx, n, k, sigma):
-    """t = 0 exactly; later within 2 % (the order of the claims, as in
-    test_grid_chemistry_gpu_against_oracle) and 4 standard deviations of a count."""
+    """t = 0 exactly; later the mean of eight calls, whose claims race, within 2 % (the order
+    of the claims, as in test_grid_chemistry_gpu_against_oracle) and 4 standard deviations of a
+    count."""
     rad = clusters(n, k, sigma, n + k)
     ref, _, _ = oracle.chem_grid(rad, seed=9)
-    r = _lib.ChemGridResult()
-    _lib.check("grid", _lib.lib().wgdna_chem_grid(ctx.h, _lib.ptr(rad), n, 16, 1000.0, 9, C.byref(r), None, None, 0))
-    got, ref = np.array(r.counts).astype(float), ref.astype(float)
-    np.testing.assert_array_equal(got[0], ref[0])
+    runs = []
+    for _ in range(8):
+        r = _lib.ChemGridResult()
+        _lib.check("grid", _lib.lib().wgdna_chem_grid(ctx.h, _lib.ptr(rad), n, 16, 1000.0, 9, C.byref(r), None, None, 0))
+        runs.append(np.array(r.counts).astype(float))
+        np.testing.assert_array_equal(runs[-1][0], ref[0])
+    got, ref = np.mean(runs, axis=0), ref.astype(float)
     assert np.all(np.abs(got - ref) <= 0.02 * ref + 4 * np.sqrt(ref + 1)), (got, ref)
 
 
