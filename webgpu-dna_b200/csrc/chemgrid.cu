@@ -18,12 +18,14 @@
 // still above the largest reaction radius, so the same pairs are in contact and
 // there are 6 times fewer to test), the radicals of a cell are stored side by side
 // (a counting sort per step) instead of chained, and are read four at a time.
-// Measured at 4096 x 1 keV (0.63 M radicals): 1614 us per react kernel with lists of
-// 1.5 nm cells, 137 us now; 1640 and 165 us per whole step.
+// Measured at 4096 x 1 keV (0.53 M radicals, all tracks from one point): 1680 us per step with
+// lists of 1.5 nm cells, 160 us now.
 //
 // The reference's walk stops after 1024 entries of a 1.5 nm cell.  While no such cell
-// (eight of 0.75 nm) holds more, no walk is stopped and the results are those of the
-// lists; a step with a fuller one walks the lists as the reference does.
+// (eight of 0.75 nm) holds more, no walk is stopped; the contacts found are rolled in the
+// order of the lists (k_cg_react), so the results are theirs, up to which of several
+// claims on one radical is the first.  A step with a fuller cell walks the lists as the
+// reference does.
 //
 // Random numbers: Philox4x32-10 with counter (radical, step, 0, 6) and the
 // call's key; the f32 Gaussians use this build's own log / sincos
@@ -250,6 +252,21 @@ __device__ __forceinline__ int cg_contact(float4* pos, uint32_t* alive, uint32_t
 //    take the radicals in index order: which of several contacts is claimed
 //    depends on when threads run, and cell order shifts the yields of a crowded
 //    origin by 0.1 % for 5 % of the time.
+//    The first contact that passes its roll wins, so the order of the rolls decides which
+//    kind of pair reacts.  It is the lists': the 27 cells of 1.5 nm one after another, a
+//    cell's radicals by falling index.  The contacts found in the 0.75 nm cells are therefore
+//    kept by their place in that walk (CG_KEEP at a time; a radical whose rolls all fail
+//    looks through the cells again for the ones after) before the first roll.  A cell that
+//    shares its bucket with another of the walk is met at both places, as in the lists:
+//    (-1, -1, z) and (1, 1, z) always do.
+//    Yields after 1 us against claims in radical order, H2O2 and H2, mean of 32 inputs of
+//    30,000 radicals in 15 clusters of sigma 0.4 nm (40 of 0.5 nm): lists -2.7 and -1.9 %
+//    (-1.6 and -0.8), rolls in the order of the 0.75 nm cells -4.2 and -2.9 (-3.2 and -2.2),
+//    now +1.0 and +0.4 (+1.6 and +0.7).  CG_KEEP 4 and 8, a call of 530,000 radicals: 12.7 ms
+//    both; 40 clusters 2.2 and 1.6 % of H2O2; in the cells' order 11.6 ms.
+constexpr uint32_t CG_LAST = 0x7fffffu;          // a contact's key: place << 23 | CG_LAST - index
+constexpr int CG_KEEP = 8;
+
 __global__ void k_cg_react(float4* pos, uint32_t* alive, const uint32_t* tab, const float4* sorted, const CgState* st,
                            uint32_t step, uint32_t* prod) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -258,37 +275,92 @@ __global__ void k_cg_react(float4* pos, uint32_t* alive, const uint32_t* tab, co
     const int ki = (int)rintf(me.w);
     if (ki < 0 || ki > 3) return;
     const int ix = cg_fine(me.x), iy = cg_fine(me.y), iz = cg_fine(me.z);
-    constexpr float R2_MAX = 0.61f * 0.61f * 1.0001f;            // cg_sigma_react's largest
-    uint32_t draw = 0;
+    const int cx = cg_cell(me.x), cy = cg_cell(me.y), cz = cg_cell(me.z);
+    // largest squared distance of a contact by the other's kind when it was sorted (an e-aq may
+    // have become an H since)
+    float r2k[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float r = k == 1 ? fmaxf(cg_sigma_react(ki, 1), cg_sigma_react(ki, 2)) : cg_sigma_react(ki, k);
+        r2k[k] = r > 0.0f ? r * r : -1.0f;
+    }
+    const float r2m = fmaxf(fmaxf(r2k[0], r2k[1]), fmaxf(r2k[2], r2k[3]));
+    uint32_t draw = 0, from = 0;
     u4 w = {0, 0, 0, 0};
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy) {
-            uint32_t word[3];                                    // three lookups in flight
+    for (;;) {
+        // the first CG_KEEP contacts from `from` on: place of the cell in the walk, falling index
+        uint32_t key[CG_KEEP];
 #pragma unroll
-            for (int dx = 0; dx < 3; ++dx) word[dx] = tab[cg_hash(ix + dx - 1, iy + dy, iz + dz)];
+        for (int k = 0; k < CG_KEEP; ++k) key[k] = CG_NONE;
+        for (int dz = -1; dz <= 1; ++dz)
+            for (int dy = -1; dy <= 1; ++dy) {
+                uint32_t word[3];                                // three lookups in flight
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx) word[dx] = tab[cg_hash(ix + dx - 1, iy + dy, iz + dz)];
 #pragma unroll 1
-            for (int dx = 0; dx < 3; ++dx) {
-                const uint32_t v = dx == 0 ? word[0] : dx == 1 ? word[1] : word[2];
-                const float4* S = sorted + (v & 0x7fffffu);
-                // four entries in flight; the last inserted first, as in the lists
-                for (int c = (int)(v >> 23) - 1; c >= 0; c -= 4) {
-                    float d2[4];
-                    uint32_t j[4];
+                for (int dx = 0; dx < 3; ++dx) {
+                    const uint32_t v = dx == 0 ? word[0] : dx == 1 ? word[1] : word[2];
+                    const float4* S = sorted + (v & 0x7fffffu);
+                    // four entries in flight
+                    for (int c = (int)(v >> 23) - 1; c >= 0; c -= 4) {
+                        float d2[4];
+                        uint32_t jw[4];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float4 q = S[max(c - u, 0)];
-                        const float ddx = me.x - q.x, ddy = me.y - q.y, ddz = me.z - q.z;
-                        d2[u] = c >= u ? ddx * ddx + ddy * ddy + ddz * ddz : 1e30f;
-                        j[u] = __float_as_uint(q.w) & 0x7fffffu;
+                        for (int u = 0; u < 4; ++u) {
+                            const float4 q = S[max(c - u, 0)];
+                            const float ddx = me.x - q.x, ddy = me.y - q.y, ddz = me.z - q.z;
+                            d2[u] = c >= u ? ddx * ddx + ddy * ddy + ddz * ddz : 1e30f;
+                            jw[u] = __float_as_uint(q.w);
+                        }
+                        if (fminf(fminf(d2[0], d2[1]), fminf(d2[2], d2[3])) > r2m) continue;
+                        uint32_t m = 0;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const uint32_t kj = jw[u] >> 23;
+                            const float lim = kj == 0u ? r2k[0] : kj == 1u ? r2k[1] : kj == 2u ? r2k[2] : kj == 3u ? r2k[3] : -1.0f;
+                            if (d2[u] <= lim && (jw[u] & CG_LAST) > i) m |= 1u << u;
+                        }
+#pragma unroll 1
+                        for (; m; m &= m - 1u) {
+                            const float4 q = S[c - (__ffs(m) - 1)];
+                            const uint32_t low = CG_LAST - (__float_as_uint(q.w) & CG_LAST);
+                            const uint32_t hq = cg_list(q);
+                            uint32_t place = 0;
+#pragma unroll 1
+                            for (int z = -1; z <= 1; ++z)
+#pragma unroll 1
+                                for (int y = -1; y <= 1; ++y)
+#pragma unroll 1
+                                    for (int x = -1; x <= 1; ++x, ++place) {
+                                        if (cg_hash(cx + x, cy + y, cz + z) != hq) continue;
+                                        uint32_t add = place << 23 | low;
+                                        bool have = add < from;
+#pragma unroll
+                                        for (int k = 0; k < CG_KEEP; ++k) have |= add == key[k];
+                                        if (have) continue;      // (two 0.75 nm cells of one bucket find it twice)
+#pragma unroll
+                                        for (int k = 0; k < CG_KEEP; ++k) {
+                                            const uint32_t old = key[k];
+                                            key[k] = min(old, add);
+                                            add = max(old, add);
+                                        }
+                                    }
+                        }
                     }
-                    if (fminf(fminf(d2[0], d2[1]), fminf(d2[2], d2[3])) > R2_MAX) continue;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (d2[u] <= R2_MAX && j[u] > i && cg_contact(pos, alive, i, ki, j[u], d2[u], step, st, draw, w, prod))
-                            return;
                 }
             }
+#pragma unroll 1
+        for (int k = 0; k < CG_KEEP; ++k) {
+            const uint32_t first = key[0], j = CG_LAST - (first & CG_LAST);
+            if (first == CG_NONE) return;
+#pragma unroll
+            for (int q = 1; q < CG_KEEP; ++q) key[q - 1] = key[q];
+            from = first + 1u;
+            const float4 q = pos[j];
+            const float ddx = me.x - q.x, ddy = me.y - q.y, ddz = me.z - q.z;
+            if (cg_contact(pos, alive, i, ki, j, ddx * ddx + ddy * ddy + ddz * ddz, step, st, draw, w, prod)) return;
         }
+    }
 }
 
 // Steps with an overfull cell: the reference's walk (chemistry.wgsl:194-266), at most
