@@ -205,7 +205,10 @@ __global__ void __launch_bounds__(CG_RB) k_cg_reserve(const float4* pos, uint32_
 //    an overfull cell also builds the reference's lists (build_hash, chemistry.wgsl:111-122).
 //    Clearing the heads and building the lists in launches of their own cost every ordinary
 //    step two that return at once, and building them in k_cg_react slowed that kernel (530,000
-//    radicals, a call: 12.4 ms with the launches, 14.2 with k_cg_react, 12.3 so).
+//    radicals, a call: 12.4 ms with the launches, 14.2 with k_cg_react, 12.3 so).  Such a step
+//    has no use for the bucket order: with 1200 radicals that stay in one cell a call of
+//    5 million takes 466 ms (488 with the order made all the same, and with 592 blocks walking
+//    the lists; 480 by lists alone).
 __global__ void k_cg_sort(const float4* pos, const uint32_t* tab, const uint32_t* cell, const uint32_t* rank, float4* sorted,
                           uint32_t* tab_old, const uint32_t* cell_old, const CgState* st, uint32_t step, int* head, int* next) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -214,7 +217,7 @@ __global__ void k_cg_sort(const float4* pos, const uint32_t* tab, const uint32_t
     const uint32_t h = cell[i];
     if (h == CG_NONE) return;                        // dead: no list leads to it
     const float4 p = pos[i];
-    if (st->dense[step & 1u]) next[i] = atomicExch(&head[cg_list(p)], (int)i);
+    if (st->dense[step & 1u]) { next[i] = atomicExch(&head[cg_list(p)], (int)i); return; }
     const uint32_t kind = (uint32_t)(int)rintf(p.w) & 7u;
     sorted[(tab[h] & 0x7fffffu) + rank[i]] = make_float4(p.x, p.y, p.z, __uint_as_float(i | (kind << 23)));
 }
@@ -456,7 +459,7 @@ cudaError_t cg_run(const CgArgs& a, cudaStream_t s, cudaGraphExec_t* cache, CgGr
                 k_cg_sort<<<nb, 256, 0, cs>>>(a.pos, tab, cell, a.rank, a.sorted, tab_old, step > 1 ? cell_old : nullptr,
                                               a.st, step, a.head, a.next);
                 k_cg_react<<<nb, 256, 0, cs>>>(a.pos, a.alive, tab, a.sorted, a.st, step, a.prod);
-                k_cg_react_list<<<592, 256, 0, cs>>>(a.st, a.pos, a.alive, a.head, a.next, step, a.prod);
+                k_cg_react_list<<<nb < 1184 ? nb : 1184, 256, 0, cs>>>(a.st, a.pos, a.alive, a.head, a.next, step, a.prod);
             }
             k_cg_count<<<296, 256, 0, cs>>>(a.pos, a.alive, a.st, a.prod, a.counts + 5 * (stage + 1));
         }
