@@ -84,6 +84,24 @@ int upload_norm(SgState* s, cudaStream_t st) {
     return WGDNA_OK;
 }
 
+int fill_state(SgState* s, cudaStream_t st) {
+    STRY(salloc(&s->p, SG_NPARAM)); STRY(salloc(&s->m, SG_NPARAM)); STRY(salloc(&s->v, SG_NPARAM));
+    STRY(salloc(&s->g, SG_NPARAM));
+    STRY(salloc(&s->W, SG_WTOTAL)); STRY(salloc(&s->WT, SG_WTOTAL));
+    STRY(salloc(&s->xmean, SG_IN)); STRY(salloc(&s->xinv, SG_IN));
+    STRY(salloc(&s->ymean, SG_OUT)); STRY(salloc(&s->ystd, SG_OUT));
+    STRY(salloc(&s->loss, 1)); STRY(salloc(&s->err, 1)); STRY(salloc(&s->acc, SG_OUT + 1));
+    STRY(salloc(&s->dbin, SG_DBIN));
+    WG_CUDA_OK(launch_dbin_table(s->dbin, st));
+    for (float* q : {s->p, s->m, s->v, s->g}) WG_CUDA_OK(cudaMemsetAsync(q, 0, SG_NPARAM * 4, st));
+    WG_CUDA_OK(cudaMemsetAsync(s->err, 0, 4, st));
+    for (int k = 0; k < SG_IN; ++k) { s->h_xmean[k] = 0.0f; s->h_xstd[k] = 1.0f; }
+    for (int k = 0; k < SG_OUT; ++k) { s->h_ymean[k] = 0.0f; s->h_ystd[k] = 1.0f; }
+    STRY(upload_norm(s, st));
+    WG_CUDA_OK(cudaStreamSynchronize(st));
+    return WGDNA_OK;
+}
+
 int ensure_state(wgdna_ctx* c, CtxView& v, SgState** out) {
     ctx_view(c, &v);
     WG_CUDA_OK(cudaSetDevice(v.device));
@@ -93,24 +111,14 @@ int ensure_state(wgdna_ctx* c, CtxView& v, SgState** out) {
         *out = *v.sg;
         return WGDNA_OK;
     }
+    // All of it on the context's stream, which does not wait for the default one, and waited
+    // for once, so that the state is complete whatever stream the next call uses.
     SgState* s = new SgState();
-    *v.sg = s;
+    const int r = fill_state(s, v.stream);
+    if (r != WGDNA_OK) { sg_free(s); return r; }
     s->mma_ns = v.mma_ns;
     s->give_up_first = v.mma_give_up_first ? 1u : 0u;
-    STRY(salloc(&s->p, SG_NPARAM)); STRY(salloc(&s->m, SG_NPARAM)); STRY(salloc(&s->v, SG_NPARAM));
-    STRY(salloc(&s->g, SG_NPARAM));
-    STRY(salloc(&s->W, SG_WTOTAL)); STRY(salloc(&s->WT, SG_WTOTAL));
-    STRY(salloc(&s->xmean, SG_IN)); STRY(salloc(&s->xinv, SG_IN));
-    STRY(salloc(&s->ymean, SG_OUT)); STRY(salloc(&s->ystd, SG_OUT));
-    STRY(salloc(&s->loss, 1)); STRY(salloc(&s->err, 1)); STRY(salloc(&s->acc, SG_OUT + 1));
-    STRY(salloc(&s->dbin, SG_DBIN));
-    WG_CUDA_OK(launch_dbin_table(s->dbin, v.stream));
-    WG_CUDA_OK(cudaMemset(s->m, 0, SG_NPARAM * 4)); WG_CUDA_OK(cudaMemset(s->v, 0, SG_NPARAM * 4));
-    WG_CUDA_OK(cudaMemset(s->g, 0, SG_NPARAM * 4)); WG_CUDA_OK(cudaMemset(s->p, 0, SG_NPARAM * 4));
-    WG_CUDA_OK(cudaMemset(s->err, 0, 4));
-    for (int k = 0; k < SG_IN; ++k) { s->h_xmean[k] = 0.0f; s->h_xstd[k] = 1.0f; }
-    for (int k = 0; k < SG_OUT; ++k) { s->h_ymean[k] = 0.0f; s->h_ystd[k] = 1.0f; }
-    STRY(upload_norm(s, v.stream));
+    *v.sg = s;
     *out = s;
     return WGDNA_OK;
 }
