@@ -1,5 +1,6 @@
 """First calls of a context while the caller's default stream is busy: what they clear or
 upload must not wait there, and so land after what follows on the context's own stream."""
+import ctypes as C
 import os
 import re
 
@@ -20,6 +21,11 @@ def on_default_stream(name):
 
 def test_surrogate_clears_nothing_on_the_default_stream():
     assert on_default_stream("surrogate_api.cu") == []
+
+
+@pytest.mark.parametrize("name", ["capi.cu", "irt.cu", "tables.cu"])
+def test_context_uploads_nothing_on_the_default_stream(name):
+    assert on_default_stream(name) == []
 
 
 def busy_default_stream():
@@ -57,3 +63,29 @@ def test_surrogate_parameters_survive_a_busy_default_stream():
     finally:
         ctx.close()
         other.close()
+
+
+@pytest.mark.gpu
+def test_context_made_while_the_default_stream_is_busy():
+    """Its first transport equals one made in quiet, and the queue of secondaries stays as
+    the transport left it."""
+    import torch
+    out = []
+    for busy in (False, True):
+        if busy:
+            busy_default_stream()
+        ctx = wgdna.Context(max_primaries=64, max_rad=2_000_000, max_sec=200_000)
+        try:
+            ctx.set_tuning(stash_spill=0, stash_keep=0)          # every secondary goes through the queue
+            p = wgdna.transport_params(64, 10000.0, 15000.0, 7.5, dna=wgdna.build_dna_target(), seed=4)
+            st = _lib.TransportStats()
+            _lib.check("transport", _lib.lib().wgdna_transport(ctx.h, C.byref(p), C.byref(st)))
+            if busy:
+                torch.cuda.synchronize()
+            res = np.zeros(64 * 8, np.float32)
+            _lib.check("copy", _lib.lib().wgdna_transport_copy_out(ctx.h, _lib.ptr(res), None, None, 0, None))
+            out.append((res, int(st.rad_n_stored), np.array(st.counters)))
+        finally:
+            ctx.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)

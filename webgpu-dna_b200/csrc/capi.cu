@@ -17,7 +17,7 @@
 #include "transport.cuh"
 
 namespace wg {
-int tables_load(const char* path, Tables* out, float** d_small, float2** d_xcw);
+int tables_load(const char* path, Tables* out, float** d_small, float2** d_xcw, cudaStream_t s);
 }
 
 using namespace wg;
@@ -260,10 +260,12 @@ extern "C" int wgdna_create(const wgdna_cfg* cfg, wgdna_ctx** out) {
     c->cfg = c0;
     std::string tp = c0.tables_path ? std::string(c0.tables_path) : lib_dir() + "/data/cross_sections.bin";
     c->cfg.tables_path = nullptr;
-    int rc = tables_load(tp.c_str(), &c->tab, &c->d_small, &c->d_xcw);
-    if (rc != WGDNA_OK) { delete c; return rc; }
     cudaError_t e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
     if (e != cudaSuccess) { wg_set_error("cudaStreamCreate: %s", cudaGetErrorString(e)); delete c; return WGDNA_ERR_CUDA; }
+    // What follows is cleared and uploaded on this stream, which does not wait for the default
+    // one: work there could otherwise hold a clear back until a transport has begun.
+    int rc = tables_load(tp.c_str(), &c->tab, &c->d_small, &c->d_xcw, c->own);
+    if (rc != WGDNA_OK) { wgdna_destroy(c); return rc; }
     c->stream = c->own;
     for (auto& ev : c->ev) cudaEventCreate(&ev);
     size_t np = c0.max_primaries, nv = (size_t)c0.vc * c0.vc * c0.vc;
@@ -284,7 +286,7 @@ extern "C" int wgdna_create(const wgdna_cfg* cfg, wgdna_ctx** out) {
     if (r == WGDNA_OK) r = dalloc(&c->d_part, c->part_cap + np + (np + 1) + 592);
     if (r == WGDNA_OK) { c->d_nsec = c->d_part + c->part_cap; c->d_first = c->d_nsec + np; c->d_share = c->d_first + np + 1; }
     if (r == WGDNA_OK) r = ensure_segments(c, (uint32_t)np);
-    if (r == WGDNA_OK && cudaMemset(c->d_secq, 0, sizeof(SecRec) * (size_t)c0.max_sec) != cudaSuccess) r = WGDNA_ERR_CUDA;
+    if (r == WGDNA_OK && cudaMemsetAsync(c->d_secq, 0, sizeof(SecRec) * (size_t)c0.max_sec, c->own) != cudaSuccess) r = WGDNA_ERR_CUDA;
     if (r == WGDNA_OK && cudaMallocHost((void**)&c->h_pin, H_PIN) != cudaSuccess) {
         cudaGetLastError();
         c->h_pin = nullptr;
@@ -579,10 +581,10 @@ static int irt_ensure(wgdna_ctx* c, uint32_t nseg, uint64_t rad_n, uint32_t cap)
     // the reaction constants live in __constant__ memory, which every device
     // holds separately: upload them once per device (the context's is current)
     static DeviceOnce consts;
-    WG_CUDA_OK(consts.run([] {
+    WG_CUDA_OK(consts.run([c] {
         IrtConst C;
         irt_constants(&C);
-        return irt_set_constants(C);
+        return irt_set_constants(C, c->stream);
     }));
     return WGDNA_OK;
 }
@@ -842,10 +844,11 @@ extern "C" int wgdna_set_dna_target(wgdna_ctx* c, double L_nm, uint32_t grid_N, 
         WG_CUDA_OK(cudaMallocHost((void**)&c->h_fib, 12 * (size_t)info.n_fibers));
         c->h_fib_cap = info.n_fibers;
     }
-    WG_CUDA_OK(cudaMemcpy(c->d_fy, fy.data(), fy.size() * 4, cudaMemcpyHostToDevice));
-    WG_CUDA_OK(cudaMemcpy(c->d_fz, fz.data(), fz.size() * 4, cudaMemcpyHostToDevice));
-    WG_CUDA_OK(cudaMemcpy(c->d_rbb0, r0.data(), r0.size() * 4, cudaMemcpyHostToDevice));
-    WG_CUDA_OK(cudaMemcpy(c->d_rbb1, r1.data(), r1.size() * 4, cudaMemcpyHostToDevice));
+    WG_CUDA_OK(cudaMemcpyAsync(c->d_fy, fy.data(), fy.size() * 4, cudaMemcpyHostToDevice, c->stream));
+    WG_CUDA_OK(cudaMemcpyAsync(c->d_fz, fz.data(), fz.size() * 4, cudaMemcpyHostToDevice, c->stream));
+    WG_CUDA_OK(cudaMemcpyAsync(c->d_rbb0, r0.data(), r0.size() * 4, cudaMemcpyHostToDevice, c->stream));
+    WG_CUDA_OK(cudaMemcpyAsync(c->d_rbb1, r1.data(), r1.size() * 4, cudaMemcpyHostToDevice, c->stream));
+    WG_CUDA_OK(cudaStreamSynchronize(c->stream));
     c->dna = info;
     return WGDNA_OK;
 }

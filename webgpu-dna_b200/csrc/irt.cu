@@ -1696,7 +1696,10 @@ __global__ void k_seg_max(const unsigned long long* off, uint32_t nseg, unsigned
 }
 
 // ------------------------------------------------------------------ host side
-cudaError_t irt_set_constants(const IrtConst& c) { return cudaMemcpyToSymbol(c_irt, &c, sizeof c); }
+cudaError_t irt_set_constants(const IrtConst& c, cudaStream_t s) {
+    const cudaError_t e = cudaMemcpyToSymbolAsync(c_irt, &c, sizeof c, 0, cudaMemcpyHostToDevice, s);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(s);
+}
 
 static int blocks_for(const void* k, int device, uint32_t limit = 0) {
     int sms = 0, per = 0;

@@ -61,7 +61,7 @@ struct IArgs {
 
 constexpr uint32_t IRT_PCAP_MIN = 1024;  // pcap of tracks of up to 480 entries
 
-cudaError_t irt_set_constants(const IrtConst& c);
+cudaError_t irt_set_constants(const IrtConst& c, cudaStream_t s);     // there when it returns
 // Resident blocks per SM of the pairing and event kernels: as many as fit, at
 // most the given number (0 = no limit; of the event kernel in blocks of 4 warps).  The heap
 // overflow is sized per track in flight, so irt_warps and launch_irt must see the

@@ -25,7 +25,7 @@ static bool find(const std::vector<Entry>& es, const char* name, uint32_t count,
     return false;
 }
 
-int tables_load(const char* path, Tables* out, float** d_small, float2** d_xcw) {
+int tables_load(const char* path, Tables* out, float** d_small, float2** d_xcw, cudaStream_t s) {
     FILE* f = fopen(path, "rb");
     if (!f) { wg_set_error("cannot open cross-section blob %s", path); return WGDNA_ERR_TABLES; }
     fseek(f, 0, SEEK_END);
@@ -112,8 +112,9 @@ int tables_load(const char* path, Tables* out, float** d_small, float2** d_xcw) 
                 small[S_GUIDE + (k * NWE_ + r) * GUIDES + m] = xwc[(size_t)k * NWE_ * NWR_ + r * NWR_ + 16 * m];
     WG_CUDA_OK(cudaMalloc(d_small, small.size() * 4));
     WG_CUDA_OK(cudaMalloc(d_xcw, xcw.size() * sizeof(float2)));
-    WG_CUDA_OK(cudaMemcpy(*d_small, small.data(), small.size() * 4, cudaMemcpyHostToDevice));
-    WG_CUDA_OK(cudaMemcpy(*d_xcw, xcw.data(), xcw.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    WG_CUDA_OK(cudaMemcpyAsync(*d_small, small.data(), small.size() * 4, cudaMemcpyHostToDevice, s));
+    WG_CUDA_OK(cudaMemcpyAsync(*d_xcw, xcw.data(), xcw.size() * sizeof(float2), cudaMemcpyHostToDevice, s));
+    WG_CUDA_OK(cudaStreamSynchronize(s));
     t.small = *d_small;
     t.xcw = *d_xcw;
     *out = t;
