@@ -218,7 +218,12 @@ template <class T> static int dalloc(T** p, size_t n) {
     if (*p) { cudaFree(*p); *p = nullptr; }
     if (n == 0) n = 1;
     cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
-    if (e != cudaSuccess) { wg_set_error("cudaMalloc(%zu bytes): %s", n * sizeof(T), cudaGetErrorString(e)); *p = nullptr; return WGDNA_ERR_NOMEM; }
+    if (e != cudaSuccess) {
+        cudaGetLastError();              // or the next launch check would report it
+        wg_set_error("cudaMalloc(%zu bytes): %s", n * sizeof(T), cudaGetErrorString(e));
+        *p = nullptr;
+        return WGDNA_ERR_NOMEM;
+    }
     return WGDNA_OK;
 }
 #define TRY(x) do { int r_ = (x); if (r_ != WGDNA_OK) return r_; } while (0)
@@ -226,6 +231,7 @@ template <class T> static int dalloc(T** p, size_t n) {
 static int ensure_segments(wgdna_ctx* c, uint32_t nseg) {
     if (nseg <= c->seg_cap) return WGDNA_OK;
     uint32_t cap = nseg < 4096 ? 4096 : nseg;
+    c->seg_cap = 0;
     TRY(dalloc(&c->d_pid_cnt, cap));
     TRY(dalloc(&c->d_pid_cur, cap));
     TRY(dalloc(&c->d_pid_off, (size_t)cap + 1));
@@ -532,6 +538,9 @@ extern "C" int wgdna_run_transport(wgdna_ctx* c, const wgdna_transport_params* p
 // ------------------------------------------------------------------ Phase C
 static void irt_constants(IrtConst* C);
 
+// A capacity is 0 until every buffer it stands for has its new size: an allocation that
+// fails leaves null pointers, which a smaller call must not take for the old buffers.
+//
 // Per-track particle slots 2*len + 64 and event slots 16*len + 2048 (the
 // kernels' tbase / ebase), per track in flight heap overflow hcap = 8*pcap + 4352
 // and pcap partners, pcap at least the largest track's particle slots
@@ -545,27 +554,32 @@ static int irt_ensure(wgdna_ctx* c, uint32_t nseg, uint64_t rad_n, uint32_t cap)
     const IrtShape shape{c->tune.irt_init_blocks_per_sm, c->tune.irt_loop_blocks_per_sm};
     size_t hov = (size_t)irt_warps(c->device, shape, nseg) * (hcap + (size_t)pcap);
     if (slots > c->irt_slots) {
+        c->irt_slots = 0;
         TRY(dalloc(&c->d_px, slots)); TRY(dalloc(&c->d_py, slots)); TRY(dalloc(&c->d_pz, slots));
         TRY(dalloc(&c->d_tb, slots)); TRY(dalloc(&c->d_sp, slots)); TRY(dalloc(&c->d_alive8, slots));
         TRY(dalloc(&c->d_lst, 6 * slots)); TRY(dalloc(&c->d_lpos, slots));
         c->irt_slots = slots;
     }
     if (evslots > c->irt_evslots) {
+        c->irt_evslots = 0;
         TRY(dalloc(&c->d_evt, evslots)); TRY(dalloc(&c->d_evab, evslots));
         c->irt_evslots = evslots;
     }
     if (hov > c->irt_hov) {
+        c->irt_hov = 0;
         TRY(dalloc(&c->d_hov_t, hov)); TRY(dalloc(&c->d_hov_ab, hov));
         c->irt_hov = hov;
     }
     c->irt_hcap = hcap;
     c->irt_pcap = pcap;
     if (slots > c->irt_pf_slots) {
+        c->irt_pf_slots = 0;
         TRY(dalloc(&c->d_pf, slots));
         TRY(dalloc(&c->d_rec, 6 * slots));
         c->irt_pf_slots = slots;
     }
     if (nseg > c->irt_tracks) {
+        c->irt_tracks = 0;
         TRY(dalloc(&c->d_track, 11 * (size_t)nseg)); TRY(dalloc(&c->d_toff, (size_t)nseg + 1));
         TRY(dalloc(&c->d_tdel, (size_t)nseg));
         c->irt_tracks = nseg;
@@ -573,6 +587,7 @@ static int irt_ensure(wgdna_ctx* c, uint32_t nseg, uint64_t rad_n, uint32_t cap)
     if (!c->d_irt_cnt) TRY(dalloc(&c->d_irt_cnt, 8));
     // a track of n entries has up to 8 n + 1024 events, in chunks of 2048 from 4097 on
     if (rad_n / 128 + 64 > c->irt_big) {
+        c->irt_big = 0;
         TRY(dalloc(&c->d_irt_big, rad_n / 128 + 64));
         c->irt_big = rad_n / 128 + 64;
     }
@@ -607,6 +622,7 @@ static int irt_run(wgdna_ctx* c, uint32_t nseg, unsigned long long maxseg, uint3
     c->curves_n = 0;
     if (c->irt_curves_on) {
         if (nseg > c->curves_cap) {
+            c->curves_cap = 0;
             TRY(dalloc(&c->d_curves, (size_t)nseg * 80));
             c->curves_cap = nseg;
         }
@@ -936,7 +952,7 @@ extern "C" int wgdna_score_indirect(wgdna_ctx* c, const float* pos, const uint32
     WG_CUDA_OK(cudaSetDevice(c->device));
     c->have_transport = false;
     TRY(hits_in(c, hits));
-    if (n > c->alive_cap) { TRY(dalloc(&c->d_alive, n)); c->alive_cap = n; }
+    if (n > c->alive_cap) { c->alive_cap = 0; TRY(dalloc(&c->d_alive, n)); c->alive_cap = n; }
     if (n) {
         WG_CUDA_OK(host_copy(&c->hc, c->device, c->d_rad_raw, pos, n * 16, cudaMemcpyHostToDevice, c->stream));
         WG_CUDA_OK(host_copy(&c->hc, c->device, c->d_alive, alive, n * 4, cudaMemcpyHostToDevice, c->stream));
@@ -1106,7 +1122,7 @@ extern "C" int wgdna_chem_grid(wgdna_ctx* c, const float* rad, uint64_t rad_n, u
     uint64_t n_all;
     if (rad) {
         n_all = rad_n;
-        if (rad_n > c->cg_rad_cap) { TRY(dalloc(&c->d_cg_rad, rad_n)); c->cg_rad_cap = rad_n; }
+        if (rad_n > c->cg_rad_cap) { c->cg_rad_cap = 0; TRY(dalloc(&c->d_cg_rad, rad_n)); c->cg_rad_cap = rad_n; }
         WG_CUDA_OK(host_copy(&c->hc, c->device, c->d_cg_rad, rad, rad_n * 16, cudaMemcpyHostToDevice, s));
         src = c->d_cg_rad;
     } else {

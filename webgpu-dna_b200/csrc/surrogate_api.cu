@@ -53,10 +53,12 @@ void sg_free(SgState* s) {
 
 namespace {
 
+// (a capacity is 0 until every buffer it stands for has its new size)
 template <class T> int salloc(T** p, size_t n) {
     if (*p) { cudaFree(*p); *p = nullptr; }
     cudaError_t e = cudaMalloc((void**)p, (n ? n : 1) * sizeof(T));
     if (e != cudaSuccess) {
+        cudaGetLastError();
         wg_set_error("cudaMalloc(%zu bytes): %s", n * sizeof(T), cudaGetErrorString(e));
         *p = nullptr;
         return WGDNA_ERR_NOMEM;
@@ -133,6 +135,7 @@ SgWeights weights(SgState* s) {
 int ensure_parts(SgState* s, uint32_t n) {
     const uint32_t k = sg_parts(n);
     if (k <= s->part_cap) return WGDNA_OK;
+    s->part_cap = 0;
     STRY(salloc(&s->part, (size_t)k * SG_NPARAM));
     s->part_cap = k;
     return WGDNA_OK;
@@ -232,6 +235,7 @@ extern "C" int wgdna_surrogate_load(wgdna_ctx* c, const float* X, const float* G
     SgState* s;
     STRY(ensure_state(c, v, &s));
     if (n > s->data_cap) {
+        s->data_cap = s->ndata = 0;
         STRY(salloc(&s->X, n * SG_IN)); STRY(salloc(&s->T, n * SG_OUT));
         s->data_cap = n;
     }
@@ -284,6 +288,7 @@ extern "C" int wgdna_surrogate_train(wgdna_ctx* c, uint32_t epochs, uint32_t bat
     const uint32_t B = (uint32_t)(batch < n ? batch : n);
     STRY(ensure_parts(s, B));
     if (n > s->perm_cap) {
+        s->perm_cap = 0;
         STRY(salloc(&s->perm, n));
         s->perm_cap = n;
     }
@@ -323,6 +328,7 @@ extern "C" int wgdna_surrogate_predict(wgdna_ctx* c, const float* X, uint64_t n,
     const float* src = s->desc;
     if (X) {
         if (n > s->desc_cap) {
+            s->desc_cap = s->desc_n = 0;
             STRY(salloc(&s->desc, n * SG_IN)); STRY(salloc(&s->pred, n * SG_OUT));
             s->desc_cap = n;
         }
@@ -353,6 +359,7 @@ extern "C" int wgdna_track_descriptors(wgdna_ctx* c, float* out, uint64_t cap, u
     if (!v.have_transport) { wg_set_error("wgdna_track_descriptors: no transport result in the context"); return WGDNA_ERR_STATE; }
     const uint64_t n = v.nseg;
     if (n > s->desc_cap) {
+        s->desc_cap = s->desc_n = 0;
         STRY(salloc(&s->desc, n * SG_IN)); STRY(salloc(&s->pred, n * SG_OUT));
         s->desc_cap = n;
     }
@@ -381,6 +388,7 @@ extern "C" int wgdna_surrogate_chemistry(wgdna_ctx* c, double* G, float* ms) {
     if (!v.have_transport) { wg_set_error("wgdna_surrogate_chemistry: no transport result in the context"); return WGDNA_ERR_STATE; }
     const uint64_t n = v.nseg;
     if (n > s->desc_cap) {
+        s->desc_cap = s->desc_n = 0;
         STRY(salloc(&s->desc, n * SG_IN)); STRY(salloc(&s->pred, n * SG_OUT));
         s->desc_cap = n;
     }
