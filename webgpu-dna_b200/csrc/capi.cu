@@ -865,6 +865,11 @@ extern "C" int wgdna_set_dna_target(wgdna_ctx* c, double L_nm, uint32_t grid_N, 
     WG_CUDA_OK(cudaMemcpyAsync(c->d_rbb0, r0.data(), r0.size() * 4, cudaMemcpyHostToDevice, c->stream));
     WG_CUDA_OK(cudaMemcpyAsync(c->d_rbb1, r1.data(), r1.size() * 4, cudaMemcpyHostToDevice, c->stream));
     WG_CUDA_OK(cudaStreamSynchronize(c->stream));
+    if (info.n_bp != c->dna.n_bp) {      // the per-site arrays are made for the new size when they are asked for
+        if (c->d_lambda) { cudaFree(c->d_lambda); c->d_lambda = nullptr; }
+        if (c->d_hits_in) { cudaFree(c->d_hits_in); c->d_hits_in = nullptr; }
+        c->have_lambda = false;
+    }
     c->dna = info;
     return WGDNA_OK;
 }
