@@ -554,7 +554,8 @@ __global__ void k_dbin_table(float2* tab) {
         const uint32_t b0 = (DBIN_E0 + threadIdx.x) << 23;
         int k = 0;
         while (k < 15 && edge[k + 1] <= b0) ++k;
-        tab[threadIdx.x] = make_float2(k < 15 ? __uint_as_float(edge[k + 1]) : __int_as_float(0x7f800000), __int_as_float(k));
+        // (no d2 is at or above a NaN: the last bin holds infinity too)
+        tab[threadIdx.x] = make_float2(__uint_as_float(k < 15 ? edge[k + 1] : 0x7fffffffu), __int_as_float(k));
     }
 }
 
@@ -591,7 +592,7 @@ __global__ void __launch_bounds__(128) k_descriptors(DescArgs a) {
             for (int t = 0; t < 3; ++t) {
                 if (i < (t == 0 ? 1u : t == 1 ? 4u : 16u)) continue;
                 const float dx = q.x - o[t].x, dy = q.y - o[t].y, dz = q.z - o[t].z;
-                const float d2 = dx * dx + dy * dy + dz * dz;
+                const float d2 = fmaxf(dx * dx + dy * dy + dz * dz, 0.0f);       // a NaN counts as 0, as in dbin
                 const int oct = min(max((int)(__float_as_uint(d2) >> 23) - DBIN_E0, 0), DBIN_N - 1);
                 const float2 b = tab[oct];
                 atomicAdd(&h[16 * t + __float_as_int(b.y) + (d2 >= b.x ? 1 : 0)], 1u);
