@@ -77,9 +77,10 @@ __device__ __forceinline__ long long near_backbone(const DnaDev& d, double x, do
     return (long long)fiber * d.n_bp_per + best_bp + (long long)best_s * d.n_bp;
 }
 
-// False only if the entry is certainly beyond reach of every fibre axis: the f32
-// offset from the nearest axis has an error below 0.03 nm for |y|, |z| up to
-// 100 um, `far` adds 0.05 nm to the reach.  A NaN goes on to the f64 geometry.
+// False only if the entry is certainly beyond reach of every fibre axis: the f32 offset
+// from the nearest axis has an error of at most (|grid_off| + 3 |y - grid_off| + sp / 2) 2^-24,
+// below 0.05 nm for |y|, |z| and |grid_off| up to 100 um, and `far` adds that to the reach (it
+// is infinite on a wider grid).  A NaN goes on to the f64 geometry.
 __device__ __forceinline__ bool maybe_near(float y, float z, float grid_off, float inv_sp, float sp, float far) {
     const float u = (y - grid_off) * inv_sp, v = (z - grid_off) * inv_sp;
     const float dy = fabsf(u - rintf(u)) * sp, dz = fabsf(v - rintf(v)) * sp;
@@ -103,7 +104,8 @@ __global__ void __launch_bounds__(FB) k_find(const float4* rad, const uint32_t* 
     const unsigned long long a = q * SEG;
     if (a >= n) return;
     const float grid_off = (float)(-(((double)d.grid_N - 1) * d.spacing) * 0.5), sp = (float)d.spacing;
-    const float inv_sp = (float)(1 / d.spacing), far = (float)(d.r_bb + r_d) + 0.05f;
+    const float inv_sp = (float)(1 / d.spacing);
+    const float far = grid_off >= -1e5f ? (float)(d.r_bb + r_d) + 0.05f : __int_as_float(0x7f800000);
     uint32_t f[6] = {0, 0, 0, 0, 0, 0}, len = 0;
     bool open = true;                             // no run has started in the segment yet
     uint32_t par = 0;                             // parity of the last run start
