@@ -1331,6 +1331,18 @@ __device__ __forceinline__ bool pair_exact(const IArgs& A, const IrtConst& C, un
 template <int W>
 constexpr int LT = W <= 4 ? IB : 32 * W;    // 16 warps per SM
 
+// One meeting of the block's IB threads, which come to it at different places of the kernel
+// (__syncthreads_count asks for one place, or one condition); how many came with `more`.
+__device__ __forceinline__ uint32_t block_meet(bool more) {
+    uint32_t n;
+    __syncwarp();
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.red.popc.u32 %0, 1, %2, p;\n\t}"
+                 : "=r"(n)
+                 : "r"((uint32_t)more), "n"(IB)
+                 : "memory");
+    return n;
+}
+
 template <int W>
 __global__ void __launch_bounds__(LT<W>, 512 / LT<W>) k_irt_loop(const __grid_constant__ IArgs A) {
     constexpr int G = LT<W> / 32 / W;            // tracks per block
@@ -1497,7 +1509,7 @@ __global__ void __launch_bounds__(LT<W>, 512 / LT<W>) k_irt_loop(const __grid_co
             const int si = S.si, sj = S.sj, ri = S.ri;
             const int np_ = C.nprod[ri];
             if (W > 1) gsync();                            // all have read the event
-            else __syncthreads_count(1);                   // the block's tracks go on together
+            else block_meet(true);                         // the block's tracks go on together
 #pragma unroll 1
             for (int pp = 0; pp < np_; ++pp) {
                 const int nsp = pp == 0 ? C.prod0[ri] : C.prod1[ri];
@@ -1660,7 +1672,7 @@ __global__ void __launch_bounds__(LT<W>, 512 / LT<W>) k_irt_loop(const __grid_co
             __syncwarp();
         }
     }
-    if (W == 1) while (__syncthreads_count(0)) {}          // until the block's last track has ended
+    if (W == 1) while (block_meet(false)) {}               // until the block's last track has ended
     if (lane == 0 && n_pairs) atomicAdd(&A.acc[10], n_pairs);
     gsync();
     if (lead) {
