@@ -125,7 +125,8 @@ typedef struct {
 
 /* Phase A + Phase B (dispatch.ts:106-145) into device memory of the context.
  * rad_buf is left in canonical order: grouped by primary, the primary's own
- * entries first, then each secondary's, each in emission order. */
+ * entries first, then each secondary's, each in emission order.  A primary with
+ * more than 8192 entries (above about 63 keV) ends in WGDNA_ERR_DEVICE. */
 int wgdna_transport(wgdna_ctx *ctx, const wgdna_transport_params *p, wgdna_transport_stats *st);
 /* Readbacks of the last transport (dispatch.ts:148-240).  Any pointer may be
  * NULL.  results: np*8 words (R struct, primary.wgsl:9); dose: vc^3 u32;

@@ -1765,9 +1765,9 @@ static bool load_wide(int device, const IArgs& a) {
 
 // Warps per track of the event kernel: two while all tracks are resident at once at 16 warps
 // per SM, more while they are at 8 per SM.  Measured (10 keV tracks on 148 SMs, ms with
-// W = 1, 2, 4, 8, 16): 64 tracks 5.96 3.46 3.13 3.02 3.07, 150: 6.34 3.90 3.56 3.47 3.83,
-// 300: 6.38 3.91 3.66 4.02 6.65, 600: 6.61 4.38 4.85 7.09 -, 1200: 6.98 6.28 8.07 - -,
-// 1800: 7.97 8.95 11.2 - -; one track of 3060 species 10.3 9.2 9.0 9.0 8.7.
+// W = 1, 2, 4, 8, 16): 64 tracks 5.12 3.09 2.88 2.80 2.87, 150: 5.46 3.15 2.89 2.80 3.57,
+// 300: 5.69 3.45 3.36 3.75 5.97, 600: 5.81 3.95 4.37 6.29 -, 1200: 6.39 5.63 7.39 - -,
+// 1800: 7.25 8.21 10.2 - -; one track of 3060 species 7.85 6.81 6.56 6.52 6.53.
 static int loop_width(int device, uint32_t nseg) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);

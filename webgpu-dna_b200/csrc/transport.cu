@@ -35,10 +35,7 @@ constexpr int STG_FLUSH = 256;     // staged rad entries written out at this lev
 constexpr int STG = STG_FLUSH + 3 * TB;   // iteration at most
 constexpr int STASH = TW * (int)TRANSPORT_STASH / 2;   // secondaries a block keeps in shared memory
 constexpr int NREC = 512;          // steps drawn ahead per iteration (few electrons)
-#ifndef WG_SHARE
-#define WG_SHARE 8
-#endif
-constexpr int SHARE = WG_SHARE;    // secondaries a block gives away per iteration while others have no work
+constexpr int SHARE = 8;           // secondaries a block gives away per iteration while others have no work
 constexpr int QTAKE = 64;          // and takes from the queue at a time
 
 __device__ __forceinline__ unsigned long long gtime() {
@@ -1238,6 +1235,9 @@ __global__ void __launch_bounds__(CTHR) k_share_scan(CanonArgs c) {
     }
 }
 
+// Entries of a primary, at most: what the sort of launch_canon holds in shared memory.  A
+// transport whose entries are placed by counting could have more, but is refused the same, so
+// that a primary does not pass or fail by whether another one's entries were dropped.
 constexpr int SEG_MAX = 8192;
 // entries to their places; the primaries' offsets and the longest segment
 __global__ void k_place(CanonArgs c) {
