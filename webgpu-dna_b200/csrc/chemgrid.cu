@@ -261,7 +261,8 @@ __device__ __forceinline__ int cg_contact(float4* pos, uint32_t* alive, uint32_t
 //    kept by their place in that walk (CG_KEEP at a time; a radical whose rolls all fail
 //    looks through the cells again for the ones after) before the first roll.  A cell that
 //    shares its bucket with another of the walk is met at both places, as in the lists:
-//    (-1, -1, z) and (1, 1, z) always do.
+//    (-1, -1, z) and (1, 1, z) always do.  (Not the lists': a position that is not a number is
+//    in contact with nothing here.)
 //    Yields after 1 us against claims in radical order, H2O2 and H2, mean of 32 inputs of
 //    30,000 radicals in 15 clusters of sigma 0.4 nm (40 of 0.5 nm): lists -2.7 and -1.9 %
 //    (-1.6 and -0.8), rolls in the order of the 0.75 nm cells -4.2 and -2.9 (-3.2 and -2.2),

@@ -849,7 +849,7 @@ __device__ __forceinline__ int move(const TArgs& A, Blk& b, int s, Dep& dep, uns
 // are alive at a time, so an iteration costs little more than its longest
 // phase path, and with more electrons the issue slots bind.
 // Measured at 4096 x 10 keV: 14.9 ms with one warp per 32 electrons taking all
-// branches one after another (7.8 lanes per instruction, 16 % issue), 4.35 ms now.
+// branches one after another (7.8 lanes per instruction, 16 % issue), 4.5 ms now.
 __global__ void __launch_bounds__(TB, 2) k_transport(TArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     float* T = reinterpret_cast<float*>(smem);
