@@ -268,6 +268,9 @@ __device__ __forceinline__ int cg_contact(float4* pos, uint32_t* alive, uint32_t
 //    (-1.6 and -0.8), rolls in the order of the 0.75 nm cells -4.2 and -2.9 (-3.2 and -2.2),
 //    now +1.0 and +0.4 (+1.6 and +0.7).  CG_KEEP 4 and 8, a call of 530,000 radicals: 12.7 ms
 //    both; 40 clusters 2.2 and 1.6 % of H2O2; in the cells' order 11.6 ms.
+//    The kept contacts cost 13 registers, and so one of 5 blocks per SM: 700 x 5 keV 12.5 ms in the
+//    cells' order, 13.8 now (lists 20.6).  In shared memory at 48 registers 13.4, but the 15
+//    clusters 32 ms instead of 18.5; a first look for any contact at all 14.3.
 constexpr uint32_t CG_LAST = 0x7fffffu;          // a contact's key: place << 23 | CG_LAST - index
 constexpr int CG_KEEP = 8;
 
